@@ -437,7 +437,7 @@ class Plan:
         _check(lib().gg_plan_set_tile_shape(self.handle, int(tile_u)))
 
     def set_slice_staging(self, mode: int = -1) -> None:
-        """Kernel-slice staging in shared memory: -1 auto, 0 off, 1 on."""
+        """Accepted (-1, 0 or 1) without effect: taps are read through L1."""
         _check(lib().gg_plan_set_slice_staging(self.handle, int(mode)))
 
     def set_batch_limit(self, max_points: int = 0) -> None:

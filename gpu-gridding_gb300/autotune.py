@@ -4,15 +4,13 @@ A plan's speed on a given GPU depends on a handful of settings that change
 no placement, norm or skip count (gg_tuning in the C header):
 
 * ``tile_u``        -- tile width (32, 16 or 8 cells; 2048-cell tiles),
-* ``slice_staging`` -- kernel slices staged in shared memory or read through L1,
+* ``slice_staging``, ``lane_groups`` -- accepted without effect,
 * ``items_per_cta`` -- how finely heavy tiles are split into work items,
 * ``sort_detail``   -- record order within a tile (plane + offset class,
   plane only, or visibility order),
 * ``ctas_per_sm``   -- resident gridding CTAs per SM (0 = as many as fit),
-* ``plane_group_mb`` -- kernel bytes per gridding pass (0 = half of L2),
+* ``plane_group_mb`` -- kernel bytes per gridding pass (0 = 3/4 of L2),
 * ``tile_order``    -- tiles taken by distance from the centre or row by row,
-* ``lane_groups``   -- on 32-wide tiles, each consumer warp takes records
-  whole (1) or as two half-warp streams (2).
 * ``tile_phases``   -- 1, 2, 4 or 8 tile grids offset by a fraction of a tile
   width; each visibility is gridded on the one that cuts its footprint
   into the fewest tile columns (the later grids' tiles as partial tiles

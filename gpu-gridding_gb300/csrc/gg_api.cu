@@ -226,10 +226,8 @@ struct gg_kernels {
   int support_max = 0;
   long long total_taps = 0;
   std::vector<int> h_support;
-  std::vector<long long> h_base, h_sbase;
-  long long total_slab_taps = 0;
-  size_t zero_half_bytes = 0;
-  DevBuf support, base, taps, tap_sum, zeros, sbase, slabs;
+  std::vector<SlicePlane> h_planes;
+  DevBuf support, planes, taps, tap_sum;
 
   StackView view() const {
     StackView v;
@@ -238,12 +236,10 @@ struct gg_kernels {
     v.omax = omax;
     v.conv_size_half = conv_size_half;
     v.support = support.as<int>();
-    v.base = base.as<long long>();
+    v.planes = planes.as<SlicePlane>();
     v.taps = taps.p;
+    v.wide = (unsigned long long)total_taps * (is_double ? 16 : 8) > 1ull << 32;
     v.tap_sum = tap_sum.as<double>();
-    v.zeros = zeros.as<char>() + zero_half_bytes;
-    v.sbase = sbase.as<long long>();
-    v.slabs = slabs.p;
     return v;
   }
 };
@@ -280,8 +276,8 @@ int validate_stack(size_t num_w_planes, const int* support, int oversample,
   return GG_OK;
 }
 
-// (Re)builds kernel stack k from a cube: sizes, tables, the re-laid slice
-// and slab stacks and the tap sums, enqueued on s.  k's device buffers are
+// (Re)builds kernel stack k from a cube: sizes, tables, the re-laid slices
+// and the tap sums, enqueued on s.  k's device buffers are
 // reused when large enough, so rebuilding one object for every call (the
 // host-pointer entry points do) allocates nothing after the first call.  A
 // host cube is copied through *stage (a local buffer when stage is NULL).
@@ -320,54 +316,42 @@ int kernels_fill(gg_kernels* k, size_t num_w_planes, const int* support,
   k->omax = (oversample + 1) / 2;
   k->conv_size_half = conv_size_half;
   k->h_support.assign(support, support + num_w_planes);
-  std::vector<long long>& base = k->h_base;
-  base.resize(num_w_planes);
-  long long total = 0;
+  std::vector<SlicePlane>& planes = k->h_planes;
+  planes.resize(num_w_planes);
+  long long total = kStackLead, limit_taps = 0;
   const long long classes = (long long)(k->omax + 1) * (k->omax + 1);
   for (size_t p = 0; p < num_w_planes; ++p) {
-    base[p] = total;
-    total += classes * slice_taps(support[p]);
+    planes[p].origin = total + kSlicePad * (long long)slice_pitch(support[p]);
+    planes[p].stride = (int)slice_stride(support[p]);
+    planes[p].support = support[p];
+    total += plane_taps(support[p], k->omax);
+    const long long F = 2LL * support[p] + 1;
+    limit_taps += classes * ((F * (F + 2 * kSlicePad) + 1) & ~1LL);
     k->support_max = std::max(k->support_max, support[p]);
   }
-  k->h_sbase.resize(num_w_planes);
-  long long qtotal = 0;
-  for (size_t p = 0; p < num_w_planes; ++p) {
-    k->h_sbase[p] = qtotal;
-    qtotal += (k->omax + 1) * slab_taps(support[p], oversample, k->omax);
-  }
-  // Slab row pitch and column bases are 16-bit fields of the gridding
-  // kernel's record descriptors.
   if ((long long)oversample * (k->support_max + 2) + k->support_max + 64 >
       32767)
     return fail(set_error(GG_ERR_UNSUPPORTED,
                           "oversample * (support + 2) = %lld exceeds this "
-                          "build's slab row limit",
+                          "build's kernel row limit",
                           (long long)oversample * (k->support_max + 2)));
-  // Record descriptors hold slab offsets plus column bases in 32 bits.
-  if (total > 0x7fffffffLL || qtotal > 0x7fffffffLL - (1LL << 24))
+  // Record descriptors index the stack's taps in 32 bits.  The limit counts
+  // both pad blocks of every slice, a little more than plane_taps, which
+  // shares them.
+  if (limit_taps > 0x7fffffffLL)
     return fail(set_error(GG_ERR_UNSUPPORTED,
                           "re-laid kernel stack has %lld taps; this build "
-                          "indexes at most 2^31-1",
-                          std::max(total, qtotal)));
+                          "indexes at most 2^31-1", limit_taps));
   k->total_taps = total;
-  k->total_slab_taps = qtotal;
-  // Zero buffer for lanes outside a footprint: a lane reads kRows = 8 rows
-  // at a stride of up to 2*s_max+1 taps either way from its middle.
-  k->zero_half_bytes = (size_t)8 * (2 * k->support_max + 1) * 2 * sizeof(Real);
   int r;
   if ((r = k->support.ensure(num_w_planes * sizeof(int))) ||
-      (r = k->base.ensure(num_w_planes * sizeof(long long))) ||
+      (r = k->planes.ensure(num_w_planes * sizeof(SlicePlane))) ||
       (r = k->taps.ensure((size_t)total * 2 * sizeof(Real))) ||
-      (r = k->zeros.ensure(2 * k->zero_half_bytes + 256)) ||
-      (r = k->sbase.ensure(num_w_planes * sizeof(long long))) ||
-      (r = k->slabs.ensure((size_t)qtotal * 2 * sizeof(Real) + 16)) ||
       (r = k->tap_sum.ensure(num_w_planes * (2 * k->omax + 1) *
                              (2 * k->omax + 1) * sizeof(double))))
     return fail(r);
   const cudaStream_t s_call = s;
   if (ss) s = ss->light;
-  if (cudaMemsetAsync(k->zeros.p, 0, k->zeros.bytes, s) != cudaSuccess)
-    return fail(set_error(GG_ERR_CUDA, "zero buffer memset failed"));
   auto cu = [&](cudaError_t e, const char* what) -> int {
     if (e == cudaSuccess) return GG_OK;
     return set_error(GG_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -375,14 +359,11 @@ int kernels_fill(gg_kernels* k, size_t num_w_planes, const int* support,
   if ((r = cu(cudaMemcpyAsync(k->support.p, support,
                               num_w_planes * sizeof(int),
                               cudaMemcpyHostToDevice, s), "support H2D")) ||
-      (r = cu(cudaMemcpyAsync(k->base.p, base.data(),
-                              num_w_planes * sizeof(long long),
-                              cudaMemcpyHostToDevice, s), "base H2D")) ||
-      (r = cu(cudaMemcpyAsync(k->sbase.p, k->h_sbase.data(),
-                              num_w_planes * sizeof(long long),
-                              cudaMemcpyHostToDevice, s), "sbase H2D")))
+      (r = cu(cudaMemcpyAsync(k->planes.p, planes.data(),
+                              num_w_planes * sizeof(SlicePlane),
+                              cudaMemcpyHostToDevice, s), "planes H2D")))
     return fail(r);
-  k->h2d_bytes += num_w_planes * (sizeof(int) + 2 * sizeof(long long));
+  k->h2d_bytes += num_w_planes * (sizeof(int) + sizeof(SlicePlane));
   const cudaStream_t s_tables = s;
   if (ss) {
     if ((r = cu(cudaEventRecord(ss->tables, s_tables), "tables event")))
@@ -469,13 +450,8 @@ int kernels_fill(gg_kernels* k, size_t num_w_planes, const int* support,
         return fail(r);
     }
   }
-  if ((r = cu(launch_stack_relayout<Real>(d_conv, v, k->taps.p, total, s,
-                                          changed),
+  if ((r = cu(launch_stack_relayout<Real>(d_conv, v, k->taps.p, s, changed),
               "relayout")))
-    return fail(r);
-  if ((r = cu(launch_stack_relayout_slabs<Real>(d_conv, v, k->slabs.p, s,
-                                                changed),
-              "slab relayout")))
     return fail(r);
   StackView raw = v;
   raw.taps = d_conv;
@@ -564,6 +540,7 @@ struct gg_plan {
   DevBuf cell, meta, vw, rec_count, rec_offset;
   DevBuf blk_norm, blk_skip, blk_macs;
   DevBuf keys0, vals0, keys1, vals1, sort_tmp, scan_tmp;
+  DevBuf recs, rec_spans;   // prepared records (launch_grid_tiles)
   DevBuf tile_start, item_a, item_b, items, split_tiles, partials, tile_slot;
   DevBuf scalars;  // device scalars, see Scalar below
   uint32_t* h_scalars = nullptr;  // pinned mirror
@@ -571,13 +548,13 @@ struct gg_plan {
   // Phase events (recorded only when profiling is enabled).
   static constexpr int kEvents = 6;
   int forced_shape = -1;  // tile shape index, -1 = chosen per call
-  int forced_stage = -1;  // slice staging 0/1, -1 = chosen per call
+  int slice_staging = -1; // as set; without effect (gg_plan_set_slice_staging)
   int items_per_cta = 4;  // work-item granularity of heavy-tile splits
   int sort_detail = 2;    // low sort-key fields: 2 plane+class, 1 plane, 0
   int ctas_per_sm = 0;    // cap on resident gridding CTAs, 0 = none
-  int plane_group_mb = 0; // slab bytes per plane group, 0 = L2 size / 2
+  int plane_group_mb = 0; // slice bytes per plane group, 0 = 3/4 of L2
   int queue_order = 0;    // tuning tile_order: 0 radius, 1 row by row
-  int lane_groups = 0;    // tuning lane_groups: 0 automatic, 1, 2
+  int lane_groups = 0;    // as set; without effect (gg_tuning)
   int tile_phases = 0;    // tuning tile_phases: 0 automatic, 1, 2, 4
   // Tile phases requested for the call being placed (0 automatic, chosen
   // with the shape; see gridding_phases).
@@ -670,7 +647,6 @@ struct gg_plan {
     unsigned long long num_points = 0;
     int num_grids = 0, grid_size = 0, num_chunks = 0, num_tiles = 0;
     int num_ctas = 0, shape = 0;
-    bool stage = false;
     uint32_t num_records = 0;
     TileGeom geom{};
     int group_span = 1;   // virtual groups per gridding launch
@@ -784,18 +760,9 @@ unsigned long long max_records_per_vis(int s_max, int shape) {
   return r;
 }
 
-// Record streams per consumer warp (TileGeom::lane_groups): half-warp
-// streams exist for the 32-wide tiles that read taps from the slab stack;
-// 0 (automatic) keeps whole warps (half-warp streams measured 4 % faster on
-// the synthetic-challenge shape, 2 % slower on the SKA-LOW one).
-int lane_groups_for(const gg_plan* plan, int tile_u, bool stage) {
-  if (tile_u != 32 || stage) return 1;
-  return plan->lane_groups == 2 ? 2 : 1;
-}
-
 // Plane groups for a call: consecutive w-planes cut into as many groups as
-// the byte budget (plan->plane_group_mb, or half the L2 cache) needs, with
-// even slab bytes per group, so that each gridding pass reads a stack slice
+// the byte budget (plan->plane_group_mb, or 3/4 of the L2 cache) needs, with
+// even slice bytes per group, so that each gridding pass reads a stack slice
 // that stays resident in L2.  At most max_groups groups (the sort key's
 // spare bits).
 // Uploads the plane -> group table when it changes; returns the number of
@@ -807,7 +774,7 @@ int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
   if (budget <= 0) {
     int l2 = 0;
     GG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, K->device));
-    budget = std::max<long long>((long long)l2 / 2, 1 << 20);
+    budget = std::max<long long>((long long)l2 / 4 * 3, 1 << 20);
   }
   max_groups = std::max(1, std::min(max_groups, 64));
   if (plan->pg_kernels == K->id && plan->pg_budget == requested &&
@@ -819,8 +786,7 @@ int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
   std::vector<long long> bytes(K->num_planes);
   long long total = 0;
   for (int p = 0; p < K->num_planes; ++p) {
-    bytes[p] = (K->omax + 1) *
-               slab_taps(K->h_support[p], K->oversample, K->omax) * tap_bytes;
+    bytes[p] = plane_taps(K->h_support[p], K->omax) * tap_bytes;
     total += bytes[p];
   }
   // More groups than allowed: widen the budget until they fit.
@@ -828,7 +794,7 @@ int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
   // As many groups as the budget needs, with even byte counts: plane p
   // joins the group that holds the middle of its bytes (a greedy fill to
   // the budget would leave the last group with the remainder, and the first
-  // groups' slabs, at the full budget, less likely to stay in L2).
+  // groups' slices, at the full budget, less likely to stay in L2).
   const long long want = std::max(1LL, (total + budget - 1) / budget);
   const double target = (double)total / (double)want;
   std::vector<int>& grp = plan->h_plane_group;
@@ -1055,7 +1021,6 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
 struct Bins {
   uint32_t total = 0;
   int shape = 0;
-  bool stage = false;
   int num_groups = 1, num_tiles = 0, grid_size = 0;
   TileGeom geom{};
   const uint32_t* keys = nullptr;
@@ -1093,9 +1058,6 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
                        "than 2^32-16; split it (batched calls do so by "
                        "grids)", records);
   }
-  const bool stage = plan->forced_stage >= 0
-                         ? plan->forced_stage != 0
-                         : ((plan->h_scalars[kShape] >> 8) & 1u) != 0;
   plan->stats.num_records = total;
   memcpy(&plan->stats.num_macs, (char*)plan->h_scalars + 32, 8);
   int key_bits = 0;
@@ -1135,7 +1097,6 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
                             plan->plane_group.as<int>(), phases);
   geom.split_tv = split ? plan->split_row / tile_v : 0;
   geom.split_mask = split_mask;
-  geom.lane_groups = lane_groups_for(plan, geom.tile_u, stage);
   const int num_tiles = num_groups * geom.tiles_total;
   plan->stats.num_plane_groups = pgroups;
   plan->split_tv = geom.split_tv;
@@ -1149,11 +1110,9 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   plan->kept.num_records = total;
   plan->kept.geom = geom;
   plan->kept.shape = shape;
-  plan->kept.stage = stage;
   plan->kept.num_tiles = num_tiles;
   b->total = total;
   b->shape = shape;
-  b->stage = stage;
   b->num_groups = num_groups;
   b->num_tiles = num_tiles;
   b->grid_size = grid_size;
@@ -1200,7 +1159,7 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
 // the distance of the tile's centre from the uv origin (the grid centre),
 // nearest first.  On telescope data the w-plane of a visibility grows with
 // its baseline, so tiles at the same distance use similar planes and the
-// CTAs running at one time share more kernel slabs in L2; the heavy
+// CTAs running at one time share more kernel slices in L2; the heavy
 // central tiles also start first.  Uploaded when the geometry changes.
 int tile_queue_order(gg_plan* plan, const TileGeom& g, int grid_size,
                      cudaStream_t s, const int** out) {
@@ -1235,11 +1194,15 @@ int tile_queue_order(gg_plan* plan, const TileGeom& g, int grid_size,
   return GG_OK;
 }
 
-// The work-item queue of binned records for num_ctas persistent CTAs: heavy
+// The work-item queue of binned records for num_ctas persistent CTAs (the
+// gridding kernel: teams of as many warps as a tile has bands): heavy
 // tiles are split into items of `chunk` records so that each of the call's
 // `passes` launches has about items_per_cta items per CTA (the gridding
 // passes of the groups; the degridder's single launch asks for as many
-// items as all of them).  Items: at most one
+// items as all of them).  Gridding chunks shorter than 1024 records are
+// made longer, up to half a CTA's share: below that the partial tiles cost
+// more than the better balance gives (2048^2, 2e5 points, 6.6e5 records:
+// 0.69 ms with chunks of 434, 0.60 with 867).  Items: at most one
 // more per tile than
 // total / chunk; partial-tile slots (split tiles only): at most
 // 2 * total / chunk, each a tile of partial sums when partial_tiles is set
@@ -1255,8 +1218,14 @@ int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
   // ends with a tail up to one item long.
   const unsigned long long f =
       (unsigned long long)plan->items_per_cta * (unsigned long long)passes;
-  const uint32_t chunk = (uint32_t)std::max<unsigned long long>(
-      64, ((unsigned long long)b.total + f * num_ctas - 1) / (f * num_ctas));
+  unsigned long long records =
+      ((unsigned long long)b.total + f * num_ctas - 1) / (f * num_ctas);
+  if (partial_tiles)
+    records = std::max(records,
+                       std::min(1024ull, (unsigned long long)b.total /
+                                             (2ull * passes * num_ctas)));
+  const uint32_t chunk =
+      (uint32_t)std::max<unsigned long long>(64, records);
   const size_t item_cap = (size_t)num_tiles + 2 * f * (size_t)num_ctas + 16;
   const size_t slot_cap = 2 * f * (size_t)num_ctas + 16;
   plan->stats.num_ctas = num_ctas;
@@ -1358,11 +1327,9 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
 
   int sms = 0;
   GG_TRY(num_sms_of_current(&sms));
-  int per_sm = grid_tiles_ctas_per_sm<Real>(geom.tile_u, b.stage,
-                                            geom.lane_groups);
+  int per_sm = grid_tiles_ctas_per_sm<Real>(geom.tile_u, view.wide);
   if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
   const int num_ctas = sms * per_sm;
-  plan->stats.slice_staging = b.stage ? 1 : 0;
   ItemBuffers ib;
   // The tile phases of a plane group share one launch, their later phases'
   // tiles added as partial tiles after it (where the kernels use the
@@ -1370,8 +1337,9 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   // Items are sized per virtual group (a phase's tiles are smaller, and
   // larger items leave longer tails).
   const int span = geom.tile_phases;
-  GG_TRY(build_work_items<Real>(plan, b, num_ctas, geom.num_groups, true, s,
-                                &ib, span));
+  GG_TRY(build_work_items<Real>(plan, b, grid_teams(num_ctas),
+                                geom.num_groups, true, s, &ib, span));
+  plan->stats.num_ctas = num_ctas;
   plan->kept.group_span = span;
   plan->kept.rec_vis = b.vals;
   plan->kept.num_ctas = num_ctas;
@@ -1405,12 +1373,16 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
     plan->direct_launched = true;
     plan->stats.num_launches += 1;
   }
+  gg_plan* T = plan->scratch ? plan->scratch : plan;
+  GG_TRY(T->recs.ensure((size_t)b.total * prepared_record_bytes<Real>()));
+  GG_TRY(T->rec_spans.ensure((size_t)b.total * 2));
   plan->mark(3, s);
   GG_CUDA(launch_grid_tiles<Real>(
-      ib.items, ib.group_items, ib.counter, sc + kDeviceError, b.vals,
+      ib.items, ib.group_items, ib.counter, T->recs.p,
+      T->rec_spans.as<unsigned short>(), b.vals,
       po.cell, po.meta, po.vw, view, geom, grid_size, d_grid, grid_stride,
       plan->partials.as<Real>(), ib.split_tiles, ib.num_split, b.num_tiles,
-      num_ctas, b.stage, s, wait_before.data(), record_after.data(),
+      num_ctas, s, wait_before.data(), record_after.data(),
       (Real*)plan->host_grid, tile_groups, span, plan->tile_slot.as<int2>(),
       plan->tile_start.as<uint32_t>()));
   plan->split_launched = upper_done >= 0;
@@ -1418,7 +1390,7 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   plan->mark(5, s);
   // each gridding launch and its partial reduction (one per virtual group,
   // or one over all the phases of a launch)
-  plan->stats.num_launches += 2 * (b.num_groups / span);
+  plan->stats.num_launches += 1 + 2 * (b.num_groups / span);
   plan->events_valid = plan->profile;
   return GG_OK;
 }
@@ -1627,13 +1599,11 @@ int batched_split(gg_plan* plan, const gg_kernels* K, int num_grids,
   for (int k = 0; k < nsub; ++k) {
     gg_plan* c = plan->subs[k].get();
     c->forced_shape = plan->forced_shape;
-    c->forced_stage = plan->forced_stage;
     c->items_per_cta = plan->items_per_cta;
     c->sort_detail = plan->sort_detail;
     c->ctas_per_sm = plan->ctas_per_sm;
     c->plane_group_mb = plan->plane_group_mb;
     c->queue_order = plan->queue_order;
-    c->lane_groups = plan->lane_groups;
     c->tile_phases = plan->tile_phases;
     const int a = g0[k], b = g0[k + 1];
     const unsigned long long v0 = h_offsets[a];
@@ -1719,14 +1689,14 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
       s));
   if (kp.num_records == 0) return GG_OK;
   const long long grid_stride = 2LL * kp.grid_size * kp.grid_size;
+  gg_plan* T = plan->scratch ? plan->scratch : plan;
   GG_CUDA(launch_grid_tiles<Real>(
       plan->items.as<WorkItem>(), plan->group_items.as<uint32_t>(),
-      sc + kCounter,
-      sc + kDeviceError, kp.rec_vis, plan->cell.as<uint32_t>(),
+      sc + kCounter, T->recs.p, T->rec_spans.as<unsigned short>(), kp.rec_vis, plan->cell.as<uint32_t>(),
       plan->meta.as<uint32_t>(), plan->vw.p, view, kp.geom, kp.grid_size,
       d_grids, grid_stride, plan->partials.as<Real>(),
       plan->split_tiles.as<int4>(), sc + kNumSplit, kp.num_tiles, kp.num_ctas,
-      kp.stage, s, nullptr, nullptr, nullptr, nullptr, kp.group_span,
+      s, nullptr, nullptr, nullptr, nullptr, kp.group_span,
       plan->tile_slot.as<int2>(), plan->tile_start.as<uint32_t>()));
   return GG_OK;
 }
@@ -1787,7 +1757,7 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
                      b.total);
   int sms = 0;
   GG_TRY(num_sms_of_current(&sms));
-  int per_sm = degrid_tiles_ctas_per_sm<Real>();
+  int per_sm = degrid_tiles_ctas_per_sm<Real>(view.wide);
   if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
   const int num_ctas = sms * per_sm;
   ItemBuffers ib;
@@ -2705,7 +2675,7 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode) {
   if (mode < -1 || mode > 1)
     return set_error(GG_ERR_INVALID_ARG,
                      "mode = %d: -1 (automatic), 0 (off) or 1 (on)", mode);
-  plan->forced_stage = mode;
+  plan->slice_staging = mode;
   return GG_OK;
 }
 
@@ -2756,7 +2726,7 @@ GG_API int gg_plan_get_tuning(const gg_plan* plan, gg_tuning* t) {
   t_last_error.clear();
   if (!plan || !t) return set_error(GG_ERR_INVALID_ARG, "plan or tuning is NULL");
   t->tile_u = plan->forced_shape < 0 ? 0 : tile_u_of_shape(plan->forced_shape);
-  t->slice_staging = plan->forced_stage;
+  t->slice_staging = plan->slice_staging;
   t->items_per_cta = plan->items_per_cta;
   t->sort_detail = plan->sort_detail;
   t->ctas_per_sm = plan->ctas_per_sm;

@@ -57,16 +57,32 @@ struct Vec2<double> { using type = double2; };
 // that matrix explicitly, for every plane and every absolute offset class
 // (cu, cv) in [0, omax]^2:
 //   S[jj][kk] = K[|cv + (jj - s)*os|][|cu + (kk - s)*os|],  jj, kk in [0, 2s]
-// at slice_base(p, cu, cv) = base[p] + (cu*(omax+1) + cv) * F^2, F = 2s+1.
 // A negative offset reads the mirrored slice: |-c + k*os| = |c + (-k)*os|,
 // so the tap of (j, k) for offsets (ou, ov) is
 //   S_{|ou|,|ov|}[s + sgn(ov)*j][s + sgn(ou)*k].
-// Each slice is contiguous (one bulk copy stages it in shared memory) and a
-// warp whose lanes hold consecutive k reads consecutive words.  Every slice
-// carries kSlicePad zero rows above and below, so a lane whose kRows
-// consecutive cells straddle the footprint's top or bottom edge reads zeros
-// there instead of testing each row.
+// A warp whose lanes hold consecutive k thus reads one contiguous run of a
+// row, whatever the offset: two 128-byte wavefronts per 32 taps, where a row
+// folded at off_u + k*os = 0 (two runs, each across line boundaries) took
+// 2.7 to 3.0 (measured with the taps in L1).  Every row ends in one zero tap
+// (row pitch 2s + 2), so a lane left or right of the footprint reads the zero
+// tap beside the row's own taps -- the end of the row above, or of the row
+// itself -- and kSlicePad zero rows lie above and below every slice (shared
+// by neighbours), so a lane whose kRows consecutive cells straddle the
+// footprint's top or bottom edge reads zeros there instead of testing each
+// row.
 constexpr int kSlicePad = 7;
+// Zero taps before the first plane, and one of them from which kRows rows of
+// the smallest pitch (2) and one column may be read either way: a record, or
+// a lane, that adds nothing.
+constexpr int kStackLead = 40;
+constexpr int kStackZero = 20;
+
+// One plane's slices, as the producers of the tile kernels look them up.
+struct alignas(16) SlicePlane {
+  long long origin;   // tap S[0][0] of the slice of class (0, 0)
+  int stride;         // taps from one class's slice to the next
+  int support;
+};
 
 struct StackView {
   int num_planes;
@@ -74,68 +90,38 @@ struct StackView {
   int omax;                 // (oversample + 1) / 2: largest |offset|
   int conv_size_half;
   const int* support;       // [P]
-  const long long* base;    // [P] first tap of plane p (complex units)
+  const SlicePlane* planes; // [P]
   const void* taps;         // float2 or double2
+  bool wide;                // more than 4 GiB of taps (load_taps)
   const double* tap_sum;    // [P][2*omax+1][2*omax+1] sum of Re(tap), FP64
-  const void* zeros;        // middle of a zero buffer that any lane's rows
-                            // (kRows rows of any slice stride) stay inside
-  const long long* sbase;   // [P] first tap of plane p in the slab stack
-  const void* slabs;        // slab stack (see below)
 };
 
-// ---------------------------------------------------------------------------
-// Slab stack: footprint rows in order, columns residue-major.
-// ---------------------------------------------------------------------------
-// For plane p and row class c = |off_v| in [0, omax] a slab holds the
-// footprint's rows j = -s..s in order, each the quadrant row
-// t = |c + j*os|, with kSlicePad zero rows before and after:
-//   slab_{p,c}[kSlicePad + j + s][r][m] = K_p[|c + j*os|][r + m*os]
-// for residues r in [0, os) and lattice indices m in [0, M), M = s + 1
-// (+1 when omax >= os, i.e. os = 1).  A negative off_v reads the slab's
-// rows in reverse (|-c + j*os| = |c + (-j)*os|).  Rows are stored by column
-// residue: the tap of footprint column k for offset ou is
-// K[.][|ou + k*os|], and on either side of the fold ou + k*os = 0 that
-// column has one residue and a lattice index that moves by one per column,
-// so a warp's lanes (consecutive k) read at most two contiguous runs of a
-// row, and a lane's rows are evenly spaced.  Each quadrant row appears in
-// the slabs of a plane about 1.5 times (against (omax + 1) times plus the
-// column mirror in the per-offset slices above), which keeps the whole
-// stack of a large W-projection setup in L2.
-__host__ __device__ inline int slab_cols_m(int s, int os, int omax) {
-  return s + 1 + (omax >= os ? 1 : 0);
+// Row pitch of a slice: its 2s + 1 taps and a zero (even, so every row
+// starts 16-byte aligned).
+__host__ __device__ inline int slice_pitch(int s) { return 2 * s + 2; }
+// Taps from one slice of a plane to the next: its rows and the pad rows.
+__host__ __device__ inline long long slice_stride(int s) {
+  return (long long)(2 * s + 1 + kSlicePad) * slice_pitch(s);
 }
-// Taps of one slab, rounded up to an even count (16-byte aligned slabs).
-__host__ __device__ inline long long slab_taps(int s, int os, int omax) {
-  return ((long long)(2 * s + 1 + 2 * kSlicePad) * os *
-              slab_cols_m(s, os, omax) + 1) & ~1LL;
+// Taps of a plane: pad rows, then the slices, each followed by pad rows.
+__host__ __device__ inline long long plane_taps(int s, int omax) {
+  return (long long)kSlicePad * slice_pitch(s) +
+         (long long)(omax + 1) * (omax + 1) * slice_stride(s);
+}
+// Index of tap S[0][0] of the plane's slice for absolute offsets (cu, cv).
+__host__ __device__ inline long long slice_origin(const SlicePlane& p,
+                                                  int omax, int cu, int cv) {
+  return p.origin + (long long)(cu * (omax + 1) + cv) * p.stride;
 }
 
-// Rows and columns of a plane's quadrant cube that the stack preparation
-// reads (slices and tap sums: |off| + s*os with |off| <= omax; slabs:
-// columns r + m*os with r < os, m < M): the square [0, E)^2 below
-// E = min(csh, 1 + max(s*os + omax, M*os - 1)).
+// Rows and columns of a plane's quadrant cube that the stack preparation may
+// read (|off| + s*os with |off| <= omax, rounded up to whole oversampling
+// steps): the square [0, E)^2.
 __host__ __device__ inline int cube_read_extent(int s, int os, int omax,
                                                 int csh) {
-  const int a = s * os + omax, b = slab_cols_m(s, os, omax) * os - 1;
-  const int e = 1 + (a > b ? a : b);
+  const int a = s * os + omax + 1, b = (s + 1 + (omax >= os ? 1 : 0)) * os;
+  const int e = a > b ? a : b;
   return e < csh ? e : csh;
-}
-
-// Taps one slice occupies: padding rows included, rounded up to an even
-// count so that every slice starts 16-byte aligned (bulk copies need it).
-__host__ __device__ inline long long slice_taps(int s) {
-  const long long F = 2 * s + 1;
-  return ((F + 2 * kSlicePad) * F + 1) & ~1LL;
-}
-
-// Index of tap S[0][0] of the slice of plane p for absolute offsets
-// (cu, cv) (the padding rows come before it).
-__host__ __device__ inline long long slice_offset(long long plane_base,
-                                                  int s, int omax, int cu,
-                                                  int cv) {
-  const long long F = 2 * s + 1;
-  return plane_base + (long long)(cu * (omax + 1) + cv) * slice_taps(s) +
-         kSlicePad * F;
 }
 
 // ---------------------------------------------------------------------------
@@ -160,7 +146,7 @@ struct PlaceParams {
 
 // Tile geometry shared by the binning and gridding kernels.
 // With plane groups (num_groups > 1) the records of a call are gridded in
-// one pass per group of consecutive w-planes, each group's kernel slabs
+// one pass per group of consecutive w-planes, each group's kernel slices
 // small enough to stay in L2 during its pass; the sort key's tile field is
 // then the virtual tile group * tiles_total + tile.
 struct TileGeom {
@@ -179,10 +165,6 @@ struct TileGeom {
   // num_groups counts them all.
   int split_tv;
   int split_mask;
-  // Record streams per consumer warp of the 32-wide gridding kernel: 1 (or
-  // 0) -- the whole warp takes each record that meets its rows; 2 -- each
-  // half-warp (16 columns) takes the records that meet its own columns.
-  int lane_groups;
   // Tile phases (1, 2, 4 or 8): the tile columns of phase p start p * tile_u /
   // tile_phases cells to the left of phase 0's, and each visibility is
   // gridded on the phase whose tiles cut its footprint into the fewest

@@ -11,7 +11,7 @@
 // the gridder's queue.  Its eight consumer warps hold the tile's grid
 // values in registers (lane = column, kRows rows per lane, as in the
 // gridder) and, for every record whose footprint meets their rows, multiply
-// them by the record's taps from the slab stack and sum across the warp by
+// them by the record's taps and sum across the warp by
 // shuffles.  The producer warp gathers and prepares the records and, once
 // the consumers are done with a buffer, adds each record's warp sums in warp
 // order and stores the record's partial result at its emission slot
@@ -59,20 +59,13 @@ template <typename Real>
 struct DegridSmem {
   using R2 = typename Vec2<Real>::type;
   R2 part[kRing][kBuf][kWarps];  // consumer warp w's sum of record t
-  int4 rec[kRing][kBuf];         // slab descriptors (slab_record)
+  uint2 rec[kRing][kBuf];        // slice_record descriptors
   uint32_t band[kRing][kBuf];    // bit w: the footprint meets warp w's rows
   uint32_t out[kRing][kBuf];     // emission slot | conjugated << 31
   int4 head[kRing];              // item, records (-1: no more work), flags
   uint64_t full[kRing];
   uint64_t empty[kRing];
 };
-
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  return __ffma2_rn(a, b, c);
-}
-__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
-  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
-}
 
 // The producer warp: takes work items from the queue, streams their records
 // through the ring and stores each finished buffer's per-record results.
@@ -154,16 +147,13 @@ __device__ bool degrid_produce(const DegridArgs<Real>& a,
           const int t = q * 32 + lane;
           if (t < nb) {
             const uint32_t m = me[q];
-            const int plane = meta_plane(m);
-            const int s = a.view.support[plane];
+            const SlicePlane plane = a.view.planes[meta_plane(m)];
+            const int s = plane.support;
             const int gu = cell_u(ce[q]), gv = cell_v(ce[q]);
-            sm.rec[slot][t] =
-                a.view.oversample == 4
-                    ? slab_record<kDegridTileU, 4>(a.view, plane, s,
-                                                   meta_ou(m), meta_ov(m),
-                                                   gu - u0, gv - v0)
-                    : slab_record<kDegridTileU>(a.view, plane, s, meta_ou(m),
-                                                meta_ov(m), gu - u0, gv - v0);
+            const int ou = meta_ou(m), ov = meta_ov(m);
+            sm.rec[slot][t] = slice_record(
+                slice_origin(plane, a.view.omax, abs(ou), abs(ov)),
+                s, ou, ov, gu - u0, gv - v0);
             uint32_t band = 0;
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) {
@@ -204,24 +194,6 @@ __device__ bool degrid_produce(const DegridArgs<Real>& a,
   return true;
 }
 
-// The kRows taps of one record for this lane from the slab stack; lanes
-// outside the footprint's columns read zeros.  (Rows of the warp outside
-// the footprint read the slab's zero padding rows.)
-template <typename R2>
-__device__ __forceinline__ void load_taps(const int4 ra,
-                                          const R2* __restrict__ slabs,
-                                          const R2* __restrict__ gzeros,
-                                          int lx, int rowl, uint64_t pol,
-                                          R2 (&out)[kRows]) {
-  const int c0 = (ra.w >> 8) & 0xFF, cw = (int)((unsigned)ra.w >> 16);
-  const bool ok = (unsigned)(lx - c0) <= (unsigned)cw;
-  const int off = (lx >= (ra.w & 0xFF) ? ra.x + lx : ra.y - lx) + rowl * ra.z;
-  const R2* p = ok ? slabs + off : gzeros;
-  const int step = ok ? ra.z : 0;
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) out[r] = ld_tap(p + r * step, pol);
-}
-
 // This lane's share of conj(c~) * g over its kRows cells, with
 // gx[r] = (g.re, g.re) and gy[r] = (g.im, g.im): P = sum t * g.re and
 // Q = sum t * g.im componentwise, so with c~ = (t.re, sgn * t.im)
@@ -242,7 +214,7 @@ __device__ __forceinline__ void dot_record(const R2 (&t)[kRows],
   im = Q.x - sgn * P.y;
 }
 
-template <typename Real>
+template <typename Real, bool kWide>
 __global__ void __launch_bounds__(kThreads, sizeof(Real) == 4 ? 2 : 1)
 k_degrid_tiles(DegridArgs<Real> a) {
   using R2 = typename Vec2<Real>::type;
@@ -255,7 +227,6 @@ k_degrid_tiles(DegridArgs<Real> a) {
       mbar_init(&sm.full[i], 1);
       mbar_init(&sm.empty[i], kWarps);
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   if (warp == kWarps) {
@@ -266,17 +237,24 @@ k_degrid_tiles(DegridArgs<Real> a) {
   const int rowl = warp * kRows;   // this lane's row 0 in the tile
   const int G = a.grid_size;
   const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
-  const R2* __restrict__ slabs = (const R2*)a.view.slabs;
-  const R2* __restrict__ gzeros = (const R2*)a.view.zeros;
+  const R2* __restrict__ taps = (const R2*)a.view.taps;
   const R2* __restrict__ grid = (const R2*)a.grid;
-  const uint64_t pol = evict_last_policy();
   const uint32_t my_bit = 1u << warp;
   R2 gx[kRows], gy[kRows];
 #pragma unroll
   for (int r = 0; r < kRows; ++r) gx[r].x = gx[r].y = gy[r].x = gy[r].y = 0;
 
+  // The taps of record t of buffer slot `slot` for this lane's rows.
+  int slot = 0;
+  auto load = [&](int t, R2 (&out)[kRows]) {
+    const uint2 d = sm.rec[slot][t];
+    const int step = slice_step(d);
+    load_taps<kWide>(taps, slice_tap(d, step, lane) + (uint32_t)(rowl * step), step,
+              out);
+  };
+
   for (unsigned k = 0;; ++k) {
-    const int slot = (int)(k % kRing);
+    slot = (int)(k % kRing);
     if (!mbar_wait(&sm.full[slot], (k / kRing) & 1)) {
       atomicExch(a.error, 1u);
       return;
@@ -312,14 +290,14 @@ k_degrid_tiles(DegridArgs<Real> a) {
         const int tA = c0 + __ffs(m) - 1;
         m &= m - 1;
         R2 ta[kRows];
-        load_taps(sm.rec[slot][tA], slabs, gzeros, lane, rowl, pol, ta);
+        load(tA, ta);
         const Real sA = (sm.out[slot][tA] >> 31) ? (Real)-1 : (Real)1;
         Real reA, imA;
         if (m) {
           const int tB = c0 + __ffs(m) - 1;
           m &= m - 1;
           R2 tb[kRows];
-          load_taps(sm.rec[slot][tB], slabs, gzeros, lane, rowl, pol, tb);
+          load(tB, tb);
           const Real sB = (sm.out[slot][tB] >> 31) ? (Real)-1 : (Real)1;
           Real reB, imB;
           dot_record(ta, gx, gy, sA, reA, imA);
@@ -385,31 +363,38 @@ __global__ void k_degrid_finish(const uint32_t* __restrict__ count,
   ((R2*)out)[i] = acc;
 }
 
-template <typename Real>
-cudaError_t prepare_degrid_kernel(size_t* smem) {
+template <typename Real, bool kWide>
+cudaError_t prepare_degrid_kernel(void** fn, size_t* smem) {
   static std::atomic<unsigned long long> opted_in{0};
+  *fn = (void*)k_degrid_tiles<Real, kWide>;
   *smem = sizeof(DegridSmem<Real>);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = 1ull << (dev & 63);
   if (dev < 64 && (opted_in.load() & bit)) return cudaSuccess;
-  e = cudaFuncSetAttribute(k_degrid_tiles<Real>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)*smem);
   if (e == cudaSuccess && dev < 64) opted_in.fetch_or(bit);
   return e;
 }
 
+template <typename Real>
+cudaError_t prepare_degrid_kernel_for(bool wide, void** fn, size_t* smem) {
+  return wide ? prepare_degrid_kernel<Real, true>(fn, smem)
+              : prepare_degrid_kernel<Real, false>(fn, smem);
+}
+
 }  // namespace
 
 template <typename Real>
-int degrid_tiles_ctas_per_sm() {
+int degrid_tiles_ctas_per_sm(bool wide) {
+  void* fn = nullptr;
   size_t smem = 0;
   int n = 0;
-  if (prepare_degrid_kernel<Real>(&smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &n, k_degrid_tiles<Real>, kThreads, smem) != cudaSuccess)
+  if (prepare_degrid_kernel_for<Real>(wide, &fn, &smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, smem) !=
+          cudaSuccess)
     n = 1;
   return n < 1 ? 1 : n;
 }
@@ -438,13 +423,14 @@ cudaError_t launch_degrid_tiles(const WorkItem* items,
   a.grid_size = grid_size;
   a.grid = grid;
   a.rec_out = (typename Vec2<Real>::type*)rec_out;
+  void* fn = nullptr;
   size_t smem = 0;
-  cudaError_t e = prepare_degrid_kernel<Real>(&smem);
+  cudaError_t e = prepare_degrid_kernel_for<Real>(view.wide, &fn, &smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
-  k_degrid_tiles<Real><<<num_ctas, kThreads, smem, s>>>(a);
-  return cudaGetLastError();
+  void* args[] = {&a};
+  return cudaLaunchKernel(fn, dim3(num_ctas), dim3(kThreads), args, smem, s);
 }
 
 template <typename Real>
@@ -458,8 +444,8 @@ cudaError_t launch_degrid_finish(const uint32_t* count, const uint32_t* offset,
   return cudaGetLastError();
 }
 
-template int degrid_tiles_ctas_per_sm<float>();
-template int degrid_tiles_ctas_per_sm<double>();
+template int degrid_tiles_ctas_per_sm<float>(bool);
+template int degrid_tiles_ctas_per_sm<double>(bool);
 template cudaError_t launch_degrid_tiles<float>(
     const WorkItem*, const uint32_t*, uint32_t*, uint32_t*, const uint32_t*,
     const uint32_t*, const uint32_t*, const uint32_t*, StackView, TileGeom,

@@ -3,29 +3,46 @@
 // The grid is cut into tiles of TW (u) x TV (v) cells.  After the sort each
 // tile's (visibility, tile) records are contiguous and ordered by (plane,
 // |offset| class); a tile's record range is cut into work items of at most
-// `chunk` records.  A persistent CTA takes work items from a queue and keeps
-// the item's whole tile in registers: lane (lx, ly) of consumer warp w owns
-// column lx and kRows consecutive rows of the warp's band.  For every record,
-// each warp whose band meets the footprint multiplies the visibility by the
-// kernel taps of its own cells and accumulates -- no atomics, no
-// shared-memory read-modify-write.  A tile with one item is then added to
-// the grid in place with one coalesced read-modify-write; a tile split over
-// several items writes one partial tile per item and k_reduce_partials (or
+// `chunk` records.  k_prepare_records turns the sorted records into
+// descriptors; then every warp of the persistent gridding kernel works by
+// itself: it takes a band of a work item (8 lane rows by the tile's columns)
+// from a queue and keeps the band's cells in registers: lane (lx, ly) owns
+// column lx and kRows consecutive rows.  For every record whose footprint
+// meets its rows the warp multiplies the visibility by the kernel taps of its
+// own cells and accumulates -- no atomics, no shared-memory
+// read-modify-write.  A tile with one item is then added to the grid in place
+// with one coalesced read-modify-write per band; a tile split over several
+// items writes one partial tile per item and k_reduce_partials (or
 // k_reduce_phases) adds them to the grid in item order, so the result does
 // not depend on scheduling.
 //
-// The CTA is warp-specialised.  One producer warp takes work items, gathers
-// and prepares their records and streams them through a ring of kRing
-// shared-memory buffers guarded by mbarriers; when a buffer is dominated by
-// one (plane, |offset|) group that is long enough to pay for it, the producer
-// also stages that group's kernel slice into one of kSlots shared-memory
-// slots with a bulk asynchronous copy (cp.async.bulk, completion tracked by
-// the buffer's mbarrier), and those records read their taps from shared
-// memory instead of L2.  Eight consumer warps accumulate.
+// The bands of a tile are far from equally loaded where the visibilities
+// crowd (in a simulation of eight warps sharing one stream of records they
+// were busy 81 % of the time on 512-station tracks over 8192^2, 44 % on
+// 128-station ones over 2048^2), so they are units of their own.
+//
+// What bounds it: each complex multiply-add needs one 8-byte tap that no
+// register holds, so a warp's 32 taps cost two cycles of the SM's L1 data
+// pipe, and a step (a record on a band, 8 rows) 16 at least; as about half of
+// the lanes and rows of a step lie inside its footprint, about half of that
+// serves no multiply-add.  The pass takes about 33 cycles a step where it
+// took 40 to 50, and the instructions issued (about 65 a step) come next.
+// What led there, passes in ms (8192^2: 2.2e6 points, uniform w; 7.8e6 track
+// points, 339 planes; 16 grids of 2048^2, 1.1e7 points):
+//                                               5.6   8.0  15.6
+//   taps of long runs no longer copied into
+//   shared memory first (the copies' slots took
+//   the L1 capacity of all other records), rows
+//   unfolded (StackView)                        5.6   5.8  11.7
+//   warps of their own, plain FMAs              5.2   5.7   8.8
+//   everything a lane needs of a record worked
+//   out once when it is queued, packed FMAs     4.6   5.4   8.7
+//   32-bit tap offsets (load_taps)              4.4   5.1   8.1
 //
 // Three warp shapes share the 2048-cell tile: TW = 32 (32 x 64 tiles, for
 // large footprints), 16 (16 x 128) and 8 (8 x 256, for small footprints,
-// where a 32-wide warp would leave most lanes outside the footprint).
+// where a 32-wide warp would leave most lanes outside the footprint).  Each
+// lane row of the narrow ones takes its own records.
 //
 // Tile phases (TileGeom::tile_phases): up to eight tile grids, each offset
 // by a strip of TW / phases columns from the last; every visibility's
@@ -41,8 +58,8 @@
 // (oskar_grid_wproj_gpu.cu:840-1309), a one-warp-per-32x16-tile kernel that
 // flushes with float atomics whenever its tile changes.
 //
-// FP32 accumulation is compensated: each buffer of records is summed in
-// plain FP32 FMA, then folded into a (hi, lo) pair by Knuth's TwoSum, so
+// FP32 accumulation is compensated: the records of each run of 128 are summed
+// in plain FP32 FMA, then folded into a (hi, lo) pair by Knuth's TwoSum, so
 // rounding error does not grow with the number of visibilities on a cell.
 #include <algorithm>
 #include <atomic>
@@ -55,19 +72,21 @@ namespace gg {
 
 namespace {
 
-constexpr int kSlots = 2;         // staged kernel slices
-constexpr int kSliceBytes = 26624;  // per slot: (2s+15)(2s+1) taps, s <= 25 (FP32)
-constexpr int kRunMin = 24;       // records of one group that pay for staging
-
-// Visibility coefficients of one record with the conjugation folded in:
-// re += a*t.re + b*t.im, im += c*t.re + d*t.im.  Stored as (a, d, c, b) so
-// that the FP32 kernel can accumulate two packed pairs per cell with FP32x2
-// FMAs, P += (a, d) * (t.re, t.im) and Q += (c, b) * (t.re, t.im), and
-// recover re = P.x + Q.y, im = Q.x + P.y when it folds a buffer.
+// A prepared record: slice_record's descriptor and the weighted visibility.
 template <typename Real>
-struct alignas(4 * sizeof(Real)) Coef {
-  Real a, d, c, b;
+struct alignas(16) Record {
+  uint2 d;
+  typename Vec2<Real>::type v;
 };
+
+// The lane-row groups (kRows rows each, at most 32) of a tile that a
+// record's footprint meets, first | last << 5, with bit 15 set where its
+// kernel is conjugated (ww > 0).
+constexpr uint32_t kSpanConj = 1u << 15;
+constexpr uint32_t kSpanNone = 31u;   // first 31, last 0: meets none
+__device__ __forceinline__ bool span_meets(uint32_t span, int group) {
+  return (int)((span >> 5) & 31u) >= group && (int)(span & 31u) <= group;
+}
 
 // Knuth's TwoSum: s + e == a + b exactly.
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
@@ -83,11 +102,12 @@ struct GridArgs {
   int group;                     // the launch's first virtual group
   int group_span;                // virtual groups in the launch
   uint32_t* counter;
-  uint32_t* error;          // set to 1 when a bounded wait runs out
   const uint32_t* rec_vis;
   const uint32_t* cell;
   const uint32_t* meta;
   const typename Vec2<Real>::type* vw;
+  Record<Real>* recs;       // prepared records, in sorted order
+  unsigned short* spans;    // and the rows they meet
   StackView view;
   TileGeom geom;
   int grid_size;
@@ -123,565 +143,297 @@ __device__ __forceinline__ void cell_ends(const uint32_t* tile_groups,
   }
 }
 
-// Shared-memory layout of one CTA (dynamic shared memory).  Without slice
-// staging the CTA needs about 50 KB, leaving the rest of the SM's unified
-// L1 / shared memory to cache the taps it reads from the global stack.
-template <typename Real, bool kStage>
-struct Smem {
+// Prepares the records of every work item of the call: one block per item at
+// a time.  HBM-bound: 4 B of index, a 32-byte sector from each of three
+// arrays per record in, 18 B (FP64: 34 B) out.
+template <typename Real, int TW>
+__global__ void __launch_bounds__(128)
+k_prepare_records(GridArgs<Real> a, int num_groups) {
   using R2 = typename Vec2<Real>::type;
-  static constexpr int kNSlots = kStage ? kSlots : 1;
-  static constexpr int kSliceTaps = kStage ? kSliceBytes / (int)sizeof(R2) : 2;
-  // Largest staged slice width F: (F + 2*kSlicePad) * F <= kSliceTaps.
-  static constexpr int kMaxStagedF = sizeof(Real) == 4 ? 51 : 33;
-  // Zero region for lanes outside a footprint: kRows rows of up to
-  // kMaxStagedF taps either way from its middle.
-  static constexpr int kZeroTaps = kStage ? 2 * kRows * kMaxStagedF + 2 : 2;
+  using WS = WarpShape<TW>;
+  const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
+  const int num_items = (int)a.group_items[num_groups];
+  for (int it = blockIdx.x; it < num_items; it += gridDim.x) {
+    const WorkItem item = a.items[it];
+    const int vg = item.tile / a.geom.tiles_total;   // virtual group
+    const int tl = (item.tile - vg * a.geom.tiles_total) % tiles_per_grid;
+    const int u0 = (tl % a.geom.tiles_u) * WS::kTileU - phase_shift(a.geom, vg);
+    const int v0 = (tl / a.geom.tiles_u) * WS::kTileV;
+    for (int i = item.rec_begin + (int)threadIdx.x; i < item.rec_end;
+         i += blockDim.x) {
+      const uint32_t vid = a.rec_vis[i];
+      const uint32_t ce = a.cell[vid], m = a.meta[vid];
+      const R2 v = a.vw[vid];
+      const SlicePlane plane = a.view.planes[meta_plane(m)];
+      const int ou = meta_ou(m), ov = meta_ov(m), s = plane.support;
+      const int gu = cell_u(ce) - u0, gv = cell_v(ce) - v0;
+      Record<Real> rec;
+      rec.d = slice_record(slice_origin(plane, a.view.omax, abs(ou), abs(ov)),
+                           s, ou, ov, gu, gv);
+      rec.v = v;
+      a.recs[i] = rec;
+      // The tile meets each of its records: clipped to it.
+      a.spans[i] = (unsigned short)(
+          (uint32_t)(max(gv - s, 0) / kRows) |
+          (uint32_t)(min(gv + s, WS::kTileV - 1) / kRows) << 5 |
+          (meta_conj(m) ? kSpanConj : 0u));
+    }
+  }
+}
+
+// A queued record of a lane-row group: everything the group's lanes need for
+// it, worked out by the one lane that queues it.  The tap of the lane at tile
+// column col in the group's row r is
+//   taps[x + r * step + su * clamp(col - gu, -S, S)]
+// with S = s + 1 (the clamped ends are zero taps) and step = +-2S; the record
+// adds (a, d) * (t.re, t.im) to the cell's P and (c, b) * (t.re, t.im) to its
+// Q, and re = P.x + Q.y, im = Q.x + P.y (FP32: two packed FMAs a cell).
+template <typename Real>
+struct alignas(16) Queued {
+  uint32_t x;
+  int gu_su;    // gu << 16 | (su & 0xFFFF)
+  int S, step;
+  Real a, d, c, b;
+};
+template <typename Real>
+__device__ __forceinline__ Queued<Real> queued(const Record<Real>& r,
+                                               uint32_t span, int group) {
+  Queued<Real> q;
+  const int z = (int)(short)(r.d.y & 0xFFFFu);
+  const int s = (int)((r.d.y >> 16) & 0x3FFFu);
+  const bool mu = (r.d.y & kMirrorU) != 0u, conj = (span & kSpanConj) != 0u;
+  q.S = s + 1;
+  q.step = slice_step(r.d);
+  q.x = r.d.x + (uint32_t)(group * kRows * q.step + s);
+  const int gu = mu ? z - s : s - z;
+  q.gu_su = (int)((uint32_t)gu << 16 | (mu ? 0xFFFFu : 1u));
+  q.a = r.v.x;
+  q.c = r.v.y;
+  q.d = conj ? -r.v.x : r.v.x;
+  q.b = conj ? r.v.y : -r.v.y;
+  return q;
+}
+
+// Shared memory of one warp of the gridding kernel.
+template <typename Real, int TW>
+struct WarpSmem {
+  using R2 = typename Vec2<Real>::type;
   static constexpr bool kComp = sizeof(Real) == 4;
-  R2 slice[kNSlots][kSliceTaps];
-  R2 zero[kZeroTaps];
-  R2 hi[kComp ? kRows : 1][kConsumers];
-  R2 lo[kComp ? kRows : 1][kConsumers];
-  int4 rec[kRing][kBuf];
-  Coef<Real> cf[kRing][kBuf];
-  uint32_t band[kRing][kBuf];
-  signed char src[kRing][kBuf];   // slice slot of the record, -1 = global
-  // Half-warp record lists of the buffer being gridded (per consumer warp:
-  // the records meeting its rows and columns 0..15, then 16..31).
-  unsigned char half_list[kWarps][2][kBuf];
-  int4 head[kRing];
-  uint64_t full[kRing];
-  uint64_t empty[kRing];
-};
-static_assert((51 + 2 * kSlicePad) * 51 <= kSliceBytes / 8, "FP32 slot size");
-static_assert((33 + 2 * kSlicePad) * 33 <= kSliceBytes / 16, "FP64 slot size");
-
-// Record data in shared memory (int4 per record).  A record whose taps are
-// read from the slab stack in global memory (src < 0) holds slab_record's
-// descriptor (gg_tiles.cuh).  A record whose slice is staged in a
-// shared-memory slot (src >= 0) holds
-//   x = org:   tap index of tile cell (0, 0) on the staged slice
-//   y = rstep: +-(2s+1), slice rows per tile row (mirrored for ov < 0)
-//   z = ulo:   first footprint column (tile-relative)
-//   w = su * (2s+1): column mirror sign and footprint width
-// so its tap for tile cell (row, col) is slice[org + row * rstep +
-// col * su]; lanes whose column lies outside [ulo, ulo + 2s] read zeros.
-//
-// Slice-slot bookkeeping of the producer (lane-uniform).
-struct SlotState {
-  int group[kSlots];       // (plane, |offset| class) held, -1 = none
-  unsigned last_k[kSlots]; // last ring buffer that referenced the slot
-  bool used[kSlots];
+  static constexpr int kQueue = 64;
+  R2 hi[kComp ? kRows : 1][32];
+  R2 lo[kComp ? kRows : 1][32];
+  // Records waiting for each lane-row group, a ring.
+  Queued<Real> queue[WarpShape<TW>::kLanesY][kQueue];
 };
 
-__device__ __forceinline__ int group_of(uint32_t meta) {
-  return meta_plane(meta) * 64 + abs(meta_ou(meta)) * 8 + abs(meta_ov(meta));
-}
+constexpr int kGridWarps = 4;    // per block of the gridding kernel
+constexpr int kGridThreads = kGridWarps * 32;
 
-// The producer warp: takes work items from the queue and streams their
-// records, staged, through the ring.  Returns false if a wait ran out.
-template <typename Real, int TW, bool kStage, bool kHalves>
-__device__ bool produce(const GridArgs<Real>& a, Smem<Real, kStage>& sm) {
-  using R2 = typename Vec2<Real>::type;
-  using WS = WarpShape<TW>;
-  const int lane = threadIdx.x & 31;
-  const int omax = a.view.omax;
-  const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
-  // The launch's items: those of its virtual groups (a plane group's tile
-  // phases, or one of them).
-  const int first_item = (int)a.group_items[a.group];
-  const int end_item = (int)a.group_items[a.group + a.group_span];
-  const R2* __restrict__ taps = (const R2*)a.view.taps;
-  SlotState st;
-  for (int x = 0; x < kSlots; ++x) {
-    st.group[x] = -1;
-    st.last_k[x] = 0;
-    st.used[x] = false;
-  }
-  unsigned k = 0;
-  for (;;) {
-    int it = 0;
-    if (lane == 0) it = first_item + (int)atomicAdd(a.counter, 1u);
-    it = __shfl_sync(0xffffffffu, it, 0);
-    const bool done = it >= end_item;
-    WorkItem item{0, 0, 0, -1};
-    int u0 = 0, v0 = 0;
-    if (!done) {
-      item = a.items[it];
-      const int vg = item.tile / a.geom.tiles_total;   // virtual group
-      const int tl = (item.tile - vg * a.geom.tiles_total) % tiles_per_grid;
-      u0 = (tl % a.geom.tiles_u) * WS::kTileU - phase_shift(a.geom, vg);
-      v0 = (tl / a.geom.tiles_u) * WS::kTileV;
-    }
-    int b0 = item.rec_begin;
-    do {
-      const int slot = (int)(k % kRing);
-      const unsigned use = k / kRing;
-      if (use > 0 && !mbar_wait(&sm.empty[slot], (use - 1) & 1)) return false;
-      int nb = -1;
-      if (!done) {
-        nb = min(kBuf, item.rec_end - b0);
-        // Gather kPerLane records per lane; their loads are independent,
-        // so they overlap.
-        uint32_t vid[kPerLane], ce[kPerLane], me[kPerLane];
-        R2 v[kPerLane];
-        int grp[kPerLane];
-#pragma unroll
-        for (int q = 0; q < kPerLane; ++q) {
-          const int t = q * 32 + lane;
-          vid[q] = t < nb ? a.rec_vis[b0 + t] : 0u;
-        }
-#pragma unroll
-        for (int q = 0; q < kPerLane; ++q) {
-          const int t = q * 32 + lane;
-          ce[q] = 0; me[q] = 0; grp[q] = -2;
-          if (t < nb) {
-            ce[q] = a.cell[vid[q]];
-            me[q] = a.meta[vid[q]];
-            v[q] = a.vw[vid[q]];
-            grp[q] = group_of(me[q]);
-          }
-        }
-        // ---- stage the slices of the buffer's dominant groups ----------
-        // Candidates: the groups of the first and the last record (records
-        // are sorted by group within a tile, so a long run covers one end).
-        if constexpr (kStage) {
-        const int last = nb - 1;
-        int cand[2];
-        uint32_t cand_meta[2];
-        cand[0] = __shfl_sync(0xffffffffu, grp[0], 0);
-        cand_meta[0] = __shfl_sync(0xffffffffu, me[0], 0);
-        {
-          int gl = grp[0];
-          uint32_t ml = me[0];
-#pragma unroll
-          for (int q = 1; q < kPerLane; ++q)
-            if (q == last / 32) { gl = grp[q]; ml = me[q]; }
-          cand[1] = __shfl_sync(0xffffffffu, gl, last % 32);
-          cand_meta[1] = __shfl_sync(0xffffffffu, ml, last % 32);
-        }
-#pragma unroll
-        for (int ci = 0; ci < 2; ++ci) {
-          const int g = cand[ci];
-          if (ci == 1 && g == cand[0]) break;
-          int cnt = 0;
-#pragma unroll
-          for (int q = 0; q < kPerLane; ++q)
-            cnt += __popc(__ballot_sync(0xffffffffu, grp[q] == g));
-          const int plane = meta_plane(cand_meta[ci]);
-          const int s = a.view.support[plane];
-          const long long bytes = slice_taps(s) * (long long)sizeof(R2);
-          bool resident = false;
-          for (int x = 0; x < kSlots; ++x) resident |= st.group[x] == g;
-          if (resident || cnt < kRunMin || bytes > kSliceBytes) continue;
-          // Take the slot used longest ago that the other candidate does
-          // not hold.
-          int x = 0;
-          for (int y = 1; y < kSlots; ++y) {
-            const bool other = st.group[x] == cand[1 - ci];
-            if (other || (st.group[y] != cand[1 - ci] &&
-                          st.last_k[y] < st.last_k[x]))
-              x = y;
-          }
-          // The slot's previous contents may still be read by a buffer in
-          // flight: wait for the consumers to finish it.
-          if (st.used[x] && st.last_k[x] + kRing > k) {
-            const unsigned kk = st.last_k[x];
-            if (!mbar_wait(&sm.empty[kk % kRing], (kk / kRing) & 1))
-              return false;
-          }
-          const long long start =
-              a.view.base[plane] +
-              (long long)(abs(meta_ou(cand_meta[ci])) * (omax + 1) +
-                          abs(meta_ov(cand_meta[ci]))) * slice_taps(s);
-          if (lane == 0) {
-            mbar_expect_tx(&sm.full[slot], (uint32_t)bytes);
-            bulk_copy_g2s(&sm.slice[x][0], taps + start, (uint32_t)bytes,
-                          &sm.full[slot]);
-          }
-          st.group[x] = g;
-          st.used[x] = true;
-          st.last_k[x] = k;
-        }
-        }  // kStage
-        // ---- prepare the records ---------------------------------------
-#pragma unroll
-        for (int q = 0; q < kPerLane; ++q) {
-          const int t = q * 32 + lane;
-          int src = -1;
-          if constexpr (kStage) {
-            for (int x = 0; x < kSlots; ++x)
-              if (grp[q] == st.group[x]) src = x;
-            // Slots referenced by this buffer stay reserved until it is
-            // done.
-            for (int x = 0; x < kSlots; ++x)
-              if (__any_sync(0xffffffffu, src == x)) st.last_k[x] = k;
-          }
-          if (t < nb) {
-            const uint32_t m = me[q];
-            const int plane = meta_plane(m);
-            const int ou = meta_ou(m), ov = meta_ov(m);
-            const int s = a.view.support[plane];
-            const int F = 2 * s + 1;
-            const int gu = cell_u(ce[q]) - u0, gv = cell_v(ce[q]) - v0;
-            const int su = ou < 0 ? -1 : 1, sv = ov < 0 ? -1 : 1;
-            if (src < 0) {
-              // Slab of (plane, |ov|); rows mirrored for ov < 0, columns by
-              // residue on either side of the fold ou + k*os = 0.
-              sm.rec[slot][t] =
-                  a.view.oversample == 4
-                      ? slab_record<TW, 4>(a.view, plane, s, ou, ov, gu, gv)
-                      : slab_record<TW>(a.view, plane, s, ou, ov, gu, gv);
-            } else {
-              // Tap index of S[0][0] relative to the padded slice start.
-              const int org = kSlicePad * F + (s - sv * gv) * F +
-                              (s - su * gu);
-              sm.rec[slot][t] = make_int4(org, sv * F, gu - s, su * F);
-            }
-            sm.src[slot][t] = (signed char)src;
-            // Bit (warp * kLanesY + lane row) = that lane row's kRows rows
-            // meet the footprint rows [gv - s, gv + s].
-            uint32_t band = 0;
-#pragma unroll
-            for (int gg = 0; gg < kWarps * WS::kLanesY; ++gg) {
-              const int r0 = gg * kRows;
-              if (gv - s <= r0 + kRows - 1 && gv + s >= r0) band |= 1u << gg;
-            }
-            if constexpr (kHalves) {
-              // Bits 8 and 9: the footprint meets tile columns 0..15,
-              // 16..31 (the two half-warps' columns).
-              if (gu - s <= 15) band |= 1u << 8;
-              if (gu + s >= 16) band |= 1u << 9;
-            }
-            sm.band[slot][t] = band;
-            Coef<Real> cf;
-            cf.a = v[q].x;
-            cf.c = v[q].y;
-            if (meta_conj(m)) { cf.b = v[q].y; cf.d = -v[q].x; }
-            else { cf.b = -v[q].y; cf.d = v[q].x; }
-            sm.cf[slot][t] = cf;
-          }
-        }
-      }
-      if (lane == 0) {
-        // item index, record count (-1 = no more work), first/last flags
-        const int flags = done ? 0 : ((b0 == item.rec_begin ? 1 : 0) |
-                                      (b0 + kBuf >= item.rec_end ? 2 : 0));
-        sm.head[slot] = make_int4(it, nb, flags, 0);
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.full[slot]);
-      ++k;
-      if (done) return true;
-      b0 += kBuf;
-    } while (b0 < item.rec_end);
-  }
-}
-
-// The kRows taps of a record with slab descriptor ra for this lane (zeros
-// outside the footprint's columns or when !inband).
-template <typename R2>
-__device__ __forceinline__ void load_slab_taps(const int4 ra, bool inband,
-                                               const R2* __restrict__ slabs,
-                                               const R2* __restrict__ gzeros,
-                                               int lx, int rowl, uint64_t pol,
-                                               R2 (&out)[kRows]) {
-  const int c0 = (ra.w >> 8) & 0xFF, cw = (int)((unsigned)ra.w >> 16);
-  const bool ok = inband && (unsigned)(lx - c0) <= (unsigned)cw;
-  const int off = (lx >= (ra.w & 0xFF) ? ra.x + lx : ra.y - lx) + rowl * ra.z;
-  const R2* p = ok ? slabs + off : gzeros;
-  const int step = ok ? ra.z : 0;
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) out[r] = ld_tap(p + r * step, pol);
-}
-
-// Loads the kRows taps of one record for this lane: from the record's
-// slice slot in shared memory, or from the slab stack (see the record
-// layout above).  Lanes outside the footprint's columns, or outside the
-// warp rows the record meets, read zeros.
-template <typename Real, int TW, bool kStage, typename R2>
-__device__ __forceinline__ void load_record(const Smem<Real, kStage>& sm,
-                                            int slot, int t,
-                                            const R2* __restrict__ slabs,
-                                            const R2* __restrict__ gzeros,
-                                            uint32_t my_bit, int lx, int rowl,
-                                            uint64_t pol, R2 (&out)[kRows]) {
-  const int4 ra = sm.rec[slot][t];
-  // With one lane row per warp (TW = 32) a warp only takes records that
-  // meet its rows; narrower tiles check the lane's own row group.
-  const bool inband = TW == 32 || (sm.band[slot][t] & my_bit) != 0u;
-  if (kStage && sm.src[slot][t] >= 0) {
-    const int src = sm.src[slot][t];
-    const bool ok =
-        inband && (unsigned)(lx - ra.z) <= (unsigned)(abs(ra.w) - 1);
-    const int off = ra.x + rowl * ra.y + lx * (ra.w < 0 ? -1 : 1);
-    const R2* p = ok ? &sm.slice[src][0] + off
-                     : &sm.zero[Smem<Real, kStage>::kZeroTaps / 2];
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) out[r] = p[r * ra.y];
-    return;
-  }
-  const int c0 = (ra.w >> 8) & 0xFF, cw = (int)((unsigned)ra.w >> 16);
-  const bool ok = inband && (unsigned)(lx - c0) <= (unsigned)cw;
-  const int off = (lx >= (ra.w & 0xFF) ? ra.x + lx : ra.y - lx) + rowl * ra.z;
-  const R2* p = ok ? slabs + off : gzeros;
-  const int step = ok ? ra.z : 0;
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) out[r] = ld_tap(p + r * step, pol);
-}
-
-// Adds one record's contribution to the lane's cells.  FP32: packed FP32x2
-// FMAs into the (P, Q) pairs (see Coef); FP64: plain FMAs into (re, im).
-template <typename Real, typename R2>
-__device__ __forceinline__ void accumulate(const Coef<Real>& c,
-                                           const R2 (&tp)[kRows],
-                                           R2 (&acc)[kRows],
-                                           R2 (&acq)[kRows]) {
-  if constexpr (sizeof(Real) == 4) {
-    const float2 cp = make_float2(c.a, c.d), cq = make_float2(c.c, c.b);
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      acc[r] = __ffma2_rn(cp, tp[r], acc[r]);
-      acq[r] = __ffma2_rn(cq, tp[r], acq[r]);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      acc[r].x = fma(c.b, tp[r].y, fma(c.a, tp[r].x, acc[r].x));
-      acc[r].y = fma(c.d, tp[r].y, fma(c.c, tp[r].x, acc[r].y));
-    }
-  }
-}
-
-template <typename Real, bool kCompensate, int TW, bool kStage, bool kHalves>
-__global__ void __launch_bounds__(kThreads, sizeof(Real) == 4 ? 2 : 1)
+template <typename Real, int TW, bool kWide>
+__global__ void __launch_bounds__(kGridThreads, sizeof(Real) == 4 ? 5 : 2)
 k_grid_tiles(GridArgs<Real> a) {
-  static_assert(!kHalves || (TW == 32 && !kStage),
-                "half-warp record streams: 32-wide tiles, taps from the "
-                "slab stack");
+  constexpr bool kCompensate = sizeof(Real) == 4;
+  // Records in flight per warp.
+  constexpr int kDepth = 2;
   using R2 = typename Vec2<Real>::type;
   using WS = WarpShape<TW>;
-  using SM = Smem<Real, kStage>;
-  constexpr int G = WS::kLanesY;
+  using SM = WarpSmem<Real, TW>;
+  constexpr int G = WS::kLanesY, Q = SM::kQueue;
   extern __shared__ __align__(16) unsigned char g_smem_raw[];
-  SM& sm = *reinterpret_cast<SM*>(g_smem_raw);
-
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < SM::kZeroTaps; i += blockDim.x) {
-    sm.zero[i].x = 0;
-    sm.zero[i].y = 0;
-  }
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kRing; ++i) {
-      mbar_init(&sm.full[i], 1);
-      mbar_init(&sm.empty[i], kWarps);
-    }
-    // Make the initialised barriers visible to the async proxy (bulk
-    // copies complete transactions on them).
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-
-  if (warp == kWarps) {
-    if (!produce<Real, TW, kStage, kHalves>(a, sm)) atomicExch(a.error, 1u);
-    return;
-  }
-
+  const int lane = threadIdx.x & 31;
+  SM& sm = reinterpret_cast<SM*>(g_smem_raw)[threadIdx.x >> 5];
   const int lx = lane % TW, ly = lane / TW;
-  const int rowl = warp * WS::kBand + ly * kRows;   // this lane's row 0
-  const int G_size = a.grid_size;
-  const R2* __restrict__ slabs = (const R2*)a.view.slabs;
-  const R2* __restrict__ gzeros = (const R2*)a.view.zeros;
-  const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
-  const uint64_t pol = evict_last_policy();
-  const uint32_t my_bit = 1u << (warp * G + ly);
-  const uint32_t warp_bits = ((1u << G) - 1u) << (warp * G);
+  const R2* __restrict__ stack = (const R2*)a.view.taps;
+  const uint32_t lt = (1u << lane) - 1u;
+  // The launch's units: the bands of its virtual groups' items.
+  const unsigned first = a.group_items[a.group];
+  const unsigned units =
+      (a.group_items[a.group + a.group_span] - first) * kWarps;
+  unsigned next = 0;
+  if (lane == 0) next = atomicAdd(a.counter, 1u);
+  for (;;) {
+    const unsigned unit = __shfl_sync(0xffffffffu, next, 0);
+    if (unit >= units) return;
+    if (lane == 0) next = atomicAdd(a.counter, 1u);   // used in the next turn
+    const WorkItem item = a.items[first + unit / kWarps];
+    const int band = (int)(unit % kWarps);
+    const int g0 = band * G;   // first lane-row group
 
-  // FP32: (P, Q) pairs of every cell (see Coef); FP64: (re, im) in acc.
-  R2 acc[kRows], acq[kRows];
+    R2 acc[kRows], acq[kRows];   // P and Q
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) acc[r].x = acc[r].y = acq[r].x = acq[r].y = 0;
-
-  for (unsigned k = 0;; ++k) {
-    const int slot = (int)(k % kRing);
-    if (!mbar_wait(&sm.full[slot], (k / kRing) & 1)) {
-      atomicExch(a.error, 1u);
-      return;
+    for (int r = 0; r < kRows; ++r) {
+      acc[r] = acq[r] = R2{};
+      if constexpr (kCompensate) sm.hi[r][lane] = sm.lo[r][lane] = R2{};
     }
-    const int4 head = sm.head[slot];
-    const int nb = head.y;
-    if (nb < 0) break;
-    if (head.z & 1) {  // first buffer of a work item
+    R2 tp[kDepth][kRows];
+    // Queue positions: `at` the oldest record not yet added (the kDepth from
+    // there on are being loaded once `primed`), tails the ends.
+    int at = 0, tails[G];
+    bool primed = false;
+#pragma unroll
+    for (int g = 0; g < G; ++g) tails[g] = 0;
+    Queued<Real>* const queue = sm.queue[ly];
+    auto load = [&](int i, R2 (&out)[kRows]) {
+      const int4 e = *(const int4*)&queue[i & (Q - 1)];
+      const int t = min(max(lx - (e.y >> 16), -e.z), e.z);
+      load_taps<kWide>(stack, (uint32_t)(e.x + (int)(short)e.y * t), e.w, out);
+    };
+    auto add = [&](int i, const R2 (&t)[kRows]) {
+      const Queued<Real>& e = queue[i & (Q - 1)];
+      R2 p, q;
+      p.x = e.a; p.y = e.d;
+      q.x = e.c; q.y = e.b;
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
-        acc[r].x = acc[r].y = acq[r].x = acq[r].y = 0;
-        if constexpr (kCompensate) {
-          sm.hi[r][threadIdx.x] = acc[r];
-          sm.lo[r][threadIdx.x] = acc[r];
+        acc[r] = fma2(p, t[r], acc[r]);
+        acq[r] = fma2(q, t[r], acq[r]);
+      }
+    };
+    // Adds queued records, kDepth at a time, while every queue holds another
+    // kDepth to load behind them.
+    auto run = [&](int end) {
+      if (!primed && end - at >= kDepth) {
+#pragma unroll
+        for (int d = 0; d < kDepth; ++d) load(at + d, tp[d]);
+        primed = true;
+      }
+      for (; end - at >= 2 * kDepth; at += kDepth) {
+#pragma unroll
+        for (int d = 0; d < kDepth; ++d) {
+          add(at + d, tp[d]);
+          load(at + kDepth + d, tp[d]);
         }
       }
-    }
-    // ---- half-warp record streams (32-wide tiles) ------------------------
-    // Each half-warp takes, in queue order, the records of the buffer that
-    // meet this warp's rows and its own 16 columns (lists built from the
-    // buffer's band bits), so a record that meets one half only runs beside
-    // another record on the other half.  Up to three records per half at a
-    // time.  Each cell still takes its records in queue order.
-    if constexpr (kHalves) {
-      const int hh = lane >> 4;
-      unsigned char* l0 = sm.half_list[warp][0];
-      unsigned char* l1 = sm.half_list[warp][1];
-      const uint32_t lt = (1u << lane) - 1u;
-      int n0 = 0, n1 = 0;
-      for (int c0 = 0; c0 < nb; c0 += 32) {
-        const uint32_t bd = c0 + lane < nb ? sm.band[slot][c0 + lane] : 0u;
-        const bool mine = (bd & warp_bits) != 0u;
-        const bool in0 = mine && (bd & 0x100u), in1 = mine && (bd & 0x200u);
-        const uint32_t b0 = __ballot_sync(0xffffffffu, in0);
-        const uint32_t b1 = __ballot_sync(0xffffffffu, in1);
-        if (in0) l0[n0 + __popc(b0 & lt)] = (unsigned char)(c0 + lane);
-        if (in1) l1[n1 + __popc(b1 & lt)] = (unsigned char)(c0 + lane);
-        n0 += __popc(b0);
-        n1 += __popc(b1);
+    };
+    // Fills every queue up to `end` with records that add nothing.
+    auto fill = [&](int end) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        if (g == ly)
+          for (int i = tails[g] + lx; i < end; i += TW) {
+            Queued<Real> none{};
+            none.x = kStackZero;
+            queue[i & (Q - 1)] = none;
+          }
+        tails[g] = max(tails[g], end);
       }
       __syncwarp();
-      const unsigned char* my = hh ? l1 : l0;
-      const int nmine = hh ? n1 : n0;
-      const int n = max(n0, n1);
-      // Entry i of this half's list; past its end the half runs the other
-      // half's entry i with its taps read as zeros (so it adds nothing).
-      const unsigned char* other = hh ? l0 : l1;
-      auto pick = [&](int i) { return (int)(i < nmine ? my[i] : other[i]); };
-      auto taps = [&](int i, int t, R2 (&out)[kRows]) {
-        load_slab_taps(sm.rec[slot][t], i < nmine, slabs, gzeros, lx, rowl,
-                       pol, out);
-      };
-      auto coef = [&](int t) -> const Coef<Real>& { return sm.cf[slot][t]; };
-      for (int i = 0; i < n; i += 3) {
-        const int tA = pick(i);
-        R2 ta[kRows];
-        taps(i, tA, ta);
-        if (n - i >= 2) {
-          const int tB = pick(i + 1);
-          R2 tb[kRows];
-          taps(i + 1, tB, tb);
-          if (n - i >= 3) {
-            const int tC = pick(i + 2);
-            R2 tc[kRows];
-            taps(i + 2, tC, tc);
-            accumulate<Real>(coef(tA), ta, acc, acq);
-            accumulate<Real>(coef(tB), tb, acc, acq);
-            accumulate<Real>(coef(tC), tc, acc, acq);
-          } else {
-            accumulate<Real>(coef(tA), ta, acc, acq);
-            accumulate<Real>(coef(tB), tb, acc, acq);
-          }
-        } else {
-          accumulate<Real>(coef(tA), ta, acc, acq);
-        }
-      }
-      __syncwarp();
-    } else
-    // ---- this warp's records: those whose footprint meets its band ------
-    for (int c0 = 0; c0 < nb; c0 += 32) {
-      const bool touch =
-          c0 + lane < nb && (sm.band[slot][c0 + lane] & warp_bits) != 0u;
-      uint32_t m = __ballot_sync(0xffffffffu, touch);
-      // Up to three records at a time (FP32; two for FP64, whose taps take
-      // twice the registers): 3 * kRows independent tap loads per lane in
-      // flight.  Each cell takes the records in queue order.
-      while (m) {
-        const int tA = c0 + __ffs(m) - 1;
-        m &= m - 1;
-        R2 ta[kRows];
-        load_record<Real, TW, kStage>(sm, slot, tA, slabs, gzeros, my_bit,
-                                      lx, rowl, pol, ta);
-        if (m) {
-          const int tB = c0 + __ffs(m) - 1;
-          m &= m - 1;
-          R2 tb[kRows];
-          load_record<Real, TW, kStage>(sm, slot, tB, slabs, gzeros, my_bit,
-                                        lx, rowl, pol, tb);
-          if (sizeof(Real) == 4 && m) {
-            const int tC = c0 + __ffs(m) - 1;
-            m &= m - 1;
-            R2 tc[kRows];
-            load_record<Real, TW, kStage>(sm, slot, tC, slabs, gzeros,
-                                          my_bit, lx, rowl, pol, tc);
-            accumulate<Real>(sm.cf[slot][tA], ta, acc, acq);
-            accumulate<Real>(sm.cf[slot][tB], tb, acc, acq);
-            accumulate<Real>(sm.cf[slot][tC], tc, acc, acq);
-          } else {
-            accumulate<Real>(sm.cf[slot][tA], ta, acc, acq);
-            accumulate<Real>(sm.cf[slot][tB], tb, acc, acq);
-          }
-        } else {
-          accumulate<Real>(sm.cf[slot][tA], ta, acc, acq);
-        }
-      }
-    }
-    if constexpr (kCompensate) {
+    };
+    auto fold = [&]() {
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
-        R2 hi = sm.hi[r][threadIdx.x], lo = sm.lo[r][threadIdx.x];
-        const float re = __fadd_rn(acc[r].x, acq[r].y);
-        const float im = __fadd_rn(acq[r].x, acc[r].y);
+        R2 hi = sm.hi[r][lane], lo = sm.lo[r][lane];
         float s, e;
-        two_sum(hi.x, re, s, e); hi.x = s; lo.x += e;
-        two_sum(hi.y, im, s, e); hi.y = s; lo.y += e;
-        sm.hi[r][threadIdx.x] = hi;
-        sm.lo[r][threadIdx.x] = lo;
-        acc[r].x = acc[r].y = acq[r].x = acq[r].y = 0;
+        two_sum(hi.x, acc[r].x + acq[r].y, s, e); hi.x = s; lo.x += e;
+        two_sum(hi.y, acq[r].x + acc[r].y, s, e); hi.y = s; lo.y += e;
+        sm.hi[r][lane] = hi;
+        sm.lo[r][lane] = lo;
+        acc[r] = acq[r] = R2{};
+      }
+    };
+
+    uint32_t span = kSpanNone;
+    Record<Real> rec;
+    auto fetch = [&](int i) {
+      span = kSpanNone;
+      if (i + lane < item.rec_end) {
+        span = a.spans[i + lane];
+        rec = a.recs[i + lane];
+      }
+    };
+    fetch(item.rec_begin);
+    for (int i = item.rec_begin; i < item.rec_end; i += 32) {
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const bool hit = span_meets(span, g0 + g);
+        const uint32_t b = __ballot_sync(0xffffffffu, hit);
+        if (hit)
+          sm.queue[g][(tails[g] + __popc(b & lt)) & (Q - 1)] =
+              queued(rec, span, g0 + g);
+        tails[g] += __popc(b);
+      }
+      if (i + 32 < item.rec_end) fetch(i + 32);
+      __syncwarp();
+      int lo = tails[0], hi = tails[0];
+#pragma unroll
+      for (int g = 1; g < G; ++g) {
+        lo = min(lo, tails[g]);
+        hi = max(hi, tails[g]);
+      }
+      run(lo);
+      // A queue without room for another 32 records goes on alone.
+      if (G > 1 && hi - at > Q - 32) {
+        fill(hi - (hi - at) % kDepth);
+        run(hi - (hi - at) % kDepth);
+      }
+      // Plain FP32 sums of at most 128 records (and the few in flight) go
+      // into the compensated (hi, lo) pair.
+      if (kCompensate && ((i - item.rec_begin) & 96) == 96) fold();
+      __syncwarp();
+    }
+    int end = tails[0];
+#pragma unroll
+    for (int g = 1; g < G; ++g) end = max(end, tails[g]);
+    if (end > at) {
+      end = at + (end - at + kDepth - 1) / kDepth * kDepth;
+      fill(end);
+      run(end);
+#pragma unroll
+      for (int d = 0; d < kDepth; ++d) add(at + d, tp[d]);
+    }
+    __syncwarp();   // the queues are free for the next unit
+    if (kCompensate) fold();
+    // An owned band that no record meets stays as it is (in direct mode its
+    // cells may still have to move between the host and the scratch grid).
+    if (end == 0 && item.slot < 0 && !a.tile_groups) continue;
+
+    // ---- flush the band ---------------------------------------------------
+    const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
+    const int rt = item.tile % a.geom.tiles_total;   // real tile
+    const int gi = rt / tiles_per_grid;
+    const int tl = rt - gi * tiles_per_grid;
+    const int vg = item.tile / a.geom.tiles_total;   // virtual group
+    R2 out[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      if constexpr (kCompensate) {
+        const R2 hi = sm.hi[r][lane], lo = sm.lo[r][lane];
+        out[r].x = hi.x + lo.x;
+        out[r].y = hi.y + lo.y;
+      } else {
+        out[r].x = acc[r].x + acq[r].y;
+        out[r].y = acq[r].x + acc[r].y;
       }
     }
-    if (head.z & 2) {  // last buffer of the work item: flush its tile
-      const WorkItem item = a.items[head.x];
-      const int rt = item.tile % a.geom.tiles_total;   // real tile
-      const int gi = rt / tiles_per_grid;
-      const int tl = rt - gi * tiles_per_grid;
-      const int vg = item.tile / a.geom.tiles_total;   // virtual group
-      const int u0 = (tl % a.geom.tiles_u) * WS::kTileU - phase_shift(a.geom, vg);
-      const int v0 = (tl / a.geom.tiles_u) * WS::kTileV;
-      R2 out[kRows];
+    if (item.slot < 0) {
+      const int col =
+          (tl % a.geom.tiles_u) * WS::kTileU - phase_shift(a.geom, vg) + lx;
+      const int row0 = (tl / a.geom.tiles_u) * WS::kTileV +
+                       (g0 + ly) * kRows;
+      // Phase tiles reach past the grid's first and last columns.
+      const bool col_in = (unsigned)col < (unsigned)a.grid_size;
+      R2 *src, *dst;
+      cell_ends<R2>(a.tile_groups, a.geom, tl / a.geom.tiles_u,
+                    col_in ? col : 0, vg,
+                    (R2*)(a.grid + (long long)gi * a.grid_stride),
+                    (R2*)a.host, src, dst);
 #pragma unroll
       for (int r = 0; r < kRows; ++r) {
-        if constexpr (kCompensate) {
-          const R2 hi = sm.hi[r][threadIdx.x], lo = sm.lo[r][threadIdx.x];
-          out[r].x = hi.x + lo.x;
-          out[r].y = hi.y + lo.y;
-        } else {
-          out[r] = acc[r];
+        const int row = row0 + r;
+        if (row < a.grid_size && col_in) {
+          const size_t off = (size_t)row * a.grid_size + col;
+          R2 old = __ldcs(src + off);
+          old.x += out[r].x;
+          old.y += out[r].y;
+          __stcs(dst + off, old);
         }
       }
-      const int col = u0 + lx;
-      if (item.slot < 0) {
-        // Phase tiles reach past the grid's first and last columns.
-        const bool col_in = (unsigned)col < (unsigned)G_size;
-        R2 *src, *dst;
-        cell_ends<R2>(a.tile_groups, a.geom, tl / a.geom.tiles_u,
-                      col_in ? col : 0, vg,
-                      (R2*)(a.grid + (long long)gi * a.grid_stride),
-                      (R2*)a.host, src, dst);
+    } else {
+      // Partial tile, thread-major: entry r * kConsumers + band * 32 + lane.
+      R2* p = a.partials + (size_t)item.slot * kCells + band * 32 + lane;
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-          const int row = v0 + rowl + r;
-          if (row < G_size && col_in) {
-            const size_t off = (size_t)row * G_size + col;
-            R2 old = __ldcs(src + off);
-            old.x += out[r].x;
-            old.y += out[r].y;
-            __stcs(dst + off, old);
-          }
-        }
-      } else {
-        // Partial tile, thread-major: entry r * kConsumers + thread.
-        R2* p = a.partials + (size_t)item.slot * kCells;
-#pragma unroll
-        for (int r = 0; r < kRows; ++r)
-          __stcs(p + r * kConsumers + threadIdx.x, out[r]);
-      }
+      for (int r = 0; r < kRows; ++r) __stcs(p + r * kConsumers, out[r]);
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.empty[slot]);
   }
 }
 
@@ -1055,21 +807,15 @@ __global__ void k_item_emit(const uint32_t* __restrict__ tile_start,
   }
 }
 
-template <typename Real, int TW, bool kStage, bool kHalves = false>
-void* grid_kernel_ptr() {
-  return (void*)k_grid_tiles<Real, std::is_same<Real, float>::value, TW,
-                             kStage, kHalves>;
-}
-
 // The kernels take more than 48 KB of dynamic shared memory: opt in before
 // querying occupancy or launching.  The opt-in is made once per device, so
 // later launches (replays captured in a CUDA graph among them) make no
 // attribute call.
-template <typename Real, int TW, bool kStage, bool kHalves = false>
+template <typename Real, int TW, bool kWide>
 cudaError_t prepare_grid_kernel(void** fn, size_t* smem) {
   static std::atomic<unsigned long long> opted_in{0};
-  *fn = grid_kernel_ptr<Real, TW, kStage, kHalves>();
-  *smem = sizeof(Smem<Real, kStage>);
+  *fn = (void*)k_grid_tiles<Real, TW, kWide>;
+  *smem = kGridWarps * sizeof(WarpSmem<Real, TW>);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -1081,18 +827,18 @@ cudaError_t prepare_grid_kernel(void** fn, size_t* smem) {
   return e;
 }
 
+template <typename Real, bool kWide>
+cudaError_t prepare_grid_kernel_of(int tile_u, void** fn, size_t* smem) {
+  return tile_u == 32   ? prepare_grid_kernel<Real, 32, kWide>(fn, smem)
+         : tile_u == 16 ? prepare_grid_kernel<Real, 16, kWide>(fn, smem)
+                        : prepare_grid_kernel<Real, 8, kWide>(fn, smem);
+}
+
 template <typename Real>
-cudaError_t prepare_grid_kernel_for(int tile_u, bool stage, void** fn,
-                                    size_t* smem, int lane_groups = 1) {
-  if (lane_groups == 2 && tile_u == 32 && !stage)
-    return prepare_grid_kernel<Real, 32, false, true>(fn, smem);
-  if (stage)
-    return tile_u == 32   ? prepare_grid_kernel<Real, 32, true>(fn, smem)
-           : tile_u == 16 ? prepare_grid_kernel<Real, 16, true>(fn, smem)
-                          : prepare_grid_kernel<Real, 8, true>(fn, smem);
-  return tile_u == 32   ? prepare_grid_kernel<Real, 32, false>(fn, smem)
-         : tile_u == 16 ? prepare_grid_kernel<Real, 16, false>(fn, smem)
-                        : prepare_grid_kernel<Real, 8, false>(fn, smem);
+cudaError_t prepare_grid_kernel_for(int tile_u, bool wide, void** fn,
+                                    size_t* smem) {
+  return wide ? prepare_grid_kernel_of<Real, true>(tile_u, fn, smem)
+              : prepare_grid_kernel_of<Real, false>(tile_u, fn, smem);
 }
 
 }  // namespace
@@ -1167,18 +913,27 @@ cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
 }
 
 template <typename Real>
-int grid_tiles_ctas_per_sm(int tile_u, bool stage, int lane_groups) {
+int grid_tiles_ctas_per_sm(int tile_u, bool wide) {
   void* fn = nullptr;
   size_t smem = 0;
   int n = 0;
-  if (prepare_grid_kernel_for<Real>(tile_u, stage, &fn, &smem,
-                                    lane_groups) !=
-          cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads,
+  if (prepare_grid_kernel_for<Real>(tile_u, wide, &fn, &smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kGridThreads,
                                                     smem) != cudaSuccess)
     n = 1;
   return n < 1 ? 1 : n;
 }
+
+int grid_teams(int num_ctas) {
+  return std::max(1, num_ctas * kGridWarps / kWarps);
+}
+
+template <typename Real>
+size_t prepared_record_bytes() {
+  return sizeof(Record<Real>);
+}
+template size_t prepared_record_bytes<float>();
+template size_t prepared_record_bytes<double>();
 
 template <typename Real>
 cudaError_t launch_reduce_phases(const int2* tile_slot, const Real* partials,
@@ -1241,14 +996,14 @@ cudaError_t launch_reduce_group(const int4* split_tiles,
 template <typename Real>
 cudaError_t launch_grid_tiles(const WorkItem* items,
                               const uint32_t* group_items,
-                              uint32_t* counter, uint32_t* error,
-                              const uint32_t* rec_vis,
+                              uint32_t* counter, void* recs,
+                              unsigned short* spans, const uint32_t* rec_vis,
                               const uint32_t* cell, const uint32_t* meta,
                               const void* vw, StackView view, TileGeom geom,
                               int grid_size, Real* grid, long long grid_stride,
                               Real* partials, const int4* split_tiles,
                               const uint32_t* num_split, int max_split,
-                              int num_ctas, bool stage, cudaStream_t s,
+                              int num_ctas, cudaStream_t s,
                               const cudaEvent_t* wait_before,
                               const cudaEvent_t* record_after,
                               Real* host_grid, const uint32_t* tile_groups,
@@ -1259,7 +1014,8 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
   a.group_items = group_items;
   a.group = 0;
   a.counter = counter;
-  a.error = error;
+  a.recs = (Record<Real>*)recs;
+  a.spans = spans;
   a.rec_vis = rec_vis;
   a.cell = cell;
   a.meta = meta;
@@ -1276,12 +1032,20 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
     return cudaErrorInvalidValue;
   void* fn = nullptr;
   size_t smem = 0;
-  cudaError_t e = prepare_grid_kernel_for<Real>(geom.tile_u, stage, &fn,
-                                                &smem, geom.lane_groups);
+  cudaError_t e = prepare_grid_kernel_for<Real>(geom.tile_u, view.wide,
+                                                &fn, &smem);
   if (e != cudaSuccess) return e;
-  void* args[] = {&a};
   const int span = group_span > 1 ? group_span : 1;
   a.group_span = span;
+  int num_groups = geom.num_groups;
+  void* prep_args[] = {&a, &num_groups};
+  e = cudaLaunchKernel(geom.tile_u == 32 ? (void*)k_prepare_records<Real, 32>
+                       : geom.tile_u == 16
+                           ? (void*)k_prepare_records<Real, 16>
+                           : (void*)k_prepare_records<Real, 8>,
+                       dim3(8 * num_ctas), dim3(128), prep_args, 0, s);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&a};
   for (int g = 0; g < geom.num_groups; g += span) {
     a.group = g;
     if (wait_before && wait_before[g]) {
@@ -1290,7 +1054,7 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
     }
     e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    e = cudaLaunchKernel(fn, dim3(num_ctas), dim3(kThreads), args, smem, s);
+    e = cudaLaunchKernel(fn, dim3(num_ctas), dim3(kGridThreads), args, smem, s);
     if (e != cudaSuccess) return e;
     if (span > 1 && tile_slot) {
       e = launch_reduce_phases<Real>(tile_slot, partials, geom, g, grid_size,
@@ -1313,18 +1077,18 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
   return cudaSuccess;
 }
 
-template int grid_tiles_ctas_per_sm<float>(int, bool, int);
-template int grid_tiles_ctas_per_sm<double>(int, bool, int);
+template int grid_tiles_ctas_per_sm<float>(int, bool);
+template int grid_tiles_ctas_per_sm<double>(int, bool);
 template cudaError_t launch_grid_tiles<float>(
-    const WorkItem*, const uint32_t*, uint32_t*, uint32_t*, const uint32_t*,
-    const uint32_t*, const uint32_t*, const void*, StackView, TileGeom, int,
-    float*, long long, float*, const int4*, const uint32_t*, int, int, bool,
+    const WorkItem*, const uint32_t*, uint32_t*, void*, unsigned short*,
+    const uint32_t*, const uint32_t*, const uint32_t*, const void*, StackView, TileGeom, int,
+    float*, long long, float*, const int4*, const uint32_t*, int, int,
     cudaStream_t, const cudaEvent_t*, const cudaEvent_t*, float*,
     const uint32_t*, int, const int2*, const uint32_t*);
 template cudaError_t launch_grid_tiles<double>(
-    const WorkItem*, const uint32_t*, uint32_t*, uint32_t*, const uint32_t*,
-    const uint32_t*, const uint32_t*, const void*, StackView, TileGeom, int,
-    double*, long long, double*, const int4*, const uint32_t*, int, int, bool,
+    const WorkItem*, const uint32_t*, uint32_t*, void*, unsigned short*,
+    const uint32_t*, const uint32_t*, const uint32_t*, const void*, StackView, TileGeom, int,
+    double*, long long, double*, const int4*, const uint32_t*, int, int,
     cudaStream_t, const cudaEvent_t*, const cudaEvent_t*, double*,
     const uint32_t*, int, const int2*, const uint32_t*);
 

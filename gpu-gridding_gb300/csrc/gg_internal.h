@@ -33,21 +33,14 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals,
                              bool* in_alt);
 
 // ---- kernel stack preparation (gg_stack.cu) -------------------------------
-// Re-lays conv_func (device, [P][csh][csh] complex) into the residue-split
-// layout and forms the FP64 tap sums in the reference's summation order.
+// Re-lays conv_func (device, [P][csh][csh] complex) into the slices of
+// StackView and forms the FP64 tap sums in the reference's summation order.
 // With `changed` given, each of these kernels returns at once while
 // *changed == 0 (a cube equal to the one the outputs were made from).
 template <typename Real>
 cudaError_t launch_stack_relayout(const Real* d_conv_func, StackView view,
-                                  void* d_taps_out, long long total_taps,
-                                  cudaStream_t s,
+                                  void* d_taps_out, cudaStream_t s,
                                   const int* changed = nullptr);
-// Fills the slab stack (view.slabs layout, planes at view.sbase).
-template <typename Real>
-cudaError_t launch_stack_relayout_slabs(const Real* d_conv_func,
-                                        StackView view, void* d_out,
-                                        cudaStream_t s,
-                                        const int* changed = nullptr);
 // support_max: the largest support of the stack (sizes the row window).
 template <typename Real>
 cudaError_t launch_tap_sums(StackView view, double* d_tap_sum,
@@ -76,13 +69,10 @@ __host__ __device__ inline int tile_v_of_shape(int shape) {
   return 2048 / (32 >> shape);
 }
 
-// Tile shape, slice staging and tile phases for a call, from its mean
+// Tile shape and tile phases for a call, from its mean
 // footprint side sqrt(macs / gridded points): narrow tiles only for tiny
-// footprints (a 32-wide warp would leave most lanes outside them); kernel
-// slices staged in shared memory (bit 8) when footprints are small enough
-// for their slices to fit the slots, otherwise the kernel keeps its shared
-// memory small so the L1 cache serves the tap loads; tile phases (bits 12
-// and 13: log2 of 1, 2, 4 or 8) four when footprints are narrower than the
+// footprints (a 32-wide warp would leave most lanes outside them); tile
+// phases (bits 12 and 13: log2 of 1, 2, 4 or 8) four when footprints are narrower than the
 // tile, where offset tile grids save the most tile crossings, else one.
 // forced_shape >= 0 overrides the shape, phases > 0 the phases.
 __host__ __device__ inline uint32_t choose_shape(unsigned long long macs,
@@ -92,11 +82,10 @@ __host__ __device__ inline uint32_t choose_shape(unsigned long long macs,
   const double side = gridded ? sqrt((double)macs / (double)gridded) : 0.0;
   int shape = forced_shape;
   if (shape < 0) shape = side >= 16.0 ? 0 : (side >= 8.0 ? 1 : 2);
-  const uint32_t stage = side < 40.0 ? 1u : 0u;
   if (phases <= 0) phases = side < (double)tile_u_of_shape(shape) ? 4 : 1;
   const uint32_t pbits =
       phases >= 8 ? 3u : (phases >= 4 ? 2u : (phases >= 2 ? 1u : 0u));
-  return (uint32_t)shape | (stage << 8) | (pbits << 12);
+  return (uint32_t)shape | (pbits << 12);
 }
 // Tile phases of a shape word made by choose_shape.
 __host__ __device__ inline int phases_of_shape(uint32_t word) {
@@ -250,7 +239,12 @@ struct ItemBuffers {
 cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
                                uint32_t num_records, uint32_t chunk,
                                ItemBuffers b, cudaStream_t s);
-// Persistent launches in virtual-group order, each over the work items of
+// Bytes of a prepared record (launch_grid_tiles' recs, one per record; spans
+// takes two more).
+template <typename Real>
+size_t prepared_record_bytes();
+// Prepares the records of every item (recs, spans), then
+// persistent launches in virtual-group order, each over the work items of
 // group_span consecutive virtual groups: with group_span = tile_phases one
 // launch per plane group takes all its tile phases (the items were built
 // with ItemBuffers::partial_phases = tile_phases: the first phase's
@@ -268,14 +262,14 @@ cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
 template <typename Real>
 cudaError_t launch_grid_tiles(const WorkItem* items,
                               const uint32_t* group_items,
-                              uint32_t* counter, uint32_t* error,
-                              const uint32_t* rec_vis,
+                              uint32_t* counter, void* recs,
+                              unsigned short* spans, const uint32_t* rec_vis,
                               const uint32_t* cell, const uint32_t* meta,
                               const void* vw, StackView view, TileGeom geom,
                               int grid_size, Real* grid, long long grid_stride,
                               Real* partials, const int4* split_tiles,
                               const uint32_t* num_split, int max_split,
-                              int num_ctas, bool stage, cudaStream_t s,
+                              int num_ctas, cudaStream_t s,
                               const cudaEvent_t* wait_before = nullptr,
                               const cudaEvent_t* record_after = nullptr,
                               Real* host_grid = nullptr,
@@ -295,10 +289,11 @@ cudaError_t launch_tile_groups(const uint32_t* tile_start,
                                const TileGeom& geom, int grid_size,
                                uint32_t* out, unsigned long long* cells,
                                cudaStream_t s);
-// stage: the kernel variant that stages kernel slices in shared memory;
-// lane_groups: TileGeom::lane_groups.
+// Resident CTAs per SM (wide: StackView::wide), and the teams of one warp per
+// band of a tile that num_ctas CTAs make.
 template <typename Real>
-int grid_tiles_ctas_per_sm(int tile_u, bool stage, int lane_groups = 1);
+int grid_tiles_ctas_per_sm(int tile_u, bool wide);
+int grid_teams(int num_ctas);
 
 // ---- accessors defined in gg_api.cu ---------------------------------------
 // Records a failure for gg_last_error() on this thread; returns code.
@@ -345,7 +340,7 @@ cudaError_t measure_fp32_fma(int num_sms, double* tflops_best, float* ms_out);
 // ---- adjoint (gg_degrid.cu) -----------------------------------------------
 // Resident CTAs per SM of the degridding kernel.
 template <typename Real>
-int degrid_tiles_ctas_per_sm();
+int degrid_tiles_ctas_per_sm(bool wide);
 // One persistent launch over the whole work-item queue (32 x 64-cell tiles
 // only): rec_out[rec_offset[v] + rank] = the record's share of
 // conj(tap) * grid for every record, rank = the record's tile among

@@ -13,7 +13,7 @@
 // beforehand with gg_kernels_create_f (that set-up step does allocate).
 //
 // Costs of this design, stated for the caller:
-// * every GPU that loads the library holds the 32 MiB array until the
+// * every GPU that loads the library holds the 48 MiB array until the
 //   process exits, whether or not it ever calls this entry point;
 // * the array is shared by all calls on a device: calls that overlap on the
 //   GPU (different streams, different host threads) race on it and must be
@@ -50,7 +50,7 @@ constexpr size_t kNoAllocMaxRecords = size_t(1) << 20;  // 1,048,576
 constexpr int kNoAllocMaxGrid = 8192;
 constexpr int kNoAllocMaxSlots = 384;    // partial tiles of split tiles
 constexpr int kNoAllocCells = 2048;      // cells per tile
-constexpr size_t kNoAllocBytes = size_t(32) << 20;
+constexpr size_t kNoAllocBytes = size_t(48) << 20;
 constexpr int kMaxDevices = 64;
 
 // The scratch memory of every no-alloc call on a device.
@@ -192,6 +192,9 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   WorkItem* items = c.take<WorkItem>(max_tiles + kNoAllocMaxSlots + 16);
   int4* split_tiles = c.take<int4>(max_tiles + 1);
   float2* partials = c.take<float2>((size_t)kNoAllocMaxSlots * kNoAllocCells);
+  unsigned char* recs =
+      c.take<unsigned char>(maxr * prepared_record_bytes<float>());
+  unsigned short* spans = c.take<unsigned short>(maxr);
   if (c.used > kNoAllocBytes)
     return record_error(GG_ERR_UNSUPPORTED,
                         "no-alloc scratch layout exceeds the array");
@@ -238,7 +241,6 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   }
   const uint32_t total = host_sc[0];
   const int shape = (int)(host_sc[5] & 0xFFu);
-  const bool stage = ((host_sc[5] >> 8) & 1u) != 0;
   if (total > kNoAllocMaxRecords)
     return record_error(GG_ERR_CAPACITY,
                         "the call needs more (visibility, tile) records than "
@@ -285,14 +287,16 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
                              s));
   int sms = 0;
   NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int num_ctas = sms * grid_tiles_ctas_per_sm<float>(geom.tile_u, stage);
-  // Work items of about total / (2 * num_ctas) records, as the allocating
+  const int num_ctas =
+      sms * grid_tiles_ctas_per_sm<float>(geom.tile_u, view.wide);
+  // Work items of about total / (2 * teams) records, as the allocating
   // path sizes them, but never so small that the split tiles need more
   // partial-tile slots than the array holds: a tile of c > chunk records
   // splits into at most 2c / chunk chunks, so split chunks
   // <= 2 * total / chunk <= kNoAllocMaxSlots.
+  const unsigned long long wanted = 2ull * grid_teams(num_ctas);
   const unsigned long long per_item =
-      ((unsigned long long)total + 2ull * num_ctas - 1) / (2ull * num_ctas);
+      ((unsigned long long)total + wanted - 1) / wanted;
   const unsigned long long min_chunk =
       (2ull * total + kNoAllocMaxSlots - 1) / kNoAllocMaxSlots;
   const uint32_t chunk = (uint32_t)std::max<unsigned long long>(
@@ -310,10 +314,10 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   ib.num_groups = 1;
   ib.scan_tmp = scan_tmp;
   NA_CUDA(launch_build_items(tile_start, num_tiles, total, chunk, ib, s));
-  NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, sc + 6, vals, cell,
+  NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, recs, spans, vals, cell,
                                    meta, vw, view, geom, grid_size, d_grid, 0,
                                    (float*)partials, split_tiles, sc + 3,
-                                   num_tiles, num_ctas, stage, s));
+                                   num_tiles, num_ctas, s));
   return GG_OK;
 }
 

@@ -1,5 +1,5 @@
 // Kernel-stack preparation: re-layout of the reference's quadrant cube into
-// the residue-split layout of StackView, and the FP64 tap sums used for the
+// the slices of StackView, and the FP64 tap sums used for the
 // grid normalisation.
 //
 // The reference re-packs its kernels on the host on every call
@@ -16,9 +16,10 @@ namespace gg {
 namespace {
 
 
-// One thread per output tap; blockIdx.y is the plane.  Output: for each
-// absolute offset class (cu, cv) the (2s+1)^2 slice S[jj][kk] =
-// K[|cv + (jj-s)*os|][|cu + (kk-s)*os|] (see StackView).
+// One warp per output row at a time; blockIdx.y is the plane.  Output: for
+// each absolute offset class (cu, cv) the (2s+1)^2 slice S[jj][kk] =
+// K[|cv + (jj-s)*os|][|cu + (kk-s)*os|] with its zero column and pad rows
+// (see StackView).
 template <typename Real>
 __global__ void k_relayout(const Real* __restrict__ conv, StackView v,
                            typename Vec2<Real>::type* __restrict__ out,
@@ -26,72 +27,35 @@ __global__ void k_relayout(const Real* __restrict__ conv, StackView v,
   using R2 = typename Vec2<Real>::type;
   if (changed && *changed == 0) return;
   const int p = blockIdx.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = blockDim.x >> 5;
   const int os = v.oversample, csh = v.conv_size_half;
   const int s = v.support[p];
-  const long long F = 2 * s + 1;
-  const long long rows = F + 2 * kSlicePad;   // padded slice rows
-  const long long stride = slice_taps(s);     // >= rows * F, even
-  const int classes = (v.omax + 1) * (v.omax + 1);
-  const long long n = (long long)classes * stride;
-  const long long base = v.base[p];
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long rem = e % stride;
-    const int kk = (int)(rem % F);
-    const int jj = (int)(rem / F) - kSlicePad;
-    const int cls = (int)(e / stride);
-    const int cu = cls / (v.omax + 1), cv = cls % (v.omax + 1);
-    const int t = abs(cv + (jj - s) * os);   // row    = |off_v + j*os|
-    const int c = abs(cu + (kk - s) * os);   // column = |off_u + k*os|
-    R2 val;
-    if (rem < rows * F && jj >= 0 && jj < F && t < csh && c < csh) {
-      const size_t src = (((size_t)p * csh + t) * csh + c) * 2;
-      val.x = conv[src];
-      val.y = conv[src + 1];
-    } else {
-      // Padding rows, and taps beyond the cube (which the reference would
-      // read out of bounds), are zero.
-      val.x = 0; val.y = 0;
+  const int F = 2 * s + 1, pitch = slice_pitch(s);
+  const int block = F + kSlicePad;
+  const int side = v.omax + 1;
+  const int rows = kSlicePad + side * side * block;
+  R2 zero;
+  zero.x = 0;
+  zero.y = 0;
+  if (p == 0 && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < kStackLead; i += blockDim.x)
+      out[i] = zero;
+  const R2* __restrict__ cube = (const R2*)conv + (size_t)p * csh * csh;
+  R2* const dst = out + v.planes[p].origin - kSlicePad * pitch;
+  for (int r = blockIdx.x * warps + warp; r < rows; r += gridDim.x * warps) {
+    const int cls = (r - kSlicePad) / block;
+    const int jj = (r - kSlicePad) - cls * block;
+    const int cu = cls / side, cv = cls - cu * side;
+    const int t = abs(cv + (jj - s) * os);   // row = |off_v + j*os|
+    // Taps beyond the cube (which the reference would read out of bounds)
+    // are zero.
+    const bool real = r >= kSlicePad && jj < F && t < csh;
+    for (int kk = lane; kk <= F; kk += 32) {
+      const int c = abs(cu + (kk - s) * os);   // column = |off_u + k*os|
+      dst[(size_t)r * pitch + kk] =
+          real && kk < F && c < csh ? cube[(size_t)t * csh + c] : zero;
     }
-    out[base + e] = val;
-  }
-}
-
-// One thread per output tap of the slab stack; blockIdx.y is the plane.
-// slab_{p,c}[kSlicePad + j + s][r][m] = K_p[|c + j*os|][r + m*os]; padding
-// rows, and taps beyond the cube, are zero.
-template <typename Real>
-__global__ void k_relayout_slabs(const Real* __restrict__ conv, StackView v,
-                                 typename Vec2<Real>::type* __restrict__ out,
-                                 const int* changed) {
-  using R2 = typename Vec2<Real>::type;
-  if (changed && *changed == 0) return;
-  const int p = blockIdx.y;
-  const int os = v.oversample, csh = v.conv_size_half;
-  const int s = v.support[p];
-  const int F = 2 * s + 1;
-  const int M = slab_cols_m(s, os, v.omax);
-  const long long row_taps = (long long)os * M;
-  const long long stride = slab_taps(s, os, v.omax);
-  const long long n = (long long)(v.omax + 1) * stride;
-  const long long base = v.sbase[p];
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const int c = (int)(e / stride);
-    const long long rem = e - c * stride;
-    const int jp = (int)(rem / row_taps) - kSlicePad;
-    const int in_row = (int)(rem % row_taps);
-    const int col = (in_row / M) + (in_row % M) * os;   // r + m*os
-    const int t = abs(c + (jp - s) * os);
-    R2 val;
-    if (jp >= 0 && jp < F && t < csh && col < csh) {
-      const size_t src = (((size_t)p * csh + t) * csh + col) * 2;
-      val.x = conv[src];
-      val.y = conv[src + 1];
-    } else {
-      val.x = 0; val.y = 0;
-    }
-    out[base + e] = val;
   }
 }
 
@@ -299,22 +263,11 @@ cudaError_t launch_cube_gather(const Real* src, StackView view, Real* dst,
 
 template <typename Real>
 cudaError_t launch_stack_relayout(const Real* d_conv_func, StackView view,
-                                  void* d_taps_out, long long total_taps,
-                                  cudaStream_t s, const int* changed) {
-  (void)total_taps;
-  dim3 grid(64, view.num_planes);
+                                  void* d_taps_out, cudaStream_t s,
+                                  const int* changed) {
+  dim3 grid(32, view.num_planes);
   k_relayout<Real><<<grid, 256, 0, s>>>(
       d_conv_func, view, (typename Vec2<Real>::type*)d_taps_out, changed);
-  return cudaGetLastError();
-}
-
-template <typename Real>
-cudaError_t launch_stack_relayout_slabs(const Real* d_conv_func,
-                                        StackView view, void* d_out,
-                                        cudaStream_t s, const int* changed) {
-  dim3 grid(64, view.num_planes);
-  k_relayout_slabs<Real><<<grid, 256, 0, s>>>(
-      d_conv_func, view, (typename Vec2<Real>::type*)d_out, changed);
   return cudaGetLastError();
 }
 
@@ -346,19 +299,11 @@ cudaError_t launch_tap_sums(StackView view, double* d_tap_sum,
 }
 
 template cudaError_t launch_stack_relayout<float>(const float*, StackView,
-                                                  void*, long long,
-                                                  cudaStream_t, const int*);
+                                                  void*, cudaStream_t,
+                                                  const int*);
 template cudaError_t launch_stack_relayout<double>(const double*, StackView,
-                                                   void*, long long,
-                                                   cudaStream_t, const int*);
-template cudaError_t launch_stack_relayout_slabs<float>(const float*,
-                                                        StackView, void*,
-                                                        cudaStream_t,
-                                                        const int*);
-template cudaError_t launch_stack_relayout_slabs<double>(const double*,
-                                                         StackView, void*,
-                                                         cudaStream_t,
-                                                         const int*);
+                                                   void*, cudaStream_t,
+                                                   const int*);
 template cudaError_t launch_cube_compare<float>(const float*, const float*,
                                                 StackView, int*, cudaStream_t);
 template cudaError_t launch_cube_compare<double>(const double*, const double*,

@@ -1,8 +1,7 @@
 // Pieces shared by the tile-owning kernels (gridding in gg_grid.cu,
-// degridding in gg_degrid.cu): the CTA shape (one producer warp, eight
-// consumer warps owning a 2048-cell tile, lane = column, kRows rows per
-// lane), the record ring, bounded mbarrier waits, tap loads with an L2
-// keep hint, and the slab-stack descriptor of a record.
+// degridding in gg_degrid.cu): the tile shape (2048 cells in eight bands,
+// lane = column, kRows rows per lane), bounded mbarrier waits, tap loads and
+// the slice descriptor of a record.
 #pragma once
 
 #include "gg_internal.h"
@@ -32,7 +31,7 @@ struct WarpShape {
   static constexpr int kTileV = kWarps * kBand;
 };
 
-// ---- mbarrier and bulk-copy helpers (shared::cta) --------------------------
+// ---- mbarrier helpers (shared::cta) --------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -47,14 +46,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .b64 st;\n\t"
       "mbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar))
-      : "memory");
-}
-// Adds `bytes` of expected asynchronous transactions to the current phase.
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile(
-      "mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(
-          smem_u32(bar)),
-      "r"(bytes)
       : "memory");
 }
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
@@ -78,71 +69,85 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
   return false;
 }
-// Bulk copy global -> shared (16-byte aligned, size a multiple of 16),
-// completing `bytes` transactions on `bar`.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src,
-                                              uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes "
-      "[%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  return __ffma2_rn(a, b, c);
+}
+__device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
 }
 
-// Read-only tap load that asks L2 to keep the line (evict_last policy):
-// the compact stack is re-read by every tile while the grid streams past.
-__device__ __forceinline__ float2 ld_tap(const float2* p, uint64_t pol) {
+// Read-only tap load.
+__device__ __forceinline__ float2 ld_tap(const float2* p) {
   float2 v;
-  asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
-      : "=f"(v.x), "=f"(v.y)
-      : "l"(p), "l"(pol));
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];"
+               : "=f"(v.x), "=f"(v.y)
+               : "l"(p));
   return v;
 }
-__device__ __forceinline__ double2 ld_tap(const double2* p, uint64_t pol) {
+__device__ __forceinline__ double2 ld_tap(const double2* p) {
   double2 v;
-  asm("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-      : "=d"(v.x), "=d"(v.y)
-      : "l"(p), "l"(pol));
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];"
+               : "=d"(v.x), "=d"(v.y)
+               : "l"(p));
   return v;
-}
-__device__ __forceinline__ uint64_t evict_last_policy() {
-  uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;"
-               : "=l"(pol));
-  return pol;
 }
 
-// Slab-stack descriptor of a record (plane with support s, offsets ou,
-// ov; footprint centre at tile-relative column gu, row gv; tiles TW wide):
-//   x = A + Cp, y = A + Cn, z = B,
-//   w = Lf | c0 << 8 | (c1 - c0) << 16
-// where A is the slab tap index of tile row 0 for a column offset of 0, B
-// the slab taps per tile row (+-row pitch; rows mirrored for ov < 0), Cp +
-// col and Cn - col the column offsets on the non-negative and the negative
-// side of the column fold (which begins at lane column Lf), and [c0, c1]
-// the footprint's columns in the tile; so the tap of tile cell (row, col)
-// is slabs[(col >= Lf ? x + col : y - col) + row * B] for c0 <= col <= c1.
-template <int TW, int OS = 0>
-__device__ __forceinline__ int4 slab_record(const StackView& v, int plane,
-                                            int s, int ou, int ov, int gu,
-                                            int gv) {
-  // OS > 0: the oversampling known at compile time (integer divisions and
-  // remainders by it become shifts and masks when it is a power of two).
-  const int os = OS > 0 ? OS : v.oversample, omax = v.omax;
-  const int M = slab_cols_m(s, os, omax);
-  const int pitch = os * M;
-  const int sb = (int)(v.sbase[plane] + abs(ov) * slab_taps(s, os, omax));
-  const int A = ov >= 0 ? sb + (s + kSlicePad - gv) * pitch
-                        : sb + (s + kSlicePad + gv) * pitch;
-  const int B = ov >= 0 ? pitch : -pitch;
-  const int ap = ((ou % os) + os) % os, an = ((-ou % os) + os) % os;
-  const int bp = (ou - ap) / os, bn = (-ou - an) / os;
-  const int Cp = ap * M + bp - gu, Cn = an * M + bn + gu;
-  // floor(ou / os); the fold lane is gu - floor(ou / os).
-  const int fl = ou >= 0 ? ou / os : -((-ou + os - 1) / os);
-  const int Lf = min(max(gu - fl, 0), TW);
-  const int c0 = max(gu - s, 0), c1 = min(gu + s, TW - 1);
-  return make_int4(A + Cp, A + Cn, B, Lf | (c0 << 8) | ((c1 - c0) << 16));
+// Descriptor of a record (plane with support s, offsets ou, ov; footprint
+// centre at tile-relative column gu, row gv) for its slice, tap S[0][0] at
+// index `origin`, row pitch `pitch`:
+//   x: tap index of slice column 0 in the slice row of tile row 0 (which
+//      may lie outside the stack, or wrap: only sums are tap indices)
+//   y: slice column of tile column 0 (bits 0-15, signed), s (16-29), and
+//      bits 30 and 31 where the columns (ou < 0) and rows (ov < 0) are
+//      mirrored
+// so with z and s from y and su, sv = -1 where mirrored, else 1, the tap of
+// tile cell (row, col) is
+//   taps[x + sv * row * pitch + clamp(z + su * col, -1, 2s + 1)]
+// where the clamped ends are zero taps.
+constexpr uint32_t kMirrorU = 1u << 30, kMirrorV = 1u << 31;
+__device__ __forceinline__ uint2 slice_record(long long origin, int s, int ou,
+                                              int ov, int gu, int gv) {
+  const int pitch = slice_pitch(s);
+  const int z = ou < 0 ? s + gu : s - gu;
+  const int row = ov < 0 ? s + gv : s - gv;
+  return make_uint2((uint32_t)(origin + (long long)row * pitch),
+                    ((uint32_t)z & 0xFFFFu) | (uint32_t)s << 16 |
+                        (ou < 0 ? kMirrorU : 0u) |
+                        (ov < 0 ? kMirrorV : 0u));
+}
+
+// Taps from one tile row to the next of descriptor d.
+__device__ __forceinline__ int slice_step(uint2 d) {
+  const int pitch = 2 * (int)((d.y >> 16) & 0x3FFFu) + 2;
+  return (int)d.y < 0 ? -pitch : pitch;
+}
+// Tap index of tile cell (0, col) of descriptor d with that step.
+__device__ __forceinline__ uint32_t slice_tap(uint2 d, int step, int col) {
+  const int z = (int)(short)(d.y & 0xFFFFu);
+  const int c = d.y & kMirrorU ? z - col : z + col;
+  return d.x + (uint32_t)min(max(c, -1), abs(step) - 1);
+}
+
+// kRows taps from `at` on, `step` taps apart.  kWide: the stack holds more
+// than 4 GiB; below that its byte offsets fit 32 bits, and each row costs one
+// 32-bit addition to a common base instead of a 64-bit one (5 % of the
+// gridding passes on 8192^2 workloads).
+template <bool kWide, typename R2>
+__device__ __forceinline__ void load_taps(const R2* __restrict__ taps,
+                                          uint32_t at, int step,
+                                          R2 (&out)[kRows]) {
+  if constexpr (kWide) {
+    const R2* p = taps + at;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) out[r] = ld_tap(p + (long long)r * step);
+  } else {
+    const uint32_t first = at * (uint32_t)sizeof(R2);
+    const uint32_t bytes = (uint32_t)step * (uint32_t)sizeof(R2);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+      out[r] = ld_tap(
+          (const R2*)((const char*)taps + (size_t)(first + r * bytes)));
+  }
 }
 
 }  // namespace

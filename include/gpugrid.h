@@ -149,7 +149,7 @@ typedef struct
     unsigned long long num_macs;        /* complex multiply-adds performed */
     unsigned long long num_launches;    /* kernels this library launched */
     int tile_u, tile_v;                 /* tile shape used */
-    int slice_staging;                  /* 1 if slices were staged */
+    int slice_staging;                  /* always 0 (see gg_plan_set_slice_staging) */
     int num_ctas;                       /* persistent gridding CTAs */
     unsigned long long chunk_records;   /* records per work item (max) */
     int num_plane_groups;               /* gridding passes (plane groups) */
@@ -164,11 +164,9 @@ GG_API int gg_plan_last_stats(const gg_plan* plan, gg_stats* stats);
  * its inputs and this setting. */
 GG_API int gg_plan_set_tile_shape(gg_plan* plan, int tile_u);
 
-/* Staging of kernel slices in shared memory by the gridding kernel (bulk
- * asynchronous copies of a (plane, offset) slice shared by many records of
- * a tile): -1 (default) decides per call from the mean footprint, 0 off,
- * 1 on.  Results are bit-identical either way: only where the taps are
- * read from changes, not the arithmetic or its order. */
+/* Staging of kernel slices in shared memory: accepted (-1, 0 or 1) and
+ * reported back, without effect.  Taps are always read through L1, which
+ * measured faster on every workload; results were bit-identical either way. */
 GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
 
 /* Launch and decomposition parameters of a plan's gridding calls, as set
@@ -177,9 +175,9 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  * settings that change how a cell's contributions are grouped or ordered
  * (tile_u, items_per_cta, sort_detail, ctas_per_sm -- through the number of
  * work items --, plane_group_mb, tile_phases) change the grid by FP32
- * rounding; slice_staging leaves it bit-identical.
+ * rounding; slice_staging has no effect.
  *   tile_u         32, 16 or 8 (cells across a tile); 0 = chosen per call
- *   slice_staging  -1 chosen per call, 0 off, 1 on (bit-identical results)
+ *   slice_staging  -1, 0 or 1; without effect
  *   items_per_cta  work items per persistent CTA in each gridding pass
  *                  that the split of heavy tiles aims for, 1..64 (default
  *                  4): more items balance the load better but write more
@@ -193,19 +191,15 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  *                  group's re-laid kernels within this many MiB (about
  *                  equal in size) and each group is gridded in its own
  *                  pass, so that a pass's kernels stay in L2; 0 (default) =
- *                  half the device's L2 cache, 0..1048576
+ *                  three quarters of the device's L2 cache, 0..1048576
  *   tile_order     order in which the persistent CTAs take the tiles: 0
  *                  (default) by distance from the grid centre (baseline
  *                  length, so w and the kernels read stay alike among the
  *                  tiles gridded at one time), 1 row by row (the tiles in
  *                  flight share grid rows: fewer pages touched at once when
  *                  the grid is the caller's host memory, used in place)
- *   lane_groups    record streams per consumer warp of the 32-wide tiles
- *                  (taps read from the slab stack): 1 -- the whole warp
- *                  takes every record that meets its 8 rows; 2 -- each
- *                  half-warp takes the records that meet its own 16
- *                  columns, so two narrow footprints are gridded side by
- *                  side; 0 (default) = 1
+ *   lane_groups    0 (default), 1 or 2; without effect (each lane row of a
+ *                  warp takes its own records)
  *   tile_phases    1, 2, 4 or 8 tile grids offset by tile_u / tile_phases
  *                  columns from one another; each visibility is gridded on
  *                  the one whose tiles cut its footprint into the fewest
@@ -430,7 +424,7 @@ GG_API int gg_plan_probe_bounded_wait(gg_plan* plan, unsigned iterations,
  * allocate device memory while they grid (a real-time loop that must not
  * stall on cudaMalloc, or code running under another framework's memory
  * pool).  This entry point has no counterpart in the reference.  All scratch
- * comes from one 32 MiB device array inside the library, held by every GPU
+ * comes from one 48 MiB device array inside the library, held by every GPU
  * that loads it until the process exits; nothing is allocated or freed by
  * the call.  The kernel-stack handle is made beforehand (that step
  * allocates).  Limits: num_points <= 131072, grid_size <= 8192, and at most

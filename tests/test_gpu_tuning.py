@@ -165,3 +165,38 @@ def test_host_tuning_applies_to_dropin(pkg, torch, wl, fp64):
     assert pkg.host_tuning() == default
     g2, ns2, nm2 = pkg.grid_f(wl)
     assert ns2 == ns and nm2 == nm
+
+
+@pytest.mark.parametrize("tile_u", [32, 16, 8])
+def test_stack_beyond_4_gib(pkg, torch, tile_u):
+    """A stack whose taps pass 4 GiB (64-bit tap offsets in the kernels)
+    grids and degrids bit for bit like a small one with the same kernels:
+    every plane of both has the same support and chirp, and all points fall
+    on the last."""
+    G, s, n = 512, 100, 600
+    rng = np.random.default_rng(3)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    uu, vv = (dev(rng.uniform(-130.0, 130.0, n)) for _ in range(2))
+    ww = dev(np.full(n, 1.0e6) * rng.choice([-1.0, 1.0], n))
+    vis, weight = dev(rng.standard_normal((n, 2))), dev(rng.uniform(1, 2, n))
+    y = dev(rng.standard_normal((G, G, 2)))
+    outs = []
+    for planes in (2, 1500):
+        stack = pkg.KernelStack.generate(
+            planes, np.full(planes, s, np.int32), 4, 4 * (s + 1),
+            np.full(planes, 3.0))
+        plan = pkg.Plan()
+        plan.set_tuning({"tile_u": tile_u, "plane_group_mb": 1048576})
+        grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+        norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+        skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+        pkg.grid_wproj_device(plan, stack, uu, vv, ww, vis, weight, 0.002,
+                              np.float32(1.0e6), G, grid, norm, skip)
+        out = torch.empty((n, 2), dtype=torch.float32, device="cuda")
+        pkg.degrid_wproj_device(plan, stack, uu, vv, ww, 0.002,
+                                np.float32(1.0e6), G, y, out)
+        outs.append([t.cpu().numpy() for t in (grid, norm, skip, out)])
+        del stack
+    assert int(outs[0][2][0]) < n // 2 and np.abs(outs[0][0]).max() > 0
+    for a, b in zip(*outs):
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
