@@ -437,71 +437,105 @@ k_grid_tiles(GridArgs<Real> a) {
   }
 }
 
+// v += the n partial values at q, one per chunk, in chunk order: added in
+// FP64 and rounded once.  Loads go out eight at a time: a heavy tile has
+// hundreds of chunks, and one load per addition would leave the pass waiting
+// out a memory latency for each.
+template <typename R2>
+__device__ __forceinline__ void add_chunks(R2& v, const R2* __restrict__ q,
+                                           int n) {
+  double sx = v.x, sy = v.y;
+  int c = 0;
+  for (; c + 8 <= n; c += 8) {
+    R2 t[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) t[j] = q[(size_t)(c + j) * kCells];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      sx += t[j].x;
+      sy += t[j].y;
+    }
+  }
+  for (; c < n; ++c) {
+    const R2 t = q[(size_t)c * kCells];
+    sx += t.x;
+    sy += t.y;
+  }
+  v.x = sx;
+  v.y = sy;
+}
+
+// The cell of thread tid in a band of a tile (one cell per thread): its row
+// and column in the band, and its entry in the tile's partials less the
+// band's part, band * 32 (the gridding kernel's thread-major layout).
+template <int TW>
+struct BandCell {
+  int row, col, entry;
+  __device__ __forceinline__ explicit BandCell(int tid)
+      : row(tid / TW), col(tid % TW),
+        entry(row % kRows * kConsumers + row / kRows * TW + col) {}
+};
+
 // grid(tile) += sum of the tile's partials in chunk order, accumulated in
 // FP64 and rounded once, for the split tiles of one plane group (a real
 // tile is split at most once per group, so the blocks of one launch never
-// share a tile).  The partial layout is the kernel's thread-major one:
-// entry e = r * kConsumers + consumer thread.
+// share a tile).  A block takes one band of a tile at a time: the chains of
+// chunks of a heavy tile, which the pass waits for, run on all its bands at
+// once.
 template <typename Real, int TW>
-__global__ void k_reduce_partials(const int4* __restrict__ split_tiles,
-                                  const uint32_t* __restrict__ num_split,
-                                  const typename Vec2<Real>::type* __restrict__ partials,
-                                  TileGeom g, int group, int G, Real* grid,
-                                  long long grid_stride, Real* host,
-                                  const uint32_t* __restrict__ tile_groups) {
+__global__ void __launch_bounds__(kConsumers, 4)
+k_reduce_partials(const int4* __restrict__ split_tiles,
+                  const uint32_t* __restrict__ num_split,
+                  const typename Vec2<Real>::type* __restrict__ partials,
+                  TileGeom g, int group, int G, Real* grid,
+                  long long grid_stride, Real* host,
+                  const uint32_t* __restrict__ tile_groups) {
   using R2 = typename Vec2<Real>::type;
   using WS = WarpShape<TW>;
   const int tiles_per_grid = g.tiles_u * g.tiles_v;
-  const int n = (int)*num_split;
-  for (int st = blockIdx.x; st < n; st += gridDim.x) {
-    const int4 d = split_tiles[st];  // virtual tile, first slot, chunks
+  const int n = (int)*num_split * kWarps;
+  const BandCell<TW> me(threadIdx.x);
+  for (int b = blockIdx.x; b < n; b += gridDim.x) {
+    const int4 d = split_tiles[b / kWarps];  // virtual tile, first slot, chunks
     if (d.x / g.tiles_total != group) continue;
+    const int band = b % kWarps;
     const int rt = d.x % g.tiles_total;
     const int gi = rt / tiles_per_grid;
     const int tl = rt - gi * tiles_per_grid;
-    const int u0 = (tl % g.tiles_u) * WS::kTileU - phase_shift(g, group);
-    const int v0 = (tl / g.tiles_u) * WS::kTileV;
-    R2* const gg = (R2*)(grid + (long long)gi * grid_stride);
-    for (int e = threadIdx.x; e < kCells; e += blockDim.x) {
-      const int r = e / kConsumers, t = e % kConsumers;
-      const int w = t >> 5, ln = t & 31;
-      const int row = v0 + w * WS::kBand + (ln / TW) * kRows + r;
-      const int col = u0 + ln % TW;
-      if (row >= G || (unsigned)col >= (unsigned)G) continue;
-      R2 *src, *dst;
-      cell_ends<R2>(tile_groups, g, tl / g.tiles_u, col, group, gg,
-                    (R2*)host, src, dst);
-      const size_t off = (size_t)row * G + col;
-      const R2 old = src[off];
-      double sx = old.x, sy = old.y;
-      for (int c = 0; c < d.z; ++c) {
-        const R2 q = partials[(size_t)(d.y + c) * kCells + e];
-        sx += q.x;
-        sy += q.y;
-      }
-      R2 nw;
-      nw.x = (Real)sx;
-      nw.y = (Real)sy;
-      dst[off] = nw;
-    }
+    const int tv = tl / g.tiles_u;
+    const int col =
+        (tl - tv * g.tiles_u) * WS::kTileU - phase_shift(g, group) + me.col;
+    const int row = tv * WS::kTileV + band * WS::kBand + me.row;
+    if (row >= G || (unsigned)col >= (unsigned)G) continue;
+    R2 *src, *dst;
+    cell_ends<R2>(tile_groups, g, tv, col, group,
+                  (R2*)(grid + (long long)gi * grid_stride), (R2*)host, src,
+                  dst);
+    const size_t off = (size_t)row * G + col;
+    R2 v = src[off];
+    add_chunks(v, partials + (size_t)d.y * kCells + band * 32 + me.entry, d.z);
+    dst[off] = v;
   }
 }
 
 // The partial tiles of one plane group's tile phases (virtual groups
 // group0 .. group0 + P - 1, one launch of the gridding kernel), added to
-// the grids in one pass: block b takes the cells of phase-0 tile position
-// b and adds to each cell, phase by phase, the partial tiles of the tile of
-// that phase that covers it (their chunks summed in FP64, rounded once per
-// phase) -- the additions, in the same order, that one reduction launch per
-// phase makes (k_reduce_partials).  A single chunk is added in the grid's
-// precision: the FP64 sum of two FP32 values rounded to FP32 is their
-// correctly rounded FP32 sum.  tile_slot[virtual tile] = (first partial
-// slot, chunks), chunks 0 when the tile has no partial tiles.  Each thread
-// keeps one column (blockDim.x a multiple of TW) and looks its phases'
-// tiles up once.  kMaxPhases >= tile_phases (4 or 8: the lookups of eight
-// phases take registers that four do not need).
+// the grids in one pass: a block takes two bands of a phase-0 tile position
+// at a time (two cells a thread) and adds to each cell, phase by phase, the partial tiles of the
+// tile of that phase that covers it (their chunks summed in FP64, rounded
+// once per phase) -- the additions, in the same order, that one reduction
+// launch per phase makes (k_reduce_partials).  A single chunk is added in
+// the grid's precision: the FP64 sum of two FP32 values rounded to FP32 is
+// their correctly rounded FP32 sum.  Those loads (the grid's cells and up to
+// four partials each) all go out before the first addition.
+// tile_slot[virtual tile] = (first partial slot, chunks), chunks 0 when the
+// tile has no partial tiles.  HBM-bound but for the heavy tiles' chains.
+// With whole tiles for a block (eight cells and, for heavy tiles, eight
+// chains of chunks a thread) it took 0.66 ms on 7.8e6 track points over
+// 8192^2 and 0.09 ms on 4e3 points over 256^2.
+// kMaxPhases >= tile_phases (4 or 8).
 template <typename Real, int TW, int kMaxPhases>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kConsumers, kMaxPhases > 4 ? 3 : 4)
 k_reduce_phases(const int2* __restrict__ tile_slot,
                 const typename Vec2<Real>::type* __restrict__ partials,
                 TileGeom g, int group0, int G, Real* grid,
@@ -510,23 +544,26 @@ k_reduce_phases(const int2* __restrict__ tile_slot,
                 const uint32_t* __restrict__ tile_start) {
   using R2 = typename Vec2<Real>::type;
   using WS = WarpShape<TW>;
-  constexpr int kTV = WS::kTileV;
-  constexpr int kRowStep = 256 / TW;    // rows between a thread's cells
   const int P = g.tile_phases;
   const int sw = 1 << g.strip_shift;
   const int real_u = g.tiles_u - 1;   // phase-0 tile columns
   const int tiles_per_grid = g.tiles_u * g.tiles_v;
-  const int n = g.num_grids * real_u * g.tiles_v;
-  const int C = threadIdx.x % TW, R0 = threadIdx.x / TW;
+  constexpr int kPairs = kWarps / 2;
+  const int n = g.num_grids * real_u * g.tiles_v * kPairs;
+  const BandCell<TW> me(threadIdx.x);
   for (int b = blockIdx.x; b < n; b += gridDim.x) {
-    const int gi = b / (real_u * g.tiles_v);
-    const int rem = b - gi * real_u * g.tiles_v;
-    const int tv = rem / real_u, tu = rem - (rem / real_u) * real_u;
-    const int col = tu * TW + C;
+    const int band = b % kPairs * 2, pos = b / kPairs;
+    const int gi = pos / (real_u * g.tiles_v);
+    const int rem = pos - gi * real_u * g.tiles_v;
+    const int tv = rem / real_u, tu = rem - tv * real_u;
+    const int col = tu * TW + me.col;
+    const int row = tv * WS::kTileV + band * WS::kBand + me.row;
+    if (col >= G || row >= G) continue;
+    const bool both = row + WS::kBand < G;
     // This column's tile in each phase: its slots and its column there.
     int2 sl[kMaxPhases];
     int cp[kMaxPhases];
-    bool mine = false;
+    bool mine = false, several = false;
 #pragma unroll
     for (int p = 0; p < kMaxPhases; ++p) {
       sl[p] = make_int2(0, 0);
@@ -534,15 +571,15 @@ k_reduce_phases(const int2* __restrict__ tile_slot,
       if (p < P) {
         const int c = col + p * sw;
         const int tc = c / TW;
-        cp[p] = c - tc * TW;
+        cp[p] = c - tc * TW - me.col;
         sl[p] = tile_slot[(size_t)(group0 + p) * g.tiles_total +
                           (size_t)gi * tiles_per_grid +
                           (size_t)tv * g.tiles_u + tc];
         mine |= sl[p].y > 0;
+        several |= sl[p].y > 1;
       }
     }
-    if (!__syncthreads_or(mine)) continue;
-    if (!mine || col >= G) continue;
+    if (!mine) continue;
     R2* gg = (R2*)(grid + (long long)gi * grid_stride);
     // Direct mode (the caller's grid at host in place, one grid): the
     // column's strip was last added to at host unless phase 0's tile here
@@ -564,78 +601,44 @@ k_reduce_phases(const int2* __restrict__ tile_slot,
       if (!added0 && first >= group0) src = (R2*)host;
       if (last < group0 + P) dst = (R2*)host;
     }
-    if constexpr (sizeof(Real) == 4 && kMaxPhases <= 4) {
-      bool several = false;
+    const size_t off0 = (size_t)row * G + col;
+    const size_t off1 = off0 + (both ? (size_t)WS::kBand * G : 0);
+    const R2* const q = partials + band * 32 + me.entry;
+    R2 v0 = src[off0], v1 = src[off1];
+    if (!several) {
+      R2 t0[kMaxPhases], t1[kMaxPhases];
 #pragma unroll
-      for (int p = 0; p < kMaxPhases; ++p) several |= sl[p].y > 1;
-      if (!several) {
-        // Every phase adds at most one chunk to this column: all of the
-        // thread's loads (its rows of the grid and of up to kMaxPhases
-        // partial tiles) go out before the first addition, so the block
-        // waits out one memory latency rather than one per row.  The
-        // additions are the loop's below, in the same order.
-        constexpr int kRowsPer = kTV / kRowStep;
-        R2 acc[kRowsPer], pv[kMaxPhases][kRowsPer];
-#pragma unroll
-        for (int i = 0; i < kRowsPer; ++i) {
-          const int R = R0 + i * kRowStep;
-          const int row = tv * kTV + R;
-          const bool in = row < G;
-          const int w = R / WS::kBand, ly = (R % WS::kBand) / kRows;
-          const int ent0 = (R % kRows) * kConsumers + w * 32 + ly * TW;
-          acc[i] = in ? src[(size_t)row * G + col] : R2{};
-#pragma unroll
-          for (int p = 0; p < kMaxPhases; ++p)
-            pv[p][i] = in && sl[p].y > 0
-                           ? partials[(size_t)sl[p].x * kCells + ent0 + cp[p]]
-                           : R2{};
-        }
-#pragma unroll
-        for (int i = 0; i < kRowsPer; ++i) {
-          const int row = tv * kTV + R0 + i * kRowStep;
-          if (row >= G) break;
-#pragma unroll
-          for (int p = 0; p < kMaxPhases; ++p) {
-            if (sl[p].y == 0) continue;
-            acc[i].x += pv[p][i].x;
-            acc[i].y += pv[p][i].y;
-          }
-          dst[(size_t)row * G + col] = acc[i];
-        }
-        continue;
+      for (int p = 0; p < kMaxPhases; ++p) {
+        const R2* qp = q + (ptrdiff_t)sl[p].x * kCells + cp[p];
+        t0[p] = sl[p].y ? qp[0] : R2{};
+        t1[p] = sl[p].y ? qp[32] : R2{};
       }
-    }
-#pragma unroll 4
-    for (int R = R0; R < kTV; R += kRowStep) {
-      const int row = tv * kTV + R;
-      if (row >= G) break;
-      // The cell's entry in a partial tile whose column is Cp (the
-      // kernel's thread-major layout: row R is warp R / kBand, lane row
-      // (R % kBand) / kRows, register row R % kRows).
-      const int w = R / WS::kBand, ly = (R % WS::kBand) / kRows;
-      const int ent0 = (R % kRows) * kConsumers + w * 32 + ly * TW;
-      R2 acc = src[(size_t)row * G + col];
 #pragma unroll
       for (int p = 0; p < kMaxPhases; ++p) {
         if (sl[p].y == 0) continue;
-        const R2* q = partials + (size_t)sl[p].x * kCells + ent0 + cp[p];
+        v0.x += t0[p].x;
+        v0.y += t0[p].y;
+        v1.x += t1[p].x;
+        v1.y += t1[p].y;
+      }
+    } else {
+#pragma unroll
+      for (int p = 0; p < kMaxPhases; ++p) {
+        const R2* qp = q + (ptrdiff_t)sl[p].x * kCells + cp[p];
         if (sl[p].y == 1) {
-          const R2 v = *q;
-          acc.x += v.x;
-          acc.y += v.y;
-        } else {
-          double sx = acc.x, sy = acc.y;
-          for (int k = 0; k < sl[p].y; ++k) {
-            const R2 v = q[(size_t)k * kCells];
-            sx += v.x;
-            sy += v.y;
-          }
-          acc.x = (Real)sx;
-          acc.y = (Real)sy;
+          const R2 t0 = qp[0], t1 = qp[32];
+          v0.x += t0.x;
+          v0.y += t0.y;
+          v1.x += t1.x;
+          v1.y += t1.y;
+        } else if (sl[p].y > 1) {
+          add_chunks(v0, qp, sl[p].y);
+          add_chunks(v1, qp + 32, sl[p].y);
         }
       }
-      dst[(size_t)row * G + col] = acc;
     }
+    dst[off0] = v0;
+    if (both) dst[off1] = v1;
   }
 }
 
@@ -942,7 +945,8 @@ cudaError_t launch_reduce_phases(const int2* tile_slot, const Real* partials,
                                  Real* host, const uint32_t* tile_groups,
                                  const uint32_t* tile_start, cudaStream_t s) {
   const long long n =
-      (long long)geom.num_grids * (geom.tiles_u - 1) * geom.tiles_v;
+      (long long)geom.num_grids * (geom.tiles_u - 1) * geom.tiles_v * kWarps /
+      2;
   if (n <= 0) return cudaSuccess;
   if (geom.tile_phases > 8) return cudaErrorInvalidValue;
   const int blocks = (int)std::min<long long>(n, 65535);
@@ -976,7 +980,7 @@ cudaError_t launch_reduce_group(const int4* split_tiles,
                                 long long grid_stride, Real* host,
                                 const uint32_t* tile_groups, cudaStream_t s) {
   if (max_split <= 0) return cudaSuccess;
-  const int blocks = std::min(max_split, 4096);
+  const int blocks = (int)std::min(8LL * max_split, 2432LL);
   using P2 = const typename Vec2<Real>::type*;
   switch (geom.tile_u) {
     case 32: k_reduce_partials<Real, 32><<<blocks, 256, 0, s>>>(
