@@ -537,7 +537,7 @@ int kernels_create(gg_kernels** out, size_t num_w_planes, const int* support,
 // ===========================================================================
 struct gg_plan {
   int device = 0;
-  DevBuf cell, meta, vw, rec_count, rec_offset;
+  DevBuf cell, meta, placed, rec_count, rec_offset;
   DevBuf blk_norm, blk_skip, blk_macs;
   DevBuf keys0, vals0, keys1, vals1, sort_tmp, scan_tmp;
   DevBuf recs, rec_spans;   // prepared records (launch_grid_tiles)
@@ -881,7 +881,6 @@ int grid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
                   Real w_scale, int grid_size,
                   unsigned long long* d_num_skipped, double* d_norm,
                   Real* d_grid, cudaStream_t s) {
-  using R2 = typename Vec2<Real>::type;
   if (!plan || !K) return set_error(GG_ERR_INVALID_ARG, "plan or kernels is NULL");
   if (K->is_double != (sizeof(Real) == 8))
     return set_error(GG_ERR_INVALID_ARG,
@@ -942,14 +941,13 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
                     const PlaceParams<Real>& pp, int forced_shape,
                     double* d_norm, unsigned long long* d_num_skipped,
                     cudaStream_t s, PlaceOut* po_out) {
-  using R2 = typename Vec2<Real>::type;
   const StackView view = K->view();
   const size_t n = pp.num_points;
   const int tiles_cap = max_tiles(pp.grid_size, 1);
   const int nblk = place_num_blocks(n);
   GG_TRY(plan->cell.ensure(n * 4 + 4));
   GG_TRY(plan->meta.ensure(n * 4 + 4));
-  if (pp.vis) GG_TRY(plan->vw.ensure(n * sizeof(R2) + sizeof(R2)));
+  if (pp.vis) GG_TRY(plan->placed.ensure(n * sizeof(Placed<Real>)));
   GG_TRY(plan->rec_count.ensure(n * 4 + 4));
   GG_TRY(plan->rec_offset.ensure(n * 4 + 4));
   GG_TRY(plan->blk_norm.ensure(nblk * sizeof(double)));
@@ -962,7 +960,7 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
   PlaceOut po;
   po.cell = plan->cell.as<uint32_t>();
   po.meta = plan->meta.as<uint32_t>();
-  po.vw = pp.vis ? plan->vw.p : nullptr;
+  po.placed = pp.vis ? plan->placed.p : nullptr;
   po.rec_count = plan->rec_count.as<uint32_t>();
   po.blk_norm = plan->blk_norm.as<double>();
   po.blk_skip = plan->blk_skip.as<unsigned long long>();
@@ -984,7 +982,8 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
       PlaceOut ok = po;
       ok.cell = po.cell + a;
       ok.meta = po.meta + a;
-      ok.vw = po.vw ? (void*)((R2*)po.vw + a) : nullptr;
+      ok.placed =
+          po.placed ? (void*)((Placed<Real>*)po.placed + a) : nullptr;
       const size_t blk = a / kPlaceBlock;
       ok.blk_norm = po.blk_norm + blk;
       ok.blk_skip = po.blk_skip + blk;
@@ -1380,7 +1379,7 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   GG_CUDA(launch_grid_tiles<Real>(
       ib.items, ib.group_items, ib.counter, T->recs.p,
       T->rec_spans.as<unsigned short>(), b.vals,
-      po.cell, po.meta, po.vw, view, geom, grid_size, d_grid, grid_stride,
+      po.placed, view, geom, grid_size, d_grid, grid_stride,
       plan->partials.as<Real>(), ib.split_tiles, ib.num_split, b.num_tiles,
       num_ctas, s, wait_before.data(), record_after.data(),
       (Real*)plan->host_grid, tile_groups, span, plan->tile_slot.as<int2>(),
@@ -1406,7 +1405,6 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
                      const Real* weight, Real cell_size_rad, Real w_scale,
                      int grid_size, unsigned long long* d_num_skipped,
                      double* d_norm, Real* d_grids, cudaStream_t s) {
-  using R2 = typename Vec2<Real>::type;
   if (!plan || !K) return set_error(GG_ERR_INVALID_ARG, "plan or kernels is NULL");
   if (K->is_double != (sizeof(Real) == 8))
     return set_error(GG_ERR_INVALID_ARG,
@@ -1465,7 +1463,7 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
 
   GG_TRY(plan->cell.ensure(n * 4 + 4));
   GG_TRY(plan->meta.ensure(n * 4 + 4));
-  GG_TRY(plan->vw.ensure(n * sizeof(R2) + sizeof(R2)));
+  GG_TRY(plan->placed.ensure((n + 1) * sizeof(Placed<Real>)));
   // Counts and offsets of records per visibility: transient (a sub-plan
   // takes its parent's).
   gg_plan* T = plan->scratch ? plan->scratch : plan;
@@ -1497,7 +1495,7 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   PlaceOut po;
   po.cell = plan->cell.as<uint32_t>();
   po.meta = plan->meta.as<uint32_t>();
-  po.vw = plan->vw.p;
+  po.placed = plan->placed.p;
   po.rec_count = T->rec_count.as<uint32_t>();
   po.blk_norm = nullptr;
   po.blk_skip = nullptr;
@@ -1679,7 +1677,7 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
   uint32_t* sc = plan->scalars.as<uint32_t>();
   const ChunkParts cp = chunk_parts(plan, kp.num_chunks);
   GG_CUDA(launch_revalue<Real>(vis, weight, plan->meta.as<uint32_t>(), view,
-                               kp.num_points, plan->vw.p,
+                               kp.num_points, plan->placed.p,
                                plan->nterm.as<double>(), s));
   GG_CUDA(launch_batch_totals(
       plan->meta.as<uint32_t>(), plan->nterm.as<double>(), view,
@@ -1692,8 +1690,8 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
   gg_plan* T = plan->scratch ? plan->scratch : plan;
   GG_CUDA(launch_grid_tiles<Real>(
       plan->items.as<WorkItem>(), plan->group_items.as<uint32_t>(),
-      sc + kCounter, T->recs.p, T->rec_spans.as<unsigned short>(), kp.rec_vis, plan->cell.as<uint32_t>(),
-      plan->meta.as<uint32_t>(), plan->vw.p, view, kp.geom, kp.grid_size,
+      sc + kCounter, T->recs.p, T->rec_spans.as<unsigned short>(), kp.rec_vis,
+      plan->placed.p, view, kp.geom, kp.grid_size,
       d_grids, grid_stride, plan->partials.as<Real>(),
       plan->split_tiles.as<int4>(), sc + kNumSplit, kp.num_tiles, kp.num_ctas,
       s, nullptr, nullptr, nullptr, nullptr, kp.group_span,

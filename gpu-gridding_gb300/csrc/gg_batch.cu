@@ -43,18 +43,19 @@ template <typename Real>
 __global__ void __launch_bounds__(kThreads)
 k_place_batched(PlaceParams<Real> p, StackView v, PlaceOut out,
                 double* __restrict__ nterm) {
-  using R2 = typename Vec2<Real>::type;
   const unsigned long long i =
       (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
   if (i >= p.num_points) return;
   const Placement r = place_one(p, v, i);
   const Real w = p.weight[i];
-  R2 vw;
-  vw.x = rmul(w, p.vis[2 * i]);
-  vw.y = rmul(w, p.vis[2 * i + 1]);
-  ((R2*)out.vw)[i] = vw;
-  out.cell[i] = pack_cell(r.gu, r.gv);
-  out.meta[i] = pack_meta(r.plane, r.ou, r.ov, r.conj_neg, r.skipped);
+  Placed<Real> o;
+  o.cell = pack_cell(r.gu, r.gv);
+  o.meta = pack_meta(r.plane, r.ou, r.ov, r.conj_neg, r.skipped);
+  o.v.x = rmul(w, p.vis[2 * i]);
+  o.v.y = rmul(w, p.vis[2 * i + 1]);
+  ((Placed<Real>*)out.placed)[i] = o;
+  out.cell[i] = o.cell;
+  out.meta[i] = o.meta;
   double t = 0.0;
   if (!r.skipped) {
     const int side = 2 * v.omax + 1;
@@ -72,7 +73,7 @@ template <typename Real>
 __global__ void __launch_bounds__(kThreads)
 k_revalue(const Real* __restrict__ vis, const Real* __restrict__ weight,
           const uint32_t* __restrict__ meta, StackView v,
-          unsigned long long n, typename Vec2<Real>::type* __restrict__ vw,
+          unsigned long long n, Placed<Real>* __restrict__ placed,
           double* __restrict__ nterm) {
   using R2 = typename Vec2<Real>::type;
   const unsigned long long i =
@@ -82,7 +83,7 @@ k_revalue(const Real* __restrict__ vis, const Real* __restrict__ weight,
   R2 o;
   o.x = rmul(w, vis[2 * i]);
   o.y = rmul(w, vis[2 * i + 1]);
-  vw[i] = o;
+  placed[i].v = o;
   const uint32_t m = meta[i];
   double t = 0.0;
   if (!meta_skipped(m)) {
@@ -196,12 +197,12 @@ cudaError_t launch_batch_totals(const uint32_t* meta, const double* nterm,
 template <typename Real>
 cudaError_t launch_revalue(const Real* vis, const Real* weight,
                            const uint32_t* meta, StackView view,
-                           unsigned long long n, void* vw, double* nterm,
+                           unsigned long long n, void* placed, double* nterm,
                            cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const unsigned nb = (unsigned)((n + kThreads - 1) / kThreads);
   k_revalue<Real><<<nb, kThreads, 0, s>>>(
-      vis, weight, meta, view, n, (typename Vec2<Real>::type*)vw, nterm);
+      vis, weight, meta, view, n, (Placed<Real>*)placed, nterm);
   return cudaGetLastError();
 }
 template cudaError_t launch_revalue<float>(const float*, const float*,

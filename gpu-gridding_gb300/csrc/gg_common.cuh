@@ -47,6 +47,16 @@ struct Vec2<float> { using type = float2; };
 template <>
 struct Vec2<double> { using type = double2; };
 
+// A placed visibility as the gridding kernel's records gather it: cell, meta
+// and the weighted visibility together, so that the gather of a record, in
+// tile order and so at random, is one sector of HBM and not three
+// (k_prepare_records on 3.1e7 track points, 5.9e7 records: see there).
+template <typename Real>
+struct alignas(4 * sizeof(Real)) Placed {
+  uint32_t cell, meta;
+  typename Vec2<Real>::type v;
+};
+
 // ---------------------------------------------------------------------------
 // Re-laid kernel stack: one dense slice per (plane, |offset| class).
 // ---------------------------------------------------------------------------

@@ -103,9 +103,7 @@ struct GridArgs {
   int group_span;                // virtual groups in the launch
   uint32_t* counter;
   const uint32_t* rec_vis;
-  const uint32_t* cell;
-  const uint32_t* meta;
-  const typename Vec2<Real>::type* vw;
+  const Placed<Real>* placed;
   Record<Real>* recs;       // prepared records, in sorted order
   unsigned short* spans;    // and the rows they meet
   StackView view;
@@ -144,12 +142,11 @@ __device__ __forceinline__ void cell_ends(const uint32_t* tile_groups,
 }
 
 // Prepares the records of every work item of the call: one block per item at
-// a time.  HBM-bound: 4 B of index, a 32-byte sector from each of three
-// arrays per record in, 18 B (FP64: 34 B) out.
+// a time.  HBM-bound: 4 B of index and one sector at random per record in,
+// 18 B (FP64: 34 B) out.
 template <typename Real, int TW>
 __global__ void __launch_bounds__(128)
 k_prepare_records(GridArgs<Real> a, int num_groups) {
-  using R2 = typename Vec2<Real>::type;
   using WS = WarpShape<TW>;
   const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
   const int num_items = (int)a.group_items[num_groups];
@@ -162,15 +159,15 @@ k_prepare_records(GridArgs<Real> a, int num_groups) {
     for (int i = item.rec_begin + (int)threadIdx.x; i < item.rec_end;
          i += blockDim.x) {
       const uint32_t vid = a.rec_vis[i];
-      const uint32_t ce = a.cell[vid], m = a.meta[vid];
-      const R2 v = a.vw[vid];
+      const Placed<Real> pt = a.placed[vid];
+      const uint32_t m = pt.meta;
       const SlicePlane plane = a.view.planes[meta_plane(m)];
       const int ou = meta_ou(m), ov = meta_ov(m), s = plane.support;
-      const int gu = cell_u(ce) - u0, gv = cell_v(ce) - v0;
+      const int gu = cell_u(pt.cell) - u0, gv = cell_v(pt.cell) - v0;
       Record<Real> rec;
       rec.d = slice_record(slice_origin(plane, a.view.omax, abs(ou), abs(ov)),
                            s, ou, ov, gu, gv);
-      rec.v = v;
+      rec.v = pt.v;
       a.recs[i] = rec;
       // The tile meets each of its records: clipped to it.
       a.spans[i] = (unsigned short)(
@@ -1002,9 +999,9 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
                               const uint32_t* group_items,
                               uint32_t* counter, void* recs,
                               unsigned short* spans, const uint32_t* rec_vis,
-                              const uint32_t* cell, const uint32_t* meta,
-                              const void* vw, StackView view, TileGeom geom,
-                              int grid_size, Real* grid, long long grid_stride,
+                              const void* placed, StackView view,
+                              TileGeom geom, int grid_size, Real* grid,
+                              long long grid_stride,
                               Real* partials, const int4* split_tiles,
                               const uint32_t* num_split, int max_split,
                               int num_ctas, cudaStream_t s,
@@ -1021,9 +1018,7 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
   a.recs = (Record<Real>*)recs;
   a.spans = spans;
   a.rec_vis = rec_vis;
-  a.cell = cell;
-  a.meta = meta;
-  a.vw = (const typename Vec2<Real>::type*)vw;
+  a.placed = (const Placed<Real>*)placed;
   a.view = view;
   a.geom = geom;
   a.grid_size = grid_size;
@@ -1085,13 +1080,13 @@ template int grid_tiles_ctas_per_sm<float>(int, bool);
 template int grid_tiles_ctas_per_sm<double>(int, bool);
 template cudaError_t launch_grid_tiles<float>(
     const WorkItem*, const uint32_t*, uint32_t*, void*, unsigned short*,
-    const uint32_t*, const uint32_t*, const uint32_t*, const void*, StackView, TileGeom, int,
+    const uint32_t*, const void*, StackView, TileGeom, int,
     float*, long long, float*, const int4*, const uint32_t*, int, int,
     cudaStream_t, const cudaEvent_t*, const cudaEvent_t*, float*,
     const uint32_t*, int, const int2*, const uint32_t*);
 template cudaError_t launch_grid_tiles<double>(
     const WorkItem*, const uint32_t*, uint32_t*, void*, unsigned short*,
-    const uint32_t*, const uint32_t*, const uint32_t*, const void*, StackView, TileGeom, int,
+    const uint32_t*, const void*, StackView, TileGeom, int,
     double*, long long, double*, const int4*, const uint32_t*, int, int,
     cudaStream_t, const cudaEvent_t*, const cudaEvent_t*, double*,
     const uint32_t*, int, const int2*, const uint32_t*);

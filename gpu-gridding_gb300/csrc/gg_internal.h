@@ -95,7 +95,7 @@ __host__ __device__ inline int phases_of_shape(uint32_t word) {
 struct PlaceOut {
   uint32_t* cell;             // [N]
   uint32_t* meta;             // [N]
-  void* vw;                   // [N] weighted visibility, Real2
+  void* placed;               // [N] Placed<Real>, null for degridding
   uint32_t* rec_count;        // [N] records (tiles touched) per visibility
   double* blk_norm;           // [num_blocks]
   unsigned long long* blk_skip;   // [num_blocks]
@@ -164,7 +164,7 @@ cudaError_t launch_place_batched(PlaceParams<Real> p, StackView view,
 template <typename Real>
 cudaError_t launch_revalue(const Real* vis, const Real* weight,
                            const uint32_t* meta, StackView view,
-                           unsigned long long n, void* vw, double* nterm,
+                           unsigned long long n, void* placed, double* nterm,
                            cudaStream_t s);
 // Deterministic per-grid totals over a chunk table (chunk c covers
 // visibilities [chunk_begin[c], chunk_begin[c+1]) of grid chunk_grid[c];
@@ -264,9 +264,9 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
                               const uint32_t* group_items,
                               uint32_t* counter, void* recs,
                               unsigned short* spans, const uint32_t* rec_vis,
-                              const uint32_t* cell, const uint32_t* meta,
-                              const void* vw, StackView view, TileGeom geom,
-                              int grid_size, Real* grid, long long grid_stride,
+                              const void* placed, StackView view,
+                              TileGeom geom, int grid_size, Real* grid,
+                              long long grid_stride,
                               Real* partials, const int4* split_tiles,
                               const uint32_t* num_split, int max_split,
                               int num_ctas, cudaStream_t s,

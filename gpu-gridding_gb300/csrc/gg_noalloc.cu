@@ -173,7 +173,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   unsigned long long* call_skip = c.take<unsigned long long>(1);
   uint32_t* cell = c.take<uint32_t>(maxp);
   uint32_t* meta = c.take<uint32_t>(maxp);
-  float2* vw = c.take<float2>(maxp);
+  Placed<float>* placed = c.take<Placed<float>>(maxp);
   uint32_t* count = c.take<uint32_t>(maxp);
   uint32_t* offset = c.take<uint32_t>(maxp);
   double* blk_norm = c.take<double>(max_blocks);
@@ -216,7 +216,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   PlaceOut po;
   po.cell = cell;
   po.meta = meta;
-  po.vw = vw;
+  po.placed = placed;
   po.rec_count = count;
   po.blk_norm = blk_norm;
   po.blk_skip = blk_skip;
@@ -314,8 +314,8 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   ib.num_groups = 1;
   ib.scan_tmp = scan_tmp;
   NA_CUDA(launch_build_items(tile_start, num_tiles, total, chunk, ib, s));
-  NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, recs, spans, vals, cell,
-                                   meta, vw, view, geom, grid_size, d_grid, 0,
+  NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, recs, spans, vals,
+                                   placed, view, geom, grid_size, d_grid, 0,
                                    (float*)partials, split_tiles, sc + 3,
                                    num_tiles, num_ctas, s));
   return GG_OK;

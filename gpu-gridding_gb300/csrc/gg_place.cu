@@ -25,7 +25,6 @@ __device__ __forceinline__ T warp_sum(T x) {
 template <typename Real>
 __global__ void __launch_bounds__(kPlaceThreads)
 k_place(PlaceParams<Real> p, StackView v, TileGeom g, PlaceOut out) {
-  using R2 = typename Vec2<Real>::type;
   const unsigned long long i =
       (unsigned long long)blockIdx.x * kPlaceThreads + threadIdx.x;
   double norm = 0.0;
@@ -34,14 +33,19 @@ k_place(PlaceParams<Real> p, StackView v, TileGeom g, PlaceOut out) {
     const Placement r = place_one(p, v, i);
     // Degridding places coordinates only (no visibilities, weights, norm).
     const Real w = p.weight ? p.weight[i] : (Real)0;
+    const uint32_t cell = pack_cell(r.gu, r.gv);
+    const uint32_t meta =
+        pack_meta(r.plane, r.ou, r.ov, r.conj_neg, r.skipped);
     if (p.vis) {
-      R2 vw;
-      vw.x = rmul(w, p.vis[2 * i]);
-      vw.y = rmul(w, p.vis[2 * i + 1]);
-      ((R2*)out.vw)[i] = vw;
+      Placed<Real> o;
+      o.cell = cell;
+      o.meta = meta;
+      o.v.x = rmul(w, p.vis[2 * i]);
+      o.v.y = rmul(w, p.vis[2 * i + 1]);
+      ((Placed<Real>*)out.placed)[i] = o;
     }
-    out.cell[i] = pack_cell(r.gu, r.gv);
-    out.meta[i] = pack_meta(r.plane, r.ou, r.ov, r.conj_neg, r.skipped);
+    out.cell[i] = cell;
+    out.meta[i] = meta;
     if (r.skipped) {
       skip = 1;
     } else {
