@@ -677,7 +677,8 @@ enum Scalar {
 // Tile shape of the degridding kernel (32 x 64 cells).
 constexpr int kDegridShape = 0;
 // 64-bit device scalars live after the 32-bit ones.
-constexpr size_t kScalar64Offset = 64;
+constexpr size_t kScalar64Offset = 32;
+static_assert(4 * kScalarCount <= kScalar64Offset, "scalars overlap");
 enum Scalar64 {
   kMacs = 0, kSkipScratch, kDirectCells, kRecords64, kScalar64Count
 };
@@ -1003,12 +1004,12 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
                                po.rec_count, s));
   GG_CUDA(exclusive_scan_u32(po.rec_count, plan->rec_offset.as<uint32_t>(), n,
                              sc + kTotalRecords, plan->scan_tmp.p, s));
-  plan->stats.num_launches = 6;  // place, finalize, count, 3-kernel scan
+  // place, finalize, count, scan
+  plan->stats.num_launches = 3 + scan_launches(n);
   plan->mark(1, s);
-  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, sc, 4 * kScalarCount,
+  // The 32-bit scalars and the MAC count behind them.
+  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, sc, kScalar64Offset + 8,
                           cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaMemcpyAsync((char*)plan->h_scalars + 32, scalar64(plan, kMacs),
-                          8, cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
   *po_out = po;
   return GG_OK;
@@ -1058,7 +1059,7 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
                        "grids)", records);
   }
   plan->stats.num_records = total;
-  memcpy(&plan->stats.num_macs, (char*)plan->h_scalars + 32, 8);
+  memcpy(&plan->stats.num_macs, (char*)plan->h_scalars + kScalar64Offset, 8);
   int key_bits = 0;
   // Tile phases (chosen with the shape; placement counted the records with
   // them): one more tile column and a phase field in the virtual group.
@@ -1144,7 +1145,7 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
     return set_error(GG_ERR_CUDA, "internal: sort pass count mismatch");
   b->keys = in_alt ? T->keys1.as<uint32_t>() : T->keys0.as<uint32_t>();
   b->vals = in_alt ? v1.as<uint32_t>() : v0.as<uint32_t>();
-  plan->stats.num_launches += 1 + 5 * (unsigned)((key_bits + 7) / 8);
+  plan->stats.num_launches += 1 + radix_launches(total, key_bits);
   plan->mark(2, s);
 
   GG_TRY(plan->tile_start.ensure((size_t)(num_tiles + 1) * 4));
@@ -1266,8 +1267,8 @@ int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
     GG_TRY(plan->partials.ensure(((size_t)slots + 1) * b.geom.tile_u *
                                  b.geom.tile_v * sizeof(R2)));
   }
-  // item counts, 2 scans, item emit
-  plan->stats.num_launches += 1 + 6 + 1;
+  // item counts, scan, item emit
+  plan->stats.num_launches += 2 + scan_launches(num_tiles);
   return GG_OK;
 }
 
@@ -1516,13 +1517,12 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
                                po.rec_count, s));
   GG_CUDA(exclusive_scan_u32(po.rec_count, T->rec_offset.as<uint32_t>(), n,
                              sc + kTotalRecords, plan->scan_tmp.p, s));
-  // place, chunk totals, finalize, count, 3-kernel scan
-  plan->stats.num_launches = (num_chunks > 0 ? 7 : 6);
+  // place, chunk totals, finalize, count, scan
+  plan->stats.num_launches = (num_chunks > 0 ? 4 : 3) + scan_launches(n);
   plan->mark(1, s);
-  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, sc, 4 * kScalarCount,
+  // The 32-bit scalars and the MAC count behind them.
+  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, sc, kScalar64Offset + 8,
                           cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaMemcpyAsync((char*)plan->h_scalars + 32, scalar64(plan, kMacs),
-                          8, cudaMemcpyDeviceToHost, s));
   GG_CUDA(cudaStreamSynchronize(s));
   GG_TRY(bin_and_grid<Real>(plan, K, n, po, grid_size, num_grids,
                             plan->grid_offsets.as<unsigned long long>(),

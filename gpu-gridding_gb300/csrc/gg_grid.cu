@@ -150,6 +150,8 @@ k_prepare_records(GridArgs<Real> a, int num_groups) {
   using WS = WarpShape<TW>;
   const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
   const int num_items = (int)a.group_items[num_groups];
+  // The first gridding launch's work counter.
+  if (blockIdx.x == 0 && threadIdx.x == 0) *a.counter = 0;
   for (int it = blockIdx.x; it < num_items; it += gridDim.x) {
     const WorkItem item = a.items[it];
     const int vg = item.tile / a.geom.tiles_total;   // virtual group
@@ -639,15 +641,23 @@ k_reduce_phases(const int2* __restrict__ tile_slot,
   }
 }
 
+// tile_start[t] = the first record of virtual tile t or a later one, by
+// binary search: the records may leave any number of tiles empty, and a
+// thread per record that writes the bounds of the tiles it passes writes
+// tens of thousands of them where they do (0.22 ms of a 24 ms call with four
+// plane groups).
 __global__ void k_tile_bounds(const uint32_t* __restrict__ keys, uint32_t n,
                               int shift, int num_tiles,
                               uint32_t* __restrict__ tile_start) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-       i <= (long long)n; i += (long long)gridDim.x * blockDim.x) {
-    const long long cur = i < n ? (long long)(keys[i] >> shift) : num_tiles;
-    const long long prev = i == 0 ? -1 : (long long)(keys[i - 1] >> shift);
-    for (long long x = prev + 1; x <= cur; ++x) tile_start[x] = (uint32_t)i;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t > num_tiles) return;
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if ((keys[mid] >> shift) < (uint32_t)t) lo = mid + 1;
+    else hi = mid;
   }
+  tile_start[t] = lo;
 }
 
 // Per tile row of a single grid, the strips (tile_u / tile_phases columns)
@@ -735,8 +745,10 @@ __global__ void k_item_counts(const uint32_t* __restrict__ tile_start,
                               const int* __restrict__ order, uint32_t chunk,
                               int partial_phases,
                               uint32_t* __restrict__ A,
-                              uint32_t* __restrict__ B) {
+                              uint32_t* __restrict__ B,
+                              uint32_t* __restrict__ num_split) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *num_split = 0;   // k_item_emit counts from here
   if (i >= num_tiles) return;
   const int T = num_tiles / num_groups;
   const int t = tile_at_rank(i, T, order);
@@ -846,8 +858,9 @@ cudaError_t prepare_grid_kernel_for(int tile_u, bool wide, void** fn,
 cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
                                int num_tiles, uint32_t* tile_start,
                                cudaStream_t s) {
-  const long long work = (long long)n + 1;
-  const int blocks = (int)std::min<long long>((work + 255) / 256, 65536);
+  // A tile per thread; with the whole key below the tile field no shift
+  // separates them, and every record is tile 0's.
+  const int blocks = num_tiles / 256 + 1;
   k_tile_bounds<<<blocks, 256, 0, s>>>(keys, n, shift, num_tiles, tile_start);
   return cudaGetLastError();
 }
@@ -890,14 +903,11 @@ cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
   const int blocks = (num_tiles + 256) / 256;   // one more thread: bounds
   const int pp = b.partial_phases > 1 ? b.partial_phases : 1;
   k_item_counts<<<blocks, 256, 0, s>>>(tile_start, num_tiles, b.num_groups,
-                                       b.tile_order, chunk, pp, A, B);
-  cudaError_t e;
-  e = exclusive_scan_u32(A, A, num_tiles, b.num_slots, b.scan_tmp, s);
-  if (e != cudaSuccess) return e;
+                                       b.tile_order, chunk, pp, A, B,
+                                       b.num_split);
   // The work counter doubles as scratch for B's total until k_item_emit.
-  e = exclusive_scan_u32(B, B, num_tiles, b.counter, b.scan_tmp, s);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(b.num_split, 0, sizeof(uint32_t), s);
+  cudaError_t e = exclusive_scan_pair_u32(A, B, num_tiles, b.num_slots,
+                                          b.counter, b.scan_tmp, s);
   if (e != cudaSuccess) return e;
   k_item_emit<<<blocks, 256, 0, s>>>(tile_start, num_tiles, b.num_groups,
                                      b.tile_order, chunk, pp, A, B,
@@ -906,10 +916,7 @@ cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
                                      b.items, b.split_tiles, b.num_split,
                                      b.num_items, b.group_items,
                                      b.tile_slot);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  // The persistent kernel's work counter starts at zero.
-  return cudaMemsetAsync(b.counter, 0, sizeof(uint32_t), s);
+  return cudaGetLastError();
 }
 
 template <typename Real>
@@ -1051,8 +1058,10 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
       e = cudaStreamWaitEvent(s, wait_before[g], 0);
       if (e != cudaSuccess) return e;
     }
-    e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
+    if (g > 0) {
+      e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
+      if (e != cudaSuccess) return e;
+    }
     e = cudaLaunchKernel(fn, dim3(num_ctas), dim3(kGridThreads), args, smem, s);
     if (e != cudaSuccess) return e;
     if (span > 1 && tile_slot) {

@@ -26,6 +26,13 @@ cudaError_t sum_u32(const uint32_t* in, size_t n, unsigned long long* total,
 // Sorts the first n pairs by key bits [0, end_bit).  Ping-pongs between
 // (keys, vals) and (keys_alt, vals_alt); on return *in_alt tells which pair
 // of buffers holds the result.  tmp must hold radix_temp_bytes(n).
+// The same for two arrays of n entries, in place and in the same launches.
+cudaError_t exclusive_scan_pair_u32(uint32_t* a, uint32_t* b, size_t n,
+                                    uint32_t* total_a, uint32_t* total_b,
+                                    void* tmp, cudaStream_t s);
+// Kernel launches of a scan of n entries (one array or a pair), and of a sort.
+int scan_launches(size_t n);
+int radix_launches(size_t n, int end_bit);
 size_t radix_temp_bytes(size_t n);
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals,
                              uint32_t* keys_alt, uint32_t* vals_alt, size_t n,

@@ -48,33 +48,33 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x,
   return result;
 }
 
-// Scan input loader (a functor, so other input forms can reuse the
-// kernels).
-struct LoadU32 {
-  const uint32_t* in;
-  __device__ __forceinline__ uint32_t operator()(size_t i) const {
-    return in[i];
-  }
+// The arrays of one scan launch: blockIdx.y takes one of two.
+struct ScanArrays {
+  const uint32_t* in[2];
+  uint32_t* out[2];
+  uint32_t* total[2];   // may be null
 };
 
-template <typename Load>
-__global__ void k_scan_reduce(Load in, size_t n,
+__global__ void k_scan_reduce(ScanArrays a, size_t n,
                               uint32_t* __restrict__ block_sums) {
+  const uint32_t* __restrict__ in = a.in[blockIdx.y];
   const size_t base = (size_t)blockIdx.x * kScanTile;
   uint32_t s = 0;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     size_t idx = base + (size_t)i * kScanThreads + threadIdx.x;
-    if (idx < n) s += in(idx);
+    if (idx < n) s += in[idx];
   }
   uint32_t total;
   block_exclusive_scan(s, &total);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
+  if (threadIdx.x == 0)
+    block_sums[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = total;
 }
 
 // Exclusive scan of the block sums in place by one block, chunk by chunk.
 __global__ void k_scan_top(uint32_t* __restrict__ sums, size_t nb,
-                           uint32_t* __restrict__ d_total) {
+                           ScanArrays a) {
+  sums += (size_t)blockIdx.y * nb;
   uint32_t carry = 0;
   for (size_t base = 0; base < nb; base += blockDim.x) {
     size_t idx = base + threadIdx.x;
@@ -84,44 +84,68 @@ __global__ void k_scan_top(uint32_t* __restrict__ sums, size_t nb,
     if (idx < nb) sums[idx] = carry + ex;
     carry += total;
   }
-  if (threadIdx.x == 0 && d_total) *d_total = carry;
+  if (threadIdx.x == 0 && a.total[blockIdx.y]) *a.total[blockIdx.y] = carry;
 }
 
-template <typename Load>
-__global__ void k_scan_down(Load in, uint32_t* __restrict__ out, size_t n,
-                            const uint32_t* __restrict__ block_offsets) {
-  __shared__ uint32_t tile[kScanTile];
-  const size_t base = (size_t)blockIdx.x * kScanTile;
+// One kScanTile of a scan by kThreads_ threads; returns the tile's sum.
+template <int kThreads_>
+__device__ __forceinline__ uint32_t scan_tile(const uint32_t* in,
+                                              uint32_t* out, size_t base,
+                                              size_t n, uint32_t before,
+                                              uint32_t* tile) {
+  constexpr int kItems = kScanTile / kThreads_;
   // Striped, coalesced load into shared memory.
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    int t = i * kScanThreads + threadIdx.x;
+  for (int i = 0; i < kItems; ++i) {
+    int t = i * kThreads_ + threadIdx.x;
     size_t idx = base + t;
-    tile[t] = idx < n ? in(idx) : 0;
+    tile[t] = idx < n ? in[idx] : 0;
   }
   __syncthreads();
-  // Each thread scans its kScanItems consecutive entries.
-  uint32_t v[kScanItems];
+  // Each thread scans its kItems consecutive entries.
+  uint32_t v[kItems];
   uint32_t s = 0;
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    v[i] = tile[threadIdx.x * kScanItems + i];
+  for (int i = 0; i < kItems; ++i) {
+    v[i] = tile[threadIdx.x * kItems + i];
     s += v[i];
   }
   uint32_t total;
-  uint32_t pre = block_exclusive_scan(s, &total) + block_offsets[blockIdx.x];
+  uint32_t pre = block_exclusive_scan(s, &total) + before;
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    tile[threadIdx.x * kScanItems + i] = pre;
+  for (int i = 0; i < kItems; ++i) {
+    tile[threadIdx.x * kItems + i] = pre;
     pre += v[i];
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    int t = i * kScanThreads + threadIdx.x;
+  for (int i = 0; i < kItems; ++i) {
+    int t = i * kThreads_ + threadIdx.x;
     size_t idx = base + t;
     if (idx < n) out[idx] = tile[t];
   }
+  __syncthreads();
+  return total;
+}
+
+__global__ void k_scan_down(ScanArrays a, size_t n,
+                            const uint32_t* __restrict__ block_offsets) {
+  __shared__ uint32_t tile[kScanTile];
+  scan_tile<kScanThreads>(
+      a.in[blockIdx.y], a.out[blockIdx.y], (size_t)blockIdx.x * kScanTile, n,
+      block_offsets[(size_t)blockIdx.y * gridDim.x + blockIdx.x], tile);
+}
+
+// A whole scan by one block (n <= kScanOneBlock): one launch instead of
+// three, which is what a short scan costs (3 to 4 us each in a small call).
+constexpr size_t kScanOneBlock = 8 * kScanTile;
+__global__ void __launch_bounds__(1024) k_scan_one(ScanArrays a, size_t n) {
+  __shared__ uint32_t tile[kScanTile];
+  uint32_t sum = 0;
+  for (size_t base = 0; base < n; base += kScanTile)
+    sum += scan_tile<1024>(a.in[blockIdx.y], a.out[blockIdx.y], base, n, sum,
+                           tile);
+  if (threadIdx.x == 0 && a.total[blockIdx.y]) *a.total[blockIdx.y] = sum;
 }
 
 // ---------------------------------------------------------------------------
@@ -132,7 +156,12 @@ constexpr int kRadixWarps = kRadixThreads / 32;
 constexpr int kRadixRounds = 16;
 constexpr int kRadixTile = kRadixThreads * kRadixRounds;  // 4096
 constexpr int kRadixDigits = 256;
+// Up to this many blocks the scatter kernel works out its run starts from the
+// histograms itself (num_blocks loads a thread, from L2): two launches a pass
+// instead of five.
+constexpr int kFewBlocks = 192;
 
+template <bool kFew>
 __global__ void __launch_bounds__(kRadixThreads)
 k_radix_hist(const uint32_t* __restrict__ keys, size_t n, int shift,
              int num_blocks, uint32_t* __restrict__ hist) {
@@ -154,8 +183,12 @@ k_radix_hist(const uint32_t* __restrict__ keys, size_t n, int shift,
   }
   __syncthreads();
   // Digit-major layout: the scan then yields, for each (digit, block), the
-  // global position of that block's first key with that digit.
-  hist[(size_t)threadIdx.x * num_blocks + blockIdx.x] = h[threadIdx.x];
+  // global position of that block's first key with that digit.  Without a
+  // scan (kFew) block-major, so that a block's threads read the counts
+  // of a digit each, block by block.
+  hist[kFew
+           ? (size_t)blockIdx.x * kRadixDigits + threadIdx.x
+           : (size_t)threadIdx.x * num_blocks + blockIdx.x] = h[threadIdx.x];
 }
 
 // Stable scatter of one 4096-key block: the keys are first ordered by digit
@@ -166,8 +199,8 @@ k_radix_hist(const uint32_t* __restrict__ keys, size_t n, int shift,
 // w * 512 + j * 32 + l of the block) against warp-private digit counters,
 // so the ranking needs no block barrier; one per-digit prefix over the
 // warps then places every key.  hist holds the block's digit counts
-// (digit-major, as k_radix_hist wrote them) and offsets their exclusive
-// scan (global start of each (digit, block) run).
+// (as k_radix_hist wrote them) and offsets, unless kFew, their exclusive scan (global start of each (digit, block) run).
+template <bool kFew>
 __global__ void __launch_bounds__(kRadixThreads, 3)
 k_radix_scatter(const uint32_t* __restrict__ keys,
                 const uint32_t* __restrict__ vals, size_t n, int shift,
@@ -184,13 +217,26 @@ k_radix_scatter(const uint32_t* __restrict__ keys,
   // the warps before it.
   __shared__ uint32_t warp_count[kRadixWarps][kRadixDigits];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t cell = (size_t)threadIdx.x * num_blocks + blockIdx.x;
-  digit_base[threadIdx.x] = offsets[cell];
+  uint32_t total, count;
+  if constexpr (kFew) {
+    uint32_t before = 0, all = 0;
+    count = hist[(size_t)blockIdx.x * kRadixDigits + threadIdx.x];
+#pragma unroll 8
+    for (int b = 0; b < num_blocks; ++b) {
+      const uint32_t c = hist[(size_t)b * kRadixDigits + threadIdx.x];
+      all += c;
+      if (b < (int)blockIdx.x) before += c;
+    }
+    digit_base[threadIdx.x] = block_exclusive_scan(all, &total) + before;
+  } else {
+    const size_t cell = (size_t)threadIdx.x * num_blocks + blockIdx.x;
+    digit_base[threadIdx.x] = offsets[cell];
+    count = hist[cell];
+  }
 #pragma unroll
   for (int w = 0; w < kRadixWarps; ++w) warp_count[w][threadIdx.x] = 0;
-  uint32_t total;
   // (block_exclusive_scan ends with a barrier: the counters are zeroed.)
-  local_start[threadIdx.x] = block_exclusive_scan(hist[cell], &total);
+  local_start[threadIdx.x] = block_exclusive_scan(count, &total);
   const uint32_t lt_mask = (1u << lane) - 1u;
   const size_t base = (size_t)blockIdx.x * kRadixTile;
   const int valid_n = (int)min((size_t)kRadixTile, n - base);
@@ -270,21 +316,31 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 size_t scan_temp_bytes(size_t n) {
   size_t nb = (n + kScanTile - 1) / kScanTile;
-  return align_up((nb + 1) * sizeof(uint32_t), 256);
+  return align_up(2 * (nb + 1) * sizeof(uint32_t), 256);
 }
 
-template <typename Load>
-static cudaError_t scan_impl(Load in, uint32_t* out, size_t n,
-                             uint32_t* d_total, void* tmp, cudaStream_t s) {
+// `arrays` scans of n entries each in the same launches; tmp holds
+// scan_temp_bytes(n) for each.
+static cudaError_t scan_impl(const ScanArrays& a, int arrays, size_t n,
+                             void* tmp, cudaStream_t s) {
   if (n == 0) {
-    if (d_total) return cudaMemsetAsync(d_total, 0, sizeof(uint32_t), s);
+    for (int i = 0; i < arrays; ++i)
+      if (a.total[i]) {
+        cudaError_t e = cudaMemsetAsync(a.total[i], 0, sizeof(uint32_t), s);
+        if (e != cudaSuccess) return e;
+      }
     return cudaSuccess;
+  }
+  if (n <= kScanOneBlock) {
+    k_scan_one<<<dim3(1, arrays), 1024, 0, s>>>(a, n);
+    return cudaGetLastError();
   }
   size_t nb = (n + kScanTile - 1) / kScanTile;
   uint32_t* sums = (uint32_t*)tmp;
-  k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, sums);
-  k_scan_top<<<1, 1024, 0, s>>>(sums, nb, d_total);
-  k_scan_down<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums);
+  k_scan_reduce<<<dim3((unsigned)nb, arrays), kScanThreads, 0, s>>>(a, n,
+                                                                    sums);
+  k_scan_top<<<dim3(1, arrays), 1024, 0, s>>>(sums, nb, a);
+  k_scan_down<<<dim3((unsigned)nb, arrays), kScanThreads, 0, s>>>(a, n, sums);
   return cudaGetLastError();
 }
 
@@ -318,7 +374,24 @@ cudaError_t sum_u32(const uint32_t* in, size_t n, unsigned long long* total,
 
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
                                uint32_t* d_total, void* tmp, cudaStream_t s) {
-  return scan_impl(LoadU32{in}, out, n, d_total, tmp, s);
+  return scan_impl({{in, nullptr}, {out, nullptr}, {d_total, nullptr}}, 1, n,
+                   tmp, s);
+}
+
+cudaError_t exclusive_scan_pair_u32(uint32_t* a, uint32_t* b, size_t n,
+                                    uint32_t* total_a, uint32_t* total_b,
+                                    void* tmp, cudaStream_t s) {
+  return scan_impl({{a, b}, {a, b}, {total_a, total_b}}, 2, n, tmp, s);
+}
+
+int scan_launches(size_t n) {
+  return n == 0 ? 0 : n <= kScanOneBlock ? 1 : 3;
+}
+int radix_launches(size_t n, int end_bit) {
+  if (n <= 1 || end_bit <= 0) return 0;
+  const size_t nb = (n + kRadixTile - 1) / kRadixTile;
+  return (end_bit + 7) / 8 *
+         (nb > kFewBlocks ? 2 + scan_launches(nb * kRadixDigits) : 2);
 }
 
 size_t radix_temp_bytes(size_t n) {
@@ -341,13 +414,20 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals,
   void* scan_tmp = (char*)tmp + 2 * hist_bytes;
   uint32_t *k_in = keys, *v_in = vals, *k_out = keys_alt, *v_out = vals_alt;
   for (int shift = 0; shift < end_bit; shift += 8) {
-    k_radix_hist<<<(unsigned)nb, kRadixThreads, 0, s>>>(k_in, n, shift,
-                                                        (int)nb, hist);
-    cudaError_t e = exclusive_scan_u32(hist, offs, nb * kRadixDigits, nullptr,
-                                       scan_tmp, s);
-    if (e != cudaSuccess) return e;
-    k_radix_scatter<<<(unsigned)nb, kRadixThreads, 0, s>>>(
-        k_in, v_in, n, shift, (int)nb, hist, offs, k_out, v_out);
+    if (nb <= kFewBlocks) {
+      k_radix_hist<true><<<(unsigned)nb, kRadixThreads, 0, s>>>(
+          k_in, n, shift, (int)nb, hist);
+      k_radix_scatter<true><<<(unsigned)nb, kRadixThreads, 0, s>>>(
+          k_in, v_in, n, shift, (int)nb, hist, offs, k_out, v_out);
+    } else {
+      k_radix_hist<false><<<(unsigned)nb, kRadixThreads, 0, s>>>(
+          k_in, n, shift, (int)nb, hist);
+      cudaError_t e = exclusive_scan_u32(hist, offs, nb * kRadixDigits,
+                                         nullptr, scan_tmp, s);
+      if (e != cudaSuccess) return e;
+      k_radix_scatter<false><<<(unsigned)nb, kRadixThreads, 0, s>>>(
+          k_in, v_in, n, shift, (int)nb, hist, offs, k_out, v_out);
+    }
     uint32_t* t;
     t = k_in; k_in = k_out; k_out = t;
     t = v_in; v_in = v_out; v_out = t;

@@ -198,3 +198,24 @@ def test_degrid_host_grid_access_modes(pkg, synthetic, torch, prec):
         pkg.set_host_grid_access(mode)
     for o in outs[1:]:
         assert np.array_equal(o.view(np.uint8), outs[0].view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [1, 2, 4096, 4097, 16384, 16385, 192 * 4096,
+                               192 * 4096 + 1])
+def test_sort_and_scan_sizes(pkg, oracle_mod, synthetic, torch, n):
+    """The sort's and the scans' launches change at these point counts (one
+    block, one-block scans, run starts worked out without a scan): the density
+    grid stays the serial sums bit for bit, and gridding the same number of
+    points matches the FP64 oracle."""
+    G, cell = 512, np.float32(1e-3)
+    uu, vv, w = _points(n, G, cell, np.float32, 5)
+    dens, ns = pkg.grid_weights_write(uu, vv, w, cell, G)
+    ref, ns_ref = oracle_mod.weights_write(uu, vv, w, cell, G)
+    assert ns == ns_ref
+    _same(dens, ref)
+    wl = synthetic.random_uniform_workload("sizes", n, 256, 4, 1, 2, seed=n,
+                                           cell_size_rad=6.4e-4)
+    g64, ns64, nm64 = oracle_mod.grid_f_fp64acc(wl)
+    g, ns, nm = pkg.grid_f(wl)
+    assert ns == ns64 and abs(nm - nm64) <= 1e-12 * abs(nm64)
+    assert max_rel(g, g64) <= 1e-5
