@@ -2228,7 +2228,8 @@ int weights_write_pipeline(gg_plan* plan, size_t n, const Real* uu,
   GG_TRY(plan->keys1.ensure(n * 4));
   GG_TRY(plan->vals1.ensure(n * 4));
   GG_TRY(plan->sort_tmp.ensure(radix_temp_bytes(n)));
-  GG_CUDA(launch_weight_keys<Real>(uu, vv, n, cell_size_rad, grid_size,
+  GG_CUDA(launch_weight_keys<Real>(uu, vv, weight, n, cell_size_rad,
+                                   grid_size,
                                    plan->keys0.as<uint32_t>(),
                                    plan->vals0.as<uint32_t>(), d_num_skipped,
                                    s));

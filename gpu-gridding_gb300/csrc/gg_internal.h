@@ -310,11 +310,12 @@ bool kernels_info(const gg_kernels* k, StackView* view, int* device,
                   bool* is_double, int* num_planes);
 
 // ---- uniform weighting (gg_weights.cu) -------------------------------------
-// Keys each point by its density cell (grid_size^2 when off the grid) and
-// counts the off-grid points into *d_num_skipped (which must start at 0).
+// Keys each point by its density cell (grid_size^2 when off the grid), its
+// value the weight's bits (FP32) or its index, and counts the off-grid points into *d_num_skipped (which must start at 0).
 template <typename Real>
 cudaError_t launch_weight_keys(const Real* uu, const Real* vv,
-                               unsigned long long n, Real cell_size_rad,
+                               const Real* weight, unsigned long long n,
+                               Real cell_size_rad,
                                int grid_size, uint32_t* keys, uint32_t* vals,
                                unsigned long long* d_num_skipped,
                                cudaStream_t s);

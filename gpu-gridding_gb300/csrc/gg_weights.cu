@@ -9,7 +9,8 @@
 // Density: the reference adds the weights into the grid one visibility at a
 // time, so each cell's sum is formed in visibility order.  Here the
 // visibilities are keyed by cell and stably sorted (visibility order kept
-// within a cell), and one thread adds each cell's run in that order onto
+// within a cell; FP32 weights are the sorted values, so the sums read them in
+// place), and one thread adds each cell's run in that order onto
 // the cell's existing value -- the same additions in the same order, so the
 // density grid is bit-identical to the serial code's.
 #include "gg_internal.h"
@@ -38,11 +39,12 @@ __device__ __forceinline__ bool weight_cell(Real uu, Real vv, Real scale,
   return true;
 }
 
-// key = cell (G*G for skipped points, which sort last), value = index.
+// key = cell (G*G for skipped points, which sort last), value = the weight
+// itself where it fits the sort's 32-bit values (FP32), else the index.
 template <typename Real>
 __global__ void __launch_bounds__(kThreads)
 k_weight_keys(const Real* __restrict__ uu, const Real* __restrict__ vv,
-              unsigned long long n, Real scale, int grid_size,
+              const Real* __restrict__ weight, unsigned long long n, Real scale, int grid_size,
               uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
               unsigned long long* __restrict__ num_skipped) {
   const unsigned long long i =
@@ -52,7 +54,8 @@ k_weight_keys(const Real* __restrict__ uu, const Real* __restrict__ vv,
     uint32_t c;
     skip = !weight_cell(uu[i], vv[i], scale, grid_size, &c);
     keys[i] = skip ? (uint32_t)((unsigned long long)grid_size * grid_size) : c;
-    vals[i] = (uint32_t)i;
+    if constexpr (sizeof(Real) == 4) vals[i] = __float_as_uint(weight[i]);
+    else vals[i] = (uint32_t)i;
   }
   const unsigned int cnt = __popc(__ballot_sync(0xffffffffu, skip));
   if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(num_skipped, cnt);
@@ -62,21 +65,46 @@ __device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ double radd(double a, double b) { return __dadd_rn(a, b); }
 
 // The first thread of each run of equal cells adds the run's weights, in
-// visibility order, onto the cell.
+// visibility order, onto the cell.  What bounds it is the longest run (the
+// cells of the shortest baselines hold thousands of points): one chain of
+// additions, so its keys and weights are loaded sixteen ahead.
 template <typename Real>
 __global__ void __launch_bounds__(kThreads)
 k_weight_runs(const uint32_t* __restrict__ keys,
               const uint32_t* __restrict__ vals, unsigned long long n,
               const Real* __restrict__ weight, unsigned long long num_cells,
               Real* __restrict__ grid) {
+  constexpr int kAhead = 16;
   const unsigned long long j =
       (unsigned long long)blockIdx.x * kThreads + threadIdx.x;
   if (j >= n) return;
   const uint32_t c = keys[j];
   if (c >= num_cells || (j > 0 && keys[j - 1] == c)) return;
-  Real g = grid[c];
-  for (unsigned long long t = j; t < n && keys[t] == c; ++t)
-    g = radd(g, weight[vals[t]]);
+  auto value = [&](unsigned long long t) -> Real {
+    if constexpr (sizeof(Real) == 4) return __uint_as_float(vals[t]);
+    else return weight[vals[t]];
+  };
+  Real g = radd(grid[c], value(j));
+  unsigned long long t = j + 1;
+  // Most runs are short: one record at a time until a few have been added.
+  for (const unsigned long long e = min(n, j + 4); t < e && keys[t] == c; ++t)
+    g = radd(g, value(t));
+  bool more = t == j + 4 && t < n && keys[t] == c;
+  while (more) {
+    uint32_t k[kAhead];
+    Real w[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      k[q] = t + q < n ? keys[t + q] : 0xFFFFFFFFu;
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) w[q] = k[q] == c ? value(t + q) : Real(0);
+    // Sorted: the run's records are the first of the sixteen.
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q)
+      if (k[q] == c) g = radd(g, w[q]);
+    more = k[kAhead - 1] == c;
+    t += kAhead;
+  }
   grid[c] = g;
 }
 
@@ -115,7 +143,8 @@ unsigned blocks_for(unsigned long long n) {
 
 template <typename Real>
 cudaError_t launch_weight_keys(const Real* uu, const Real* vv,
-                               unsigned long long n, Real cell_size_rad,
+                               const Real* weight, unsigned long long n,
+                               Real cell_size_rad,
                                int grid_size, uint32_t* keys, uint32_t* vals,
                                unsigned long long* d_num_skipped,
                                cudaStream_t s) {
@@ -124,7 +153,7 @@ cudaError_t launch_weight_keys(const Real* uu, const Real* vv,
   // the call's precision.
   const Real scale = (Real)grid_size * cell_size_rad;
   k_weight_keys<Real><<<blocks_for(n), kThreads, 0, s>>>(
-      uu, vv, n, scale, grid_size, keys, vals, d_num_skipped);
+      uu, vv, weight, n, scale, grid_size, keys, vals, d_num_skipped);
   return cudaGetLastError();
 }
 
@@ -154,11 +183,13 @@ cudaError_t launch_weights_read(const Real* uu, const Real* vv,
 }
 
 template cudaError_t launch_weight_keys<float>(const float*, const float*,
+                                               const float*,
                                                unsigned long long, float, int,
                                                uint32_t*, uint32_t*,
                                                unsigned long long*,
                                                cudaStream_t);
 template cudaError_t launch_weight_keys<double>(const double*, const double*,
+                                                const double*,
                                                 unsigned long long, double,
                                                 int, uint32_t*, uint32_t*,
                                                 unsigned long long*,
