@@ -1202,7 +1202,10 @@ int tile_queue_order(gg_plan* plan, const TileGeom& g, int grid_size,
 // items as all of them).  Gridding chunks shorter than 1024 records are
 // made longer, up to half a CTA's share: below that the partial tiles cost
 // more than the better balance gives (2048^2, 2e5 points, 6.6e5 records:
-// 0.69 ms with chunks of 434, 0.60 with 867).  Items: at most one
+// 0.69 ms with chunks of 434, 0.60 with 867).  FP64 gridding takes twice the
+// items and no such minimum: a record costs it four times as much, a unit's
+// tail likewise (the same points: 2.87 ms with chunks of 1084, 2.43 with 542,
+// 2.35 with 271, 2.34 with 136).  Items: at most one
 // more per tile than
 // total / chunk; partial-tile slots (split tiles only): at most
 // 2 * total / chunk, each a tile of partial sums when partial_tiles is set
@@ -1216,11 +1219,12 @@ int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
   const int num_tiles = b.num_tiles;
   // items_per_cta items per CTA in each of the call's passes: every pass
   // ends with a tail up to one item long.
-  const unsigned long long f =
-      (unsigned long long)plan->items_per_cta * (unsigned long long)passes;
+  const bool grid64 = partial_tiles && sizeof(Real) == 8;
+  const unsigned long long f = (unsigned long long)plan->items_per_cta *
+                               (unsigned long long)passes * (grid64 ? 2 : 1);
   unsigned long long records =
       ((unsigned long long)b.total + f * num_ctas - 1) / (f * num_ctas);
-  if (partial_tiles)
+  if (partial_tiles && !grid64)
     records = std::max(records,
                        std::min(1024ull, (unsigned long long)b.total /
                                              (2ull * passes * num_ctas)));

@@ -78,6 +78,13 @@ struct alignas(16) Record {
   uint2 d;
   typename Vec2<Real>::type v;
 };
+// FP64: also the tile rows of the footprint (in what would be padding).
+template <>
+struct alignas(16) Record<double> {
+  uint2 d;
+  int row0, row1;
+  double2 v;
+};
 
 // The lane-row groups (kRows rows each, at most 32) of a tile that a
 // record's footprint meets, first | last << 5, with bit 15 set where its
@@ -170,6 +177,10 @@ k_prepare_records(GridArgs<Real> a, int num_groups) {
       rec.d = slice_record(slice_origin(plane, a.view.omax, abs(ou), abs(ov)),
                            s, ou, ov, gu, gv);
       rec.v = pt.v;
+      if constexpr (sizeof(Real) == 8) {
+        rec.row0 = gv - s;
+        rec.row1 = gv + s;
+      }
       a.recs[i] = rec;
       // The tile meets each of its records: clipped to it.
       a.spans[i] = (unsigned short)(
@@ -186,18 +197,16 @@ k_prepare_records(GridArgs<Real> a, int num_groups) {
 //   taps[x + r * step + su * clamp(col - gu, -S, S)]
 // with S = s + 1 (the clamped ends are zero taps) and step = +-2S; the record
 // adds (a, d) * (t.re, t.im) to the cell's P and (c, b) * (t.re, t.im) to its
-// Q, and re = P.x + Q.y, im = Q.x + P.y (FP32: two packed FMAs a cell).
-template <typename Real>
+// Q, and re = P.x + Q.y, im = Q.x + P.y (two packed FMAs a cell).
 struct alignas(16) Queued {
   uint32_t x;
   int gu_su;    // gu << 16 | (su & 0xFFFF)
   int S, step;
-  Real a, d, c, b;
+  float a, d, c, b;
 };
-template <typename Real>
-__device__ __forceinline__ Queued<Real> queued(const Record<Real>& r,
-                                               uint32_t span, int group) {
-  Queued<Real> q;
+__device__ __forceinline__ Queued queued(const Record<float>& r, uint32_t span,
+                                         int group) {
+  Queued q;
   const int z = (int)(short)(r.d.y & 0xFFFFu);
   const int s = (int)((r.d.y >> 16) & 0x3FFFu);
   const bool mu = (r.d.y & kMirrorU) != 0u, conj = (span & kSpanConj) != 0u;
@@ -214,29 +223,25 @@ __device__ __forceinline__ Queued<Real> queued(const Record<Real>& r,
 }
 
 // Shared memory of one warp of the gridding kernel.
-template <typename Real, int TW>
+template <int TW>
 struct WarpSmem {
-  using R2 = typename Vec2<Real>::type;
-  static constexpr bool kComp = sizeof(Real) == 4;
   static constexpr int kQueue = 64;
-  R2 hi[kComp ? kRows : 1][32];
-  R2 lo[kComp ? kRows : 1][32];
+  float2 hi[kRows][32];
+  float2 lo[kRows][32];
   // Records waiting for each lane-row group, a ring.
-  Queued<Real> queue[WarpShape<TW>::kLanesY][kQueue];
+  Queued queue[WarpShape<TW>::kLanesY][kQueue];
 };
 
 constexpr int kGridWarps = 4;    // per block of the gridding kernel
 constexpr int kGridThreads = kGridWarps * 32;
 
-template <typename Real, int TW, bool kWide>
-__global__ void __launch_bounds__(kGridThreads, sizeof(Real) == 4 ? 5 : 2)
-k_grid_tiles(GridArgs<Real> a) {
-  constexpr bool kCompensate = sizeof(Real) == 4;
-  // Records in flight per warp.
-  constexpr int kDepth = 2;
-  using R2 = typename Vec2<Real>::type;
+template <int TW, bool kWide>
+__global__ void __launch_bounds__(kGridThreads, 5)
+k_grid_tiles(GridArgs<float> a) {
+  constexpr int kDepth = 2;   // records in flight per warp
+  using R2 = float2;
   using WS = WarpShape<TW>;
-  using SM = WarpSmem<Real, TW>;
+  using SM = WarpSmem<TW>;
   constexpr int G = WS::kLanesY, Q = SM::kQueue;
   extern __shared__ __align__(16) unsigned char g_smem_raw[];
   const int lane = threadIdx.x & 31;
@@ -262,7 +267,7 @@ k_grid_tiles(GridArgs<Real> a) {
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
       acc[r] = acq[r] = R2{};
-      if constexpr (kCompensate) sm.hi[r][lane] = sm.lo[r][lane] = R2{};
+      sm.hi[r][lane] = sm.lo[r][lane] = R2{};
     }
     R2 tp[kDepth][kRows];
     // Queue positions: `at` the oldest record not yet added (the kDepth from
@@ -271,14 +276,14 @@ k_grid_tiles(GridArgs<Real> a) {
     bool primed = false;
 #pragma unroll
     for (int g = 0; g < G; ++g) tails[g] = 0;
-    Queued<Real>* const queue = sm.queue[ly];
+    Queued* const queue = sm.queue[ly];
     auto load = [&](int i, R2 (&out)[kRows]) {
       const int4 e = *(const int4*)&queue[i & (Q - 1)];
       const int t = min(max(lx - (e.y >> 16), -e.z), e.z);
       load_taps<kWide>(stack, (uint32_t)(e.x + (int)(short)e.y * t), e.w, out);
     };
     auto add = [&](int i, const R2 (&t)[kRows]) {
-      const Queued<Real>& e = queue[i & (Q - 1)];
+      const Queued& e = queue[i & (Q - 1)];
       R2 p, q;
       p.x = e.a; p.y = e.d;
       q.x = e.c; q.y = e.b;
@@ -310,7 +315,7 @@ k_grid_tiles(GridArgs<Real> a) {
       for (int g = 0; g < G; ++g) {
         if (g == ly)
           for (int i = tails[g] + lx; i < end; i += TW) {
-            Queued<Real> none{};
+            Queued none{};
             none.x = kStackZero;
             queue[i & (Q - 1)] = none;
           }
@@ -332,7 +337,7 @@ k_grid_tiles(GridArgs<Real> a) {
     };
 
     uint32_t span = kSpanNone;
-    Record<Real> rec;
+    Record<float> rec;
     auto fetch = [&](int i) {
       span = kSpanNone;
       if (i + lane < item.rec_end) {
@@ -367,7 +372,7 @@ k_grid_tiles(GridArgs<Real> a) {
       }
       // Plain FP32 sums of at most 128 records (and the few in flight) go
       // into the compensated (hi, lo) pair.
-      if (kCompensate && ((i - item.rec_begin) & 96) == 96) fold();
+      if (((i - item.rec_begin) & 96) == 96) fold();
       __syncwarp();
     }
     int end = tails[0];
@@ -381,7 +386,7 @@ k_grid_tiles(GridArgs<Real> a) {
       for (int d = 0; d < kDepth; ++d) add(at + d, tp[d]);
     }
     __syncwarp();   // the queues are free for the next unit
-    if (kCompensate) fold();
+    fold();
     // An owned band that no record meets stays as it is (in direct mode its
     // cells may still have to move between the host and the scratch grid).
     if (end == 0 && item.slot < 0 && !a.tile_groups) continue;
@@ -395,14 +400,9 @@ k_grid_tiles(GridArgs<Real> a) {
     R2 out[kRows];
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
-      if constexpr (kCompensate) {
-        const R2 hi = sm.hi[r][lane], lo = sm.lo[r][lane];
-        out[r].x = hi.x + lo.x;
-        out[r].y = hi.y + lo.y;
-      } else {
-        out[r].x = acc[r].x + acq[r].y;
-        out[r].y = acq[r].x + acc[r].y;
-      }
+      const R2 hi = sm.hi[r][lane], lo = sm.lo[r][lane];
+      out[r].x = hi.x + lo.x;
+      out[r].y = hi.y + lo.y;
     }
     if (item.slot < 0) {
       const int col =
@@ -433,6 +433,179 @@ k_grid_tiles(GridArgs<Real> a) {
 #pragma unroll
       for (int r = 0; r < kRows; ++r) __stcs(p + r * kConsumers, out[r]);
     }
+  }
+}
+
+// A queued record of the FP64 kernel: its footprint clipped to the warp's band,
+// w columns of n cells, row by row.  Cell i of it lies in row i / w, column
+// i % w: band cell `cell` + row * TW + column, tap x + row * step + su *
+// column.  (a, d, c, b): the coefficients of t.re (a, c) and t.im (b, d) in re
+// and im.
+struct alignas(16) Queued64 {
+  uint32_t x;
+  int su, step, cell;
+  int n, w;
+  float inv_w;
+  double a, b, c, d;
+};
+
+constexpr int kBandCells = kCells / kWarps;   // 256
+
+struct WarpSmem64 {
+  double2 acc[kBandCells];
+  Queued64 queue[32];
+};
+
+// The gridding kernel in FP64.  The FP64 pipe bounds it (a warp's FMA takes
+// 12 cycles of the SM however few of its lanes are active, four of them for
+// 32 cells), so the lanes take a record's cells in the band packed row by row,
+// whatever the footprint's position, instead of a column each: of the cells
+// of a record on a band about half are inside its footprint (2048^2, 2e5
+// points, 128 planes, support 4 to 24), of the packed ones 95 %.  The band's
+// sums lie in shared memory, a read and a write of 16 bytes a cell that the
+// pipe hides; a warp adds its records one after the other, so no two lanes
+// meet in a cell.  That workload's pass: 4.1 ms with a column a lane and
+// band rows in registers, 2.15 so (the multiply-adds alone 1.73).  Eight
+// cells a lane in flight, three blocks: 2.15; four cells and four to six
+// blocks 2.18 to 2.2, as the units in flight at the end are more.
+template <int TW>
+__global__ void __launch_bounds__(kGridThreads, 3)
+k_grid_tiles_f64(GridArgs<double> a) {
+  using WS = WarpShape<TW>;
+  constexpr int kAhead = 8;   // cells of a lane in flight
+  extern __shared__ __align__(16) unsigned char g_smem_raw[];
+  const int lane = threadIdx.x & 31;
+  WarpSmem64& sm =
+      reinterpret_cast<WarpSmem64*>(g_smem_raw)[threadIdx.x >> 5];
+  const double2* __restrict__ stack = (const double2*)a.view.taps;
+  const unsigned first = a.group_items[a.group];
+  const unsigned units =
+      (a.group_items[a.group + a.group_span] - first) * kWarps;
+  unsigned next = 0;
+  if (lane == 0) next = atomicAdd(a.counter, 1u);
+  for (;;) {
+    const unsigned unit = __shfl_sync(0xffffffffu, next, 0);
+    if (unit >= units) return;
+    if (lane == 0) next = atomicAdd(a.counter, 1u);   // used in the next turn
+    const WorkItem item = a.items[first + unit / kWarps];
+    const int band = (int)(unit % kWarps);
+    const int row0 = band * WS::kBand;
+    for (int i = lane; i < kBandCells; i += 32) sm.acc[i] = double2{};
+    bool any = false;
+    uint32_t span = kSpanNone;
+    Record<double> rec;
+    auto fetch = [&](int i) {
+      span = kSpanNone;
+      if (i + lane < item.rec_end) {
+        span = a.spans[i + lane];
+        rec = a.recs[i + lane];
+      }
+    };
+    fetch(item.rec_begin);
+    for (int i0 = item.rec_begin; i0 < item.rec_end; i0 += 32) {
+      // The lane's record, clipped to the band and the tile.
+      const int s = (int)((rec.d.y >> 16) & 0x3FFFu);
+      const bool mu = (rec.d.y & kMirrorU) != 0u;
+      const int z = (int)(short)(rec.d.y & 0xFFFFu);
+      const int gu = mu ? z - s : s - z;
+      const int c0 = max(gu - s, 0), c1 = min(gu + s, TW - 1);
+      const uint32_t g0 = (uint32_t)(band * WS::kLanesY);
+      const bool hit = (int)((span >> 5) & 31u) >= (int)g0 &&
+                       (int)(span & 31u) < (int)g0 + WS::kLanesY && c0 <= c1;
+      const uint32_t b = __ballot_sync(0xffffffffu, hit);
+      if (hit) {
+        const int step = slice_step(rec.d);
+        const int r0 = max(rec.row0 - row0, 0);
+        const int r1 = min(rec.row1 - row0, WS::kBand - 1);
+        Queued64 q;
+        q.w = c1 - c0 + 1;
+        q.n = q.w * (r1 - r0 + 1);
+        q.inv_w = 1.0f / (float)q.w;
+        q.su = mu ? -1 : 1;
+        q.step = step;
+        q.cell = r0 * TW + c0;
+        q.x = rec.d.x +
+              (uint32_t)((row0 + r0) * step + (mu ? z - c0 : z + c0));
+        const bool conj = (span & kSpanConj) != 0u;
+        q.a = rec.v.x;
+        q.c = rec.v.y;
+        q.d = conj ? -rec.v.x : rec.v.x;
+        q.b = conj ? rec.v.y : -rec.v.y;
+        sm.queue[__popc(b & ((1u << lane) - 1u))] = q;
+      }
+      const int count = __popc(b);
+      any |= count > 0;
+      if (i0 + 32 < item.rec_end) fetch(i0 + 32);
+      __syncwarp();
+      for (int k = 0; k < count; ++k) {
+        const Queued64& q = sm.queue[k];
+        const int n = q.n, w = q.w, step = q.step, su = q.su;
+        const uint32_t x = q.x;
+        const float inv_w = q.inv_w;
+        const double ca = q.a, cb = q.b, cc = q.c, cd = q.d;
+        double2* const acc = sm.acc + q.cell;
+        // Up to eight of the lane's cells at a time: their taps' loads
+        // overlap.
+        for (int i = lane; i < n; i += 32 * kAhead) {
+          double2 t[kAhead];
+          int at[kAhead];
+#pragma unroll
+          for (int j = 0; j < kAhead; ++j) {
+            const int e = i + 32 * j;
+            const int row = (int)(((float)e + 0.5f) * inv_w);
+            const int col = e - row * w;
+            at[j] = row * TW + col;
+            t[j] = double2{};
+            if (e < n)
+              t[j] = ld_tap(stack + (x + (uint32_t)(row * step + su * col)));
+          }
+#pragma unroll
+          for (int j = 0; j < kAhead; ++j) {
+            if (i + 32 * j >= n) break;
+            double2 v = acc[at[j]];
+            v.x = fma(cb, t[j].y, fma(ca, t[j].x, v.x));
+            v.y = fma(cd, t[j].y, fma(cc, t[j].x, v.y));
+            acc[at[j]] = v;
+          }
+        }
+        __syncwarp();   // the next record may add to these cells
+      }
+    }
+    __syncwarp();
+    // An owned band that no record meets: as in k_grid_tiles.
+    if (!any && item.slot < 0 && !a.tile_groups) continue;
+    const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
+    const int rt = item.tile % a.geom.tiles_total;   // real tile
+    const int gi = rt / tiles_per_grid;
+    const int tl = rt - gi * tiles_per_grid;
+    const int vg = item.tile / a.geom.tiles_total;   // virtual group
+    const int u0 =
+        (tl % a.geom.tiles_u) * WS::kTileU - phase_shift(a.geom, vg);
+    const int v0 = (tl / a.geom.tiles_u) * WS::kTileV + row0;
+    for (int i = lane; i < kBandCells; i += 32) {
+      const double2 out = sm.acc[i];
+      const int r = i / TW, c = i % TW;
+      if (item.slot < 0) {
+        const int col = u0 + c, row = v0 + r;
+        if (row >= a.grid_size || (unsigned)col >= (unsigned)a.grid_size)
+          continue;
+        double2 *src, *dst;
+        cell_ends<double2>(a.tile_groups, a.geom, tl / a.geom.tiles_u, col,
+                           vg,
+                           (double2*)(a.grid + (long long)gi * a.grid_stride),
+                           (double2*)a.host, src, dst);
+        const size_t off = (size_t)row * a.grid_size + col;
+        double2 old = __ldcs(src + off);
+        old.x += out.x;
+        old.y += out.y;
+        __stcs(dst + off, old);
+      } else {
+        // Partial tile entry of band row r, column c (see BandCell).
+        const int e = r % kRows * kConsumers + r / kRows * TW + c;
+        __stcs(a.partials + (size_t)item.slot * kCells + band * 32 + e, out);
+      }
+    }
+    __syncwarp();   // acc is free for the next unit
   }
 }
 
@@ -826,8 +999,13 @@ __global__ void k_item_emit(const uint32_t* __restrict__ tile_start,
 template <typename Real, int TW, bool kWide>
 cudaError_t prepare_grid_kernel(void** fn, size_t* smem) {
   static std::atomic<unsigned long long> opted_in{0};
-  *fn = (void*)k_grid_tiles<Real, TW, kWide>;
-  *smem = kGridWarps * sizeof(WarpSmem<Real, TW>);
+  if constexpr (sizeof(Real) == 4) {
+    *fn = (void*)k_grid_tiles<TW, kWide>;
+    *smem = kGridWarps * sizeof(WarpSmem<TW>);
+  } else {
+    *fn = (void*)k_grid_tiles_f64<TW>;
+    *smem = kGridWarps * sizeof(WarpSmem64);
+  }
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -849,8 +1027,10 @@ cudaError_t prepare_grid_kernel_of(int tile_u, void** fn, size_t* smem) {
 template <typename Real>
 cudaError_t prepare_grid_kernel_for(int tile_u, bool wide, void** fn,
                                     size_t* smem) {
-  return wide ? prepare_grid_kernel_of<Real, true>(tile_u, fn, smem)
-              : prepare_grid_kernel_of<Real, false>(tile_u, fn, smem);
+  return wide && sizeof(Real) == 4
+             ? prepare_grid_kernel_of<Real, sizeof(Real) == 4>(tile_u, fn,
+                                                               smem)
+             : prepare_grid_kernel_of<Real, false>(tile_u, fn, smem);
 }
 
 }  // namespace
