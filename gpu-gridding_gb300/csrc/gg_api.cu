@@ -1025,16 +1025,63 @@ struct Bins {
   TileGeom geom{};
   const uint32_t* keys = nullptr;
   const uint32_t* vals = nullptr;
+  int low_bits = 0;                  // key bits below the tile
+  const int* tile_order = nullptr;   // degridding: tile_queue_order's
 };
+
+// Queue order of the tiles of one group: grid by grid, and within a grid by
+// the distance of the tile's centre from the uv origin (the grid centre),
+// nearest first.  On telescope data the w-plane of a visibility grows with
+// its baseline, so tiles at the same distance use similar planes and the
+// CTAs running at one time share more kernel slices in L2; the heavy
+// central tiles also start first.  *rank (if asked for): each tile's place in
+// that order.  Uploaded when the geometry changes.
+int tile_queue_order(gg_plan* plan, const TileGeom& g, int grid_size,
+                     cudaStream_t s, const int** out, const int** rank = nullptr) {
+  const int key[5] = {grid_size, g.tile_u, g.tile_v, g.num_grids,
+                      plan->queue_order};
+  if (!std::equal(key, key + 5, plan->to_key) ||
+      (int)plan->h_tile_order.size() != 2 * g.tiles_total) {
+    const int tpg = g.tiles_u * g.tiles_v;
+    std::vector<long long> r2(g.tiles_total);
+    for (int l = 0; l < g.tiles_total; ++l) {
+      const int tl = l % tpg;
+      const long long du =
+          (long long)(tl % g.tiles_u) * g.tile_u + g.tile_u / 2 - grid_size / 2;
+      const long long dv =
+          (long long)(tl / g.tiles_u) * g.tile_v + g.tile_v / 2 - grid_size / 2;
+      r2[l] = plan->queue_order == 1 ? l : du * du + dv * dv;
+    }
+    std::vector<int>& ord = plan->h_tile_order;
+    ord.resize(2 * (size_t)g.tiles_total);
+    const auto end = ord.begin() + g.tiles_total;
+    for (int l = 0; l < g.tiles_total; ++l) ord[l] = l;
+    std::stable_sort(ord.begin(), end, [&](int a, int b) {
+      const int ga = a / tpg, gb = b / tpg;
+      return ga != gb ? ga < gb : r2[a] < r2[b];
+    });
+    for (int l = 0; l < g.tiles_total; ++l) end[ord[l]] = l;
+    GG_TRY(plan->tile_order.ensure(ord.size() * sizeof(int)));
+    GG_CUDA(cudaMemcpyAsync(plan->tile_order.p, ord.data(),
+                            ord.size() * sizeof(int), cudaMemcpyHostToDevice,
+                            s));
+    std::copy(key, key + 5, plan->to_key);
+  }
+  *out = plan->tile_order.as<int>();
+  if (rank) *rank = *out + g.tiles_total;
+  return GG_OK;
+}
 
 // After the host has read back the record total and the tile shape: plane
 // groups, tile geometry, record emission, the sort and the tile bounds.
 // Batched calls pass the device array of per-grid visibility offsets.
+// Degridding (degrid): the records are sorted by their tiles' places in the
+// queue order instead, no tile bounds, and `points` is filled.
 template <typename Real>
 int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
                 const PlaceOut& po, int grid_size, int num_grids,
                 const unsigned long long* d_grid_offsets, cudaStream_t s,
-                Bins* b) {
+                Bins* b, bool degrid = false) {
   const StackView view = K->view();
   if (plan->h_scalars[kDeviceError])
     return set_error(GG_ERR_CUDA,
@@ -1117,7 +1164,14 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   b->num_tiles = num_tiles;
   b->grid_size = grid_size;
   b->geom = geom;
+  b->low_bits = low_bits;
   if (total == 0) return GG_OK;
+  const int* tile_rank = nullptr;
+  if (degrid) {
+    GG_TRY(tile_queue_order(plan, geom, grid_size, s, &b->tile_order,
+                            &tile_rank));
+    GG_TRY(plan->placed.ensure(n * 16));
+  }
 
   // The sorted values stay with the plan (replays read them); the keys,
   // the values' other side and the sort scratch are transient and, for a
@@ -1136,7 +1190,8 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
                               T->rec_offset.as<uint32_t>(), n, view, geom,
                               0, 0, T->keys0.as<uint32_t>(),
                               v0.as<uint32_t>(), s, d_grid_offsets,
-                              num_grids));
+                              num_grids, tile_rank,
+                              degrid ? plan->placed.p : nullptr));
   bool in_alt = false;
   GG_CUDA(radix_sort_pairs(T->keys0.as<uint32_t>(), v0.as<uint32_t>(),
                            T->keys1.as<uint32_t>(), v1.as<uint32_t>(), total,
@@ -1147,6 +1202,7 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   b->vals = in_alt ? v1.as<uint32_t>() : v0.as<uint32_t>();
   plan->stats.num_launches += 1 + radix_launches(total, key_bits);
   plan->mark(2, s);
+  if (degrid) return GG_OK;
 
   GG_TRY(plan->tile_start.ensure((size_t)(num_tiles + 1) * 4));
   GG_CUDA(launch_tile_bounds(b->keys, total, low_bits, num_tiles,
@@ -1155,52 +1211,11 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   return GG_OK;
 }
 
-// Queue order of the tiles of one group: grid by grid, and within a grid by
-// the distance of the tile's centre from the uv origin (the grid centre),
-// nearest first.  On telescope data the w-plane of a visibility grows with
-// its baseline, so tiles at the same distance use similar planes and the
-// CTAs running at one time share more kernel slices in L2; the heavy
-// central tiles also start first.  Uploaded when the geometry changes.
-int tile_queue_order(gg_plan* plan, const TileGeom& g, int grid_size,
-                     cudaStream_t s, const int** out) {
-  const int key[5] = {grid_size, g.tile_u, g.tile_v, g.num_grids,
-                      plan->queue_order};
-  if (!std::equal(key, key + 5, plan->to_key) ||
-      (int)plan->h_tile_order.size() != g.tiles_total) {
-    const int tpg = g.tiles_u * g.tiles_v;
-    std::vector<long long> r2(g.tiles_total);
-    for (int l = 0; l < g.tiles_total; ++l) {
-      const int tl = l % tpg;
-      const long long du =
-          (long long)(tl % g.tiles_u) * g.tile_u + g.tile_u / 2 - grid_size / 2;
-      const long long dv =
-          (long long)(tl / g.tiles_u) * g.tile_v + g.tile_v / 2 - grid_size / 2;
-      r2[l] = plan->queue_order == 1 ? l : du * du + dv * dv;
-    }
-    std::vector<int>& ord = plan->h_tile_order;
-    ord.resize(g.tiles_total);
-    for (int l = 0; l < g.tiles_total; ++l) ord[l] = l;
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
-      const int ga = a / tpg, gb = b / tpg;
-      return ga != gb ? ga < gb : r2[a] < r2[b];
-    });
-    GG_TRY(plan->tile_order.ensure(ord.size() * sizeof(int)));
-    GG_CUDA(cudaMemcpyAsync(plan->tile_order.p, ord.data(),
-                            ord.size() * sizeof(int), cudaMemcpyHostToDevice,
-                            s));
-    std::copy(key, key + 5, plan->to_key);
-  }
-  *out = plan->tile_order.as<int>();
-  return GG_OK;
-}
-
-// The work-item queue of binned records for num_ctas persistent CTAs (the
-// gridding kernel: teams of as many warps as a tile has bands): heavy
-// tiles are split into items of `chunk` records so that each of the call's
-// `passes` launches has about items_per_cta items per CTA (the gridding
-// passes of the groups; the degridder's single launch asks for as many
-// items as all of them).  Gridding chunks shorter than 1024 records are
-// made longer, up to half a CTA's share: below that the partial tiles cost
+// The work-item queue of binned records for num_ctas teams of as many
+// resident warps as a tile has bands: heavy tiles are split into items of
+// `chunk` records so that each of the call's `passes` launches has about
+// items_per_cta items per team.  Chunks shorter than 1024 records are made
+// longer, up to half a team's share: below that the partial tiles cost
 // more than the better balance gives (2048^2, 2e5 points, 6.6e5 records:
 // 0.69 ms with chunks of 434, 0.60 with 867).  FP64 gridding takes twice the
 // items and no such minimum: a record costs it four times as much, a unit's
@@ -1208,23 +1223,21 @@ int tile_queue_order(gg_plan* plan, const TileGeom& g, int grid_size,
 // 2.35 with 271, 2.34 with 136).  Items: at most one
 // more per tile than
 // total / chunk; partial-tile slots (split tiles only): at most
-// 2 * total / chunk, each a tile of partial sums when partial_tiles is set
-// (gridding; the degridder's items write no tile).
+// 2 * total / chunk, each a tile of partial sums.
 template <typename Real>
 int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
-                     bool partial_tiles, cudaStream_t s, ItemBuffers* ib,
-                     int launch_span = 1) {
+                     cudaStream_t s, ItemBuffers* ib, int launch_span = 1) {
   using R2 = typename Vec2<Real>::type;
   uint32_t* sc = plan->scalars.as<uint32_t>();
   const int num_tiles = b.num_tiles;
   // items_per_cta items per CTA in each of the call's passes: every pass
   // ends with a tail up to one item long.
-  const bool grid64 = partial_tiles && sizeof(Real) == 8;
+  const bool grid64 = sizeof(Real) == 8;
   const unsigned long long f = (unsigned long long)plan->items_per_cta *
                                (unsigned long long)passes * (grid64 ? 2 : 1);
   unsigned long long records =
       ((unsigned long long)b.total + f * num_ctas - 1) / (f * num_ctas);
-  if (partial_tiles && !grid64)
+  if (!grid64)
     records = std::max(records,
                        std::min(1024ull, (unsigned long long)b.total /
                                              (2ull * passes * num_ctas)));
@@ -1242,8 +1255,8 @@ int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
   // Gridding launches that take all the tile phases of a plane group
   // (launch_span = tile_phases): every tile of a later phase writes partial
   // tiles, as many as the scans count (read back below).
-  const int pphases = partial_tiles && launch_span > 1 ? launch_span : 1;
-  if (partial_tiles && pphases == 1)
+  const int pphases = std::max(launch_span, 1);
+  if (pphases == 1)
     GG_TRY(plan->partials.ensure(slot_cap * b.geom.tile_u * b.geom.tile_v *
                                  sizeof(R2)));
   GG_TRY(plan->group_items.ensure((size_t)(b.num_groups + 1) * 4));
@@ -1342,7 +1355,7 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   // larger items leave longer tails).
   const int span = geom.tile_phases;
   GG_TRY(build_work_items<Real>(plan, b, grid_teams(num_ctas),
-                                geom.num_groups, true, s, &ib, span));
+                                geom.num_groups, s, &ib, span));
   plan->stats.num_ctas = num_ctas;
   plan->kept.group_span = span;
   plan->kept.rec_vis = b.vals;
@@ -1733,7 +1746,7 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
   if (dev != K->device || dev != plan->device)
     return set_error(GG_ERR_INVALID_ARG,
                      "plan, kernel stack and current device differ");
-  // The gridder's placement, records and work items (32 x 64-cell tiles;
+  // The gridder's placement and records (32 x 64-cell tiles;
   // geometry kept for a batched replay is discarded), then the tile
   // kernel and the per-visibility sums.
   plan->stats = gg_stats{};
@@ -1748,7 +1761,8 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
   GG_TRY(place_and_count<Real>(plan, K, pp, kDegridShape, nullptr, nullptr, s,
                                &po));
   Bins b;
-  GG_TRY(bin_records<Real>(plan, K, n, po, grid_size, 1, nullptr, s, &b));
+  GG_TRY(bin_records<Real>(plan, K, n, po, grid_size, 1, nullptr, s, &b,
+                           true));
   if (b.total == 0) {
     GG_CUDA(cudaMemsetAsync(d_out, 0, 2 * n * sizeof(Real), s));
     return GG_OK;
@@ -1762,19 +1776,15 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
   int per_sm = degrid_tiles_ctas_per_sm<Real>(view.wide);
   if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
   const int num_ctas = sms * per_sm;
-  ItemBuffers ib;
-  // One launch over the queue of all plane groups, as many items as the
-  // gridding's passes together.
-  GG_TRY(build_work_items<Real>(plan, b, num_ctas, b.num_groups, false, s,
-                                &ib));
+  plan->stats.num_ctas = num_ctas;
   GG_TRY(plan->rec_out.ensure((size_t)b.total * 2 * sizeof(Real)));
   uint32_t* sc = plan->scalars.as<uint32_t>();
   if (plan->grid_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->grid_wait, 0));
   if (plan->stack_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->stack_wait, 0));
   GG_CUDA(launch_degrid_tiles<Real>(
-      ib.items, ib.num_items, ib.counter, sc + kDeviceError, b.vals, po.cell,
-      po.meta, plan->rec_offset.as<uint32_t>(), view, b.geom, grid_size,
-      d_grid, plan->rec_out.p, num_ctas, s));
+      b.keys, b.vals, b.total, b.low_bits, b.tile_order, plan->placed.p,
+      sc + kCounter, view, b.geom, grid_size, d_grid, plan->rec_out.p,
+      num_ctas, s));
   GG_CUDA(launch_degrid_finish<Real>(po.rec_count,
                                      plan->rec_offset.as<uint32_t>(),
                                      plan->rec_out.p, n, d_out, s));

@@ -6,25 +6,33 @@
 //   out_i = sum over the footprint of conj(c~_i(cell)) * grid(cell).
 //
 // It runs on the gridder's records: after placement, emission and the sort,
-// each 32 x 64-cell tile's (visibility, tile) records are contiguous, and a
-// persistent CTA takes work items (a tile and a range of its records) from
-// the gridder's queue.  Its eight consumer warps hold the tile's grid
-// values in registers (lane = column, kRows rows per lane, as in the
-// gridder) and, for every record whose footprint meets their rows, multiply
-// them by the record's taps and sum across the warp by
-// shuffles.  The producer warp gathers and prepares the records and, once
-// the consumers are done with a buffer, adds each record's warp sums in warp
-// order and stores the record's partial result at its emission slot
-// (rec_offset[visibility] + its tile's rank among the visibility's tiles).
+// each 32 x 64-cell tile's (visibility, tile) records are contiguous, tiles in
+// queue order.  Every warp works by itself: it takes a unit of up to 128
+// consecutive records, prepares them in its shared memory, and goes through
+// the tile's eight bands with the band's grid values in registers (lane =
+// column, kRows rows per lane, as in the gridder): for each record that meets
+// the band it multiplies them by the record's taps, sums over the warp and
+// adds that to the record's sum.  Each record's sum goes to its emission slot
+// (rec_offset[visibility] + its tile's rank among the visibility's tiles);
 // k_degrid_finish then adds each visibility's partial results in emission
-// order.  Nothing is accumulated with atomics, so the result does
-// not depend on scheduling.  With tile phases (see gg_grid.cu) a
-// visibility's records are on its phase's tiles; the degridder only reads
-// the grid, so the tiles of all phases share its one launch.
+// order.  Nothing is accumulated with atomics, and a record's sums are formed
+// alike whatever unit it is in, so the result does not depend on scheduling.
+// With tile phases (see gg_grid.cu) a visibility's records are on its phase's
+// tiles; the degridder only reads the grid, so the tiles of all phases share
+// its one launch.
+//
+// What bounds it: the instructions issued, some 100 a record and band (issue
+// slots 65 % in use, the L1 data pipe 52 %), of which the sum over the warp
+// is a dozen.  In FP64 the FP64 pipe (16 cycles of the SM for a warp's FMA).
+// Calls in ms, with a block of eight band warps and a producer sharing a
+// stream of records -> warps of their own: 2e5 points on 2048^2 0.513 ->
+// 0.467; 7.8e6 track points on 8192^2 (support 4 to 72) 7.9 -> 6.8; the
+// former in FP64 5.4 -> 2.9 (the multiply-adds alone 1.7).
 //
 // The reference has no degridder; this one is pinned by the dot-product
 // identity <G x, y> = <x, G^H y> against the forward kernel and by the FP64
 // oracle.
+#include <algorithm>
 #include <atomic>
 
 #include "gg_internal.h"
@@ -36,17 +44,50 @@ namespace {
 
 constexpr int kDegridTileU = 32;
 using DegridShape = WarpShape<kDegridTileU>;
+constexpr int kDegridWarps = 4;    // per block
+constexpr int kDegridThreads = kDegridWarps * 32;
+constexpr int kUnit = 128;         // records of a unit, at most
+constexpr int kPerLane = kUnit / 32;
+// A unit with fewer records a tile than this takes its records' grid values
+// one by one: tile by tile, each band would wait out a memory latency for a
+// record or two.  2e5 points on 2048^2: 0.485 ms so, 0.53 tile by tile; 3, 6
+// and 12 records a tile as the line measure the same within 1 %.
+constexpr int kSparse = 6;
+constexpr uint32_t kConj = 1u << 31;
+
+// The records are cut into units of 128, then (from record `begin64` on) of
+// 64, then (from `begin32` on) of 32, two of 32 and four of 64 a warp: a
+// launch ends with units that are short for the warps that still have one
+// (2e5 points on 2048^2, 6.6e5 records: 0.47 ms, half as many
+// short units 0.475 to 0.48, none of 32 0.50; 1.5e7 records: no difference).
+struct DegridUnits {
+  uint32_t total;              // records
+  uint32_t begin64, begin32;   // multiples of 128
+};
+__device__ __forceinline__ uint2 degrid_unit(const DegridUnits& c,
+                                             uint32_t unit) {
+  const uint32_t n128 = c.begin64 / 128, n64 = (c.begin32 - c.begin64) / 64;
+  uint32_t b, n;
+  if (unit < n128) {
+    b = unit * 128; n = 128;
+  } else if (unit - n128 < n64) {
+    b = c.begin64 + (unit - n128) * 64; n = 64;
+  } else {
+    b = c.begin32 + (unit - n128 - n64) * 32; n = 32;
+  }
+  return make_uint2(b, min(b + n, c.total));
+}
 
 template <typename Real>
 struct DegridArgs {
-  const WorkItem* items;
-  const uint32_t* num_items;  // queue length (device scalar)
+  DegridUnits cut;
+  uint32_t num_units;
   uint32_t* counter;
-  uint32_t* error;            // set to 1 when a bounded wait runs out
-  const uint32_t* rec_vis;    // sorted records: visibility index
-  const uint32_t* cell;
-  const uint32_t* meta;
-  const uint32_t* rec_offset; // first emission slot of each visibility
+  const uint32_t* rec_key;    // sorted records: keys (tile << low_bits | ...)
+  const uint32_t* rec_vis;    // and visibility indices
+  int low_bits;
+  const int* tile_order;      // tile at each place of the queue order
+  const uint4* points;        // per visibility: cell, meta, emission slot
   StackView view;
   TileGeom geom;
   int grid_size;
@@ -54,288 +95,338 @@ struct DegridArgs {
   typename Vec2<Real>::type* rec_out;  // partial result per emission slot
 };
 
-// Shared-memory layout of one CTA (dynamic shared memory).
+// Shared memory of one warp.  A record's int4: the tap index of the footprint
+// centre's column in the slice row of tile row 0; conjugated << 31 | columns
+// mirrored << 30 | the centre's tile column (16 bits); support + 1; taps from
+// one tile row to the next.  Record kUnit adds nothing.
 template <typename Real>
-struct DegridSmem {
+struct DegridWarp {
   using R2 = typename Vec2<Real>::type;
-  R2 part[kRing][kBuf][kWarps];  // consumer warp w's sum of record t
-  uint2 rec[kRing][kBuf];        // slice_record descriptors
-  uint32_t band[kRing][kBuf];    // bit w: the footprint meets warp w's rows
-  uint32_t out[kRing][kBuf];     // emission slot | conjugated << 31
-  int4 head[kRing];              // item, records (-1: no more work), flags
-  uint64_t full[kRing];
-  uint64_t empty[kRing];
+  int4 rec[kUnit + 1];
+  R2 sum[kUnit];
+  uint32_t out[kUnit];          // emission slot
+  int2 origin[kUnit + 1];       // grid column and row of the tile's first cell
+  // FP32: the tile's place, the bands it meets (first | last << 8), and the
+  // records that meet a band with fillers up to a multiple of four.
+  uint32_t tile[kUnit];
+  unsigned short span[kUnit];
+  alignas(4) unsigned char queue[kUnit + 4];
+  short row0[kUnit];            // FP64: the footprint's first tile row
 };
 
-// The producer warp: takes work items from the queue, streams their records
-// through the ring and stores each finished buffer's per-record results.
-// Returns false if a wait ran out.
+// v[2 j + c] summed over the warp for c = 0, 1 of the four records j: the
+// lane's result is that of j = lane >> 3, c = (lane >> 2) & 1.  Halving the
+// values a lane holds at each of the first three steps takes 9 shuffles
+// where a tree per value takes 40.
 template <typename Real>
-__device__ bool degrid_produce(const DegridArgs<Real>& a,
-                               DegridSmem<Real>& sm) {
-  using R2 = typename Vec2<Real>::type;
-  const int lane = threadIdx.x & 31;
-  const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
-  const int end_item = (int)*a.num_items;
-  // Buffer kb is done: add each record's warp sums (the warps its band bits
-  // name, in warp order) and store them at the record's emission slot.
-  auto flush = [&](unsigned kb) {
-    const int slot = (int)(kb % kRing);
-    const int nb = sm.head[slot].y;
-    for (int t = lane; t < nb; t += 32) {
-      const uint32_t band = sm.band[slot][t];
-      R2 acc;
-      acc.x = 0;
-      acc.y = 0;
+__device__ __forceinline__ Real warp_sum_4x2(const Real (&v)[8], int lane) {
+  Real a[4], b[2];
 #pragma unroll
-      for (int w = 0; w < kWarps; ++w) {
-        if (band & (1u << w)) {
-          acc.x += sm.part[slot][t][w].x;
-          acc.y += sm.part[slot][t][w].y;
-        }
-      }
-      a.rec_out[sm.out[slot][t] & 0x7FFFFFFFu] = acc;
-    }
-  };
-  unsigned k = 0;
-  bool done = false;
-  while (!done) {
-    int it = 0;
-    if (lane == 0) it = (int)atomicAdd(a.counter, 1u);
-    it = __shfl_sync(0xffffffffu, it, 0);
-    done = it >= end_item;
-    WorkItem item{0, 0, 0, -1};
-    int tu = 0, tv = 0, sh = 0;
-    if (!done) {
-      item = a.items[it];
-      const int tl = (item.tile % a.geom.tiles_total) % tiles_per_grid;
-      tu = tl % a.geom.tiles_u;
-      tv = tl / a.geom.tiles_u;
-      sh = phase_shift(a.geom, item.tile / a.geom.tiles_total);
-    }
-    const int u0 = tu * DegridShape::kTileU - sh;
-    const int v0 = tv * DegridShape::kTileV;
-    int b0 = item.rec_begin;
-    do {
-      const int slot = (int)(k % kRing);
-      const unsigned use = k / kRing;
-      if (use > 0) {
-        if (!mbar_wait(&sm.empty[slot], (use - 1) & 1)) return false;
-        flush(k - kRing);
-      }
-      int nb = -1;
-      if (!done) {
-        nb = min(kBuf, item.rec_end - b0);
-        uint32_t vid[kPerLane], ce[kPerLane], me[kPerLane], off[kPerLane];
-#pragma unroll
-        for (int q = 0; q < kPerLane; ++q) {
-          const int t = q * 32 + lane;
-          vid[q] = t < nb ? a.rec_vis[b0 + t] : 0u;
-        }
-#pragma unroll
-        for (int q = 0; q < kPerLane; ++q) {
-          const int t = q * 32 + lane;
-          ce[q] = 0; me[q] = 0; off[q] = 0;
-          if (t < nb) {
-            ce[q] = a.cell[vid[q]];
-            me[q] = a.meta[vid[q]];
-            off[q] = a.rec_offset[vid[q]];
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < kPerLane; ++q) {
-          const int t = q * 32 + lane;
-          if (t < nb) {
-            const uint32_t m = me[q];
-            const SlicePlane plane = a.view.planes[meta_plane(m)];
-            const int s = plane.support;
-            const int gu = cell_u(ce[q]), gv = cell_v(ce[q]);
-            const int ou = meta_ou(m), ov = meta_ov(m);
-            sm.rec[slot][t] = slice_record(
-                slice_origin(plane, a.view.omax, abs(ou), abs(ov)),
-                s, ou, ov, gu - u0, gv - v0);
-            uint32_t band = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) {
-              const int r0 = v0 + w * kRows;
-              if (gv - s <= r0 + kRows - 1 && gv + s >= r0) band |= 1u << w;
-            }
-            sm.band[slot][t] = band;
-            // Rank of this tile among the visibility's tiles, in the order
-            // k_emit writes them (tile rows outer, tile columns inner, on
-            // the visibility's tile phase).
-            const int tu0 = (gu - s + sh) / DegridShape::kTileU;
-            const int tu1 = (gu + s + sh) / DegridShape::kTileU;
-            const int tv0 = (gv - s) / DegridShape::kTileV;
-            const uint32_t rank =
-                (uint32_t)((tv - tv0) * (tu1 - tu0 + 1) + (tu - tu0));
-            sm.out[slot][t] = (off[q] + rank) |
-                              (meta_conj(m) ? 0x80000000u : 0u);
-          }
-        }
-      }
-      if (lane == 0) {
-        const int flags = done ? 0 : ((b0 == item.rec_begin ? 1 : 0) |
-                                      (b0 + kBuf >= item.rec_end ? 2 : 0));
-        sm.head[slot] = make_int4(it, nb, flags, 0);
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.full[slot]);
-      ++k;
-      b0 += kBuf;
-    } while (!done && b0 < item.rec_end);
+  for (int j = 0; j < 4; ++j) {
+    const bool up = (lane & 16) != 0;
+    a[j] = up ? v[j + 4] : v[j];
+    a[j] += __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + 4], 16);
   }
-  // Buffer k - 1 is the end marker; the kRing - 1 data buffers before it
-  // have not been reused, so their results are still to be stored.
-  for (unsigned kb = k >= kRing ? k - kRing : 0u; kb + 2 <= k; ++kb) {
-    if (!mbar_wait(&sm.empty[kb % kRing], (kb / kRing) & 1)) return false;
-    flush(kb);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const bool up = (lane & 8) != 0;
+    b[j] = up ? a[j + 2] : a[j];
+    b[j] += __shfl_xor_sync(0xffffffffu, up ? a[j] : a[j + 2], 8);
   }
-  return true;
+  const bool up = (lane & 4) != 0;
+  Real r = up ? b[1] : b[0];
+  r += __shfl_xor_sync(0xffffffffu, up ? b[0] : b[1], 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  return r;
 }
 
-// This lane's share of conj(c~) * g over its kRows cells, with
-// gx[r] = (g.re, g.re) and gy[r] = (g.im, g.im): P = sum t * g.re and
-// Q = sum t * g.im componentwise, so with c~ = (t.re, sgn * t.im)
-//   re = P.x + sgn * Q.y,  im = Q.x - sgn * P.y.
-template <typename R2, typename Real>
-__device__ __forceinline__ void dot_record(const R2 (&t)[kRows],
-                                           const R2 (&gx)[kRows],
-                                           const R2 (&gy)[kRows], Real sgn,
-                                           Real& re, Real& im) {
-  R2 P, Q;
-  P.x = P.y = Q.x = Q.y = 0;
+// This lane's share of conj(c~) * g over its kRows cells, with g = (re, im)
+// and gs = (im, re): X = sum (t.re g.re, t.im g.im) and Y = sum (t.re g.im,
+// t.im g.re), so with c~ = (t.re, sgn * t.im)
+//   re = X.x + sgn * X.y,  im = Y.x - sgn * Y.y.
+__device__ __forceinline__ void dot_record(const float2 (&t)[kRows],
+                                           const float2 (&g)[kRows],
+                                           const float2 (&gs)[kRows],
+                                           int flags, float& re, float& im) {
+  float2 X{}, Y{};
 #pragma unroll
   for (int r = 0; r < kRows; ++r) {
-    P = fma2(t[r], gx[r], P);
-    Q = fma2(t[r], gy[r], Q);
+    X = fma2(t[r], g[r], X);
+    Y = fma2(t[r], gs[r], Y);
   }
-  re = P.x + sgn * Q.y;
-  im = Q.x - sgn * P.y;
+  const float sgn = __int_as_float(((uint32_t)flags & kConj) | 0x3F800000u);
+  re = fmaf(sgn, X.y, X.x);
+  im = fmaf(-sgn, Y.y, Y.x);
 }
 
 template <typename Real, bool kWide>
-__global__ void __launch_bounds__(kThreads, sizeof(Real) == 4 ? 2 : 1)
+__global__ void __launch_bounds__(kDegridThreads, sizeof(Real) == 4 ? 4 : 3)
 k_degrid_tiles(DegridArgs<Real> a) {
   using R2 = typename Vec2<Real>::type;
-  using SM = DegridSmem<Real>;
+  using SM = DegridWarp<Real>;
+  constexpr bool kPacked = sizeof(Real) == 8;
   extern __shared__ __align__(16) unsigned char g_smem_raw[];
-  SM& sm = *reinterpret_cast<SM*>(g_smem_raw);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kRing; ++i) {
-      mbar_init(&sm.full[i], 1);
-      mbar_init(&sm.empty[i], kWarps);
-    }
-  }
-  __syncthreads();
-  if (warp == kWarps) {
-    if (!degrid_produce<Real>(a, sm)) atomicExch(a.error, 1u);
-    return;
-  }
-
-  const int rowl = warp * kRows;   // this lane's row 0 in the tile
+  const int lane = threadIdx.x & 31;
+  SM& sm = reinterpret_cast<SM*>(g_smem_raw)[threadIdx.x >> 5];
   const int G = a.grid_size;
-  const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
   const R2* __restrict__ taps = (const R2*)a.view.taps;
   const R2* __restrict__ grid = (const R2*)a.grid;
-  const uint32_t my_bit = 1u << warp;
-  R2 gx[kRows], gy[kRows];
+  const uint32_t lt = (1u << lane) - 1u;
+  if (lane == 0) {
+    sm.rec[kUnit] = make_int4((int)kStackZero, 0, 0, 0);
+    sm.origin[kUnit] = make_int2(0, 0);
+  }
+  unsigned next = 0;
+  if (lane == 0) next = atomicAdd(a.counter, 1u);
+  for (;;) {
+    const unsigned unit = __shfl_sync(0xffffffffu, next, 0);
+    if (unit >= a.num_units) return;
+    if (lane == 0) next = atomicAdd(a.counter, 1u);   // used in the next turn
+    const uint2 range = degrid_unit(a.cut, unit);
+    const int nb = (int)(range.y - range.x);
+    // Prepare the records.
+    uint4 pt[kPerLane];
+    uint32_t key[kPerLane];
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) gx[r].x = gx[r].y = gy[r].x = gy[r].y = 0;
-
-  // The taps of record t of buffer slot `slot` for this lane's rows.
-  int slot = 0;
-  auto load = [&](int t, R2 (&out)[kRows]) {
-    const uint2 d = sm.rec[slot][t];
-    const int step = slice_step(d);
-    load_taps<kWide>(taps, slice_tap(d, step, lane) + (uint32_t)(rowl * step), step,
-              out);
-  };
-
-  for (unsigned k = 0;; ++k) {
-    slot = (int)(k % kRing);
-    if (!mbar_wait(&sm.full[slot], (k / kRing) & 1)) {
-      atomicExch(a.error, 1u);
-      return;
-    }
-    const int4 head = sm.head[slot];
-    const int nb = head.y;
-    if (nb < 0) break;
-    if (head.z & 1) {  // first buffer of a work item: load its tile
-      const WorkItem item = a.items[head.x];
-      const int tl = (item.tile % a.geom.tiles_total) % tiles_per_grid;
-      // Tiles of later phases start left of phase 0's (and may reach past
-      // either edge of the grid).
-      const int col = (tl % a.geom.tiles_u) * DegridShape::kTileU + lane -
-                      phase_shift(a.geom, item.tile / a.geom.tiles_total);
-      const int row0 = (tl / a.geom.tiles_u) * DegridShape::kTileV + rowl;
-      const bool col_in = (unsigned)col < (unsigned)G;
-#pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        R2 g;
-        g.x = g.y = 0;
-        if (row0 + r < G && col_in) g = grid[(size_t)(row0 + r) * G + col];
-        gx[r].x = gx[r].y = g.x;
-        gy[r].x = gy[r].y = g.y;
+    for (int q = 0; q < kPerLane; ++q) {
+      const int t = q * 32 + lane;
+      if (t < nb) {
+        key[q] = a.rec_key[range.x + t];
+        pt[q] = a.points[a.rec_vis[range.x + t]];
       }
     }
-    for (int c0 = 0; c0 < nb; c0 += 32) {
-      const bool touch =
-          c0 + lane < nb && (sm.band[slot][c0 + lane] & my_bit) != 0u;
-      uint32_t m = __ballot_sync(0xffffffffu, touch);
-      // Two records at a time: 2 * kRows independent tap loads per lane in
-      // flight, and one shuffle tree for the pair.
-      while (m) {
-        const int tA = c0 + __ffs(m) - 1;
-        m &= m - 1;
-        R2 ta[kRows];
-        load(tA, ta);
-        const Real sA = (sm.out[slot][tA] >> 31) ? (Real)-1 : (Real)1;
-        Real reA, imA;
-        if (m) {
-          const int tB = c0 + __ffs(m) - 1;
-          m &= m - 1;
-          R2 tb[kRows];
-          load(tB, tb);
-          const Real sB = (sm.out[slot][tB] >> 31) ? (Real)-1 : (Real)1;
-          Real reB, imB;
-          dot_record(ta, gx, gy, sA, reA, imA);
-          dot_record(tb, gx, gy, sB, reB, imB);
-          // Lanes 0-15 keep record A, lanes 16-31 record B.
-          const bool upper = (lane & 16) != 0;
-          Real kre = upper ? reB : reA, kim = upper ? imB : imA;
-          kre += __shfl_xor_sync(0xffffffffu, upper ? reA : reB, 16);
-          kim += __shfl_xor_sync(0xffffffffu, upper ? imA : imB, 16);
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) {
-            kre += __shfl_xor_sync(0xffffffffu, kre, o);
-            kim += __shfl_xor_sync(0xffffffffu, kim, o);
-          }
-          if ((lane & 15) == 0) {
-            R2 v;
-            v.x = kre;
-            v.y = kim;
-            sm.part[slot][upper ? tB : tA][warp] = v;
-          }
+    for (int q = 0; q < kPerLane; ++q) {
+      const int t = q * 32 + lane;
+      if (t < nb) {
+        const uint32_t tile = a.low_bits >= 32 ? 0u : key[q] >> a.low_bits;
+        const int vg = (int)(tile / (uint32_t)a.geom.tiles_total);
+        const int tl =
+            a.tile_order[tile - (uint32_t)vg * (uint32_t)a.geom.tiles_total];
+        const int tv = tl / a.geom.tiles_u, tu = tl - tv * a.geom.tiles_u;
+        const int sh = phase_shift(a.geom, vg);
+        const int u0 = tu * DegridShape::kTileU - sh;
+        const int v0 = tv * DegridShape::kTileV;
+        const uint32_t m = pt[q].y;
+        const SlicePlane plane = a.view.planes[meta_plane(m)];
+        const int s = plane.support;
+        const int gu = cell_u(pt[q].x), gv = cell_v(pt[q].x);
+        const int ou = meta_ou(m), ov = meta_ov(m);
+        const uint2 d = slice_record(
+            slice_origin(plane, a.view.omax, abs(ou), abs(ov)), s, ou, ov,
+            gu - u0, gv - v0);
+        sm.rec[t] = make_int4(
+            (int)(d.x + (uint32_t)s),
+            (int)(((uint32_t)(gu - u0) & 0xFFFFu) | (d.y & kMirrorU) |
+                  (meta_conj(m) ? kConj : 0u)),
+            s + 1, slice_step(d));
+        sm.origin[t] = make_int2(u0, v0);
+        const int top = gv - s - v0;
+        if constexpr (kPacked) {
+          sm.row0[t] = (short)top;
         } else {
-          dot_record(ta, gx, gy, sA, reA, imA);
+          sm.tile[t] = tile;
+          sm.span[t] = (unsigned short)(
+              (uint32_t)(max(top, 0) / kRows) |
+              (uint32_t)(min(top + 2 * s, DegridShape::kTileV - 1) / kRows)
+                  << 8);
+        }
+        sm.sum[t] = R2{};
+        // Rank of this tile among the visibility's tiles, in the order
+        // k_emit writes them (tile rows outer, tile columns inner, on the
+        // visibility's tile phase).
+        const int tu0 = (gu - s + sh) / DegridShape::kTileU;
+        const int tu1 = (gu + s + sh) / DegridShape::kTileU;
+        const int tv0 = (gv - s) / DegridShape::kTileV;
+        sm.out[t] = pt[q].z +
+                    (uint32_t)((tv - tv0) * (tu1 - tu0 + 1) + (tu - tu0));
+      }
+    }
+    __syncwarp();
+    // Adds the warp sums of the four records named by the bytes of w.
+    auto store = [&](uint32_t w, const Real (&v)[8]) {
+      const Real r = warp_sum_4x2(v, lane);
+      const uint32_t t = w >> (lane >> 3 << 3) & 0xFFu;
+      if ((lane & 3) == 0 && t < kUnit)
+        ((Real*)sm.sum)[2 * t + ((lane >> 2) & 1)] += r;
+    };
+    if constexpr (kPacked) {
+      // As in the FP64 gridder the lanes take a record's cells packed row by
+      // row; the grid values come straight from the grid.
+      constexpr int kAhead = 8;   // cells of a lane in flight
+      for (int t0 = 0; t0 < nb; t0 += 4) {
+        uint32_t word = 0;
+        Real v[8];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            reA += __shfl_xor_sync(0xffffffffu, reA, o);
-            imA += __shfl_xor_sync(0xffffffffu, imA, o);
+        for (int j = 0; j < 4; ++j) {
+          const int t = min(t0 + j, kUnit);
+          word |= (uint32_t)(t < nb ? t : kUnit) << (8 * j);
+          Real re = 0, im = 0;
+          if (t < nb) {
+            const int4 e = sm.rec[t];
+            const int gu = (int)(short)e.y, s = e.z - 1;
+            const int su = e.y & kMirrorU ? -1 : 1;
+            const bool conj = e.y < 0;
+            const int c0 = max(gu - s, 0);
+            const int w = min(gu + s, kDegridTileU - 1) - c0 + 1;
+            const int top = sm.row0[t];
+            const int r0 = max(top, 0);
+            const int n =
+                w * (min(top + 2 * s, DegridShape::kTileV - 1) - r0 + 1);
+            const float inv_w = 1.0f / (float)w;
+            const uint32_t x = (uint32_t)(e.x + r0 * e.w + su * (c0 - gu));
+            const int2 o = sm.origin[t];
+            const R2* const cells = grid + (size_t)(o.y + r0) * G + o.x + c0;
+            for (int k = lane; k < n; k += 32 * kAhead) {
+              R2 tap[kAhead], cell[kAhead];
+#pragma unroll
+              for (int h = 0; h < kAhead; ++h) {
+                const int l = k + 32 * h;
+                const int row = (int)(((float)l + 0.5f) * inv_w);
+                const int c = l - row * w;
+                tap[h] = cell[h] = R2{};
+                if (l < n) {
+                  tap[h] =
+                      ld_tap(taps + (x + (uint32_t)(row * e.w + su * c)));
+                  cell[h] = cells[(size_t)row * G + c];
+                }
+              }
+#pragma unroll
+              for (int h = 0; h < kAhead; ++h) {
+                if (k + 32 * h >= n) break;
+                const Real ti = conj ? -tap[h].y : tap[h].y;
+                re = fma(ti, cell[h].y, fma(tap[h].x, cell[h].x, re));
+                im = fma(-ti, cell[h].x, fma(tap[h].x, cell[h].y, im));
+              }
+            }
           }
-          if (lane == 0) {
-            R2 v;
-            v.x = reA;
-            v.y = imA;
-            sm.part[slot][tA][warp] = v;
+          v[2 * j] = re;
+          v[2 * j + 1] = im;
+        }
+        __syncwarp();
+        store(word, v);
+      }
+    } else {
+      R2 g[kRows], gs[kRows];   // grid values (re, im) and (im, re)
+      int band = 0;
+      auto load_grid = [&](int2 o) {
+        const int row0 = o.y + band * kRows, col = o.x + lane;
+        // Tiles of later phases start left of phase 0's (and may reach past
+        // either edge of the grid).
+        const bool col_in = (unsigned)col < (unsigned)G;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          g[r] = R2{};
+          if (row0 + r < G && col_in) g[r] = grid[(size_t)(row0 + r) * G + col];
+        }
+      };
+      auto swap_grid = [&]() {
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          gs[r].x = g[r].y;
+          gs[r].y = g[r].x;
+        }
+      };
+      auto load = [&](uint32_t t, R2 (&out)[kRows], int& y) {
+        const int4 e = sm.rec[t & 0xFFu];
+        const int c = min(max(lane - (int)(short)e.y, -e.z), e.z);
+        y = e.y;
+        load_taps<kWide>(
+            taps,
+            (uint32_t)(e.x + band * kRows * e.w + (e.y & kMirrorU ? -c : c)), e.w,
+            out);
+      };
+      // Queues the records from `begin` on, of the same tile if `tile` is
+      // set, that meet the band; returns how many, fillers included.
+      auto enqueue = [&](int begin, bool same) {
+        const uint32_t tile = sm.tile[begin];
+        int count = 0;
+        __syncwarp();
+        for (int t = begin + lane; t - lane < nb; t += 32) {
+          const uint32_t span = t < nb ? sm.span[t] : 0xFFu;
+          const bool hit = (int)(span & 0xFFu) <= band &&
+                           (int)(span >> 8) >= band &&
+                           (!same || sm.tile[t] == tile);
+          const uint32_t b = __ballot_sync(0xffffffffu, hit);
+          if (hit) sm.queue[count + __popc(b & lt)] = (unsigned char)t;
+          count += __popc(b);
+        }
+        const int end = (count + 3) & ~3;
+        if (count + lane < end) sm.queue[count + lane] = kUnit;
+        __syncwarp();
+        return end;
+      };
+      const uint32_t* const queue = (const uint32_t*)sm.queue;
+      int tiles = 0;
+      for (int t = lane; t - lane < nb; t += 32)
+        tiles += __popc(__ballot_sync(
+            0xffffffffu,
+            t < nb && (t == 0 || sm.tile[t] != sm.tile[t - 1])));
+      if (tiles * kSparse > nb) {
+        // Few records a tile: band by band over all of them, each with its
+        // own grid values.
+        for (band = 0; band < kWarps; ++band) {
+          const int end = enqueue(0, false);
+          for (int i = 0; i < end; i += 4) {
+            const uint32_t w = queue[i / 4];
+            Real v[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              R2 t[kRows];
+              int y;
+              load(w >> (8 * j), t, y);
+              load_grid(sm.origin[w >> (8 * j) & 0xFFu]);
+              swap_grid();
+              dot_record(t, g, gs, y, v[2 * j], v[2 * j + 1]);
+            }
+            store(w, v);
           }
+        }
+      } else {
+        for (int begin = 0; begin < nb;) {
+          for (band = 0; band < kWarps; ++band) {
+            const int end = enqueue(begin, true);
+            if (end == 0) continue;
+            R2 ta[kRows], tb[kRows];   // two records' taps in flight
+            int ya = 0, yb = 0;
+            uint32_t w = queue[0];
+            load_grid(sm.origin[begin]);
+            load(w, ta, ya);
+            load(w >> 8, tb, yb);
+            swap_grid();
+            for (int i = 4;; i += 4) {
+              const uint32_t wn = i < end ? queue[i / 4] : w;
+              Real v[8];
+              dot_record(ta, g, gs, ya, v[0], v[1]);
+              load(w >> 16, ta, ya);
+              dot_record(tb, g, gs, yb, v[2], v[3]);
+              load(w >> 24, tb, yb);
+              dot_record(ta, g, gs, ya, v[4], v[5]);
+              if (i < end) load(wn, ta, ya);
+              dot_record(tb, g, gs, yb, v[6], v[7]);
+              if (i < end) load(wn >> 8, tb, yb);
+              store(w, v);
+              if (i >= end) break;
+              w = wn;
+            }
+          }
+          const uint32_t tile = sm.tile[begin];
+          int same = 0;
+          for (int t = begin + lane; t - lane < nb; t += 32)
+            same += __popc(__ballot_sync(0xffffffffu,
+                                         t < nb && sm.tile[t] == tile));
+          begin += same;
         }
       }
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.empty[slot]);
+#pragma unroll
+    for (int q = 0; q < kPerLane; ++q) {
+      const int t = q * 32 + lane;
+      if (t < nb) a.rec_out[sm.out[t]] = sm.sum[t];
+    }
+    __syncwarp();
   }
 }
 
@@ -367,7 +458,7 @@ template <typename Real, bool kWide>
 cudaError_t prepare_degrid_kernel(void** fn, size_t* smem) {
   static std::atomic<unsigned long long> opted_in{0};
   *fn = (void*)k_degrid_tiles<Real, kWide>;
-  *smem = sizeof(DegridSmem<Real>);
+  *smem = kDegridWarps * sizeof(DegridWarp<Real>);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -393,31 +484,37 @@ int degrid_tiles_ctas_per_sm(bool wide) {
   size_t smem = 0;
   int n = 0;
   if (prepare_degrid_kernel_for<Real>(wide, &fn, &smem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kThreads, smem) !=
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kDegridThreads,
+                                                    smem) !=
           cudaSuccess)
     n = 1;
   return n < 1 ? 1 : n;
 }
 
 template <typename Real>
-cudaError_t launch_degrid_tiles(const WorkItem* items,
-                                const uint32_t* num_items, uint32_t* counter,
-                                uint32_t* error, const uint32_t* rec_vis,
-                                const uint32_t* cell, const uint32_t* meta,
-                                const uint32_t* rec_offset, StackView view,
-                                TileGeom geom, int grid_size, const Real* grid,
-                                void* rec_out, int num_ctas, cudaStream_t s) {
+cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
+                                const uint32_t* rec_vis, uint32_t total,
+                                int low_bits, const int* tile_order,
+                                const void* points, uint32_t* counter,
+                                StackView view, TileGeom geom, int grid_size,
+                                const Real* grid, void* rec_out, int num_ctas,
+                                cudaStream_t s) {
   if (geom.tile_u != kDegridTileU || geom.tile_v != DegridShape::kTileV)
     return cudaErrorInvalidValue;
   DegridArgs<Real> a;
-  a.items = items;
-  a.num_items = num_items;
+  const uint32_t warps = (uint32_t)num_ctas * kDegridWarps;
+  a.cut.total = total;
+  a.cut.begin32 = (total - std::min(total, 64 * warps)) / 128 * 128;
+  a.cut.begin64 =
+      (a.cut.begin32 - std::min(a.cut.begin32, 256 * warps)) / 128 * 128;
+  a.num_units = a.cut.begin64 / 128 + (a.cut.begin32 - a.cut.begin64) / 64 +
+                (total - a.cut.begin32 + 31) / 32;
   a.counter = counter;
-  a.error = error;
+  a.rec_key = rec_key;
   a.rec_vis = rec_vis;
-  a.cell = cell;
-  a.meta = meta;
-  a.rec_offset = rec_offset;
+  a.low_bits = low_bits;
+  a.tile_order = tile_order;
+  a.points = (const uint4*)points;
   a.view = view;
   a.geom = geom;
   a.grid_size = grid_size;
@@ -430,7 +527,8 @@ cudaError_t launch_degrid_tiles(const WorkItem* items,
   e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
   void* args[] = {&a};
-  return cudaLaunchKernel(fn, dim3(num_ctas), dim3(kThreads), args, smem, s);
+  return cudaLaunchKernel(fn, dim3(num_ctas), dim3(kDegridThreads), args, smem,
+                          s);
 }
 
 template <typename Real>
@@ -447,13 +545,11 @@ cudaError_t launch_degrid_finish(const uint32_t* count, const uint32_t* offset,
 template int degrid_tiles_ctas_per_sm<float>(bool);
 template int degrid_tiles_ctas_per_sm<double>(bool);
 template cudaError_t launch_degrid_tiles<float>(
-    const WorkItem*, const uint32_t*, uint32_t*, uint32_t*, const uint32_t*,
-    const uint32_t*, const uint32_t*, const uint32_t*, StackView, TileGeom,
-    int, const float*, void*, int, cudaStream_t);
+    const uint32_t*, const uint32_t*, uint32_t, int, const int*, const void*,
+    uint32_t*, StackView, TileGeom, int, const float*, void*, int, cudaStream_t);
 template cudaError_t launch_degrid_tiles<double>(
-    const WorkItem*, const uint32_t*, uint32_t*, uint32_t*, const uint32_t*,
-    const uint32_t*, const uint32_t*, const uint32_t*, StackView, TileGeom,
-    int, const double*, void*, int, cudaStream_t);
+    const uint32_t*, const uint32_t*, uint32_t, int, const int*, const void*,
+    uint32_t*, StackView, TileGeom, int, const double*, void*, int, cudaStream_t);
 template cudaError_t launch_degrid_finish<float>(const uint32_t*,
                                                  const uint32_t*, const void*,
                                                  unsigned long long, float*,

@@ -155,9 +155,14 @@ cudaError_t launch_emit_records(const uint32_t* cell, const uint32_t* meta,
                                 uint32_t* vals, cudaStream_t s,
                                 const unsigned long long* grid_offsets =
                                     nullptr,
-                                int num_grids = 1);
+                                int num_grids = 1,
+                                const int* tile_rank = nullptr,
+                                void* points = nullptr);
 // grid_offsets (device, num_grids + 1): batched calls, where visibility i
 // belongs to the grid g with grid_offsets[g] <= i < grid_offsets[g + 1].
+// tile_rank and points (device; degridding): keys hold each tile's
+// tile_rank[tile] in place of its index, and points[i] (16 bytes) becomes
+// visibility i's cell, meta and first emission slot.
 
 // ---- batched calls (gg_batch.cu) ------------------------------------------
 // Per-visibility placement for a batched call: like launch_place, but the
@@ -349,18 +354,20 @@ cudaError_t measure_fp32_fma(int num_sms, double* tflops_best, float* ms_out);
 // Resident CTAs per SM of the degridding kernel.
 template <typename Real>
 int degrid_tiles_ctas_per_sm(bool wide);
-// One persistent launch over the whole work-item queue (32 x 64-cell tiles
-// only): rec_out[rec_offset[v] + rank] = the record's share of
-// conj(tap) * grid for every record, rank = the record's tile among
-// visibility v's tiles in emission order.
+// One persistent launch over all `total` records, sorted by (tile's place in
+// the queue order tile_order, ...) with the tile's place above the keys'
+// low_bits (32 x 64-cell tiles only): rec_out[rec_offset[v] + rank] = the
+// record's share of conj(tap) * grid for every record, rank = the record's
+// tile among visibility v's tiles in emission order; points as
+// launch_emit_records writes them.
 template <typename Real>
-cudaError_t launch_degrid_tiles(const WorkItem* items,
-                                const uint32_t* num_items, uint32_t* counter,
-                                uint32_t* error, const uint32_t* rec_vis,
-                                const uint32_t* cell, const uint32_t* meta,
-                                const uint32_t* rec_offset, StackView view,
-                                TileGeom geom, int grid_size, const Real* grid,
-                                void* rec_out, int num_ctas, cudaStream_t s);
+cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
+                                const uint32_t* rec_vis, uint32_t total,
+                                int low_bits, const int* tile_order,
+                                const void* points, uint32_t* counter,
+                                StackView view, TileGeom geom, int grid_size,
+                                const Real* grid, void* rec_out, int num_ctas,
+                                cudaStream_t s);
 // out[v] = the sum of visibility v's count[v] partial results from
 // rec_out[offset[v]] on, in order.
 template <typename Real>

@@ -217,7 +217,8 @@ __global__ void k_emit(const uint32_t* __restrict__ cell,
                        uint32_t* __restrict__ keys,
                        uint32_t* __restrict__ vals,
                        const unsigned long long* __restrict__ grid_offsets,
-                       int num_grids) {
+                       int num_grids, const int* __restrict__ tile_rank,
+                       uint4* __restrict__ points) {
   const unsigned long long i =
       (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -253,11 +254,13 @@ __global__ void k_emit(const uint32_t* __restrict__ cell,
   const int low_bits = g.plane_bits + g.phase_bits;
   const uint32_t tiles_per_grid = (uint32_t)g.tiles_u * (uint32_t)g.tiles_v;
   uint32_t pos = rec_offset[i];
+  if (points) points[i] = make_uint4(c, m, pos, 0u);
   const uint32_t vid = (uint32_t)(vis_offset + i);
   for (int tv = tv0; tv <= tv1; ++tv) {
     for (int tu = tu0; tu <= tu1; ++tu) {
       uint32_t tile = (uint32_t)grid_index * tiles_per_grid +
                       (uint32_t)tv * g.tiles_u + (uint32_t)tu;
+      if (tile_rank) tile = (uint32_t)tile_rank[tile];
       if (g.num_groups > 1) {
         uint32_t group = g.plane_group ? (uint32_t)g.plane_group[plane] : 0u;
         if (g.split_tv > 0) {
@@ -382,12 +385,13 @@ cudaError_t launch_emit_records(const uint32_t* cell, const uint32_t* meta,
                                 unsigned long long vis_offset, uint32_t* keys,
                                 uint32_t* vals, cudaStream_t s,
                                 const unsigned long long* grid_offsets,
-                                int num_grids) {
+                                int num_grids, const int* tile_rank,
+                                void* points) {
   if (n == 0) return cudaSuccess;
   const unsigned nb = (unsigned)((n + 255) / 256);
   k_emit<<<nb, 256, 0, s>>>(cell, meta, rec_offset, n, view, geom,
                             grid_index, vis_offset, keys, vals, grid_offsets,
-                            num_grids);
+                            num_grids, tile_rank, (uint4*)points);
   return cudaGetLastError();
 }
 

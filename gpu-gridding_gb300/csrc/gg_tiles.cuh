@@ -13,11 +13,7 @@ namespace {
 constexpr int kRows = 8;          // rows per lane (registers)
 constexpr int kWarps = 8;         // consumer warps per CTA
 constexpr int kConsumers = kWarps * 32;
-constexpr int kThreads = kConsumers + 32;  // + one producer warp
 constexpr int kCells = kConsumers * kRows; // 2048 cells per tile
-constexpr int kRing = 4;          // record buffers in flight
-constexpr int kBuf = 128;         // records per buffer
-constexpr int kPerLane = kBuf / 32;
 static_assert(kRows - 1 <= kSlicePad, "slices need kRows-1 padding rows");
 // Bound on every mbarrier wait (each failed probe sleeps ~100 ns): a wait
 // that runs out (> ~1 s) sets the error flag and the CTA returns.
@@ -39,14 +35,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)),
                "r"(count)
                : "memory");
-}
-// Release-arrive: the caller's earlier shared-memory writes are visible to
-// a thread whose wait observes the phase completion.
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile(
-      "{\n\t.reg .b64 st;\n\t"
-      "mbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar))
-      : "memory");
 }
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;

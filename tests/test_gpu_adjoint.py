@@ -218,3 +218,31 @@ def test_degrid_bit_identical_across_tunings(pkg, synthetic, torch):
         if t.get("plane_group_mb") == 1:
             assert plan.stats()["num_plane_groups"] > 1
         assert np.array_equal(got.view(np.uint32), base.view(np.uint32)), t
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("n,size,s_min,s_max,phases", [
+    (30, 200, 2, 6, 1),          # less than one unit of records
+    (600, 2048, 4, 20, 0),       # a record or two a tile
+    (5_000, 333, 31, 41, 4),     # footprints wider than a tile and phases
+    (900_000, 512, 1, 3, 0),     # every unit length, tiles of many units
+    (20_000, 1000, 2, 16, 2)])   # units across several tiles
+def test_degrid_units(pkg, oracle_mod, synthetic, torch, prec, n, size, s_min,
+                      s_max, phases):
+    """Degridding over units of records shorter and longer than a tile's, with
+    grid values per tile and per record.  Each result passes at most 36 rounded
+    additions in FP32 (8 rows, 5 lane steps, 8 bands, up to 15 records) and 150
+    in FP64 (128 cells of a lane, 5 lane steps, up to 15 records); the sum of
+    its terms' moduli is taken as up to 2 s_max + 1 times the largest result,
+    as for terms of random phase."""
+    wl = synthetic.random_uniform_workload("units", n, size, 16, s_min, s_max,
+                                           seed=n)
+    s = _setup(pkg, torch, wl, prec)
+    s["plan"].set_tuning({"tile_phases": phases})
+    rng = np.random.default_rng(n)
+    y = rng.standard_normal((wl.grid_size, wl.grid_size, 2)).astype(np.float32)
+    out = _adjoint(pkg, torch, s, torch.from_numpy(y).cuda().to(s["dt"]))
+    oracle = oracle_mod.degrid_fp64 if prec == "f" else oracle_mod.degrid_d
+    tol = 36 * 2.0**-24 if prec == "f" else 150 * 2.0**-53
+    assert max_rel(out.cpu().numpy(), oracle(wl, y.astype(np.float64))) <= \
+        tol * (2 * s_max + 1)
