@@ -1213,38 +1213,43 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
 
 // The work-item queue of binned records for num_ctas teams of as many
 // resident warps as a tile has bands: heavy tiles are split into items of
-// `chunk` records so that each of the call's `passes` launches has about
-// items_per_cta items per team.  Chunks shorter than 1024 records are made
-// longer, up to half a team's share: below that the partial tiles cost
-// more than the better balance gives (2048^2, 2e5 points, 6.6e5 records:
-// 0.69 ms with chunks of 434, 0.60 with 867).  FP64 gridding takes twice the
-// items and no such minimum: a record costs it four times as much, a unit's
-// tail likewise (the same points: 2.87 ms with chunks of 1084, 2.43 with 542,
-// 2.35 with 271, 2.34 with 136).  Items: at most one
-// more per tile than
-// total / chunk; partial-tile slots (split tiles only): at most
-// 2 * total / chunk, each a tile of partial sums.
+// `chunk` records so that each gridding launch (there is one for every
+// launch_span of the `passes` virtual groups) has about twice items_per_cta
+// items per team, four times that where the launch takes several tile phases
+// (every later phase's tile is a partial tile anyhow), 64 at most: a launch
+// ends with a tail up to one item long.  In ms with 4, 8, 16 and 32 items a
+// team: one phase, 7.8e6 track points on 2048^2 7.78, 7.17, 6.85, 6.67; 2.15e6
+// uniform ones on 8192^2 4.89, 4.92, 4.99, 5.06; four phases, 8, 16 and 32
+// items: 1.1e7 points on 16 grids of 2048^2 9.46, 9.10, 8.86; 7.8e6 track
+// points on 2048^2 5.40, 5.17, 5.19.
+// FP32 chunks shorter than 512 records are made longer, up to half a team's
+// share: below that the partial tiles cost more than the better balance gives
+// (track points on 2048^2, four phases: 1e6 0.64 ms so and 0.69 to 0.78 with
+// chunks of 512 to 128 records).  FP64 has no such minimum, as a record costs
+// it several times as much (2e5 points on 2048^2: 2.43 ms with chunks of 542
+// records, 2.35 with 271, 2.34 with 136).
+// Items: at most one more per tile than total / chunk; partial-tile slots
+// (split tiles only): at most 2 * total / chunk, each a tile of partial sums.
 template <typename Real>
 int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
                      cudaStream_t s, ItemBuffers* ib, int launch_span = 1) {
   using R2 = typename Vec2<Real>::type;
   uint32_t* sc = plan->scalars.as<uint32_t>();
   const int num_tiles = b.num_tiles;
-  // items_per_cta items per CTA in each of the call's passes: every pass
-  // ends with a tail up to one item long.
-  const bool grid64 = sizeof(Real) == 8;
-  const unsigned long long f = (unsigned long long)plan->items_per_cta *
-                               (unsigned long long)passes * (grid64 ? 2 : 1);
+  const unsigned long long f =
+      std::min((launch_span > 1 ? 4ull : 2ull) *
+                   (unsigned long long)plan->items_per_cta, 64ull) *
+      (unsigned long long)(passes / std::max(launch_span, 1));
   unsigned long long records =
       ((unsigned long long)b.total + f * num_ctas - 1) / (f * num_ctas);
-  if (!grid64)
+  if (sizeof(Real) == 4)
     records = std::max(records,
-                       std::min(1024ull, (unsigned long long)b.total /
+                       std::min(512ull, (unsigned long long)b.total /
                                              (2ull * passes * num_ctas)));
   const uint32_t chunk =
       (uint32_t)std::max<unsigned long long>(64, records);
-  const size_t item_cap = (size_t)num_tiles + 2 * f * (size_t)num_ctas + 16;
-  const size_t slot_cap = 2 * f * (size_t)num_ctas + 16;
+  const size_t slot_cap = 2 * (size_t)(b.total / chunk) + 16;
+  const size_t item_cap = (size_t)num_tiles + slot_cap;
   plan->stats.num_ctas = num_ctas;
   plan->stats.chunk_records = chunk;
   GG_TRY(plan->item_a.ensure((size_t)num_tiles * 4 + 4));

@@ -231,3 +231,28 @@ def test_fp64_footprints_packed_over_lanes(pkg, oracle_mod, synthetic, torch,
     want, skipped, _ = oracle_mod.grid_d(wl)
     assert int(skip.item()) == skipped
     assert max_rel(grid.cpu().numpy(), want) <= 1e-12
+
+
+@pytest.mark.parametrize("phases", [1, 4])
+@pytest.mark.parametrize("chunks", [1, 2, 15, 16, 17, 41])
+def test_chunks_of_one_tile(pkg, oracle_mod, synthetic, torch, chunks,
+                            phases):
+    """A tile cut into `chunks` chunks of 64 records, whose partial sums are
+    added sixteen at a time as (hi, lo) pairs: below, at and above one and two
+    such groups.  Each partial is rounded once, the products of weights and
+    visibilities once, the sum once: 3 * 2^-24 of the sum of moduli, here up to
+    5 times the largest cell."""
+    wl = synthetic.random_uniform_workload("chunks", 64 * chunks, 256, 4, 2, 3,
+                                           seed=chunks)
+    # All centres inside the tile to the right of and above the grid's centre.
+    extent = 1.0 / wl.cell_size_rad / 256
+    rng = np.random.default_rng(chunks)
+    wl.uu[:] = rng.uniform(12.0, 20.0, wl.num_points) * extent
+    wl.vv[:] = rng.uniform(12.0, 20.0, wl.num_points) * extent
+    plan = pkg.Plan()
+    plan.set_tuning({"tile_u": 32, "tile_phases": phases})
+    got = _grid(pkg, torch, wl, plan, pkg.KernelStack.from_workload(wl, "f"))
+    want = oracle_mod.grid_f_fp64acc(wl)
+    assert plan.stats()["chunk_records"] == 64
+    assert got[2] == want[1] == 0
+    assert max_rel(got[0], want[0]) <= 3 * 2.0**-24 * 5
