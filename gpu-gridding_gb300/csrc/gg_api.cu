@@ -557,8 +557,9 @@ struct gg_plan {
   int lane_groups = 0;    // as set; without effect (gg_tuning)
   int tile_phases = 0;    // tuning tile_phases: 0 automatic, 1, 2, 4
   // Tile phases requested for the call being placed (0 automatic, chosen
-  // with the shape; see gridding_phases).
+  // with the shape; see gridding_phases), and choose_shape's `tiles`.
   int call_phases = 1;
+  long long call_tiles = -1;
   // Batched calls larger than one sort can index (see batched_split): the
   // grids are cut into sub-batches, each gridded by its own sub-plan, which
   // keeps its geometry for replays.  A sub-plan takes the sort's transient
@@ -838,11 +839,22 @@ int max_tiles(int grid_size, int num_grids) {
   return m * num_grids;
 }
 
+// Tiles (2048 cells) of num_grids grids, for choose_shape.
+long long grid_tiles(int grid_size, int num_grids) {
+  return (long long)num_grids * grid_size * grid_size / 2048;
+}
+
 // Tile phases requested for a gridding call (TileGeom::tile_phases): the
 // plan's setting (0: chosen with the tile shape, see choose_shape), or 1
 // where eight phases' extra sort-key bits and the split passes' would not
 // fit 32-bit keys.
-int gridding_phases(const gg_plan* plan, int grid_size, int num_grids) {
+template <typename Real>
+int gridding_phases(const gg_plan* plan, int grid_size, int num_grids,
+                    bool degrid = false) {
+  // The FP64 gridder packs a footprint's cells over its lanes: offset tile
+  // grids save it records, not lanes (100 000 points, support 3 to 18: 2048^2
+  // 0.85 ms with one phase, 0.96 with four; 8192^2 1.06 and 1.62).
+  if (sizeof(Real) == 8 && !degrid && plan->tile_phases == 0) return 1;
   if (ceil_log2((unsigned long long)max_tiles(grid_size, num_grids)) + 3 + 2 >
       32)
     return 1;
@@ -925,7 +937,8 @@ int grid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
     return GG_OK;
   }
   PlaceOut po;
-  plan->call_phases = gridding_phases(plan, grid_size, 1);
+  plan->call_phases = gridding_phases<Real>(plan, grid_size, 1);
+  plan->call_tiles = grid_tiles(grid_size, 1);
   GG_TRY(place_and_count<Real>(plan, K, pp, plan->forced_shape, d_norm,
                                d_num_skipped, s, &po));
   return bin_and_grid<Real>(plan, K, n, po, grid_size, 1, nullptr, d_grid, 0,
@@ -999,7 +1012,7 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
                                 n, forced_shape,
                                 pp.defer_norm ? nullptr : d_norm,
                                 d_num_skipped, scalar64(plan, kMacs),
-                                sc + kShape, s, plan->call_phases));
+                                sc + kShape, s, plan->call_phases, plan->call_tiles));
   GG_CUDA(launch_count_records(po.cell, po.meta, n, view, sc + kShape,
                                po.rec_count, s));
   GG_CUDA(exclusive_scan_u32(po.rec_count, plan->rec_offset.as<uint32_t>(), n,
@@ -1524,7 +1537,8 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   po.blk_skip = nullptr;
   po.blk_macs = nullptr;
   const ChunkParts cp = chunk_parts(plan, num_chunks);
-  plan->call_phases = gridding_phases(plan, grid_size, num_grids);
+  plan->call_phases = gridding_phases<Real>(plan, grid_size, num_grids);
+  plan->call_tiles = grid_tiles(grid_size, num_grids);
 
   plan->mark(0, s);
   GG_CUDA(launch_place_batched<Real>(pp, view, po, plan->nterm.as<double>(),
@@ -1534,7 +1548,7 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
       plan->chunk_begin.as<unsigned long long>(), num_grids,
       plan->grid_chunk0.as<int>(), cp.norm, cp.skip, cp.macs,
       plan->forced_shape, d_norm, d_num_skipped, scalar64(plan, kMacs),
-      sc + kShape, s, plan->call_phases));
+      sc + kShape, s, plan->call_phases, plan->call_tiles));
   GG_CUDA(launch_count_records(po.cell, po.meta, n, view, sc + kShape,
                                po.rec_count, s));
   GG_CUDA(exclusive_scan_u32(po.rec_count, T->rec_offset.as<uint32_t>(), n,
@@ -1762,7 +1776,8 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
   const size_t n = num_points;
   const StackView view = K->view();
   PlaceOut po;
-  plan->call_phases = gridding_phases(plan, grid_size, 1);
+  plan->call_phases = gridding_phases<Real>(plan, grid_size, 1, true);
+  plan->call_tiles = -1;
   GG_TRY(place_and_count<Real>(plan, K, pp, kDegridShape, nullptr, nullptr, s,
                                &po));
   Bins b;

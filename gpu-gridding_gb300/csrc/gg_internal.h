@@ -76,20 +76,37 @@ __host__ __device__ inline int tile_v_of_shape(int shape) {
   return 2048 / (32 >> shape);
 }
 
-// Tile shape and tile phases for a call, from its mean
-// footprint side sqrt(macs / gridded points): narrow tiles only for tiny
-// footprints (a 32-wide warp would leave most lanes outside them); tile
-// phases (bits 12 and 13: log2 of 1, 2, 4 or 8) four when footprints are narrower than the
-// tile, where offset tile grids save the most tile crossings, else one.
+// Tile shape and tile phases for a call, from its mean footprint side
+// sqrt(macs / gridded points): narrow tiles only for tiny footprints (a
+// 32-wide warp would leave most lanes outside them); tile phases (bits 12 and
+// 13: log2 of 1, 2, 4 or 8) four when footprints are narrower than the tile,
+// where offset tile grids save the most tile crossings, and the call has
+// enough of them for its `tiles` tiles, else one.  What four phases save
+// grows with the MACs (more per MAC in narrow tiles), what they cost (the
+// partial tiles of the later phases and their addition) with the tiles.
+// Measured, ms with one and four phases (track points, 32-wide tiles where
+// support reaches 44, 16-wide for 18): 7.8e6 on 2048^2, support 44 6.85 and
+// 5.17, 18 3.09 and 2.50; on 8192^2 6.57 and 5.69, 3.07 and 3.03; 1e6 on
+// 2048^2 1.16 and 1.05, 0.63 and 0.64; on 8192^2 1.26 and 1.61, 0.75 and
+// 1.17; 4e3 uniform points on 256^2 0.14 and 0.17.
+// tiles < 0: degridding, whose phases cost nothing and save 10 % of large
+// calls.
 // forced_shape >= 0 overrides the shape, phases > 0 the phases.
 __host__ __device__ inline uint32_t choose_shape(unsigned long long macs,
                                                  unsigned long long gridded,
                                                  int forced_shape,
-                                                 int phases = 1) {
+                                                 int phases = 1,
+                                                 long long tiles = -1) {
   const double side = gridded ? sqrt((double)macs / (double)gridded) : 0.0;
   int shape = forced_shape;
   if (shape < 0) shape = side >= 16.0 ? 0 : (side >= 8.0 ? 1 : 2);
-  if (phases <= 0) phases = side < (double)tile_u_of_shape(shape) ? 4 : 1;
+  const int tu = tile_u_of_shape(shape);
+  if (phases <= 0)
+    phases = side < (double)tu &&
+                     (tiles < 0 || (double)macs * (32 / tu) >
+                                       7e4 * (double)tiles + 1.5e8)
+                 ? 4
+                 : 1;
   const uint32_t pbits =
       phases >= 8 ? 3u : (phases >= 4 ? 2u : (phases >= 2 ? 1u : 0u));
   return (uint32_t)shape | (pbits << 12);
@@ -137,7 +154,7 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   unsigned long long* d_num_skipped,
                                   unsigned long long* d_macs,
                                   uint32_t* d_shape, cudaStream_t s,
-                                  int phases = 1);
+                                  int phases = 1, long long tiles = -1);
 // count[i] = tiles of shape *d_shape touched by visibility i on its tile
 // phase (footprint_phase; 0 if skipped).
 cudaError_t launch_count_records(const uint32_t* cell, const uint32_t* meta,
@@ -193,7 +210,8 @@ cudaError_t launch_batch_totals(const uint32_t* meta, const double* nterm,
                                 int forced_shape, double* d_norm,
                                 unsigned long long* d_num_skipped,
                                 unsigned long long* d_macs, uint32_t* d_shape,
-                                cudaStream_t s, int phases = 1);
+                                cudaStream_t s, int phases = 1,
+                                long long tiles = -1);
 
 // ---- work decomposition and gridding (gg_grid.cu) -------------------------
 cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,

@@ -121,7 +121,7 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
                                  const unsigned long long* __restrict__ blk_skip,
                                  const unsigned long long* __restrict__ blk_macs,
                                  int num_blocks, unsigned long long n_points,
-                                 int forced_shape, int phases,
+                                 int forced_shape, int phases, long long tiles,
                                  double* d_norm,
                                  unsigned long long* d_num_skipped,
                                  unsigned long long* d_macs,
@@ -168,7 +168,7 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
       if (d_num_skipped) *d_num_skipped = s;
       if (d_macs) *d_macs = m;
       if (d_shape)
-        *d_shape = choose_shape(m, n_points - s, forced_shape, phases);
+        *d_shape = choose_shape(m, n_points - s, forced_shape, phases, tiles);
     }
   }
 }
@@ -338,9 +338,9 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   unsigned long long* d_num_skipped,
                                   unsigned long long* d_macs,
                                   uint32_t* d_shape, cudaStream_t s,
-                                  int phases) {
+                                  int phases, long long tiles) {
   k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, blk_skip, blk_macs,
-                                      num_blocks, n, forced_shape, phases,
+                                      num_blocks, n, forced_shape, phases, tiles,
                                       d_norm, d_num_skipped, d_macs, d_shape);
   return cudaGetLastError();
 }
@@ -364,7 +364,7 @@ cudaError_t launch_norm_terms(const uint32_t* meta, const Real* weight,
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, nullptr, nullptr, nb, n, 0,
-                                      1, d_norm, nullptr, nullptr, nullptr);
+                                      1, -1, d_norm, nullptr, nullptr, nullptr);
   return cudaGetLastError();
 }
 
