@@ -9,7 +9,8 @@ no placement, norm or skip count (gg_tuning in the C header):
 * ``sort_detail``   -- record order within a tile (plane + offset class,
   plane only, or visibility order),
 * ``ctas_per_sm``   -- resident gridding CTAs per SM (0 = as many as fit),
-* ``plane_group_mb`` -- kernel bytes per gridding pass (0 = 3/4 of L2),
+* ``plane_group_mb`` -- kernel bytes per gridding pass (0 = 3/4 of L2
+  for the planes that the call uses),
 * ``tile_order``    -- tiles taken by distance from the centre or row by row,
 * ``tile_phases``   -- 1, 2, 4 or 8 tile grids offset by a fraction of a tile
   width; each visibility is gridded on the one that cuts its footprint

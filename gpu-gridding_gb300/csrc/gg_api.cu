@@ -615,9 +615,9 @@ struct gg_plan {
   DevBuf plane_group, group_items;
   std::vector<int> h_plane_group;
   unsigned long long pg_kernels = 0;   // id of the kernel stack
-  long long pg_budget = -1;           // requested budget (bytes)
-  int pg_max_groups = 0;
+  long long pg_want = 0;              // groups asked for
   int pg_groups = 1;
+  bool plane_use = false;   // the call's plane use is in h_scalars
   bool profile = false;
   bool events_valid = false;
   cudaEvent_t ev[kEvents] = {};
@@ -684,15 +684,19 @@ enum Scalar64 {
   kMacs = 0, kSkipScratch, kDirectCells, kRecords64, kScalar64Count
 };
 
+// Behind those, launch_plane_use's bins.
+constexpr size_t kUseOffset = kScalar64Offset + kScalar64Count * 8;
+constexpr size_t kScalarBytes = kUseOffset + kPlaneBins * 4;
+
 unsigned long long* scalar64(gg_plan* p, int i) {
   return (unsigned long long*)((char*)p->scalars.p + kScalar64Offset) + i;
 }
 
 int plan_init(gg_plan* p) {
   GG_TRY(current_device(&p->device));
-  GG_TRY(p->scalars.ensure(kScalar64Offset + kScalar64Count * 8));
+  GG_TRY(p->scalars.ensure(kScalarBytes));
   GG_CUDA(cudaMemset(p->scalars.p, 0, p->scalars.bytes));
-  GG_CUDA(cudaMallocHost(&p->h_scalars, 64));
+  GG_CUDA(cudaMallocHost(&p->h_scalars, kScalarBytes));
   return GG_OK;
 }
 
@@ -762,42 +766,116 @@ unsigned long long max_records_per_vis(int s_max, int shape) {
   return r;
 }
 
+// Slice bytes of plane p.
+long long plane_bytes(const gg_kernels* K, int p) {
+  return plane_taps(K->h_support[p], K->omax) * (K->is_double ? 16 : 8);
+}
+
+// Slice bytes per plane group: the plan's setting, or 3/4 of the L2 cache.
+int plane_budget(const gg_plan* plan, const gg_kernels* K, long long* budget) {
+  *budget = (long long)plan->plane_group_mb << 20;
+  if (*budget <= 0) {
+    int l2 = 0;
+    GG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, K->device));
+    *budget = std::max<long long>((long long)l2 / 4 * 3, 1 << 20);
+  }
+  return GG_OK;
+}
+
+// Reads the call's scalars back (the 32-bit ones and the MAC count behind
+// them) and waits for them.  Where the stack is larger than the automatic
+// budget, how much the planes are used comes with them (used_bytes).
+int read_scalars(gg_plan* plan, const gg_kernels* K, const uint32_t* meta,
+                 unsigned long long n, cudaStream_t s) {
+  plan->plane_use = false;
+  if (plan->plane_group_mb <= 0 && n > 0) {
+    long long budget, total = 0;
+    GG_TRY(plane_budget(plan, K, &budget));
+    for (int p = 0; p < K->num_planes; ++p) total += plane_bytes(K, p);
+    plan->plane_use = total > budget;
+  }
+  if (plan->plane_use) {
+    GG_CUDA(launch_plane_use(meta, n, K->num_planes,
+                             (uint32_t*)((char*)plan->scalars.p + kUseOffset),
+                             s));
+    plan->stats.num_launches += 1;
+  }
+  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, plan->scalars.p,
+                          plan->plane_use ? kScalarBytes : kScalar64Offset + 8,
+                          cudaMemcpyDeviceToHost, s));
+  GG_CUDA(cudaStreamSynchronize(s));
+  return GG_OK;
+}
+
+// Slice bytes that 95 % of the call's taps come from, the most used bins of
+// planes first; the whole stack where that is more than four fifths of it (one
+// used evenly).  The planes of a telescope's visibilities crowd near zero: of a stack of 327 MB (601 planes,
+// support 4 to 72), 512-station tracks take 95 % of their taps from 67 MB,
+// 128-station ones from 114, uniform w from 290.
+long long used_bytes(const gg_plan* plan, const gg_kernels* K) {
+  const uint32_t* use =
+      (const uint32_t*)((const char*)plan->h_scalars + kUseOffset);
+  long long bytes[kPlaneBins] = {}, total = 0;
+  double taps[kPlaneBins] = {}, sum = 0;
+  int planes[kPlaneBins] = {}, order[kPlaneBins];
+  for (int p = 0; p < K->num_planes; ++p) {
+    const int b = (int)((long long)p * kPlaneBins / K->num_planes);
+    const double side = 2.0 * K->h_support[p] + 1.0;
+    bytes[b] += plane_bytes(K, p);
+    taps[b] += side * side;
+    ++planes[b];
+  }
+  for (int b = 0; b < kPlaneBins; ++b) {
+    order[b] = b;
+    total += bytes[b];
+    taps[b] = planes[b] ? taps[b] / planes[b] * use[b] : 0.0;
+    sum += taps[b];
+  }
+  std::stable_sort(order, order + kPlaneBins, [&](int a, int b) {
+    return taps[a] * (double)bytes[b] > taps[b] * (double)bytes[a];
+  });
+  double at = 0;
+  long long used = 0;
+  for (int k = 0; k < kPlaneBins && at < 0.95 * sum; ++k) {
+    at += taps[order[k]];
+    used += bytes[order[k]];
+  }
+  return used > total / 5 * 4 ? total : used;
+}
+
 // Plane groups for a call: consecutive w-planes cut into as many groups as
 // the byte budget (plan->plane_group_mb, or 3/4 of the L2 cache) needs, with
 // even slice bytes per group, so that each gridding pass reads a stack slice
-// that stays resident in L2.  At most max_groups groups (the sort key's
-// spare bits).
+// that stays resident in L2.  With the automatic budget only the bytes in use
+// count (used_bytes): groups cost tracks more partial tiles and tails than
+// they save misses (601 planes, support 4 to 72, ms with one, two and four
+// groups: 512 stations, 7.8e6 points 6.47, 6.78, 7.87; 128 stations, 2e6
+// points 3.30, 3.15, 3.03; 6e5 points of uniform w 8.31, 5.87, 5.14).  At most
+// max_groups groups (the sort key's spare bits).
 // Uploads the plane -> group table when it changes; returns the number of
 // groups in *num_groups.
 int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
                  cudaStream_t s, int* num_groups) {
-  long long budget = (long long)plan->plane_group_mb << 20;
-  const long long requested = budget;
-  if (budget <= 0) {
-    int l2 = 0;
-    GG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, K->device));
-    budget = std::max<long long>((long long)l2 / 4 * 3, 1 << 20);
-  }
+  long long budget;
+  GG_TRY(plane_budget(plan, K, &budget));
   max_groups = std::max(1, std::min(max_groups, 64));
-  if (plan->pg_kernels == K->id && plan->pg_budget == requested &&
-      plan->pg_max_groups == max_groups) {
-    *num_groups = plan->pg_groups;
-    return GG_OK;
-  }
-  const long long tap_bytes = K->is_double ? 16 : 8;
   std::vector<long long> bytes(K->num_planes);
   long long total = 0;
   for (int p = 0; p < K->num_planes; ++p) {
-    bytes[p] = plane_taps(K->h_support[p], K->omax) * tap_bytes;
+    bytes[p] = plane_bytes(K, p);
     total += bytes[p];
   }
-  // More groups than allowed: widen the budget until they fit.
-  budget = std::max(budget, (total + max_groups - 1) / max_groups);
+  const long long in_use = plan->plane_use ? used_bytes(plan, K) : total;
   // As many groups as the budget needs, with even byte counts: plane p
   // joins the group that holds the middle of its bytes (a greedy fill to
   // the budget would leave the last group with the remainder, and the first
   // groups' slices, at the full budget, less likely to stay in L2).
-  const long long want = std::max(1LL, (total + budget - 1) / budget);
+  const long long want = std::min<long long>(
+      max_groups, std::max(1LL, (in_use + budget - 1) / budget));
+  if (plan->pg_kernels == K->id && plan->pg_want == want) {
+    *num_groups = plan->pg_groups;
+    return GG_OK;
+  }
   const double target = (double)total / (double)want;
   std::vector<int>& grp = plan->h_plane_group;
   grp.assign(K->num_planes, 0);
@@ -820,8 +898,7 @@ int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
                           (size_t)K->num_planes * sizeof(int),
                           cudaMemcpyHostToDevice, s));
   plan->pg_kernels = K->id;
-  plan->pg_budget = requested;
-  plan->pg_max_groups = max_groups;
+  plan->pg_want = want;
   plan->pg_groups = groups;
   *num_groups = groups;
   return GG_OK;
@@ -1020,10 +1097,7 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
   // place, finalize, count, scan
   plan->stats.num_launches = 3 + scan_launches(n);
   plan->mark(1, s);
-  // The 32-bit scalars and the MAC count behind them.
-  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, sc, kScalar64Offset + 8,
-                          cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaStreamSynchronize(s));
+  GG_TRY(read_scalars(plan, K, po.meta, n, s));
   *po_out = po;
   return GG_OK;
 }
@@ -1556,10 +1630,7 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   // place, chunk totals, finalize, count, scan
   plan->stats.num_launches = (num_chunks > 0 ? 4 : 3) + scan_launches(n);
   plan->mark(1, s);
-  // The 32-bit scalars and the MAC count behind them.
-  GG_CUDA(cudaMemcpyAsync(plan->h_scalars, sc, kScalar64Offset + 8,
-                          cudaMemcpyDeviceToHost, s));
-  GG_CUDA(cudaStreamSynchronize(s));
+  GG_TRY(read_scalars(plan, K, po.meta, n, s));
   GG_TRY(bin_and_grid<Real>(plan, K, n, po, grid_size, num_grids,
                             plan->grid_offsets.as<unsigned long long>(),
                             d_grids, grid_stride, s));

@@ -155,6 +155,11 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   unsigned long long* d_macs,
                                   uint32_t* d_shape, cudaStream_t s,
                                   int phases = 1, long long tiles = -1);
+// use[b] = how many of up to 8192 placed points, evenly taken, are gridded with
+// planes p of bin b = p * kPlaneBins / num_planes.
+constexpr int kPlaneBins = 256;
+cudaError_t launch_plane_use(const uint32_t* meta, unsigned long long n,
+                             int num_planes, uint32_t* use, cudaStream_t s);
 // count[i] = tiles of shape *d_shape touched by visibility i on its tile
 // phase (footprint_phase; 0 if skipped).
 cudaError_t launch_count_records(const uint32_t* cell, const uint32_t* meta,

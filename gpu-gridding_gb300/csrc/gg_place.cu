@@ -173,6 +173,32 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
   }
 }
 
+// One block of 1024 threads, eight points each, their loads in flight
+// together: a few microseconds.
+__global__ void __launch_bounds__(1024)
+k_plane_use(const uint32_t* __restrict__ meta, unsigned long long n,
+            int num_planes, uint32_t* __restrict__ use) {
+  __shared__ uint32_t s_use[kPlaneBins];
+  constexpr int kEach = 8;
+  const unsigned long long samples =
+      n < kEach * 1024ull ? n : kEach * 1024ull;
+  if (threadIdx.x < kPlaneBins) s_use[threadIdx.x] = 0u;
+  __syncthreads();
+  uint32_t m[kEach];
+#pragma unroll
+  for (int j = 0; j < kEach; ++j) {
+    const unsigned long long k = j * 1024ull + threadIdx.x;
+    m[j] = k < samples ? meta[k * n / samples] : (1u << 25);
+  }
+#pragma unroll
+  for (int j = 0; j < kEach; ++j)
+    if (!meta_skipped(m[j]))
+      atomicAdd(&s_use[(long long)meta_plane(m[j]) * kPlaneBins / num_planes],
+                1u);
+  __syncthreads();
+  if (threadIdx.x < kPlaneBins) use[threadIdx.x] = s_use[threadIdx.x];
+}
+
 // Records per visibility: tiles of the chosen shape its footprint touches
 // (on its tile phase, see footprint_phase).
 __global__ void k_count(const uint32_t* __restrict__ cell,
@@ -365,6 +391,12 @@ cudaError_t launch_norm_terms(const uint32_t* meta, const Real* weight,
   if (e != cudaSuccess) return e;
   k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, nullptr, nullptr, nb, n, 0,
                                       1, -1, d_norm, nullptr, nullptr, nullptr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_plane_use(const uint32_t* meta, unsigned long long n,
+                             int num_planes, uint32_t* use, cudaStream_t s) {
+  k_plane_use<<<1, 1024, 0, s>>>(meta, n, num_planes, use);
   return cudaGetLastError();
 }
 

@@ -191,7 +191,9 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  *                  group's re-laid kernels within this many MiB (about
  *                  equal in size) and each group is gridded in its own
  *                  pass, so that a pass's kernels stay in L2; 0 (default) =
- *                  three quarters of the device's L2 cache, 0..1048576
+ *                  three quarters of the device's L2 cache for the
+ *                  planes that the call's points use (one pass where these
+ *                  fit, whatever the others take), 0..1048576
  *   tile_order     order in which the persistent CTAs take the tiles: 0
  *                  (default) by distance from the grid centre (baseline
  *                  length, so w and the kernels read stay alike among the

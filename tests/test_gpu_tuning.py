@@ -256,3 +256,40 @@ def test_chunks_of_one_tile(pkg, oracle_mod, synthetic, torch, chunks,
     assert plan.stats()["chunk_records"] == 64
     assert got[2] == want[1] == 0
     assert max_rel(got[0], want[0]) <= 3 * 2.0**-24 * 5
+
+
+@pytest.mark.parametrize("n,top,groups", [
+    (20_000, 600, 4),      # planes used evenly: the whole stack of 350 MB
+    (20_000, 120, 1),      # the lowest fifth: 5.6 MB
+    (300, 600, 3),         # 245 MB
+    (1, 1, 1),
+    (5_000, 0, 1)])        # all outside the grid: none used
+def test_plane_groups_by_use(pkg, torch, n, top, groups):
+    """The automatic number of plane groups follows the bytes of the planes
+    that the points use, and changes the grid by rounding only (the tuning
+    tests' bound)."""
+    G, planes = 512, 601
+    sup = np.rint(np.linspace(4, 72, planes)).astype(np.int32)
+    stack = pkg.KernelStack.generate(planes, sup, 4, 4 * 73,
+                                     np.full(planes, 3.0))
+    rng = np.random.default_rng(n + top)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    far = 1e6 if top == 0 else 1.0
+    uu, vv = (dev(far * rng.uniform(60.0, 150.0, n)) for _ in range(2))
+    p = np.rint(top * np.sqrt(rng.random(n)))
+    args = (stack, uu, vv, dev(p * p), dev(rng.standard_normal((n, 2))),
+            dev(rng.uniform(1, 2, n)), 0.002, np.float32(1.0), G)
+    outs = []
+    for tuning in ({}, {"plane_group_mb": 1048576}):
+        plan = pkg.Plan()
+        plan.set_tuning(tuning)
+        grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+        norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+        skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+        pkg.grid_wproj_device(plan, *args, grid, norm, skip)
+        outs.append((grid.cpu().numpy(), float(norm.item()),
+                     int(skip.item()), plan.stats()["num_plane_groups"]))
+    assert outs[0][3] == groups and outs[1][3] == 1
+    assert outs[0][1:3] == outs[1][1:3]
+    if outs[0][2] < n:
+        assert max_rel(outs[0][0], outs[1][0]) <= 1e-5
