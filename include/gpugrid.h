@@ -178,10 +178,11 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  * rounding; slice_staging has no effect.
  *   tile_u         32, 16 or 8 (cells across a tile); 0 = chosen per call
  *   slice_staging  -1, 0 or 1; without effect
- *   items_per_cta  work items per persistent CTA in each gridding pass
- *                  that the split of heavy tiles aims for, 1..64 (default
- *                  4): more items balance the load better but write more
- *                  partial tiles
+ *   items_per_cta  half the work items (with tile phases a quarter) per
+ *                  team of resident warps in each gridding pass that the
+ *                  split of heavy tiles aims for, 1..64 (default 4; at most
+ *                  64 items a team): more items balance the load better but
+ *                  write more partial tiles
  *   sort_detail    order of a tile's records: 2 (default) by w-plane then
  *                  kernel-offset class, 1 by w-plane, 0 visibility order
  *   ctas_per_sm    resident gridding CTAs per SM, 0 (default) = as many as
@@ -209,7 +210,8 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  *                  all in one pass per plane group (the tiles of later
  *                  grids add partial tiles after it); 0 (default): four
  *                  when the call's mean footprint is narrower than the
- *                  tile, else one
+ *                  tile and there are enough of them per tile to repay
+ *                  those (FP32 gridding; degridding: always), else one
  * gg_plan_set_tile_shape and gg_plan_set_slice_staging set the first two
  * fields alone. */
 typedef struct
