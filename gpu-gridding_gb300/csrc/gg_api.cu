@@ -1265,7 +1265,7 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   // sub-plan, its parent's.
   gg_plan* T = plan->scratch ? plan->scratch : plan;
   const bool alt_final =
-      total > 1 && key_bits > 0 && ((key_bits + 7) / 8) % 2 == 1;
+      total > 1 && key_bits > 0 && radix_passes(key_bits) % 2 == 1;
   DevBuf& v0 = alt_final ? T->vals0 : plan->vals0;
   DevBuf& v1 = alt_final ? plan->vals1 : T->vals1;
   GG_TRY(T->keys0.ensure((size_t)total * 4));

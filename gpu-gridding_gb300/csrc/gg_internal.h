@@ -32,6 +32,7 @@ cudaError_t exclusive_scan_pair_u32(uint32_t* a, uint32_t* b, size_t n,
                                     void* tmp, cudaStream_t s);
 // Kernel launches of a scan of n entries (one array or a pair), and of a sort.
 int scan_launches(size_t n);
+int radix_passes(int end_bit);
 int radix_launches(size_t n, int end_bit);
 size_t radix_temp_bytes(size_t n);
 cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals,

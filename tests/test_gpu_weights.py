@@ -219,3 +219,17 @@ def test_sort_and_scan_sizes(pkg, oracle_mod, synthetic, torch, n):
     g, ns, nm = pkg.grid_f(wl)
     assert ns == ns64 and abs(nm - nm64) <= 1e-12 * abs(nm64)
     assert max_rel(g, g64) <= 1e-5
+
+
+@pytest.mark.parametrize("G", [15, 16, 22, 23, 255, 300, 511, 600, 5000, 8192])
+@pytest.mark.parametrize("n", [3000, 192 * 4096 + 77])
+def test_sort_digit_widths(pkg, oracle_mod, n, G):
+    """Cell counts on both sides of where the sort changes between digits of
+    eight and of nine bits (8 | 9 | 16 | 17, 18 | 19 | 25 to 27 key bits), with
+    and without the scan launches: the serial sums bit for bit."""
+    cell = np.float32(1e-3)
+    uu, vv, w = _points(n, G, cell, np.float32, G)
+    dens, ns = pkg.grid_weights_write(uu, vv, w, cell, G)
+    ref, ns_ref = oracle_mod.weights_write(uu, vv, w, cell, G)
+    assert ns == ns_ref
+    _same(dens, ref)
