@@ -6,8 +6,8 @@ no placement, norm or skip count (gg_tuning in the C header):
 * ``tile_u``        -- tile width (32, 16 or 8 cells; 2048-cell tiles),
 * ``slice_staging``, ``lane_groups`` -- accepted without effect,
 * ``items_per_cta`` -- how finely heavy tiles are split into work items,
-* ``sort_detail``   -- record order within a tile (plane + offset class,
-  plane only, or visibility order),
+* ``sort_detail``   -- record order within a tile (by plane where it pays,
+  by plane, or visibility order),
 * ``ctas_per_sm``   -- resident gridding CTAs per SM (0 = as many as fit),
 * ``plane_group_mb`` -- kernel bytes per gridding pass (0 = 3/4 of L2
   for the planes that the call uses),

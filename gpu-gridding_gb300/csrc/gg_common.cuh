@@ -163,8 +163,7 @@ struct TileGeom {
   int tile_u, tile_v;        // cells per tile
   int tiles_u, tiles_v;      // tiles per grid side
   int num_grids;
-  int plane_bits, phase_bits;  // low key fields below the tile index
-  int phase_side;            // 2*omax+1... stored as omax+1 (|off| classes)
+  int plane_bits;            // key bits of the plane, below the tile index
   int num_groups;            // plane groups (passes), >= 1
   int tiles_total;           // num_grids * tiles_u * tiles_v
   const int* plane_group;    // [P] group of each plane (num_groups > 1)

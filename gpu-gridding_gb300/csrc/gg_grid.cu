@@ -1,9 +1,9 @@
 // Tile-owning gridding.
 //
 // The grid is cut into tiles of TW (u) x TV (v) cells.  After the sort each
-// tile's (visibility, tile) records are contiguous and ordered by (plane,
-// |offset| class); a tile's record range is cut into work items of at most
-// `chunk` records.  k_prepare_records turns the sorted records into
+// tile's (visibility, tile) records are contiguous (ordered by plane where
+// there are many plane groups); a tile's record range is cut into work items
+// of at most `chunk` records.  k_prepare_records turns the sorted records into
 // descriptors; then every warp of the persistent gridding kernel works by
 // itself: it takes a band of a work item (8 lane rows by the tile's columns)
 // from a queue and keeps the band's cells in registers: lane (lx, ly) owns

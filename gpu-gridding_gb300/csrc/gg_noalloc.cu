@@ -266,24 +266,16 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   set_strips(geom, grid_size);
   const int num_tiles = geom.tiles_u * geom.tiles_v;
   const int tile_bits = ceil_log2_u((unsigned long long)num_tiles);
-  int plane_bits = ceil_log2_u((unsigned long long)num_planes);
-  int phase_bits =
-      ceil_log2_u((unsigned long long)(view.omax + 1) * (view.omax + 1));
-  if (tile_bits + plane_bits + phase_bits > 32) phase_bits = 0;
-  if (tile_bits + plane_bits + phase_bits > 32) plane_bits = 0;
-  geom.plane_bits = plane_bits;
-  geom.phase_bits = phase_bits;
-  geom.phase_side = view.omax + 1;
-  const int low_bits = plane_bits + phase_bits;
+  geom.plane_bits = 0;   // records of a tile in visibility order
 
   NA_CUDA(launch_emit_records(cell, meta, offset, num_points, view, geom, 0,
                               0, keys0, vals0, s));
   bool in_alt = false;
   NA_CUDA(radix_sort_pairs(keys0, vals0, keys1, vals1, total,
-                           tile_bits + low_bits, sort_tmp, s, &in_alt));
+                           tile_bits, sort_tmp, s, &in_alt));
   const uint32_t* keys = in_alt ? keys1 : keys0;
   const uint32_t* vals = in_alt ? vals1 : vals0;
-  NA_CUDA(launch_tile_bounds(keys, total, low_bits, num_tiles, tile_start,
+  NA_CUDA(launch_tile_bounds(keys, total, 0, num_tiles, tile_start,
                              s));
   int sms = 0;
   NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -232,9 +232,8 @@ __global__ void k_count(const uint32_t* __restrict__ cell,
 }
 
 // One thread per visibility writes one record per tile its footprint
-// touches.  Key = (tile, plane, |offset| class) so that after the sort each
-// tile's records are contiguous and grouped by kernel slice; value = the
-// visibility index.
+// touches.  Key = (tile, plane if plane_bits) so that after the sort each
+// tile's records are contiguous; value = the visibility index.
 __global__ void k_emit(const uint32_t* __restrict__ cell,
                        const uint32_t* __restrict__ meta,
                        const uint32_t* __restrict__ rec_offset,
@@ -273,11 +272,9 @@ __global__ void k_emit(const uint32_t* __restrict__ cell,
   const int sh = phase << g.strip_shift;
   const int tu0 = (gu - s + sh) >> tws, tu1 = (gu + s + sh) >> tws;
   const int tv0 = (gv - s) >> ths, tv1 = (gv + s) >> ths;
-  const int au = abs(meta_ou(m)), av = abs(meta_ov(m));
   uint32_t low = 0;
-  if (g.phase_bits > 0) low = (uint32_t)(au * (v.omax + 1) + av);
-  if (g.plane_bits > 0) low |= (uint32_t)plane << g.phase_bits;
-  const int low_bits = g.plane_bits + g.phase_bits;
+  if (g.plane_bits > 0) low = (uint32_t)plane;
+  const int low_bits = g.plane_bits;
   const uint32_t tiles_per_grid = (uint32_t)g.tiles_u * (uint32_t)g.tiles_v;
   uint32_t pos = rec_offset[i];
   if (points) points[i] = make_uint4(c, m, pos, 0u);

@@ -1,7 +1,7 @@
 // Device-wide exclusive scan and stable LSD radix sort of (key, value)
-// pairs.  These order the (visibility, tile) records by (grid, tile, plane,
-// offset class) so the gridding kernel sees each tile's records contiguously
-// and grouped by kernel slice.  The reference bins with an atomic bucket
+// pairs.  These order the (visibility, tile) records by (grid, tile), some
+// calls' by plane too, so the gridding kernel sees each tile's records
+// contiguously.  The reference bins with an atomic bucket
 // scatter whose in-bucket order changes from run to run
 // (oskar_grid_wproj_gpu.cu:520-649); this sort is stable, so the record
 // order -- and with it the accumulation order -- is the same on every call.

@@ -183,8 +183,9 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  *                  split of heavy tiles aims for, 1..64 (default 4; at most
  *                  64 items a team): more items balance the load better but
  *                  write more partial tiles
- *   sort_detail    order of a tile's records: 2 (default) by w-plane then
- *                  kernel-offset class, 1 by w-plane, 0 visibility order
+ *   sort_detail    order of a tile's records: 2 (default) by w-plane where
+ *                  that pays (three plane groups or more), 1 by w-plane, 0
+ *                  visibility order
  *   ctas_per_sm    resident gridding CTAs per SM, 0 (default) = as many as
  *                  fit, else min(that, what fits), 1..32
  *   plane_group_mb kernel bytes per gridding pass: the w-planes are cut
