@@ -1392,11 +1392,12 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
                  const PlaceOut& po, int grid_size, int num_grids,
                  const unsigned long long* d_grid_offsets, Real* d_grid,
                  long long grid_stride, cudaStream_t s) {
-  const StackView view = K->view();
+  StackView view = K->view();
   uint32_t* sc = plan->scalars.as<uint32_t>();
   Bins b;
   GG_TRY(bin_records<Real>(plan, K, n, po, grid_size, num_grids,
                            d_grid_offsets, s, &b));
+  view.wide |= b.total >= kWideRecords;
   if (plan->stack_wait) {
     // The stack was built beside placement and binning.
     GG_CUDA(cudaStreamWaitEvent(s, plan->stack_wait, 0));
@@ -1783,7 +1784,8 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
     return set_error(GG_ERR_INVALID_ARG, "an input array is NULL");
   if (!d_grids || !d_norm || !d_num_skipped)
     return set_error(GG_ERR_INVALID_ARG, "an output pointer is NULL");
-  const StackView view = K->view();
+  StackView view = K->view();
+  view.wide |= kp.num_records >= kWideRecords;
   uint32_t* sc = plan->scalars.as<uint32_t>();
   const ChunkParts cp = chunk_parts(plan, kp.num_chunks);
   GG_CUDA(launch_revalue<Real>(vis, weight, plan->meta.as<uint32_t>(), view,

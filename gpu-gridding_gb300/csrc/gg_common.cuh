@@ -94,6 +94,9 @@ struct alignas(16) SlicePlane {
   int support;
 };
 
+// From here on FP32 gridding takes record positions as unsigned (wide view).
+constexpr uint32_t kWideRecords = (1u << 31) - 64;
+
 struct StackView {
   int num_planes;
   int oversample;
@@ -102,7 +105,8 @@ struct StackView {
   const int* support;       // [P]
   const SlicePlane* planes; // [P]
   const void* taps;         // float2 or double2
-  bool wide;                // more than 4 GiB of taps (load_taps)
+  bool wide;                // more than 4 GiB of taps (load_taps), or a call
+                            // with kWideRecords records or more
   const double* tap_sum;    // [P][2*omax+1][2*omax+1] sum of Re(tap), FP64
 };
 
@@ -216,11 +220,32 @@ __host__ __device__ inline int footprint_phase(int c0, int c1,
 }
 
 // Work item of the gridding kernel: a range of sorted records of one tile.
+// Record positions take all 32 bits (a call has up to 2^32 - 16 records): a
+// position plus a stride may wrap, so loops from kWideRecords on test the
+// distance to rec_end.  No item is empty.
 struct WorkItem {
   int tile;        // global tile index (grid * tiles_per_grid + tile)
-  int rec_begin;
-  int rec_end;
+  uint32_t rec_begin;
+  uint32_t rec_end;
   int slot;        // partial-tile slot, or -1 when the item owns the tile
 };
+
+// Chunks of at most `chunk` records that `count` records make, and the item of
+// chunk j of the records [begin, end).
+__host__ __device__ inline uint32_t num_chunks(uint32_t count,
+                                               uint32_t chunk) {
+  return count / chunk + (count % chunk != 0 ? 1u : 0u);
+}
+__host__ __device__ inline WorkItem chunk_item(int tile, uint32_t begin,
+                                               uint32_t end, uint32_t chunk,
+                                               uint32_t j, int slot) {
+  WorkItem w;
+  w.tile = tile;
+  w.rec_begin = begin + j * chunk;
+  const uint32_t left = end - w.rec_begin;
+  w.rec_end = w.rec_begin + (left < chunk ? left : chunk);
+  w.slot = slot;
+  return w;
+}
 
 }  // namespace gg
