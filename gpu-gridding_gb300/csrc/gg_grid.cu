@@ -622,40 +622,55 @@ k_grid_tiles_f64(GridArgs<double> a) {
   }
 }
 
-// A sum in more than the call's precision: FP64 as it is, FP32 as a (hi, lo)
-// pair.  An FP64 addition takes 16 cycles of the SM a warp, as does the
-// conversion of what it adds, and the tiles with hundreds of chunks lie on a
-// few SMs.  Calls with FP64 sums and so, ms: 1e6 track points on 1024^2, four
-// tile phases, 1.66 and 1.11; 2e5 uniform points on 2048^2 0.456 and 0.425.
+// A sum in more than the call's precision.  FP32: the sum split over three
+// floats by two TwoSums an addition, as an FP64 addition takes 16 cycles of the
+// SM a warp, as does the conversion of what it adds, and the tiles with
+// hundreds of chunks lie on a few SMs.  Only lo's own additions round: after
+// settle() mid and lo are at most 2^-24 and 2^-48 of hi, so while sixteen
+// values are added |mid| < 17 * 2^-24 and |lo| < 2^9 * 2^-48 of the largest
+// sum so far, and an addition loses less than 2^-63 of it, where FP64 loses
+// up to 2^-53.  Calls with FP64 sums and so, ms: 2e5
+// uniform points on 2048^2 0.443 and 0.409; track points, four tile phases, 1e6
+// on 1024^2 1.10 and 0.74, 7.8e6 on 2048^2 5.66 and 4.98.
 struct WideSum32 {
-  float hi, lo;
-  __device__ __forceinline__ explicit WideSum32(float v) : hi(v), lo(0) {}
+  float hi, mid, lo;
+  __device__ __forceinline__ explicit WideSum32(float v)
+      : hi(v), mid(0), lo(0) {}
   __device__ __forceinline__ void add(float v) {
     float e;
     two_sum(hi, v, hi, e);
+    two_sum(mid, e, mid, e);
     lo += e;
   }
-  // An infinite sum's error term is not a number.
+  __device__ __forceinline__ void settle() {
+    two_sum(hi, mid, hi, mid);
+    two_sum(mid, lo, mid, lo);
+  }
+  // The three added from the small end, rounded once (twice where the sum
+  // lies within 2^-24 of its last place from a tie).
   __device__ __forceinline__ float value() const {
-    return isfinite(hi) ? hi + lo : hi;
+    float a, b, c, d;
+    two_sum(hi, mid, a, b);
+    two_sum(b, lo, c, d);
+    two_sum(a, c, a, c);
+    return a + (c + d);
   }
 };
 struct WideSum64 {
   double s;
   __device__ __forceinline__ explicit WideSum64(double v) : s(v) {}
   __device__ __forceinline__ void add(double v) { s += v; }
+  __device__ __forceinline__ void settle() {}
   __device__ __forceinline__ double value() const { return s; }
 };
 
-// v += the n partial values at q, one per chunk, in chunk order, rounded
+// v + the n partial values at q, one per chunk, in chunk order, rounded
 // once.  Loads go out sixteen at a time: a heavy tile has hundreds of chunks,
 // and one load per addition would leave the pass waiting out a memory latency
 // for each.
-template <typename R2>
-__device__ __forceinline__ void add_chunks(R2& v, const R2* __restrict__ q,
-                                           int n) {
-  using Sum = std::conditional_t<sizeof(R2) == 8, WideSum32, WideSum64>;
-  constexpr int kAhead = sizeof(R2) == 8 ? 16 : 8;
+template <typename Sum, int kAhead, typename R2>
+__device__ __forceinline__ R2 sum_chunks(R2 v, const R2* __restrict__ q,
+                                         int n) {
   Sum sx(v.x), sy(v.y);
   int c = 0;
   for (; c + kAhead <= n; c += kAhead) {
@@ -667,6 +682,8 @@ __device__ __forceinline__ void add_chunks(R2& v, const R2* __restrict__ q,
       sx.add(t[j].x);
       sy.add(t[j].y);
     }
+    sx.settle();
+    sy.settle();
   }
   for (; c < n; ++c) {
     const R2 t = q[(size_t)c * kCells];
@@ -675,6 +692,21 @@ __device__ __forceinline__ void add_chunks(R2& v, const R2* __restrict__ q,
   }
   v.x = sx.value();
   v.y = sy.value();
+  return v;
+}
+
+// v += the n partial values at q.  An FP32 sum that leaves FP32's range on the
+// way, or meets an infinity, is formed again in FP64: only the end counts.
+template <typename R2>
+__device__ __forceinline__ void add_chunks(R2& v, const R2* __restrict__ q,
+                                           int n) {
+  if constexpr (sizeof(R2) == 8) {
+    const R2 r = sum_chunks<WideSum32, 16>(v, q, n);
+    v = isfinite(r.x) && isfinite(r.y) ? r
+                                       : sum_chunks<WideSum64, 1>(v, q, n);
+  } else {
+    v = sum_chunks<WideSum64, 8>(v, q, n);
+  }
 }
 
 // The cell of thread tid in a band of a tile (one cell per thread): its row
@@ -688,8 +720,8 @@ struct BandCell {
         entry(row % kRows * kConsumers + row / kRows * TW + col) {}
 };
 
-// grid(tile) += sum of the tile's partials in chunk order, accumulated in
-// FP64 and rounded once, for the split tiles of one plane group (a real
+// grid(tile) += sum of the tile's partials in chunk order, accumulated as
+// add_chunks does and rounded once, for the split tiles of one plane group (a real
 // tile is split at most once per group, so the blocks of one launch never
 // share a tile).  A block takes one band of a tile at a time: the chains of
 // chunks of a heavy tile, which the pass waits for, run on all its bands at
@@ -734,7 +766,7 @@ k_reduce_partials(const int4* __restrict__ split_tiles,
 // group0 .. group0 + P - 1, one launch of the gridding kernel), added to
 // the grids in one pass: a block takes two bands of a phase-0 tile position
 // at a time (two cells a thread) and adds to each cell, phase by phase, the partial tiles of the
-// tile of that phase that covers it (their chunks summed in FP64, rounded
+// tile of that phase that covers it (their chunks summed by add_chunks, rounded
 // once per phase) -- the additions, in the same order, that one reduction
 // launch per phase makes (k_reduce_partials).  A single chunk is added in
 // the grid's precision: the FP64 sum of two FP32 values rounded to FP32 is

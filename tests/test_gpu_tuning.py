@@ -8,6 +8,7 @@ it in its cache and takes it from there on the next call.
 from __future__ import annotations
 
 import importlib
+import math
 
 import numpy as np
 import pytest
@@ -293,3 +294,50 @@ def test_plane_groups_by_use(pkg, torch, n, top, groups):
     assert outs[0][1:3] == outs[1][1:3]
     if outs[0][2] < n:
         assert max_rel(outs[0][0], outs[1][0]) <= 1e-5
+
+
+@pytest.mark.parametrize("phases", [1, 4])
+@pytest.mark.parametrize("start,parts", [
+    (0.0, [2.0**28, 2.0**-23, 15.0, -2.0**28, -15.0]),
+    (-15.0, [2.0**28] * 17 + [2.0**-23, 15.0] + [-2.0**28] * 17),
+    (3e38, [3e38, -3e38]),
+    (1.0, [3e38, 3e38, -3e38, -3e38]),
+    (2e38, [2e38, 1.0]),
+    (float("inf"), [1.0, 2.0]),
+    (float("inf"), [-3e38] * 17)])
+def test_chunk_sums_keep_fp64_range_and_bits(pkg, torch, start, parts, phases):
+    """A tile's partial sums are added to the grid with an FP64 sum's range
+    and no fewer bits, then rounded once: each chunk's first record brings one
+    of `parts`, and the cell is no further from the exact sum than FP64
+    additions in chunk order leave it."""
+    G, n = 256, 64 * len(parts)
+    cube = torch.zeros((1, 2, 2, 2), dtype=torch.float32, device="cuda")
+    cube[0, 0, 0, 0] = 1.0
+    stack = pkg.KernelStack(1, np.zeros(1, np.int32), 1, 2, cube, "f")
+    vis = torch.zeros((n, 2), dtype=torch.float32, device="cuda")
+    p = torch.tensor(parts, dtype=torch.float32, device="cuda")
+    vis[::64, 0], vis[::64, 1] = p, -p
+    at = lambda v: torch.full((n,), float(v), device="cuda")
+    plan = pkg.Plan()
+    plan.set_tuning({"tile_u": 32, "tile_phases": phases})
+    grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+    grid[G // 2 + 5, G // 2 + 3, 0] = start
+    grid[G // 2 + 5, G // 2 + 3, 1] = -start
+    norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+    skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+    pkg.grid_wproj_device(plan, stack, at(-3), at(5), at(0), vis, at(1),
+                          np.float32(1 / G), np.float32(1.0), G, grid, norm,
+                          skip)
+    assert plan.stats()["chunk_records"] == 64
+    want = np.float64(np.float32(start))
+    for x in parts:
+        want += np.float64(np.float32(x))
+    with np.errstate(over="ignore"):
+        want = np.float32(want)
+    exact = math.fsum([start] + parts)
+    got = grid.cpu().numpy()
+    re, im = got[G // 2 + 5, G // 2 + 3]
+    assert re == -im
+    assert re == want or abs(re - exact) <= abs(want - exact)
+    got[G // 2 + 5, G // 2 + 3] = 0
+    assert not got.any()
