@@ -287,7 +287,7 @@ size_t prepared_record_bytes();
 // single-chunk tiles are added to the grid by the launch, every other item
 // writes a partial tile); with group_span = 1 one launch per virtual group.
 // Each launch is followed by the reduction of its virtual groups' partial
-// tiles in group order (grid += their partials in chunk order, add_chunks; all
+// tiles in group order (grid += their partials in chunk order; all
 // the phases of a launch in one pass over the grid when tile_slot, the
 // item builder's map, is given): the grid takes the groups' and phases'
 // contributions in order.
