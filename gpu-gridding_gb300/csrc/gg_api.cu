@@ -818,18 +818,22 @@ long long used_bytes(const gg_plan* plan, const gg_kernels* K) {
     taps[b] += side * side;
     ++planes[b];
   }
+  // Bins without planes (stacks of fewer than kPlaneBins) stay out: with no
+  // bytes they would compare as equal to every other.
+  int n = 0;
   for (int b = 0; b < kPlaneBins; ++b) {
-    order[b] = b;
+    if (!planes[b]) continue;
+    order[n++] = b;
     total += bytes[b];
-    taps[b] = planes[b] ? taps[b] / planes[b] * use[b] : 0.0;
+    taps[b] = taps[b] / planes[b] * use[b];
     sum += taps[b];
   }
-  std::stable_sort(order, order + kPlaneBins, [&](int a, int b) {
+  std::stable_sort(order, order + n, [&](int a, int b) {
     return taps[a] * (double)bytes[b] > taps[b] * (double)bytes[a];
   });
   double at = 0;
   long long used = 0;
-  for (int k = 0; k < kPlaneBins && at < 0.95 * sum; ++k) {
+  for (int k = 0; k < n && at < 0.95 * sum; ++k) {
     at += taps[order[k]];
     used += bytes[order[k]];
   }

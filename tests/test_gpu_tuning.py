@@ -341,3 +341,43 @@ def test_chunk_sums_keep_fp64_range_and_bits(pkg, torch, start, parts, phases):
     assert re == want or abs(re - exact) <= abs(want - exact)
     got[G // 2 + 5, G // 2 + 3] = 0
     assert not got.any()
+
+
+def _auto_groups(pkg, torch, planes, s_min, s_max, plane, seed=1):
+    """Plane groups of a default call whose points use the given planes."""
+    sup = np.rint(np.linspace(s_min, s_max, planes)).astype(np.int32)
+    stack = pkg.KernelStack.generate(planes, sup, 4, 4 * (s_max + 1),
+                                     np.full(planes, 3.0))
+    G, n = 512, len(plane)
+    rng = np.random.default_rng(seed)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    uu, vv = (dev(rng.uniform(-50.0, 50.0, n)) for _ in range(2))
+    p = np.asarray(plane, np.float64)
+    grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+    norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+    skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+    plan = pkg.Plan()
+    pkg.grid_wproj_device(plan, stack, uu, vv, dev(p * p),
+                          dev(rng.standard_normal((n, 2))),
+                          dev(rng.uniform(1, 2, n)), 0.002, np.float32(1.0),
+                          G, grid, norm, skip)
+    return plan.stats()["num_plane_groups"]
+
+
+@pytest.mark.parametrize("planes,s_min,s_max,lowest,mb", [
+    (200, 4, 72, 170, 41),     # of 118 MB
+    (128, 60, 100, 109, 55),   # of 257 MB
+    (128, 60, 100, 0, None),   # all
+    (300, 40, 72, 0, None)])   # all, more planes than bins
+def test_plane_groups_of_few_planes(pkg, torch, planes, s_min, s_max, lowest,
+                                    mb):
+    """The bytes in use of stacks with fewer planes than the sample has bins,
+    whose upper planes the points use, make the groups: three quarters of L2
+    each."""
+    p = np.random.default_rng(planes).integers(lowest, planes, 20_000)
+    if mb is None:   # 7 + 9 * (2 s + 8) rows of 2 s + 2 taps a plane
+        sup = np.rint(np.linspace(s_min, s_max, planes))
+        mb = float(np.sum(8 * (7 + 9 * (2 * sup + 8)) * (2 * sup + 2))) / 1e6
+    budget = torch.cuda.get_device_properties(0).L2_cache_size // 4 * 3
+    assert _auto_groups(pkg, torch, planes, s_min, s_max,
+                        p) == math.ceil(mb * 1e6 / budget)
