@@ -156,7 +156,7 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   unsigned long long* d_macs,
                                   uint32_t* d_shape, cudaStream_t s,
                                   int phases = 1, long long tiles = -1);
-// use[b] = how many of up to 8192 placed points, evenly taken, are gridded with
+// use[b] = how many of up to 8192 placed points, evenly spread, are gridded with
 // planes p of bin b = p * kPlaneBins / num_planes.
 constexpr int kPlaneBins = 256;
 cudaError_t launch_plane_use(const uint32_t* meta, unsigned long long n,

@@ -187,8 +187,15 @@ k_plane_use(const uint32_t* __restrict__ meta, unsigned long long n,
   uint32_t m[kEach];
 #pragma unroll
   for (int j = 0; j < kEach; ++j) {
+    // One point of each of `samples` equal stretches, at the fractional part
+    // of k times the golden ratio in it: always the first would be the same
+    // few baselines of time-major data whose baselines divide the stretch.
     const unsigned long long k = j * 1024ull + threadIdx.x;
-    m[j] = k < samples ? meta[k * n / samples] : (1u << 25);
+    const unsigned long long at = k * n / samples;
+    const unsigned long long len = (k + 1) * n / samples - at;
+    m[j] = k < samples
+               ? meta[at + (len * ((uint32_t)k * 2654435769u) >> 32)]
+               : (1u << 25);
   }
 #pragma unroll
   for (int j = 0; j < kEach; ++j)

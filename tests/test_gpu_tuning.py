@@ -381,3 +381,17 @@ def test_plane_groups_of_few_planes(pkg, torch, planes, s_min, s_max, lowest,
     budget = torch.cuda.get_device_properties(0).L2_cache_size // 4 * 3
     assert _auto_groups(pkg, torch, planes, s_min, s_max,
                         p) == math.ceil(mb * 1e6 / budget)
+
+
+@pytest.mark.parametrize("baselines", [1, 8, 64])
+def test_plane_groups_of_time_major_points(pkg, torch, baselines):
+    """The sample behind the automatic groups meets every baseline where their
+    number divides the stride of 8192 samples in time-major points: the first
+    baseline has w = 0, the others use the stack's 350 MB evenly."""
+    times = 64 * 8192 // baselines
+    rng = np.random.default_rng(baselines)
+    p = np.rint(600 * np.sqrt(rng.random((times, baselines))))
+    p[:, 0] = 0 if baselines > 1 else p[:, 0]
+    p = p.reshape(-1)
+    got = _auto_groups(pkg, torch, 601, 4, 72, p)
+    assert got == _auto_groups(pkg, torch, 601, 4, 72, rng.permutation(p)) == 4
