@@ -246,3 +246,57 @@ def test_degrid_units(pkg, oracle_mod, synthetic, torch, prec, n, size, s_min,
     tol = 36 * 2.0**-24 if prec == "f" else 150 * 2.0**-53
     assert max_rel(out.cpu().numpy(), oracle(wl, y.astype(np.float64))) <= \
         tol * (2 * s_max + 1)
+
+
+@pytest.mark.parametrize("n,size", [(20_000, 8192), (4_000, 4099)])
+def test_gridding_and_degridding_in_turn_on_one_plan(pkg, synthetic, torch, n,
+                                                     size):
+    """A plan that grids (one tile phase) and degrids (four) in turn, as a
+    training step does, gives what plans of their own give, in about their
+    time: nothing that depends on the geometry is worked out anew each time.
+    (The margin is half as much again and 0.2 ms: the tiles' order alone took
+    a millisecond a call.)"""
+    wl = synthetic.random_uniform_workload("turns", n, size, 32, 2, 8, seed=n)
+    G = wl.grid_size
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    stack = pkg.KernelStack.from_workload(wl, "f")
+    uvw = (dev(wl.uu), dev(wl.vv), dev(wl.ww))
+    vis, weight = dev(wl.vis), dev(wl.weight)
+    geometry = (np.float32(wl.cell_size_rad), np.float32(wl.w_scale), G)
+    grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+    norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+    skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+    y = dev(np.random.default_rng(1).standard_normal((G, G, 2),
+                                                     dtype=np.float32))
+
+    def step(forward, backward):
+        out = torch.empty((n, 2), dtype=torch.float32, device="cuda")
+        grid.zero_()
+        pkg.grid_wproj_device(forward, stack, *uvw, vis, weight, *geometry,
+                              grid, norm, skip)
+        pkg.degrid_wproj_device(backward, stack, *uvw, *geometry, y, out)
+        return grid.cpu(), out.cpu()
+
+    def ms(forward, backward):
+        best = float("inf")
+        for _ in range(12):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(4):
+                grid.zero_()
+                pkg.grid_wproj_device(forward, stack, *uvw, vis, weight,
+                                      *geometry, grid, norm, skip)
+                pkg.degrid_wproj_device(backward, stack, *uvw, *geometry, y,
+                                        out)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) / 4)
+        return best
+
+    out = torch.empty((n, 2), dtype=torch.float32, device="cuda")
+    one, two, three = pkg.Plan(), pkg.Plan(), pkg.Plan()
+    for _ in range(2):
+        for got, want in zip(step(one, one), step(two, three)):
+            assert torch.equal(got, want)
+    assert ms(one, one) <= 1.5 * ms(two, three) + 0.2
