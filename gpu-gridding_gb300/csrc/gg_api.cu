@@ -769,29 +769,26 @@ long long plane_bytes(const gg_kernels* K, int p) {
   return plane_taps(K->h_support[p], K->omax) * (K->is_double ? 16 : 8);
 }
 
-// Slice bytes per plane group: the plan's setting, or 3/4 of the L2 cache.
-int plane_budget(const gg_plan* plan, const gg_kernels* K, long long* budget) {
-  *budget = (long long)plan->plane_group_mb << 20;
-  if (*budget <= 0) {
-    int l2 = 0;
-    GG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, K->device));
-    *budget = std::max<long long>((long long)l2 / 4 * 3, 1 << 20);
-  }
+long long stack_bytes(const gg_kernels* K) {
+  return K->total_taps * (K->is_double ? 16 : 8);
+}
+
+// Slice bytes that a pass's taps may come from without leaving L2.
+int cache_budget(const gg_kernels* K, long long* budget) {
+  int l2 = 0;
+  GG_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, K->device));
+  *budget = gg::cache_budget(l2);
   return GG_OK;
 }
 
 // Reads the call's scalars back (the 32-bit ones and the MAC count behind
-// them) and waits for them.  Where the stack is larger than the automatic
-// budget, how much the planes are used comes with them (used_bytes).
+// them) and waits for them.  Where the stack is larger than the cache's share,
+// how much the planes are used comes with them (used_bytes).
 int read_scalars(gg_plan* plan, const gg_kernels* K, const uint32_t* meta,
                  unsigned long long n, cudaStream_t s) {
-  plan->plane_use = false;
-  if (plan->plane_group_mb <= 0 && n > 0) {
-    long long budget, total = 0;
-    GG_TRY(plane_budget(plan, K, &budget));
-    for (int p = 0; p < K->num_planes; ++p) total += plane_bytes(K, p);
-    plan->plane_use = total > budget;
-  }
+  long long budget;
+  GG_TRY(cache_budget(K, &budget));
+  plan->plane_use = n > 0 && stack_bytes(K) > budget;
   if (plan->plane_use) {
     GG_CUDA(launch_plane_use(meta, n, K->num_planes,
                              (uint32_t*)((char*)plan->scalars.p + kUseOffset),
@@ -805,7 +802,7 @@ int read_scalars(gg_plan* plan, const gg_kernels* K, const uint32_t* meta,
   return GG_OK;
 }
 
-// Slice bytes that 95 % of the call's taps come from, the most used bins of
+// Slice bytes that 95 % of the call's taps come from (read_scalars), the most used bins of
 // planes first; the whole stack where that is more than four fifths of it (one
 // used evenly).  The planes of a telescope's visibilities crowd near zero: of a stack of 327 MB (601 planes,
 // support 4 to 72), 512-station tracks take 95 % of their taps from 67 MB,
@@ -856,10 +853,13 @@ long long used_bytes(const gg_plan* plan, const gg_kernels* K) {
 // max_groups groups (the sort key's spare bits).
 // Uploads the plane -> group table when it changes; returns the number of
 // groups in *num_groups.
+// *cached: whether the slices that a group's taps come from fit the cache.
 int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
-                 cudaStream_t s, int* num_groups) {
-  long long budget;
-  GG_TRY(plane_budget(plan, K, &budget));
+                 cudaStream_t s, int* num_groups, bool* cached) {
+  long long cache;
+  GG_TRY(cache_budget(K, &cache));
+  const long long set = (long long)plan->plane_group_mb << 20;
+  const long long budget = set > 0 ? set : cache;
   max_groups = std::max(1, std::min(max_groups, 64));
   std::vector<long long> bytes(K->num_planes);
   long long total = 0;
@@ -868,14 +868,16 @@ int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
     total += bytes[p];
   }
   const long long in_use = plan->plane_use ? used_bytes(plan, K) : total;
+  const long long counted = set > 0 ? total : in_use;
   // As many groups as the budget needs, with even byte counts: plane p
   // joins the group that holds the middle of its bytes (a greedy fill to
   // the budget would leave the last group with the remainder, and the first
   // groups' slices, at the full budget, less likely to stay in L2).
   const long long want = std::min<long long>(
-      max_groups, std::max(1LL, (in_use + budget - 1) / budget));
+      max_groups, std::max(1LL, (counted + budget - 1) / budget));
   if (plan->pg_kernels == K->id && plan->pg_want == want) {
     *num_groups = plan->pg_groups;
+    *cached = in_use <= cache * plan->pg_groups;
     return GG_OK;
   }
   const double target = (double)total / (double)want;
@@ -903,6 +905,7 @@ int plane_groups(gg_plan* plan, const gg_kernels* K, int max_groups,
   plan->pg_want = want;
   plan->pg_groups = groups;
   *num_groups = groups;
+  *cached = in_use <= cache * groups;
   return GG_OK;
 }
 
@@ -1220,10 +1223,11 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
                      plan->split_row > 0 && plan->split_row < grid_size &&
                      plan->split_row % tile_v == 0;
   int pgroups = 1;
+  bool cached = true;
   GG_TRY(plane_groups(plan, K,
                       spare <= 0 ? 1
                                  : (1 << std::min(6, spare)) - (split ? 2 : 0),
-                      s, &pgroups));
+                      s, &pgroups, &cached));
   // One plane group: its two passes serve both the upload and the copy
   // back.  Otherwise the first group's split waits for the upload in two
   // halves and the last group's split overlaps the copy back.
@@ -1237,9 +1241,14 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   // and offset class (setting 2's former order): 2.15e6 uniform points on
   // 8192^2, 714 planes, two groups 4.80, 4.88, 4.93; 3.1e7 track points 22.3,
   // 22.7, 22.9; degridding 7.8e6 6.66, 6.79, 6.80; 6e5 uniform points, 601
-  // planes, four groups 5.34, 5.14, 5.16.
+  // planes, four groups 5.34, 5.14, 5.16.  When gridding, by plane
+  // too where a group's slices leave the cache (a budget was set, or the key
+  // has no bits for more groups): one group, by plane against visibility
+  // order, 8.31 and 9.04 (601 planes, 350 MB), 5.78 and 6.49 (64, 208 MB), 5.50
+  // and 6.24 (714, 179 MB); degridding gains nothing from it (9.47 and 9.34).
   const bool by_plane =
-      plan->sort_detail == 1 || (plan->sort_detail == 2 && pgroups > 2);
+      plan->sort_detail == 1 ||
+      (plan->sort_detail == 2 && (pgroups > 2 || (!cached && !degrid)));
   TileGeom geom = make_geom(shape, grid_size, num_grids, K, &key_bits,
                             by_plane, num_groups,
                             plan->plane_group.as<int>(), phases);

@@ -338,6 +338,14 @@ int record_error(int code, const char* message);
 bool kernels_info(const gg_kernels* k, StackView* view, int* device,
                   bool* is_double, int* num_planes);
 
+// Slice bytes that a gridding pass's taps may come from without leaving an L2
+// cache of l2 bytes: three quarters of it (the grid and the records stream
+// through the rest).
+inline long long cache_budget(int l2) {
+  const long long b = (long long)l2 / 4 * 3;
+  return b > (1 << 20) ? b : 1 << 20;
+}
+
 // ---- uniform weighting (gg_weights.cu) -------------------------------------
 // Keys each point by its density cell (grid_size^2 when off the grid), its
 // value the weight's bits (FP32) or its index, and counts the off-grid points into *d_num_skipped (which must start at 0).

@@ -395,3 +395,35 @@ def test_plane_groups_of_time_major_points(pkg, torch, baselines):
     p = p.reshape(-1)
     got = _auto_groups(pkg, torch, 601, 4, 72, p)
     assert got == _auto_groups(pkg, torch, 601, 4, 72, rng.permutation(p)) == 4
+
+
+@pytest.mark.parametrize("top,planes_mb,by_plane", [
+    (600, 1048576, True),    # 350 MB in one pass
+    (600, 300, True),        # 175 MB a pass
+    (120, 1048576, False),   # 5.6 MB in use
+    (600, 0, True)])         # four groups
+def test_record_order_follows_the_cache(pkg, torch, top, planes_mb, by_plane):
+    """sort_detail 2 orders a tile's records by plane where there are three
+    plane groups or more, or a pass's slices leave the cache: the launches are
+    those of sort_detail 1 (more key bits, so more sorting passes), else those
+    of sort_detail 0, and so is the grid, bit for bit."""
+    G, n = 2048, 20_000
+    sup = np.rint(np.linspace(4, 72, 601)).astype(np.int32)
+    stack = pkg.KernelStack.generate(601, sup, 4, 4 * 73, np.full(601, 3.0))
+    rng = np.random.default_rng(top)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    uu, vv = (dev(rng.uniform(-200.0, 200.0, n)) for _ in range(2))
+    p = np.rint(top * np.sqrt(rng.random(n)))
+    args = (stack, uu, vv, dev(p * p), dev(rng.standard_normal((n, 2))),
+            dev(rng.uniform(1, 2, n)), 0.002, np.float32(1.0), G)
+    outs = []
+    for detail in (2, 1 if by_plane else 0):
+        plan = pkg.Plan()
+        plan.set_tuning({"plane_group_mb": planes_mb, "sort_detail": detail})
+        grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+        norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+        skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+        pkg.grid_wproj_device(plan, *args, grid, norm, skip)
+        outs.append((plan.stats()["num_launches"], grid))
+    assert outs[0][0] == outs[1][0]
+    assert torch.equal(outs[0][1], outs[1][1])
