@@ -48,7 +48,13 @@ using namespace gg;
 constexpr size_t kNoAllocMaxPoints = size_t(1) << 17;   // 131,072
 constexpr size_t kNoAllocMaxRecords = size_t(1) << 20;  // 1,048,576
 constexpr int kNoAllocMaxGrid = 8192;
-constexpr int kNoAllocMaxSlots = 384;    // partial tiles of split tiles
+// Partial tiles of split tiles: some of their own, the others in the place of
+// the sort's keys and its unsorted values, which the tile bounds are the last
+// to read.  With the former alone a heavy call had half an item a team (601
+// planes of support 4 to 72, 6e4 points on 1024^2: 2.20 ms, so 1.25; 339 planes
+// to 60, 1e5 points on 2048^2: 1.96, 1.30).
+constexpr int kNoAllocOwnSlots = 384;
+constexpr int kNoAllocMaxSlots = 1152;
 constexpr int kNoAllocCells = 2048;      // cells per tile
 constexpr size_t kNoAllocBytes = size_t(48) << 20;
 constexpr int kMaxDevices = 64;
@@ -181,17 +187,21 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   unsigned long long* blk_macs = c.take<unsigned long long>(max_blocks);
   void* scan_tmp =
       c.take<unsigned char>(scan_temp_bytes(std::max<size_t>(maxp, max_tiles)));
-  uint32_t* keys0 = c.take<uint32_t>(maxr);
-  uint32_t* vals0 = c.take<uint32_t>(maxr);
-  uint32_t* keys1 = c.take<uint32_t>(maxr);
-  uint32_t* vals1 = c.take<uint32_t>(maxr);
+  uint32_t* vals = c.take<uint32_t>(maxr);   // sorted
   void* sort_tmp = c.take<unsigned char>(radix_temp_bytes(maxr));
   uint32_t* tile_start = c.take<uint32_t>(max_tiles + 1);
   uint32_t* item_a = c.take<uint32_t>(max_tiles + 1);
   uint32_t* item_b = c.take<uint32_t>(max_tiles + 1);
   WorkItem* items = c.take<WorkItem>(max_tiles + kNoAllocMaxSlots + 16);
   int4* split_tiles = c.take<int4>(max_tiles + 1);
-  float2* partials = c.take<float2>((size_t)kNoAllocMaxSlots * kNoAllocCells);
+  float2* partials = c.take<float2>((size_t)kNoAllocOwnSlots * kNoAllocCells);
+  uint32_t* keys0 = c.take<uint32_t>(maxr);
+  uint32_t* keys1 = c.take<uint32_t>(maxr);
+  uint32_t* vals_other = c.take<uint32_t>(maxr);
+  static_assert((kNoAllocMaxSlots - kNoAllocOwnSlots) * kNoAllocCells *
+                        sizeof(float2) ==
+                    3 * kNoAllocMaxRecords * sizeof(uint32_t),
+                "the partial tiles run through the sort's buffers");
   unsigned char* recs =
       c.take<unsigned char>(maxr * prepared_record_bytes<float>());
   unsigned short* spans = c.take<unsigned short>(maxr);
@@ -268,13 +278,18 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   const int tile_bits = ceil_log2_u((unsigned long long)num_tiles);
   geom.plane_bits = 0;   // records of a tile in visibility order
 
+  // The sort ends in `vals`: it starts there if its passes are even in number.
+  const bool odd = total > 1 && radix_passes(tile_bits) % 2 == 1;
+  uint32_t* vals0 = odd ? vals_other : vals;
+  uint32_t* vals1 = odd ? vals : vals_other;
   NA_CUDA(launch_emit_records(cell, meta, offset, num_points, view, geom, 0,
                               0, keys0, vals0, s));
   bool in_alt = false;
   NA_CUDA(radix_sort_pairs(keys0, vals0, keys1, vals1, total,
                            tile_bits, sort_tmp, s, &in_alt));
+  if (in_alt != odd)
+    return record_error(GG_ERR_CUDA, "internal: sort pass count mismatch");
   const uint32_t* keys = in_alt ? keys1 : keys0;
-  const uint32_t* vals = in_alt ? vals1 : vals0;
   NA_CUDA(launch_tile_bounds(keys, total, 0, num_tiles, tile_start,
                              s));
   int sms = 0;

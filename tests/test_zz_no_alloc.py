@@ -216,3 +216,61 @@ def test_noalloc_reports_an_earlier_bounded_wait_failure(pkg, synthetic):
     torch.cuda.synchronize()
     assert int(outs[2].item()) == 0
     assert probe(0, None) == 1   # iterations outside 1..1048576
+
+
+@pytest.mark.parametrize("G", [1024, 4096])
+def test_noalloc_heavy_tiles(pkg, G):
+    """Calls whose tiles are split over all of the array's partial tiles (some
+    of them in the place of the sort's buffers): the grid is a plan's within
+    the tuning tests' bound, norm and skips are equal, and so is the time but
+    for the last items: some 580 of them for 380 teams of warps take at most
+    two turns where one and a half would do, 4/3, and 0.1 ms for the launches."""
+    import torch
+    fn = _noalloc_fn(pkg.lib())
+    n = 60_000
+    sup = np.rint(np.linspace(4, 72, 601)).astype(np.int32)
+    stack = pkg.KernelStack.generate(601, sup, 4, 4 * 73, np.full(601, 3.0))
+    rng = np.random.default_rng(G)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    r = 0.12 * np.abs(rng.standard_normal(n)).clip(max=3.0) / 0.002
+    t = rng.uniform(0, 2 * np.pi, n)
+    p = np.rint(600 * np.sqrt(rng.random(n)))
+    arrs = (dev(r * np.cos(t)), dev(r * np.sin(t)),
+            dev(p * p * rng.choice([-1.0, 1.0], n)),
+            dev(rng.standard_normal((n, 2))), dev(rng.uniform(1, 2, n)))
+    cell, wsc = np.float32(0.002), np.float32(1.0)
+    stream = torch.cuda.current_stream()
+    plan = pkg.Plan()
+    plan.set_tuning({"tile_phases": 1, "sort_detail": 0,
+                     "plane_group_mb": 1048576})
+    uu, vv, ww, vis, weight = arrs
+
+    def by_plan(grid, norm, skip):
+        pkg.grid_wproj_device(plan, stack, uu, vv, ww, vis, weight, cell, wsc,
+                              G, grid, norm, skip, stream)
+
+    def noalloc(grid, norm, skip):
+        assert _call(fn, stack, n, arrs, cell, wsc, G, (grid, norm, skip),
+                     stream) == 0, pkg.last_error()
+
+    ms, outs = [], []
+    for f in (by_plan, noalloc):
+        o = (torch.zeros((G, G, 2), dtype=torch.float32, device="cuda"),
+             torch.zeros(1, dtype=torch.float64, device="cuda"),
+             torch.zeros(1, dtype=torch.int64, device="cuda"))
+        f(*o)
+        torch.cuda.synchronize()
+        outs.append([x.cpu().numpy().copy() for x in o])
+        best = float("inf")
+        for _ in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            for _ in range(3):
+                f(*o)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b) / 3)
+        ms.append(best)
+    assert outs[0][2] == outs[1][2] and outs[0][1] == outs[1][1]
+    assert max_rel(outs[1][0], outs[0][0]) <= 1e-5
+    assert ms[1] <= 4.0 / 3.0 * ms[0] + 0.1
