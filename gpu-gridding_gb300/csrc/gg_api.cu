@@ -69,6 +69,10 @@ int set_error(int code, const char* fmt, ...) {
 // ===========================================================================
 // Device buffers
 // ===========================================================================
+// Set while a call makes its second attempt after an allocation failed: its
+// buffers get no headroom and its optional ones are left out (with_memory).
+thread_local bool t_tight = false;
+
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -81,11 +85,12 @@ struct DevBuf {
     p = nullptr;
     bytes = 0;
   }
-  // Grows to at least n bytes (with 25% headroom); contents are not kept.
+  // Grows to at least n bytes (with 25% headroom, see t_tight); contents are
+  // not kept.
   int ensure(size_t n) {
     if (n <= bytes && p) return GG_OK;
     release();
-    size_t want = std::max<size_t>(n + n / 4, 256);
+    size_t want = std::max<size_t>(t_tight ? n : n + n / 4, 256);
     cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
       p = nullptr;
@@ -537,10 +542,15 @@ int kernels_create(gg_kernels** out, size_t num_w_planes, const int* support,
 // ===========================================================================
 struct gg_plan {
   int device = 0;
-  DevBuf cell, meta, placed, rec_count, rec_offset;
+  DevBuf placed, rec_count, rec_offset;   // placed: PlacedPoints
   DevBuf blk_norm, blk_skip, blk_macs;
-  DevBuf keys0, vals0, keys1, vals1, sort_tmp, scan_tmp;
-  DevBuf recs, rec_spans;   // prepared records (launch_grid_tiles)
+  // The sorted values; and, for as long as a call needs them, the sort's keys
+  // and its other side of the values (SortParts) and, in their place once the
+  // tile bounds are known, the prepared records (RecordParts).
+  DevBuf vals, work, sort_tmp, scan_tmp;
+  size_t work_refused = SIZE_MAX;   // smallest size that work could not get
+  size_t tight_from = SIZE_MAX;  // points of calls that are short of memory
+  bool norm_added = false;  // the call's norm has reached the caller's
   DevBuf tile_start, item_a, item_b, items, split_tiles, partials, tile_slot;
   DevBuf scalars;  // device scalars, see Scalar below
   uint32_t* h_scalars = nullptr;  // pinned mirror
@@ -562,9 +572,9 @@ struct gg_plan {
   long long call_tiles = -1;
   // Batched calls larger than one sort can index (see batched_split): the
   // grids are cut into sub-batches, each gridded by its own sub-plan, which
-  // keeps its geometry for replays.  A sub-plan takes the sort's transient
-  // buffers (keys, the unsorted side of the values, sort and count scratch)
-  // from `scratch`, its parent, so they exist once.
+  // keeps its geometry for replays.  A sub-plan takes the transient buffers
+  // (`work`, sort and count scratch) from `scratch`, its parent, so they exist
+  // once.
   gg_plan* scratch = nullptr;
   // Inputs of a host call arriving in pieces (set by the drop-in around
   // its gridding pipeline): placement of points [in_chunk_end[k-1],
@@ -645,7 +655,7 @@ struct gg_plan {
   DevBuf tile_groups;
   bool direct_launched = false;
   // Geometry kept by the last batched call for replays on new amplitudes:
-  // placement (cell, meta), sorted records, work items and launch shape.
+  // placement, sorted values, work items and launch shape.
   struct Kept {
     bool valid = false;
     const gg_kernels* kernels = nullptr;
@@ -665,6 +675,15 @@ struct gg_plan {
   }
   void mark(int i, cudaStream_t s) {
     if (profile) cudaEventRecord(ev[i], s);
+  }
+  // Frees what the calls work in (not a host call's uploaded inputs).
+  void release_scratch() {
+    for (DevBuf* b : {&placed, &rec_count, &rec_offset, &blk_norm, &blk_skip,
+                      &blk_macs, &vals, &work, &sort_tmp, &scan_tmp,
+                      &tile_start, &item_a, &item_b, &items, &split_tiles,
+                      &partials, &tile_slot, &nterm, &chunk_part, &rec_out})
+      b->release();
+    work_refused = SIZE_MAX;
   }
 };
 
@@ -692,6 +711,76 @@ enum Scalar64 {
 // Behind those, launch_plane_use's bins.
 constexpr size_t kUseOffset = kScalar64Offset + kScalar64Count * 8;
 constexpr size_t kScalarBytes = kUseOffset + kPlaneBins * 4;
+
+// Runs the allocations and launches of a call of n points, `call`.  Where an
+// allocation fails they run once more on buffers allocated anew: without
+// headroom, without those that only save time (prepared records, degridding's
+// slots beside the points), and with work items as coarse as four for each of
+// two blocks an SM (FP64 one), so that the call takes no more memory than its
+// points and the sort of its records need.  Later calls of half as many points
+// or more on the plan run so at once.
+template <typename F>
+int with_memory(gg_plan* plan, size_t n, F call) {
+  struct Restore {
+    const bool before = t_tight;
+    ~Restore() { t_tight = before; }
+  } restore;
+  plan->norm_added = false;
+  t_tight = n >= plan->tight_from;
+  const int r = call();
+  if (r != GG_ERR_NO_MEMORY) return r;
+  plan->release_scratch();
+  if (plan->scratch) plan->scratch->release_scratch();
+  plan->tight_from = std::min(plan->tight_from, std::max<size_t>(n / 2, 1));
+  t_tight = true;
+  t_last_error.clear();
+  return call();
+}
+
+constexpr size_t round_256(size_t n) { return (n + 255) & ~size_t(255); }
+
+// The sort's transient arrays of n records in a work buffer, and the prepared
+// records that follow in their place.
+struct SortParts {
+  uint32_t *keys0, *keys1, *vals;
+  SortParts(const DevBuf& work, size_t n) {
+    const size_t a = round_256(n * 4);
+    keys0 = work.as<uint32_t>();
+    keys1 = (uint32_t*)(work.as<char>() + a);
+    vals = (uint32_t*)(work.as<char>() + 2 * a);
+  }
+  static size_t bytes(size_t n) { return 3 * round_256(n * 4); }
+};
+template <typename Real>
+struct RecordParts {
+  void* recs = nullptr;              // null: not prepared
+  unsigned short* spans = nullptr;
+  RecordParts(const DevBuf& work, size_t n) {
+    if (!work.p || work.bytes < bytes(n)) return;
+    recs = work.p;
+    spans = (unsigned short*)(work.as<char>() +
+                              round_256(n * prepared_record_bytes<Real>()));
+  }
+  static size_t bytes(size_t n) {
+    return round_256(n * prepared_record_bytes<Real>()) + n * 2;
+  }
+};
+
+// plan's work buffer for sorting n records, and for preparing them too where
+// that much memory can be had.
+template <typename Real>
+int ensure_work(gg_plan* plan, size_t n, bool prepare) {
+  const size_t sort = SortParts::bytes(n);
+  const size_t both = std::max(sort, RecordParts<Real>::bytes(n));
+  DevBuf& w = plan->work;
+  if (prepare && !t_tight &&
+      (both <= w.bytes || both < plan->work_refused || sort > w.bytes)) {
+    if (w.ensure(both) == GG_OK) return GG_OK;
+    plan->work_refused = both;
+    t_last_error.clear();
+  }
+  return w.ensure(sort);
+}
 
 unsigned long long* scalar64(gg_plan* p, int i) {
   return (unsigned long long*)((char*)p->scalars.p + kScalar64Offset) + i;
@@ -784,13 +873,13 @@ int cache_budget(const gg_kernels* K, long long* budget) {
 // Reads the call's scalars back (the 32-bit ones and the MAC count behind
 // them) and waits for them.  Where the stack is larger than the cache's share,
 // how much the planes are used comes with them (used_bytes).
-int read_scalars(gg_plan* plan, const gg_kernels* K, const uint32_t* meta,
+int read_scalars(gg_plan* plan, const gg_kernels* K, PlacedPoints points,
                  unsigned long long n, cudaStream_t s) {
   long long budget;
   GG_TRY(cache_budget(K, &budget));
   plan->plane_use = n > 0 && stack_bytes(K) > budget;
   if (plan->plane_use) {
-    GG_CUDA(launch_plane_use(meta, n, K->num_planes,
+    GG_CUDA(launch_plane_use(points, n, K->num_planes,
                              (uint32_t*)((char*)plan->scalars.p + kUseOffset),
                              s));
     plan->stats.num_launches += 1;
@@ -1018,13 +1107,15 @@ int grid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
     GG_CUDA(cudaMemsetAsync(d_num_skipped, 0, sizeof(unsigned long long), s));
     return GG_OK;
   }
-  PlaceOut po;
   plan->call_phases = gridding_phases<Real>(plan, grid_size, 1);
   plan->call_tiles = grid_tiles(grid_size, 1);
-  GG_TRY(place_and_count<Real>(plan, K, pp, plan->forced_shape, d_norm,
-                               d_num_skipped, s, &po));
-  return bin_and_grid<Real>(plan, K, n, po, grid_size, 1, nullptr, d_grid, 0,
-                            s);
+  return with_memory(plan, n, [&]() -> int {
+    PlaceOut po;
+    GG_TRY(place_and_count<Real>(plan, K, pp, plan->forced_shape, d_norm,
+                                 d_num_skipped, s, &po));
+    return bin_and_grid<Real>(plan, K, n, po, grid_size, 1, nullptr, d_grid, 0,
+                              s);
+  });
 }
 
 // The first half of a single-grid call, shared by gridding and degridding:
@@ -1041,9 +1132,9 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
   const size_t n = pp.num_points;
   const int tiles_cap = max_tiles(pp.grid_size, 1);
   const int nblk = place_num_blocks(n);
-  GG_TRY(plan->cell.ensure(n * 4 + 4));
-  GG_TRY(plan->meta.ensure(n * 4 + 4));
-  if (pp.vis) GG_TRY(plan->placed.ensure(n * sizeof(Placed<Real>)));
+  const unsigned stride =
+      pp.vis ? sizeof(Placed<Real>) : t_tight ? sizeof(uint2) : sizeof(uint4);
+  GG_TRY(plan->placed.ensure(n * stride));
   GG_TRY(plan->rec_count.ensure(n * 4 + 4));
   GG_TRY(plan->rec_offset.ensure(n * 4 + 4));
   GG_TRY(plan->blk_norm.ensure(nblk * sizeof(double)));
@@ -1054,9 +1145,7 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
 
   plan->mark(0, s);
   PlaceOut po;
-  po.cell = plan->cell.as<uint32_t>();
-  po.meta = plan->meta.as<uint32_t>();
-  po.placed = pp.vis ? plan->placed.p : nullptr;
+  po.points = {plan->placed.as<unsigned char>(), stride};
   po.rec_count = plan->rec_count.as<uint32_t>();
   po.blk_norm = plan->blk_norm.as<double>();
   po.blk_skip = plan->blk_skip.as<unsigned long long>();
@@ -1076,10 +1165,7 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
       pk.weight = pp.weight ? pp.weight + a : nullptr;
       pk.num_points = b - a;
       PlaceOut ok = po;
-      ok.cell = po.cell + a;
-      ok.meta = po.meta + a;
-      ok.placed =
-          po.placed ? (void*)((Placed<Real>*)po.placed + a) : nullptr;
+      ok.points.p = po.points.p + a * stride;
       const size_t blk = a / kPlaceBlock;
       ok.blk_norm = po.blk_norm + blk;
       ok.blk_skip = po.blk_skip + blk;
@@ -1092,17 +1178,19 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
   }
   GG_CUDA(launch_place_finalize(po.blk_norm, po.blk_skip, po.blk_macs, nblk,
                                 n, forced_shape,
-                                pp.defer_norm ? nullptr : d_norm,
+                                pp.defer_norm || plan->norm_added ? nullptr
+                                                                  : d_norm,
                                 d_num_skipped, scalar64(plan, kMacs),
                                 sc + kShape, s, plan->call_phases, plan->call_tiles));
-  GG_CUDA(launch_count_records(po.cell, po.meta, n, view, sc + kShape,
-                               po.rec_count, s));
+  if (!pp.defer_norm) plan->norm_added = true;
+  GG_CUDA(launch_count_records(po.points, n, view, sc + kShape, po.rec_count,
+                               s));
   GG_CUDA(exclusive_scan_u32(po.rec_count, plan->rec_offset.as<uint32_t>(), n,
                              sc + kTotalRecords, plan->scan_tmp.p, s));
   // place, finalize, count, scan
   plan->stats.num_launches = 3 + scan_launches(n);
   plan->mark(1, s);
-  GG_TRY(read_scalars(plan, K, po.meta, n, s));
+  GG_TRY(read_scalars(plan, K, po.points, n, s));
   *po_out = po;
   return GG_OK;
 }
@@ -1280,7 +1368,6 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   if (degrid) {
     GG_TRY(tile_queue_order(plan, geom, grid_size, true, s, &b->tile_order,
                             &tile_rank));
-    GG_TRY(plan->placed.ensure(n * 16));
   }
 
   // The sorted values stay with the plan (replays read them); the keys,
@@ -1289,27 +1376,23 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   gg_plan* T = plan->scratch ? plan->scratch : plan;
   const bool alt_final =
       total > 1 && key_bits > 0 && radix_passes(key_bits) % 2 == 1;
-  DevBuf& v0 = alt_final ? T->vals0 : plan->vals0;
-  DevBuf& v1 = alt_final ? plan->vals1 : T->vals1;
-  GG_TRY(T->keys0.ensure((size_t)total * 4));
-  GG_TRY(v0.ensure((size_t)total * 4));
-  GG_TRY(T->keys1.ensure((size_t)total * 4));
-  GG_TRY(v1.ensure((size_t)total * 4));
+  GG_TRY(ensure_work<Real>(T, total, !degrid));
+  GG_TRY(plan->vals.ensure((size_t)total * 4));
   GG_TRY(T->sort_tmp.ensure(radix_temp_bytes(total)));
-  GG_CUDA(launch_emit_records(po.cell, po.meta,
-                              T->rec_offset.as<uint32_t>(), n, view, geom,
-                              0, 0, T->keys0.as<uint32_t>(),
-                              v0.as<uint32_t>(), s, d_grid_offsets,
+  const SortParts sort(T->work, total);
+  uint32_t* v0 = alt_final ? sort.vals : plan->vals.as<uint32_t>();
+  uint32_t* v1 = alt_final ? plan->vals.as<uint32_t>() : sort.vals;
+  GG_CUDA(launch_emit_records(po.points, T->rec_offset.as<uint32_t>(), n, view,
+                              geom, 0, 0, sort.keys0, v0, s, d_grid_offsets,
                               num_grids, tile_rank,
-                              degrid ? plan->placed.p : nullptr));
+                              degrid && po.points.stride == 16));
   bool in_alt = false;
-  GG_CUDA(radix_sort_pairs(T->keys0.as<uint32_t>(), v0.as<uint32_t>(),
-                           T->keys1.as<uint32_t>(), v1.as<uint32_t>(), total,
-                           key_bits, T->sort_tmp.p, s, &in_alt));
+  GG_CUDA(radix_sort_pairs(sort.keys0, v0, sort.keys1, v1, total, key_bits,
+                           T->sort_tmp.p, s, &in_alt));
   if (in_alt != alt_final)
     return set_error(GG_ERR_CUDA, "internal: sort pass count mismatch");
-  b->keys = in_alt ? T->keys1.as<uint32_t>() : T->keys0.as<uint32_t>();
-  b->vals = in_alt ? v1.as<uint32_t>() : v0.as<uint32_t>();
+  b->keys = in_alt ? sort.keys1 : sort.keys0;
+  b->vals = plan->vals.as<uint32_t>();
   plan->stats.num_launches += 1 + radix_launches(total, key_bits);
   plan->mark(2, s);
   if (degrid) return GG_OK;
@@ -1356,6 +1439,13 @@ int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
     records = std::max(records,
                        std::min(512ull, (unsigned long long)b.total /
                                              (2ull * passes * num_ctas)));
+  if (t_tight) {
+    int sms = 0;
+    GG_TRY(num_sms_of_current(&sms));
+    const unsigned long long items =
+        4ull * passes * sms * (sizeof(Real) == 4 ? 2 : 1);
+    records = std::max(records, (b.total + items - 1) / items);
+  }
   const uint32_t chunk =
       (uint32_t)std::max<unsigned long long>(64, records);
   const size_t slot_cap = 2 * (size_t)(b.total / chunk) + 16;
@@ -1422,8 +1512,9 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   if (plan->stack_wait) {
     // The stack was built beside placement and binning.
     GG_CUDA(cudaStreamWaitEvent(s, plan->stack_wait, 0));
-    if (plan->norm_out) {
-      GG_CUDA(launch_norm_terms<Real>(po.meta, (const Real*)plan->norm_weight,
+    if (plan->norm_out && !plan->norm_added) {
+      plan->norm_added = true;
+      GG_CUDA(launch_norm_terms<Real>(po.points, (const Real*)plan->norm_weight,
                                       n, view, plan->blk_norm.as<double>(),
                                       plan->norm_out, s));
       plan->stats.num_launches += 2;
@@ -1508,13 +1599,11 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
     plan->stats.num_launches += 1;
   }
   gg_plan* T = plan->scratch ? plan->scratch : plan;
-  GG_TRY(T->recs.ensure((size_t)b.total * prepared_record_bytes<Real>()));
-  GG_TRY(T->rec_spans.ensure((size_t)b.total * 2));
+  const RecordParts<Real> prepared(T->work, b.total);
   plan->mark(3, s);
   GG_CUDA(launch_grid_tiles<Real>(
-      ib.items, ib.group_items, ib.counter, T->recs.p,
-      T->rec_spans.as<unsigned short>(), b.vals,
-      po.placed, view, geom, grid_size, d_grid, grid_stride,
+      ib.items, ib.group_items, ib.counter, prepared.recs, prepared.spans,
+      b.vals, po.points.p, view, geom, grid_size, d_grid, grid_stride,
       plan->partials.as<Real>(), ib.split_tiles, ib.num_split, b.num_tiles,
       num_ctas, s, wait_before.data(), record_after.data(),
       (Real*)plan->host_grid, tile_groups, span, plan->tile_slot.as<int2>(),
@@ -1524,7 +1613,8 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   plan->mark(5, s);
   // each gridding launch and its partial reduction (one per virtual group,
   // or one over all the phases of a launch)
-  plan->stats.num_launches += 1 + 2 * (b.num_groups / span);
+  plan->stats.num_launches +=
+      (prepared.recs ? 1 : 0) + 2 * (b.num_groups / span);
   plan->events_valid = plan->profile;
   return GG_OK;
 }
@@ -1534,12 +1624,12 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
 // grid is d_grids + g * grid_size^2 * 2.  One placement pass, one sort and
 // one persistent tile-gridding launch cover every grid.
 template <typename Real>
-int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
-                     const unsigned long long* h_offsets, const Real* uu,
-                     const Real* vv, const Real* ww, const Real* vis,
-                     const Real* weight, Real cell_size_rad, Real w_scale,
-                     int grid_size, unsigned long long* d_num_skipped,
-                     double* d_norm, Real* d_grids, cudaStream_t s) {
+int batched_attempt(gg_plan* plan, const gg_kernels* K, int num_grids,
+                    const unsigned long long* h_offsets, const Real* uu,
+                    const Real* vv, const Real* ww, const Real* vis,
+                    const Real* weight, Real cell_size_rad, Real w_scale,
+                    int grid_size, unsigned long long* d_num_skipped,
+                    double* d_norm, Real* d_grids, cudaStream_t s) {
   if (!plan || !K) return set_error(GG_ERR_INVALID_ARG, "plan or kernels is NULL");
   if (K->is_double != (sizeof(Real) == 8))
     return set_error(GG_ERR_INVALID_ARG,
@@ -1596,8 +1686,6 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   const int num_chunks = (int)chunk_begin.size();
   chunk_begin.push_back(n);
 
-  GG_TRY(plan->cell.ensure(n * 4 + 4));
-  GG_TRY(plan->meta.ensure(n * 4 + 4));
   GG_TRY(plan->placed.ensure((n + 1) * sizeof(Placed<Real>)));
   // Counts and offsets of records per visibility: transient (a sub-plan
   // takes its parent's).
@@ -1628,9 +1716,7 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   pp.grid_centre = grid_size / 2;
   pp.num_points = n;
   PlaceOut po;
-  po.cell = plan->cell.as<uint32_t>();
-  po.meta = plan->meta.as<uint32_t>();
-  po.placed = plan->placed.p;
+  po.points = {plan->placed.as<unsigned char>(), sizeof(Placed<Real>)};
   po.rec_count = T->rec_count.as<uint32_t>();
   po.blk_norm = nullptr;
   po.blk_skip = nullptr;
@@ -1643,19 +1729,21 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   GG_CUDA(launch_place_batched<Real>(pp, view, po, plan->nterm.as<double>(),
                                      s));
   GG_CUDA(launch_batch_totals(
-      po.meta, plan->nterm.as<double>(), view, num_chunks,
+      po.points, plan->nterm.as<double>(), view, num_chunks,
       plan->chunk_begin.as<unsigned long long>(), num_grids,
       plan->grid_chunk0.as<int>(), cp.norm, cp.skip, cp.macs,
-      plan->forced_shape, d_norm, d_num_skipped, scalar64(plan, kMacs),
-      sc + kShape, s, plan->call_phases, plan->call_tiles));
-  GG_CUDA(launch_count_records(po.cell, po.meta, n, view, sc + kShape,
-                               po.rec_count, s));
+      plan->forced_shape, plan->norm_added ? nullptr : d_norm, d_num_skipped,
+      scalar64(plan, kMacs), sc + kShape, s, plan->call_phases,
+      plan->call_tiles));
+  plan->norm_added = true;
+  GG_CUDA(launch_count_records(po.points, n, view, sc + kShape, po.rec_count,
+                               s));
   GG_CUDA(exclusive_scan_u32(po.rec_count, T->rec_offset.as<uint32_t>(), n,
                              sc + kTotalRecords, plan->scan_tmp.p, s));
   // place, chunk totals, finalize, count, scan
   plan->stats.num_launches = (num_chunks > 0 ? 4 : 3) + scan_launches(n);
   plan->mark(1, s);
-  GG_TRY(read_scalars(plan, K, po.meta, n, s));
+  GG_TRY(read_scalars(plan, K, po.points, n, s));
   GG_TRY(bin_and_grid<Real>(plan, K, n, po, grid_size, num_grids,
                             plan->grid_offsets.as<unsigned long long>(),
                             d_grids, grid_stride, s));
@@ -1668,6 +1756,16 @@ int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
   kp.num_chunks = num_chunks;
   kp.valid = true;
   return GG_OK;
+}
+
+template <typename Real, typename... Args>
+int batched_pipeline(gg_plan* plan, const gg_kernels* K, int num_grids,
+                     const unsigned long long* h_offsets, Args... args) {
+  if (!plan || num_grids < 1 || !h_offsets)
+    return set_error(GG_ERR_INVALID_ARG, "need a plan, a grid and offsets");
+  return with_memory(plan, h_offsets[num_grids], [&]() -> int {
+    return batched_attempt<Real>(plan, K, num_grids, h_offsets, args...);
+  });
 }
 
 // A batched call whose records might not fit the 32-bit record indices of
@@ -1809,22 +1907,23 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
   view.wide |= kp.num_records >= kWideRecords;
   uint32_t* sc = plan->scalars.as<uint32_t>();
   const ChunkParts cp = chunk_parts(plan, kp.num_chunks);
-  GG_CUDA(launch_revalue<Real>(vis, weight, plan->meta.as<uint32_t>(), view,
-                               kp.num_points, plan->placed.p,
-                               plan->nterm.as<double>(), s));
+  GG_CUDA(launch_revalue<Real>(vis, weight, view, kp.num_points,
+                               plan->placed.p, plan->nterm.as<double>(), s));
   GG_CUDA(launch_batch_totals(
-      plan->meta.as<uint32_t>(), plan->nterm.as<double>(), view,
+      {plan->placed.as<unsigned char>(), sizeof(Placed<Real>)}, plan->nterm.as<double>(), view,
       kp.num_chunks, plan->chunk_begin.as<unsigned long long>(),
       kp.num_grids, plan->grid_chunk0.as<int>(), cp.norm, cp.skip, cp.macs,
       kp.shape, d_norm, d_num_skipped, scalar64(plan, kMacs), sc + kShape,
       s));
   if (kp.num_records == 0) return GG_OK;
   const long long grid_stride = 2LL * kp.grid_size * kp.grid_size;
-  gg_plan* T = plan->scratch ? plan->scratch : plan;
+  // A sub-plan's records go where its parent's last sub-batch had them, if that
+  // is large enough.
+  const RecordParts<Real> prepared(
+      plan->scratch ? plan->scratch->work : plan->work, kp.num_records);
   GG_CUDA(launch_grid_tiles<Real>(
       plan->items.as<WorkItem>(), plan->group_items.as<uint32_t>(),
-      sc + kCounter, T->recs.p, T->rec_spans.as<unsigned short>(), kp.rec_vis,
-      plan->placed.p, view, kp.geom, kp.grid_size,
+      sc + kCounter, prepared.recs, prepared.spans, kp.rec_vis, plan->placed.p, view, kp.geom, kp.grid_size,
       d_grids, grid_stride, plan->partials.as<Real>(),
       plan->split_tiles.as<int4>(), sc + kNumSplit, kp.num_tiles, kp.num_ctas,
       s, nullptr, nullptr, nullptr, nullptr, kp.group_span,
@@ -1872,41 +1971,43 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
   plan->subs_valid = false;
   const size_t n = num_points;
   const StackView view = K->view();
-  PlaceOut po;
   plan->call_phases = gridding_phases<Real>(plan, grid_size, 1, true);
   plan->call_tiles = -1;
-  GG_TRY(place_and_count<Real>(plan, K, pp, kDegridShape, nullptr, nullptr, s,
-                               &po));
-  Bins b;
-  GG_TRY(bin_records<Real>(plan, K, n, po, grid_size, 1, nullptr, s, &b,
-                           true));
-  if (b.total == 0) {
-    GG_CUDA(cudaMemsetAsync(d_out, 0, 2 * n * sizeof(Real), s));
+  return with_memory(plan, n, [&]() -> int {
+    PlaceOut po;
+    GG_TRY(place_and_count<Real>(plan, K, pp, kDegridShape, nullptr, nullptr, s,
+                                 &po));
+    Bins b;
+    GG_TRY(bin_records<Real>(plan, K, n, po, grid_size, 1, nullptr, s, &b,
+                             true));
+    if (b.total == 0) {
+      GG_CUDA(cudaMemsetAsync(d_out, 0, 2 * n * sizeof(Real), s));
+      return GG_OK;
+    }
+    if (b.total > 0x7FFFFFFFu)
+      return set_error(GG_ERR_UNSUPPORTED,
+                       "%u records: degridding takes at most 2^31 - 1 per call",
+                       b.total);
+    int sms = 0;
+    GG_TRY(num_sms_of_current(&sms));
+    int per_sm = degrid_tiles_ctas_per_sm<Real>(view.wide);
+    if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
+    const int num_ctas = sms * per_sm;
+    plan->stats.num_ctas = num_ctas;
+    GG_TRY(plan->rec_out.ensure((size_t)b.total * 2 * sizeof(Real)));
+    uint32_t* sc = plan->scalars.as<uint32_t>();
+    if (plan->grid_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->grid_wait, 0));
+    if (plan->stack_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->stack_wait, 0));
+    GG_CUDA(launch_degrid_tiles<Real>(
+        b.keys, b.vals, b.total, b.low_bits, b.tile_order, po.points,
+        plan->rec_offset.as<uint32_t>(), sc + kCounter, view, b.geom,
+        grid_size, d_grid, plan->rec_out.p, num_ctas, s));
+    GG_CUDA(launch_degrid_finish<Real>(po.rec_count,
+                                       plan->rec_offset.as<uint32_t>(),
+                                       plan->rec_out.p, n, d_out, s));
+    plan->stats.num_launches += 2;
     return GG_OK;
-  }
-  if (b.total > 0x7FFFFFFFu)
-    return set_error(GG_ERR_UNSUPPORTED,
-                     "%u records: degridding takes at most 2^31 - 1 per call",
-                     b.total);
-  int sms = 0;
-  GG_TRY(num_sms_of_current(&sms));
-  int per_sm = degrid_tiles_ctas_per_sm<Real>(view.wide);
-  if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
-  const int num_ctas = sms * per_sm;
-  plan->stats.num_ctas = num_ctas;
-  GG_TRY(plan->rec_out.ensure((size_t)b.total * 2 * sizeof(Real)));
-  uint32_t* sc = plan->scalars.as<uint32_t>();
-  if (plan->grid_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->grid_wait, 0));
-  if (plan->stack_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->stack_wait, 0));
-  GG_CUDA(launch_degrid_tiles<Real>(
-      b.keys, b.vals, b.total, b.low_bits, b.tile_order, plan->placed.p,
-      sc + kCounter, view, b.geom, grid_size, d_grid, plan->rec_out.p,
-      num_ctas, s));
-  GG_CUDA(launch_degrid_finish<Real>(po.rec_count,
-                                     plan->rec_offset.as<uint32_t>(),
-                                     plan->rec_out.p, n, d_out, s));
-  plan->stats.num_launches += 2;
-  return GG_OK;
+  });
 }
 
 // True when every page of [p, p + bytes) is resident.  A page the process
@@ -2082,13 +2183,16 @@ int dropin(size_t num_w_planes, const int* support, int oversample,
   const size_t n = num_points;
   const size_t grid_bytes = (size_t)grid_size * grid_size * 2 * sizeof(Real);
   const size_t row_bytes = (size_t)grid_size * 2 * sizeof(Real);
-  GG_TRY(plan->in_grid.ensure(grid_bytes));
-  GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_ww.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vis.ensure(2 * n * sizeof(Real) + 16));
-  GG_TRY(plan->in_weight.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_misc.ensure(64));
+  GG_TRY(with_memory(plan, n, [&]() -> int {
+    GG_TRY(plan->in_grid.ensure(grid_bytes));
+    GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_ww.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vis.ensure(2 * n * sizeof(Real) + 16));
+    GG_TRY(plan->in_weight.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_misc.ensure(64));
+    return GG_OK;
+  }));
   double* d_norm = plan->in_misc.as<double>();
   unsigned long long* d_skip = (unsigned long long*)(plan->in_misc.as<char>() + 8);
   GG_TRY(ensure_copy_stream(st));
@@ -2354,29 +2458,25 @@ int weights_write_pipeline(gg_plan* plan, size_t n, const Real* uu,
   plan->subs_valid = false;
   GG_CUDA(cudaMemsetAsync(d_num_skipped, 0, sizeof(unsigned long long), s));
   if (n == 0) return GG_OK;
-  GG_TRY(plan->keys0.ensure(n * 4));
-  GG_TRY(plan->vals0.ensure(n * 4));
-  GG_TRY(plan->keys1.ensure(n * 4));
-  GG_TRY(plan->vals1.ensure(n * 4));
-  GG_TRY(plan->sort_tmp.ensure(radix_temp_bytes(n)));
-  GG_CUDA(launch_weight_keys<Real>(uu, vv, weight, n, cell_size_rad,
-                                   grid_size,
-                                   plan->keys0.as<uint32_t>(),
-                                   plan->vals0.as<uint32_t>(), d_num_skipped,
-                                   s));
-  const int key_bits =
-      ceil_log2((unsigned long long)grid_size * grid_size + 1);
-  bool in_alt = false;
-  GG_CUDA(radix_sort_pairs(plan->keys0.as<uint32_t>(),
-                           plan->vals0.as<uint32_t>(),
-                           plan->keys1.as<uint32_t>(),
-                           plan->vals1.as<uint32_t>(), n, key_bits,
-                           plan->sort_tmp.p, s, &in_alt));
-  GG_CUDA(launch_weight_runs<Real>(
-      in_alt ? plan->keys1.as<uint32_t>() : plan->keys0.as<uint32_t>(),
-      in_alt ? plan->vals1.as<uint32_t>() : plan->vals0.as<uint32_t>(), n,
-      weight, grid_size, d_grid, s));
-  return GG_OK;
+  return with_memory(plan, n, [&]() -> int {
+    GG_TRY(ensure_work<Real>(plan, n, false));
+    GG_TRY(plan->vals.ensure(n * 4));
+    GG_TRY(plan->sort_tmp.ensure(radix_temp_bytes(n)));
+    const SortParts sort(plan->work, n);
+    uint32_t* vals = plan->vals.as<uint32_t>();
+    GG_CUDA(launch_weight_keys<Real>(uu, vv, weight, n, cell_size_rad,
+                                     grid_size, sort.keys0, vals,
+                                     d_num_skipped, s));
+    const int key_bits =
+        ceil_log2((unsigned long long)grid_size * grid_size + 1);
+    bool in_alt = false;
+    GG_CUDA(radix_sort_pairs(sort.keys0, vals, sort.keys1, sort.vals, n,
+                             key_bits, plan->sort_tmp.p, s, &in_alt));
+    GG_CUDA(launch_weight_runs<Real>(in_alt ? sort.keys1 : sort.keys0,
+                                     in_alt ? sort.vals : vals, n, weight,
+                                     grid_size, d_grid, s));
+    return GG_OK;
+  });
 }
 
 template <typename Real>
@@ -2416,11 +2516,14 @@ int weights_write_host(size_t n, const Real* uu, const Real* vv,
   GG_TRY(ensure_device_plan(st));
   gg_plan* plan = st->plan;
   const size_t grid_bytes = (size_t)grid_size * grid_size * sizeof(Real);
-  GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_weight.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_grid.ensure(grid_bytes));
-  GG_TRY(plan->in_misc.ensure(64));
+  GG_TRY(with_memory(plan, n, [&]() -> int {
+    GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_weight.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_grid.ensure(grid_bytes));
+    GG_TRY(plan->in_misc.ensure(64));
+    return GG_OK;
+  }));
   unsigned long long* d_skip = plan->in_misc.as<unsigned long long>();
   if (n) {
     GG_CUDA(cudaMemcpyAsync(plan->in_uu.p, uu, n * sizeof(Real),
@@ -2465,12 +2568,15 @@ int weights_read_host(size_t n, const Real* uu, const Real* vv,
   GG_TRY(ensure_device_plan(st));
   gg_plan* plan = st->plan;
   const size_t grid_bytes = (size_t)grid_size * grid_size * sizeof(Real);
-  GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_weight.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vis.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_grid.ensure(grid_bytes));
-  GG_TRY(plan->in_misc.ensure(64));
+  GG_TRY(with_memory(plan, n, [&]() -> int {
+    GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_weight.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vis.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_grid.ensure(grid_bytes));
+    GG_TRY(plan->in_misc.ensure(64));
+    return GG_OK;
+  }));
   unsigned long long* d_skip = plan->in_misc.as<unsigned long long>();
   if (n) {
     GG_CUDA(cudaMemcpyAsync(plan->in_uu.p, uu, n * sizeof(Real),
@@ -2525,11 +2631,14 @@ int degrid_host(size_t num_w_planes, const int* support, int oversample,
   gg_plan* plan = st->plan;
   const size_t n = num_points;
   const size_t grid_bytes = (size_t)grid_size * grid_size * 2 * sizeof(Real);
-  GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_ww.ensure(n * sizeof(Real) + 16));
-  GG_TRY(plan->in_vis.ensure(2 * n * sizeof(Real) + 16));
-  GG_TRY(plan->in_grid.ensure(grid_bytes));
+  GG_TRY(with_memory(plan, n, [&]() -> int {
+    GG_TRY(plan->in_uu.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vv.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_ww.ensure(n * sizeof(Real) + 16));
+    GG_TRY(plan->in_vis.ensure(2 * n * sizeof(Real) + 16));
+    GG_TRY(plan->in_grid.ensure(grid_bytes));
+    return GG_OK;
+  }));
   // As in the gridding call: the coordinates go up first on the side
   // stream, the kernel stack is built beside placement on the stack stream
   // behind them, and the grid follows the coordinates on the side stream;

@@ -53,9 +53,7 @@ k_place_batched(PlaceParams<Real> p, StackView v, PlaceOut out,
   o.meta = pack_meta(r.plane, r.ou, r.ov, r.conj_neg, r.skipped);
   o.v.x = rmul(w, p.vis[2 * i]);
   o.v.y = rmul(w, p.vis[2 * i + 1]);
-  ((Placed<Real>*)out.placed)[i] = o;
-  out.cell[i] = o.cell;
-  out.meta[i] = o.meta;
+  ((Placed<Real>*)out.points.p)[i] = o;
   double t = 0.0;
   if (!r.skipped) {
     const int side = 2 * v.omax + 1;
@@ -72,8 +70,7 @@ k_place_batched(PlaceParams<Real> p, StackView v, PlaceOut out,
 template <typename Real>
 __global__ void __launch_bounds__(kThreads)
 k_revalue(const Real* __restrict__ vis, const Real* __restrict__ weight,
-          const uint32_t* __restrict__ meta, StackView v,
-          unsigned long long n, Placed<Real>* __restrict__ placed,
+          StackView v, unsigned long long n, Placed<Real>* __restrict__ placed,
           double* __restrict__ nterm) {
   using R2 = typename Vec2<Real>::type;
   const unsigned long long i =
@@ -84,7 +81,7 @@ k_revalue(const Real* __restrict__ vis, const Real* __restrict__ weight,
   o.x = rmul(w, vis[2 * i]);
   o.y = rmul(w, vis[2 * i + 1]);
   placed[i].v = o;
-  const uint32_t m = meta[i];
+  const uint32_t m = placed[i].meta;
   double t = 0.0;
   if (!meta_skipped(m)) {
     const int side = 2 * v.omax + 1;
@@ -98,7 +95,7 @@ k_revalue(const Real* __restrict__ vis, const Real* __restrict__ weight,
 
 // One block per chunk of one grid.
 __global__ void __launch_bounds__(kThreads)
-k_chunk_totals(const uint32_t* __restrict__ meta,
+k_chunk_totals(PlacedPoints points,
                const double* __restrict__ nterm, StackView v,
                const unsigned long long* __restrict__ chunk_begin,
                double* __restrict__ chunk_norm,
@@ -109,7 +106,7 @@ k_chunk_totals(const uint32_t* __restrict__ meta,
   double n = 0.0;
   unsigned long long skip = 0, macs = 0;
   for (unsigned long long i = b + threadIdx.x; i < e; i += kThreads) {
-    const uint32_t m = meta[i];
+    const uint32_t m = points.at(i).y;
     if (meta_skipped(m)) {
       ++skip;
     } else {
@@ -149,8 +146,8 @@ k_batch_finalize(int num_grids, const int* __restrict__ grid_chunk0,
       macs += chunk_macs[c];
       points += chunk_begin[c + 1] - chunk_begin[c];
     }
-    d_norm[g] += n;
-    d_num_skipped[g] = sk;
+    if (d_norm) d_norm[g] += n;
+    if (d_num_skipped) d_num_skipped[g] = sk;
     skips += sk;
   }
   points = block_sum(points);
@@ -173,7 +170,7 @@ cudaError_t launch_place_batched(PlaceParams<Real> p, StackView view,
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_totals(const uint32_t* meta, const double* nterm,
+cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
                                 StackView view, int num_chunks,
                                 const unsigned long long* chunk_begin,
                                 int num_grids, const int* grid_chunk0,
@@ -186,7 +183,7 @@ cudaError_t launch_batch_totals(const uint32_t* meta, const double* nterm,
                                 cudaStream_t s, int phases, long long tiles) {
   if (num_chunks > 0)
     k_chunk_totals<<<num_chunks, kThreads, 0, s>>>(
-        meta, nterm, view, chunk_begin, chunk_norm, chunk_skip, chunk_macs);
+        points, nterm, view, chunk_begin, chunk_norm, chunk_skip, chunk_macs);
   k_batch_finalize<<<1, kThreads, 0, s>>>(
       num_grids, grid_chunk0, chunk_begin, chunk_norm, chunk_skip,
       chunk_macs, forced_shape, phases, tiles, d_norm, d_num_skipped, d_macs,
@@ -196,23 +193,20 @@ cudaError_t launch_batch_totals(const uint32_t* meta, const double* nterm,
 
 template <typename Real>
 cudaError_t launch_revalue(const Real* vis, const Real* weight,
-                           const uint32_t* meta, StackView view,
-                           unsigned long long n, void* placed, double* nterm,
-                           cudaStream_t s) {
+                           StackView view, unsigned long long n, void* placed,
+                           double* nterm, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const unsigned nb = (unsigned)((n + kThreads - 1) / kThreads);
   k_revalue<Real><<<nb, kThreads, 0, s>>>(
-      vis, weight, meta, view, n, (Placed<Real>*)placed, nterm);
+      vis, weight, view, n, (Placed<Real>*)placed, nterm);
   return cudaGetLastError();
 }
 template cudaError_t launch_revalue<float>(const float*, const float*,
-                                           const uint32_t*, StackView,
-                                           unsigned long long, void*, double*,
-                                           cudaStream_t);
+                                           StackView, unsigned long long,
+                                           void*, double*, cudaStream_t);
 template cudaError_t launch_revalue<double>(const double*, const double*,
-                                            const uint32_t*, StackView,
-                                            unsigned long long, void*,
-                                            double*, cudaStream_t);
+                                            StackView, unsigned long long,
+                                            void*, double*, cudaStream_t);
 
 template cudaError_t launch_place_batched<float>(PlaceParams<float>,
                                                  StackView, PlaceOut, double*,

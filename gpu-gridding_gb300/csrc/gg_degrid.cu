@@ -88,7 +88,8 @@ struct DegridArgs {
   const uint32_t* rec_vis;    // and visibility indices
   int low_bits;
   const int* tile_order;      // tile at each place of the queue order
-  const uint4* points;        // per visibility: cell, meta, emission slot
+  const void* points;         // per visibility: cell, meta, emission slot; or,
+  const uint32_t* rec_offset; // where given, the slots, points cell and meta
   StackView view;
   TileGeom geom;
   int grid_size;
@@ -194,7 +195,13 @@ k_degrid_tiles(DegridArgs<Real> a) {
       const int t = q * 32 + lane;
       if (t < nb) {
         key[q] = a.rec_key[range.x + t];
-        pt[q] = a.points[a.rec_vis[range.x + t]];
+        const uint32_t vid = a.rec_vis[range.x + t];
+        if (a.rec_offset) {
+          const uint2 c = ((const uint2*)a.points)[vid];
+          pt[q] = make_uint4(c.x, c.y, a.rec_offset[vid], 0u);
+        } else {
+          pt[q] = ((const uint4*)a.points)[vid];
+        }
       }
     }
 #pragma unroll
@@ -496,7 +503,8 @@ template <typename Real>
 cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
                                 const uint32_t* rec_vis, uint32_t total,
                                 int low_bits, const int* tile_order,
-                                const void* points, uint32_t* counter,
+                                PlacedPoints points,
+                                const uint32_t* rec_offset, uint32_t* counter,
                                 StackView view, TileGeom geom, int grid_size,
                                 const Real* grid, void* rec_out, int num_ctas,
                                 cudaStream_t s) {
@@ -515,7 +523,8 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
   a.rec_vis = rec_vis;
   a.low_bits = low_bits;
   a.tile_order = tile_order;
-  a.points = (const uint4*)points;
+  a.points = points.p;
+  a.rec_offset = points.stride == 16 ? nullptr : rec_offset;
   a.view = view;
   a.geom = geom;
   a.grid_size = grid_size;
@@ -546,11 +555,11 @@ cudaError_t launch_degrid_finish(const uint32_t* count, const uint32_t* offset,
 template int degrid_tiles_ctas_per_sm<float>(bool);
 template int degrid_tiles_ctas_per_sm<double>(bool);
 template cudaError_t launch_degrid_tiles<float>(
-    const uint32_t*, const uint32_t*, uint32_t, int, const int*, const void*,
-    uint32_t*, StackView, TileGeom, int, const float*, void*, int, cudaStream_t);
+    const uint32_t*, const uint32_t*, uint32_t, int, const int*, PlacedPoints,
+    const uint32_t*, uint32_t*, StackView, TileGeom, int, const float*, void*, int, cudaStream_t);
 template cudaError_t launch_degrid_tiles<double>(
-    const uint32_t*, const uint32_t*, uint32_t, int, const int*, const void*,
-    uint32_t*, StackView, TileGeom, int, const double*, void*, int, cudaStream_t);
+    const uint32_t*, const uint32_t*, uint32_t, int, const int*, PlacedPoints,
+    const uint32_t*, uint32_t*, StackView, TileGeom, int, const double*, void*, int, cudaStream_t);
 template cudaError_t launch_degrid_finish<float>(const uint32_t*,
                                                  const uint32_t*, const void*,
                                                  unsigned long long, float*,

@@ -148,46 +148,60 @@ __device__ __forceinline__ void cell_ends(const uint32_t* tile_groups,
   }
 }
 
+// The first column and row of a virtual tile.
+template <int TW>
+__device__ __forceinline__ int2 tile_origin(const TileGeom& g, int tile) {
+  using WS = WarpShape<TW>;
+  const int vg = tile / g.tiles_total;   // virtual group
+  const int tl = (tile - vg * g.tiles_total) % (g.tiles_u * g.tiles_v);
+  return make_int2((tl % g.tiles_u) * WS::kTileU - phase_shift(g, vg),
+                   (tl / g.tiles_u) * WS::kTileV);
+}
+
+// The prepared record of visibility vid in the tile that starts at `tile`.
+template <typename Real, int TW>
+__device__ __forceinline__ void prepare_record(const GridArgs<Real>& a,
+                                               int2 tile, uint32_t vid,
+                                               Record<Real>& rec,
+                                               uint32_t& span) {
+  const Placed<Real> pt = a.placed[vid];
+  const uint32_t m = pt.meta;
+  const SlicePlane plane = a.view.planes[meta_plane(m)];
+  const int ou = meta_ou(m), ov = meta_ov(m), s = plane.support;
+  const int gu = cell_u(pt.cell) - tile.x, gv = cell_v(pt.cell) - tile.y;
+  rec.d = slice_record(slice_origin(plane, a.view.omax, abs(ou), abs(ov)), s,
+                       ou, ov, gu, gv);
+  rec.v = pt.v;
+  if constexpr (sizeof(Real) == 8) {
+    rec.row0 = gv - s;
+    rec.row1 = gv + s;
+  }
+  // The tile meets each of its records: clipped to it.
+  span = (uint32_t)(max(gv - s, 0) / kRows) |
+         (uint32_t)(min(gv + s, WarpShape<TW>::kTileV - 1) / kRows) << 5 |
+         (meta_conj(m) ? kSpanConj : 0u);
+}
+
 // Prepares the records of every work item of the call: one block per item at
 // a time.  HBM-bound: 4 B of index and one sector at random per record in,
 // 18 B (FP64: 34 B) out.
 template <typename Real, int TW>
 __global__ void __launch_bounds__(128)
 k_prepare_records(GridArgs<Real> a, int num_groups) {
-  using WS = WarpShape<TW>;
-  const int tiles_per_grid = a.geom.tiles_u * a.geom.tiles_v;
   const int num_items = (int)a.group_items[num_groups];
   // The first gridding launch's work counter.
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.counter = 0;
   for (int it = blockIdx.x; it < num_items; it += gridDim.x) {
     const WorkItem item = a.items[it];
-    const int vg = item.tile / a.geom.tiles_total;   // virtual group
-    const int tl = (item.tile - vg * a.geom.tiles_total) % tiles_per_grid;
-    const int u0 = (tl % a.geom.tiles_u) * WS::kTileU - phase_shift(a.geom, vg);
-    const int v0 = (tl / a.geom.tiles_u) * WS::kTileV;
+    const int2 tile = tile_origin<TW>(a.geom, item.tile);
     const uint32_t n = item.rec_end - item.rec_begin;
     for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
       const uint32_t i = item.rec_begin + k;
-      const uint32_t vid = a.rec_vis[i];
-      const Placed<Real> pt = a.placed[vid];
-      const uint32_t m = pt.meta;
-      const SlicePlane plane = a.view.planes[meta_plane(m)];
-      const int ou = meta_ou(m), ov = meta_ov(m), s = plane.support;
-      const int gu = cell_u(pt.cell) - u0, gv = cell_v(pt.cell) - v0;
       Record<Real> rec;
-      rec.d = slice_record(slice_origin(plane, a.view.omax, abs(ou), abs(ov)),
-                           s, ou, ov, gu, gv);
-      rec.v = pt.v;
-      if constexpr (sizeof(Real) == 8) {
-        rec.row0 = gv - s;
-        rec.row1 = gv + s;
-      }
+      uint32_t span;
+      prepare_record<Real, TW>(a, tile, a.rec_vis[i], rec, span);
       a.recs[i] = rec;
-      // The tile meets each of its records: clipped to it.
-      a.spans[i] = (unsigned short)(
-          (uint32_t)(max(gv - s, 0) / kRows) |
-          (uint32_t)(min(gv + s, WS::kTileV - 1) / kRows) << 5 |
-          (meta_conj(m) ? kSpanConj : 0u));
+      a.spans[i] = (unsigned short)span;
     }
   }
 }
@@ -236,7 +250,9 @@ struct WarpSmem {
 constexpr int kGridWarps = 4;    // per block of the gridding kernel
 constexpr int kGridThreads = kGridWarps * 32;
 
-template <int TW, bool kWide>
+// kPrepared: the records come from k_prepare_records; else (a call for which
+// those do not fit the device's memory) every band's warp prepares them itself.
+template <int TW, bool kWide, bool kPrepared>
 __global__ void __launch_bounds__(kGridThreads, 5)
 k_grid_tiles(GridArgs<float> a) {
   constexpr int kDepth = 2;   // records in flight per warp
@@ -351,8 +367,13 @@ k_grid_tiles(GridArgs<float> a) {
     auto fetch = [&](Pos i) {
       span = kSpanNone;
       if (before_end(i, lane)) {
-        span = a.spans[i + lane];
-        rec = a.recs[i + lane];
+        if constexpr (kPrepared) {
+          span = a.spans[i + lane];
+          rec = a.recs[i + lane];
+        } else {
+          prepare_record<float, TW>(a, tile_origin<TW>(a.geom, item.tile),
+                                    a.rec_vis[i + lane], rec, span);
+        }
       }
     };
     fetch((Pos)item.rec_begin);
@@ -479,7 +500,7 @@ struct WarpSmem64 {
 // band rows in registers, 2.15 so (the multiply-adds alone 1.73).  Eight
 // cells a lane in flight, three blocks: 2.15; four cells and four to six
 // blocks 2.18 to 2.2, as the units in flight at the end are more.
-template <int TW>
+template <int TW, bool kPrepared>
 __global__ void __launch_bounds__(kGridThreads, 3)
 k_grid_tiles_f64(GridArgs<double> a) {
   using WS = WarpShape<TW>;
@@ -508,8 +529,13 @@ k_grid_tiles_f64(GridArgs<double> a) {
     auto fetch = [&](uint32_t i) {
       span = kSpanNone;
       if ((uint32_t)lane < item.rec_end - i) {
-        span = a.spans[i + lane];
-        rec = a.recs[i + lane];
+        if constexpr (kPrepared) {
+          span = a.spans[i + lane];
+          rec = a.recs[i + lane];
+        } else {
+          prepare_record<double, TW>(a, tile_origin<TW>(a.geom, item.tile),
+                                     a.rec_vis[i + lane], rec, span);
+        }
       }
     };
     fetch(item.rec_begin);
@@ -1060,14 +1086,14 @@ __global__ void k_item_emit(const uint32_t* __restrict__ tile_start,
 // querying occupancy or launching.  The opt-in is made once per device, so
 // later launches (replays captured in a CUDA graph among them) make no
 // attribute call.
-template <typename Real, int TW, bool kWide>
+template <typename Real, int TW, bool kWide, bool kPrepared>
 cudaError_t prepare_grid_kernel(void** fn, size_t* smem) {
   static std::atomic<unsigned long long> opted_in{0};
   if constexpr (sizeof(Real) == 4) {
-    *fn = (void*)k_grid_tiles<TW, kWide>;
+    *fn = (void*)k_grid_tiles<TW, kWide, kPrepared>;
     *smem = kGridWarps * sizeof(WarpSmem<TW>);
   } else {
-    *fn = (void*)k_grid_tiles_f64<TW>;
+    *fn = (void*)k_grid_tiles_f64<TW, kPrepared>;
     *smem = kGridWarps * sizeof(WarpSmem64);
   }
   int dev = 0;
@@ -1081,20 +1107,24 @@ cudaError_t prepare_grid_kernel(void** fn, size_t* smem) {
   return e;
 }
 
-template <typename Real, bool kWide>
+template <typename Real, bool kWide, bool kPrepared>
 cudaError_t prepare_grid_kernel_of(int tile_u, void** fn, size_t* smem) {
-  return tile_u == 32   ? prepare_grid_kernel<Real, 32, kWide>(fn, smem)
-         : tile_u == 16 ? prepare_grid_kernel<Real, 16, kWide>(fn, smem)
-                        : prepare_grid_kernel<Real, 8, kWide>(fn, smem);
+  return tile_u == 32
+             ? prepare_grid_kernel<Real, 32, kWide, kPrepared>(fn, smem)
+         : tile_u == 16
+             ? prepare_grid_kernel<Real, 16, kWide, kPrepared>(fn, smem)
+             : prepare_grid_kernel<Real, 8, kWide, kPrepared>(fn, smem);
 }
 
+// Unprepared records: the wide kernel, which takes every call.
 template <typename Real>
-cudaError_t prepare_grid_kernel_for(int tile_u, bool wide, void** fn,
-                                    size_t* smem) {
-  return wide && sizeof(Real) == 4
-             ? prepare_grid_kernel_of<Real, sizeof(Real) == 4>(tile_u, fn,
-                                                               smem)
-             : prepare_grid_kernel_of<Real, false>(tile_u, fn, smem);
+cudaError_t prepare_grid_kernel_for(int tile_u, bool wide, bool prepared,
+                                    void** fn, size_t* smem) {
+  constexpr bool kF32 = sizeof(Real) == 4;
+  if (!prepared)
+    return prepare_grid_kernel_of<Real, kF32, false>(tile_u, fn, smem);
+  return wide ? prepare_grid_kernel_of<Real, kF32, true>(tile_u, fn, smem)
+              : prepare_grid_kernel_of<Real, false, true>(tile_u, fn, smem);
 }
 
 }  // namespace
@@ -1168,7 +1198,8 @@ int grid_tiles_ctas_per_sm(int tile_u, bool wide) {
   void* fn = nullptr;
   size_t smem = 0;
   int n = 0;
-  if (prepare_grid_kernel_for<Real>(tile_u, wide, &fn, &smem) != cudaSuccess ||
+  if (prepare_grid_kernel_for<Real>(tile_u, wide, true, &fn, &smem) !=
+          cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kGridThreads,
                                                     smem) != cudaSuccess)
     n = 1;
@@ -1282,19 +1313,21 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
     return cudaErrorInvalidValue;
   void* fn = nullptr;
   size_t smem = 0;
-  cudaError_t e = prepare_grid_kernel_for<Real>(geom.tile_u, view.wide,
-                                                &fn, &smem);
+  cudaError_t e = prepare_grid_kernel_for<Real>(
+      geom.tile_u, view.wide, recs != nullptr, &fn, &smem);
   if (e != cudaSuccess) return e;
   const int span = group_span > 1 ? group_span : 1;
   a.group_span = span;
   int num_groups = geom.num_groups;
   void* prep_args[] = {&a, &num_groups};
-  e = cudaLaunchKernel(geom.tile_u == 32 ? (void*)k_prepare_records<Real, 32>
-                       : geom.tile_u == 16
-                           ? (void*)k_prepare_records<Real, 16>
-                           : (void*)k_prepare_records<Real, 8>,
-                       dim3(8 * num_ctas), dim3(128), prep_args, 0, s);
-  if (e != cudaSuccess) return e;
+  if (recs) {
+    e = cudaLaunchKernel(geom.tile_u == 32 ? (void*)k_prepare_records<Real, 32>
+                         : geom.tile_u == 16
+                             ? (void*)k_prepare_records<Real, 16>
+                             : (void*)k_prepare_records<Real, 8>,
+                         dim3(8 * num_ctas), dim3(128), prep_args, 0, s);
+    if (e != cudaSuccess) return e;
+  }
   void* args[] = {&a};
   for (int g = 0; g < geom.num_groups; g += span) {
     a.group = g;
@@ -1302,7 +1335,7 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
       e = cudaStreamWaitEvent(s, wait_before[g], 0);
       if (e != cudaSuccess) return e;
     }
-    if (g > 0) {
+    if (g > 0 || !recs) {
       e = cudaMemsetAsync(counter, 0, sizeof(uint32_t), s);
       if (e != cudaSuccess) return e;
     }

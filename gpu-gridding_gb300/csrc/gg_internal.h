@@ -118,9 +118,7 @@ __host__ __device__ inline int phases_of_shape(uint32_t word) {
 }
 
 struct PlaceOut {
-  uint32_t* cell;             // [N]
-  uint32_t* meta;             // [N]
-  void* placed;               // [N] Placed<Real>, null for degridding
+  PlacedPoints points;        // [N] Placed<Real>, or pairs for degridding
   uint32_t* rec_count;        // [N] records (tiles touched) per visibility
   double* blk_norm;           // [num_blocks]
   unsigned long long* blk_skip;   // [num_blocks]
@@ -139,7 +137,7 @@ cudaError_t launch_store_f64(double* p, double v, cudaStream_t s);
 // the placed meta and the stack's tap sums, reduced in k_place's block
 // order, then *d_norm += their sum exactly as launch_place_finalize would.
 template <typename Real>
-cudaError_t launch_norm_terms(const uint32_t* meta, const Real* weight,
+cudaError_t launch_norm_terms(PlacedPoints points, const Real* weight,
                               unsigned long long n, StackView view,
                               double* blk_norm, double* d_norm,
                               cudaStream_t s);
@@ -159,18 +157,17 @@ cudaError_t launch_place_finalize(const double* blk_norm,
 // use[b] = how many of up to 8192 placed points, evenly spread, are gridded with
 // planes p of bin b = p * kPlaneBins / num_planes.
 constexpr int kPlaneBins = 256;
-cudaError_t launch_plane_use(const uint32_t* meta, unsigned long long n,
+cudaError_t launch_plane_use(PlacedPoints points, unsigned long long n,
                              int num_planes, uint32_t* use, cudaStream_t s);
 // count[i] = tiles of shape *d_shape touched by visibility i on its tile
 // phase (footprint_phase; 0 if skipped).
-cudaError_t launch_count_records(const uint32_t* cell, const uint32_t* meta,
-                                 unsigned long long n, StackView view,
-                                 const uint32_t* d_shape, uint32_t* count,
-                                 cudaStream_t s);
+cudaError_t launch_count_records(PlacedPoints points, unsigned long long n,
+                                 StackView view, const uint32_t* d_shape,
+                                 uint32_t* count, cudaStream_t s);
 template <typename Real>
 cudaError_t launch_place_only(PlaceParams<Real> p, StackView view, int* out,
                               cudaStream_t s);
-cudaError_t launch_emit_records(const uint32_t* cell, const uint32_t* meta,
+cudaError_t launch_emit_records(PlacedPoints points,
                                 const uint32_t* rec_offset,
                                 unsigned long long n, StackView view,
                                 TileGeom geom, int grid_index,
@@ -180,12 +177,12 @@ cudaError_t launch_emit_records(const uint32_t* cell, const uint32_t* meta,
                                     nullptr,
                                 int num_grids = 1,
                                 const int* tile_rank = nullptr,
-                                void* points = nullptr);
+                                bool write_slots = false);
 // grid_offsets (device, num_grids + 1): batched calls, where visibility i
 // belongs to the grid g with grid_offsets[g] <= i < grid_offsets[g + 1].
-// tile_rank and points (device; degridding): keys hold each tile's
-// tile_rank[tile] in place of its index, and points[i] (16 bytes) becomes
-// visibility i's cell, meta and first emission slot.
+// tile_rank (device; degridding): keys hold each tile's tile_rank[tile] in
+// place of its index.  write_slots: every gridded point's first emission slot
+// goes behind its cell and meta (points 16 bytes apart).
 
 // ---- batched calls (gg_batch.cu) ------------------------------------------
 // Per-visibility placement for a batched call: like launch_place, but the
@@ -195,18 +192,17 @@ template <typename Real>
 cudaError_t launch_place_batched(PlaceParams<Real> p, StackView view,
                                  PlaceOut out, double* nterm, cudaStream_t s);
 // Weighted visibilities and norm terms for new amplitudes and weights on
-// an existing placement (meta).
+// an existing placement.
 template <typename Real>
 cudaError_t launch_revalue(const Real* vis, const Real* weight,
-                           const uint32_t* meta, StackView view,
-                           unsigned long long n, void* placed, double* nterm,
-                           cudaStream_t s);
+                           StackView view, unsigned long long n, void* placed,
+                           double* nterm, cudaStream_t s);
 // Deterministic per-grid totals over a chunk table (chunk c covers
 // visibilities [chunk_begin[c], chunk_begin[c+1]) of grid chunk_grid[c];
 // grid g owns chunks [grid_chunk0[g], grid_chunk0[g+1])):
 // d_norm[g] += sum of nterm, d_num_skipped[g] = skips, *d_macs = total
 // MACs, *d_shape = choose_shape(total MACs, gridded, forced_shape).
-cudaError_t launch_batch_totals(const uint32_t* meta, const double* nterm,
+cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
                                 StackView view, int num_chunks,
                                 const unsigned long long* chunk_begin,
                                 int num_grids, const int* grid_chunk0,
@@ -279,8 +275,8 @@ cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
 // takes two more).
 template <typename Real>
 size_t prepared_record_bytes();
-// Prepares the records of every item (recs, spans), then
-// persistent launches in virtual-group order, each over the work items of
+// Prepares the records of every item (recs, spans; without recs the gridding
+// kernel prepares them itself, for each band anew), then persistent launches in virtual-group order, each over the work items of
 // group_span consecutive virtual groups: with group_span = tile_phases one
 // launch per plane group takes all its tile phases (the items were built
 // with ItemBuffers::partial_phases = tile_phases: the first phase's
@@ -390,13 +386,14 @@ int degrid_tiles_ctas_per_sm(bool wide);
 // the queue order tile_order, ...) with the tile's place above the keys'
 // low_bits (32 x 64-cell tiles only): rec_out[rec_offset[v] + rank] = the
 // record's share of conj(tap) * grid for every record, rank = the record's
-// tile among visibility v's tiles in emission order; points as
-// launch_emit_records writes them.
+// tile among visibility v's tiles in emission order.  points: 16 bytes apart
+// with the slots that launch_emit_records wrote, or 8 bytes apart.
 template <typename Real>
 cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
                                 const uint32_t* rec_vis, uint32_t total,
                                 int low_bits, const int* tile_order,
-                                const void* points, uint32_t* counter,
+                                PlacedPoints points,
+                                const uint32_t* rec_offset, uint32_t* counter,
                                 StackView view, TileGeom geom, int grid_size,
                                 const Real* grid, void* rec_out, int num_ctas,
                                 cudaStream_t s);

@@ -177,8 +177,6 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   // only once the call is accepted.
   double* call_norm = c.take<double>(1);
   unsigned long long* call_skip = c.take<unsigned long long>(1);
-  uint32_t* cell = c.take<uint32_t>(maxp);
-  uint32_t* meta = c.take<uint32_t>(maxp);
   Placed<float>* placed = c.take<Placed<float>>(maxp);
   uint32_t* count = c.take<uint32_t>(maxp);
   uint32_t* offset = c.take<uint32_t>(maxp);
@@ -224,9 +222,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   pp.grid_centre = grid_size / 2;
   pp.num_points = num_points;
   PlaceOut po;
-  po.cell = cell;
-  po.meta = meta;
-  po.placed = placed;
+  po.points = {(unsigned char*)placed, sizeof(Placed<float>)};
   po.rec_count = count;
   po.blk_norm = blk_norm;
   po.blk_skip = blk_skip;
@@ -236,8 +232,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   NA_CUDA(launch_place_finalize(blk_norm, blk_skip, blk_macs, nblk,
                                 num_points, -1, call_norm, call_skip, macs,
                                 sc + 5, s));
-  NA_CUDA(launch_count_records(cell, meta, num_points, view, sc + 5, count,
-                               s));
+  NA_CUDA(launch_count_records(po.points, num_points, view, sc + 5, count, s));
   NA_CUDA(exclusive_scan_u32(count, offset, num_points, sc + 0, scan_tmp, s));
   uint32_t host_sc[8] = {0};
   NA_CUDA(cudaMemcpyAsync(host_sc, sc, sizeof(host_sc),
@@ -282,8 +277,8 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   const bool odd = total > 1 && radix_passes(tile_bits) % 2 == 1;
   uint32_t* vals0 = odd ? vals_other : vals;
   uint32_t* vals1 = odd ? vals : vals_other;
-  NA_CUDA(launch_emit_records(cell, meta, offset, num_points, view, geom, 0,
-                              0, keys0, vals0, s));
+  NA_CUDA(launch_emit_records(po.points, offset, num_points, view, geom, 0, 0,
+                              keys0, vals0, s));
   bool in_alt = false;
   NA_CUDA(radix_sort_pairs(keys0, vals0, keys1, vals1, total,
                            tile_bits, sort_tmp, s, &in_alt));

@@ -42,10 +42,10 @@ k_place(PlaceParams<Real> p, StackView v, TileGeom g, PlaceOut out) {
       o.meta = meta;
       o.v.x = rmul(w, p.vis[2 * i]);
       o.v.y = rmul(w, p.vis[2 * i + 1]);
-      ((Placed<Real>*)out.placed)[i] = o;
+      ((Placed<Real>*)out.points.p)[i] = o;
+    } else {
+      *(uint2*)(out.points.p + i * out.points.stride) = make_uint2(cell, meta);
     }
-    out.cell[i] = cell;
-    out.meta[i] = meta;
     if (r.skipped) {
       skip = 1;
     } else {
@@ -90,13 +90,13 @@ k_place(PlaceParams<Real> p, StackView v, TileGeom g, PlaceOut out) {
 // bit-identical to what k_place would have written.
 template <typename Real>
 __global__ void __launch_bounds__(kPlaceThreads)
-k_norm_terms(const uint32_t* __restrict__ meta, const Real* __restrict__ weight,
+k_norm_terms(PlacedPoints points, const Real* __restrict__ weight,
              unsigned long long n, StackView v, double* __restrict__ blk_norm) {
   const unsigned long long i =
       (unsigned long long)blockIdx.x * kPlaceThreads + threadIdx.x;
   double norm = 0.0;
   if (i < n) {
-    const uint32_t m = meta[i];
+    const uint32_t m = points.at(i).y;
     if (!meta_skipped(m)) {
       const int side = 2 * v.omax + 1;
       const double ts = v.tap_sum[((size_t)meta_plane(m) * side +
@@ -176,7 +176,7 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
 // One block of 1024 threads, eight points each, their loads in flight
 // together: a few microseconds.
 __global__ void __launch_bounds__(1024)
-k_plane_use(const uint32_t* __restrict__ meta, unsigned long long n,
+k_plane_use(PlacedPoints points, unsigned long long n,
             int num_planes, uint32_t* __restrict__ use) {
   __shared__ uint32_t s_use[kPlaneBins];
   constexpr int kEach = 8;
@@ -194,7 +194,7 @@ k_plane_use(const uint32_t* __restrict__ meta, unsigned long long n,
     const unsigned long long at = k * n / samples;
     const unsigned long long len = (k + 1) * n / samples - at;
     m[j] = k < samples
-               ? meta[at + (len * ((uint32_t)k * 2654435769u) >> 32)]
+               ? points.at(at + (len * ((uint32_t)k * 2654435769u) >> 32)).y
                : (1u << 25);
   }
 #pragma unroll
@@ -208,15 +208,14 @@ k_plane_use(const uint32_t* __restrict__ meta, unsigned long long n,
 
 // Records per visibility: tiles of the chosen shape its footprint touches
 // (on its tile phase, see footprint_phase).
-__global__ void k_count(const uint32_t* __restrict__ cell,
-                        const uint32_t* __restrict__ meta,
-                        unsigned long long n, StackView v,
+__global__ void k_count(PlacedPoints points, unsigned long long n, StackView v,
                         const uint32_t* __restrict__ d_shape,
                         uint32_t* __restrict__ count) {
   const unsigned long long i =
       (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t m = meta[i];
+  const uint2 point = points.at(i);
+  const uint32_t m = point.y;
   uint32_t c = 0;
   if (!meta_skipped(m)) {
     const uint32_t word = *d_shape;
@@ -225,7 +224,7 @@ __global__ void k_count(const uint32_t* __restrict__ cell,
     // (32 >> shape) / phases columns: divisions become shifts.
     const int tws = 5 - shape, ths = 6 + shape;
     const int sws = tws - (phases >= 8 ? 3 : phases >= 4 ? 2 : phases >= 2);
-    const uint32_t ce = cell[i];
+    const uint32_t ce = point.x;
     const int gu = cell_u(ce), gv = cell_v(ce);
     const int s = v.support[meta_plane(m)];
     const int sh = phases > 1
@@ -241,8 +240,7 @@ __global__ void k_count(const uint32_t* __restrict__ cell,
 // One thread per visibility writes one record per tile its footprint
 // touches.  Key = (tile, plane if plane_bits) so that after the sort each
 // tile's records are contiguous; value = the visibility index.
-__global__ void k_emit(const uint32_t* __restrict__ cell,
-                       const uint32_t* __restrict__ meta,
+__global__ void k_emit(PlacedPoints points,
                        const uint32_t* __restrict__ rec_offset,
                        unsigned long long n, StackView v, TileGeom g,
                        int grid_index, unsigned long long vis_offset,
@@ -250,11 +248,12 @@ __global__ void k_emit(const uint32_t* __restrict__ cell,
                        uint32_t* __restrict__ vals,
                        const unsigned long long* __restrict__ grid_offsets,
                        int num_grids, const int* __restrict__ tile_rank,
-                       uint4* __restrict__ points) {
+                       bool write_slots) {
   const unsigned long long i =
       (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint32_t m = meta[i];
+  const uint2 point = points.at(i);
+  const uint32_t m = point.y;
   if (meta_skipped(m)) return;
   if (grid_offsets) {
     // Batched call: the grid of visibility i is the channel whose range
@@ -266,7 +265,7 @@ __global__ void k_emit(const uint32_t* __restrict__ cell,
     }
     grid_index = lo;
   }
-  const uint32_t c = cell[i];
+  const uint32_t c = point.x;
   const int gu = cell_u(c), gv = cell_v(c);
   const int plane = meta_plane(m);
   const int s = v.support[plane];
@@ -284,7 +283,7 @@ __global__ void k_emit(const uint32_t* __restrict__ cell,
   const int low_bits = g.plane_bits;
   const uint32_t tiles_per_grid = (uint32_t)g.tiles_u * (uint32_t)g.tiles_v;
   uint32_t pos = rec_offset[i];
-  if (points) points[i] = make_uint4(c, m, pos, 0u);
+  if (write_slots) *(uint32_t*)(points.p + i * points.stride + 8) = pos;
   const uint32_t vid = (uint32_t)(vis_offset + i);
   for (int tv = tv0; tv <= tv1; ++tv) {
     for (int tu = tu0; tu <= tu1; ++tu) {
@@ -383,13 +382,13 @@ cudaError_t launch_store_f64(double* p, double v, cudaStream_t s) {
 }
 
 template <typename Real>
-cudaError_t launch_norm_terms(const uint32_t* meta, const Real* weight,
+cudaError_t launch_norm_terms(PlacedPoints points, const Real* weight,
                               unsigned long long n, StackView view,
                               double* blk_norm, double* d_norm,
                               cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   const int nb = place_num_blocks(n);
-  k_norm_terms<Real><<<nb, kPlaceThreads, 0, s>>>(meta, weight, n, view,
+  k_norm_terms<Real><<<nb, kPlaceThreads, 0, s>>>(points, weight, n, view,
                                                  blk_norm);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
@@ -398,23 +397,22 @@ cudaError_t launch_norm_terms(const uint32_t* meta, const Real* weight,
   return cudaGetLastError();
 }
 
-cudaError_t launch_plane_use(const uint32_t* meta, unsigned long long n,
+cudaError_t launch_plane_use(PlacedPoints points, unsigned long long n,
                              int num_planes, uint32_t* use, cudaStream_t s) {
-  k_plane_use<<<1, 1024, 0, s>>>(meta, n, num_planes, use);
+  k_plane_use<<<1, 1024, 0, s>>>(points, n, num_planes, use);
   return cudaGetLastError();
 }
 
-cudaError_t launch_count_records(const uint32_t* cell, const uint32_t* meta,
-                                 unsigned long long n, StackView view,
-                                 const uint32_t* d_shape, uint32_t* count,
-                                 cudaStream_t s) {
+cudaError_t launch_count_records(PlacedPoints points, unsigned long long n,
+                                 StackView view, const uint32_t* d_shape,
+                                 uint32_t* count, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  k_count<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cell, meta, n, view,
-                                                     d_shape, count);
+  k_count<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(points, n, view, d_shape,
+                                                     count);
   return cudaGetLastError();
 }
 
-cudaError_t launch_emit_records(const uint32_t* cell, const uint32_t* meta,
+cudaError_t launch_emit_records(PlacedPoints points,
                                 const uint32_t* rec_offset,
                                 unsigned long long n, StackView view,
                                 TileGeom geom, int grid_index,
@@ -422,19 +420,19 @@ cudaError_t launch_emit_records(const uint32_t* cell, const uint32_t* meta,
                                 uint32_t* vals, cudaStream_t s,
                                 const unsigned long long* grid_offsets,
                                 int num_grids, const int* tile_rank,
-                                void* points) {
+                                bool write_slots) {
   if (n == 0) return cudaSuccess;
   const unsigned nb = (unsigned)((n + 255) / 256);
-  k_emit<<<nb, 256, 0, s>>>(cell, meta, rec_offset, n, view, geom,
-                            grid_index, vis_offset, keys, vals, grid_offsets,
-                            num_grids, tile_rank, (uint4*)points);
+  k_emit<<<nb, 256, 0, s>>>(points, rec_offset, n, view, geom, grid_index,
+                            vis_offset, keys, vals, grid_offsets, num_grids,
+                            tile_rank, write_slots);
   return cudaGetLastError();
 }
 
-template cudaError_t launch_norm_terms<float>(const uint32_t*, const float*,
+template cudaError_t launch_norm_terms<float>(PlacedPoints, const float*,
                                               unsigned long long, StackView,
                                               double*, double*, cudaStream_t);
-template cudaError_t launch_norm_terms<double>(const uint32_t*, const double*,
+template cudaError_t launch_norm_terms<double>(PlacedPoints, const double*,
                                                unsigned long long, StackView,
                                                double*, double*, cudaStream_t);
 template cudaError_t launch_place<float>(PlaceParams<float>, StackView,
