@@ -13,7 +13,7 @@
 // beforehand with gg_kernels_create_f (that set-up step does allocate).
 //
 // Costs of this design, stated for the caller:
-// * every GPU that loads the library holds the 48 MiB array until the
+// * every GPU that loads the library holds the 32 MiB array until the
 //   process exits, whether or not it ever calls this entry point;
 // * the array is shared by all calls on a device: calls that overlap on the
 //   GPU (different streams, different host threads) race on it and must be
@@ -50,13 +50,15 @@ constexpr size_t kNoAllocMaxRecords = size_t(1) << 20;  // 1,048,576
 constexpr int kNoAllocMaxGrid = 8192;
 // Partial tiles of split tiles: some of their own, the others in the place of
 // the sort's keys and its unsorted values, which the tile bounds are the last
-// to read.  With the former alone a heavy call had half an item a team (601
-// planes of support 4 to 72, 6e4 points on 1024^2: 2.20 ms, so 1.25; 339 planes
-// to 60, 1e5 points on 2048^2: 1.96, 1.30).
-constexpr int kNoAllocOwnSlots = 384;
-constexpr int kNoAllocMaxSlots = 1152;
+// to read.  Heavy calls, ms, with 384 partial tiles in all and with 1376: 601
+// planes of support 4 to 72, 6e4 points on 1024^2, 2.20 and 1.29; 339 planes to
+// 60, 1e5 points on 2048^2, 1.96 and 1.24.
+// The gridding kernel prepares the records itself: 18 MiB for prepared ones
+// would make the array 50 MiB and gain nothing (1.27 and 1.28 with 48 MiB).
+constexpr int kNoAllocOwnSlots = 608;
+constexpr int kNoAllocMaxSlots = 1376;
 constexpr int kNoAllocCells = 2048;      // cells per tile
-constexpr size_t kNoAllocBytes = size_t(48) << 20;
+constexpr size_t kNoAllocBytes = size_t(32) << 20;
 constexpr int kMaxDevices = 64;
 
 // The scratch memory of every no-alloc call on a device.
@@ -200,9 +202,6 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
                         sizeof(float2) ==
                     3 * kNoAllocMaxRecords * sizeof(uint32_t),
                 "the partial tiles run through the sort's buffers");
-  unsigned char* recs =
-      c.take<unsigned char>(maxr * prepared_record_bytes<float>());
-  unsigned short* spans = c.take<unsigned short>(maxr);
   if (c.used > kNoAllocBytes)
     return record_error(GG_ERR_UNSUPPORTED,
                         "no-alloc scratch layout exceeds the array");
@@ -316,7 +315,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   ib.num_groups = 1;
   ib.scan_tmp = scan_tmp;
   NA_CUDA(launch_build_items(tile_start, num_tiles, total, chunk, ib, s));
-  NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, recs, spans, vals,
+  NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, nullptr, nullptr, vals,
                                    placed, view, geom, grid_size, d_grid, 0,
                                    (float*)partials, split_tiles, sc + 3,
                                    num_tiles, num_ctas, s));

@@ -429,7 +429,7 @@ GG_API int gg_plan_probe_bounded_wait(gg_plan* plan, unsigned iterations,
  * allocate device memory while they grid (a real-time loop that must not
  * stall on cudaMalloc, or code running under another framework's memory
  * pool).  This entry point has no counterpart in the reference.  All scratch
- * comes from one 48 MiB device array inside the library, held by every GPU
+ * comes from one 32 MiB device array inside the library, held by every GPU
  * that loads it until the process exits; nothing is allocated or freed by
  * the call.  The kernel-stack handle is made beforehand (that step
  * allocates).  Limits: num_points <= 131072, grid_size <= 8192, and at most

@@ -274,3 +274,36 @@ def test_noalloc_heavy_tiles(pkg, G):
     assert outs[0][2] == outs[1][2] and outs[0][1] == outs[1][1]
     assert max_rel(outs[1][0], outs[0][0]) <= 1e-5
     assert ms[1] <= 4.0 / 3.0 * ms[0] + 0.1
+
+
+SIZE = r"""
+import importlib, sys
+import ctypes, torch
+sys.path[:0] = [{root!r}, {root!r} + "/tests"]
+from test_zz_no_alloc import _noalloc_fn
+pkg = importlib.import_module("gpu-gridding_gb300")
+import numpy as np
+x = torch.zeros((1, 2, 2, 2), device="cuda")
+stack = pkg.KernelStack(1, np.zeros(1, np.int32), 1, 2, x, "f")
+y = torch.zeros(64, device="cuda")
+torch.cuda.synchronize()
+before = torch.cuda.mem_get_info()[0]
+assert _noalloc_fn(pkg.lib())(stack.handle, 0, 0, 0, 0, 0, 0, 1.0, 1.0, 4,
+                              y.data_ptr(), y.data_ptr(), y.data_ptr(),
+                              torch.cuda.current_stream().cuda_stream) == 0
+torch.cuda.synchronize()
+print("held", before - torch.cuda.mem_get_info()[0])
+"""
+
+
+def test_noalloc_array_is_32_mib(pkg):
+    """The array that the first no-alloc call on a device brings with it, in a
+    process of its own: 32 MiB and at most 8 for the code beside it."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    r = subprocess.run([sys.executable, "-c", SIZE.format(root=ROOT)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    held = int(r.stdout.split()[-1])
+    assert 0 <= held <= 40 << 20
