@@ -39,7 +39,9 @@ from typing import Callable, Dict, Iterable, Optional
 import numpy as np
 
 CACHE_ENV = "GPUGRID_TUNE_CACHE"
-CACHE_VERSION = 8
+#: Raised when a setting's meaning, an automatic choice or the kernels that were
+#: timed change: settings found for others are not applied.
+CACHE_VERSION = 9
 
 #: The plan's settings before any tuning (each call chooses shape/staging).
 DEFAULT_TUNING = {"tile_u": 0, "slice_staging": -1, "items_per_cta": 4,
@@ -89,8 +91,9 @@ def tuning_key(grid_size: int, num_w_planes: int, max_support: int,
 
 
 class TuningCache:
-    """JSON file of tuned settings: {"version": 2, "devices": {name: {key:
-    {setting: value, ..., "ms": t}}}}."""
+    """JSON file of tuned settings: {"version": CACHE_VERSION, "devices":
+    {name: {key: {setting: value, ..., "ms": t}}}}.  A file of another version
+    is treated as empty."""
 
     def __init__(self, path: Optional[str] = None):
         self.path = path or default_cache_path()

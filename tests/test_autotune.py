@@ -145,3 +145,18 @@ def test_host_search_keeps_the_fastest(at):
     assert (0, 64) in tried and (1, 64) in tried
     assert {t["tile_phases"] for t in applied} >= {0, 1, 2}
     assert got["ms"] >= 0
+
+
+@pytest.mark.parametrize("version", [2, 8])
+def test_cache_ignores_settings_of_earlier_kernels(at, tmp_path, version):
+    """Settings that were found when items_per_cta, plane_group_mb,
+    sort_detail 2 and the automatic phases meant something else."""
+    p = tmp_path / "tuning.json"
+    entry = dict(at.DEFAULT_TUNING, plane_group_mb=64, tile_phases=2, ms=1.0)
+    p.write_text(json.dumps({"version": version,
+                             "devices": {"GB300": {"k": entry}}}))
+    c = at.TuningCache(str(p))
+    assert c.get("GB300", "k") is None
+    c.put("GB300", "k", entry)
+    c.save()
+    assert at.TuningCache(str(p)).get("GB300", "k") == entry
