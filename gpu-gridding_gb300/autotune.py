@@ -48,7 +48,11 @@ DEFAULT_TUNING = {"tile_u": 0, "slice_staging": -1, "items_per_cta": 4,
                   "sort_detail": 2, "ctas_per_sm": 0, "plane_group_mb": 0,
                   "tile_order": 0, "lane_groups": 0, "tile_phases": 0}
 
-#: Values tried per setting, in search order.
+#: Settings without effect: kept in gg_tuning and in the dictionaries, never timed
+#: (noise would choose among their values).
+WITHOUT_EFFECT = ("slice_staging", "lane_groups")
+
+#: Values per setting, in search order (:func:`timed_space` of it is tried).
 SEARCH_SPACE = (
     (("tile_u", "slice_staging"),
      [(0, -1), (32, 0), (32, 1), (16, 0), (16, 1), (8, 0), (8, 1)]),
@@ -61,6 +65,19 @@ SEARCH_SPACE = (
     (("lane_groups",), [(0,), (2,)]),
     (("tile_phases",), [(0,), (2,), (4,), (8,)]),
 )
+
+
+def timed_space(space: Iterable = SEARCH_SPACE) -> list:
+    """``space`` without the settings of :data:`WITHOUT_EFFECT` and the values
+    that differ in those alone."""
+    out = []
+    for names, values in space:
+        keep = [i for i, name in enumerate(names)
+                if name not in WITHOUT_EFFECT]
+        if keep:
+            out.append((tuple(names[i] for i in keep), list(dict.fromkeys(
+                tuple(v[i] for i in keep) for v in values))))
+    return out
 
 
 def default_cache_path() -> str:
@@ -281,7 +298,7 @@ def autotune(pkg, plan, stack, uu, vv, ww, vis, weight, cell_size_rad,
         except pkg.GridError:
             return math.inf
 
-    best, best_ms, trials = search(measure)
+    best, best_ms, trials = search(measure, timed_space())
     del grids
     plan.set_tuning(best)
     entry = dict(best, ms=best_ms)

@@ -160,3 +160,34 @@ def test_cache_ignores_settings_of_earlier_kernels(at, tmp_path, version):
     c.put("GB300", "k", entry)
     c.save()
     assert at.TuningCache(str(p)).get("GB300", "k") == entry
+
+
+def test_settings_without_effect_are_not_timed(at):
+    space = at.timed_space()
+    names = [n for group, _ in space for n in group]
+    assert set(names) == set(at.DEFAULT_TUNING) - set(at.WITHOUT_EFFECT)
+    assert dict(space)[("tile_u",)] == [(0,), (32,), (16,), (8,)]
+    for group, values in space:
+        assert len(set(values)) == len(values)
+        assert all(len(v) == len(group) for v in values)
+    seen = []
+    at.search(lambda t: seen.append(t) or 1.0, space)
+    for name in at.WITHOUT_EFFECT:
+        assert {t[name] for t in seen} == {at.DEFAULT_TUNING[name]}
+
+
+def test_autotune_times_that_space(at, monkeypatch, tmp_path):
+    torch = pytest.importorskip("torch")
+    import types
+    got = []
+    monkeypatch.setattr(at, "_device_name", lambda _: "GB300")
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: None)
+    monkeypatch.setattr(at, "search", lambda measure, space: got.append(space)
+                        or (dict(at.DEFAULT_TUNING), 1.0, {}))
+    stack = types.SimpleNamespace(num_w_planes=2, support=[1, 2], oversample=4,
+                                  precision="f")
+    plan = types.SimpleNamespace(set_tuning=lambda t: None)
+    x = torch.zeros(4)
+    at.autotune(None, plan, stack, x, x, x, x, x, 1.0, 1.0, 8,
+                cache=at.TuningCache(str(tmp_path / "t.json")))
+    assert got == [at.timed_space()]
