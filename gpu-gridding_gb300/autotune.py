@@ -8,7 +8,8 @@ no placement, norm or skip count (gg_tuning in the C header):
 * ``items_per_cta`` -- how finely heavy tiles are split into work items,
 * ``sort_detail``   -- record order within a tile (by plane where it pays,
   by plane, or visibility order),
-* ``ctas_per_sm``   -- resident gridding CTAs per SM (0 = as many as fit),
+* ``ctas_per_sm``   -- resident teams of eight warps per SM (0 = as many as
+  fit),
 * ``plane_group_mb`` -- kernel bytes per gridding pass (0 = 3/4 of L2
   for the planes that the call uses),
 * ``tile_order``    -- tiles taken by distance from the centre or row by row,

@@ -561,7 +561,7 @@ struct gg_plan {
   int slice_staging = -1; // as set; without effect (gg_plan_set_slice_staging)
   int items_per_cta = 4;  // work-item granularity of heavy-tile splits
   int sort_detail = 2;    // records of a tile by plane: 2 where it pays, 1, 0
-  int ctas_per_sm = 0;    // cap on resident gridding CTAs, 0 = none
+  int ctas_per_sm = 0;    // cap on resident teams of eight warps, 0 = none
   int plane_group_mb = 0; // slice bytes per plane group, 0 = 3/4 of L2
   int queue_order = 0;    // tuning tile_order: 0 radius, 1 row by row
   int lane_groups = 0;    // as set; without effect (gg_tuning)
@@ -1553,7 +1553,8 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   int sms = 0;
   GG_TRY(num_sms_of_current(&sms));
   int per_sm = grid_tiles_ctas_per_sm<Real>(geom.tile_u, view.wide);
-  if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
+  if (plan->ctas_per_sm > 0)
+    per_sm = std::min(per_sm, plan->ctas_per_sm * kBlocksPerTeam);
   const int num_ctas = sms * per_sm;
   ItemBuffers ib;
   // The tile phases of a plane group share one launch, their later phases'
@@ -1564,7 +1565,6 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   const int span = geom.tile_phases;
   GG_TRY(build_work_items<Real>(plan, b, grid_teams(num_ctas),
                                 geom.num_groups, s, &ib, span));
-  plan->stats.num_ctas = num_ctas;
   plan->kept.group_span = span;
   plan->kept.rec_vis = b.vals;
   plan->kept.num_ctas = num_ctas;
@@ -1991,9 +1991,10 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
     int sms = 0;
     GG_TRY(num_sms_of_current(&sms));
     int per_sm = degrid_tiles_ctas_per_sm<Real>(view.wide);
-    if (plan->ctas_per_sm > 0) per_sm = std::min(per_sm, plan->ctas_per_sm);
+    if (plan->ctas_per_sm > 0)
+      per_sm = std::min(per_sm, plan->ctas_per_sm * kBlocksPerTeam);
     const int num_ctas = sms * per_sm;
-    plan->stats.num_ctas = num_ctas;
+    plan->stats.num_ctas = grid_teams(num_ctas);
     GG_TRY(plan->rec_out.ensure((size_t)b.total * 2 * sizeof(Real)));
     uint32_t* sc = plan->scalars.as<uint32_t>();
     if (plan->grid_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->grid_wait, 0));

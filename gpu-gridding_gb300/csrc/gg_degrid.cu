@@ -47,6 +47,7 @@ constexpr int kDegridTileU = 32;
 using DegridShape = WarpShape<kDegridTileU>;
 constexpr int kDegridWarps = 4;    // per block
 constexpr int kDegridThreads = kDegridWarps * 32;
+static_assert(kDegridWarps * kBlocksPerTeam == kWarps, "a team");
 constexpr int kUnit = 128;         // records of a unit, at most
 constexpr int kPerLane = kUnit / 32;
 // A unit with fewer records a tile than this takes its records' grid values

@@ -249,6 +249,7 @@ struct WarpSmem {
 
 constexpr int kGridWarps = 4;    // per block of the gridding kernel
 constexpr int kGridThreads = kGridWarps * 32;
+static_assert(kGridWarps * kBlocksPerTeam == kWarps, "a team");
 
 // kPrepared: the records come from k_prepare_records; else (a call for which
 // those do not fit the device's memory) every band's warp prepares them itself.
@@ -1207,7 +1208,7 @@ int grid_tiles_ctas_per_sm(int tile_u, bool wide) {
 }
 
 int grid_teams(int num_ctas) {
-  return std::max(1, num_ctas * kGridWarps / kWarps);
+  return std::max(1, num_ctas / kBlocksPerTeam);
 }
 
 template <typename Real>

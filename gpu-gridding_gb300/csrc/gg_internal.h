@@ -321,8 +321,12 @@ cudaError_t launch_tile_groups(const uint32_t* tile_start,
                                const TileGeom& geom, int grid_size,
                                uint32_t* out, unsigned long long* cells,
                                cudaStream_t s);
-// Resident CTAs per SM (wide: StackView::wide), and the teams of one warp per
-// band of a tile that num_ctas CTAs make.
+// Blocks of the tile kernels that make a team: a warp for each of a tile's
+// eight bands.  What a caller sets and reads are teams (ctas_per_sm, num_ctas),
+// as a block of the kernels before these had those eight warps.
+constexpr int kBlocksPerTeam = 2;
+// Resident blocks per SM (wide: StackView::wide), and the teams that num_ctas
+// blocks make.
 template <typename Real>
 int grid_tiles_ctas_per_sm(int tile_u, bool wide);
 int grid_teams(int num_ctas);

@@ -150,7 +150,7 @@ typedef struct
     unsigned long long num_launches;    /* kernels this library launched */
     int tile_u, tile_v;                 /* tile shape used */
     int slice_staging;                  /* always 0 (see gg_plan_set_slice_staging) */
-    int num_ctas;                       /* persistent gridding CTAs */
+    int num_ctas;                       /* resident teams of eight warps */
     unsigned long long chunk_records;   /* records per work item (max) */
     int num_plane_groups;               /* gridding passes (plane groups) */
 } gg_stats;
@@ -186,8 +186,9 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  *   sort_detail    order of a tile's records: 2 (default) by w-plane where
  *                  that pays (three plane groups or more), 1 by w-plane, 0
  *                  visibility order
- *   ctas_per_sm    resident gridding CTAs per SM, 0 (default) = as many as
- *                  fit, else min(that, what fits), 1..32
+ *   ctas_per_sm    resident teams of eight warps (one for each band of a
+ *                  tile) per SM, 0 (default) = as many as fit, else min(that,
+ *                  what fits), 1..32
  *   plane_group_mb kernel bytes per gridding pass: the w-planes are cut
  *                  into as few groups of consecutive planes as keep each
  *                  group's re-laid kernels within this many MiB (about

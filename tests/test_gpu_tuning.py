@@ -427,3 +427,42 @@ def test_record_order_follows_the_cache(pkg, torch, top, planes_mb, by_plane):
         outs.append((plan.stats()["num_launches"], grid))
     assert outs[0][0] == outs[1][0]
     assert torch.equal(outs[0][1], outs[1][1])
+
+
+def test_ctas_per_sm_counts_eight_warps(pkg, torch):
+    """ctas_per_sm caps teams of eight warps, the warps of a tile's bands: two
+    an SM are sixteen warps where twenty fit, so a call takes at most 20 / 16 of
+    the time and 0.1 ms, and one an SM at most 20 / 8."""
+    G, n, planes = 2048, 200_000, 64
+    sup = np.rint(np.linspace(20, 72, planes)).astype(np.int32)
+    stack = pkg.KernelStack.generate(planes, sup, 4, 4 * 73,
+                                     np.full(planes, 3.0))
+    rng = np.random.default_rng(5)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+    uu, vv = (dev(rng.uniform(-200.0, 200.0, n)) for _ in range(2))
+    p = rng.integers(0, planes, n).astype(np.float64)
+    args = (stack, uu, vv, dev(p * p), dev(rng.standard_normal((n, 2))),
+            dev(rng.uniform(1, 2, n)), 0.002, np.float32(1.0), G)
+    grid = torch.zeros((G, G, 2), dtype=torch.float32, device="cuda")
+    norm = torch.zeros(1, dtype=torch.float64, device="cuda")
+    skip = torch.zeros(1, dtype=torch.int64, device="cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def ms(ctas):
+        plan = pkg.Plan()
+        plan.set_tuning({"ctas_per_sm": ctas})
+        best = float("inf")
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            pkg.grid_wproj_device(plan, *args, grid, norm, skip)
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        teams = plan.stats()["num_ctas"]
+        assert teams <= (ctas or 32) * sms and teams >= sms
+        return best
+
+    free = ms(0)
+    assert ms(2) <= 1.25 * free + 0.1
+    assert ms(1) <= 2.5 * free + 0.1
