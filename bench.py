@@ -221,7 +221,8 @@ def parse_args():
     ap.add_argument("--tile-shape", type=int, default=0,
                     help="force the tile width (32, 16, 8); 0 = automatic")
     ap.add_argument("--staging", type=int, default=-1,
-                    help="kernel-slice staging: -1 automatic, 0 off, 1 on")
+                    help="accepted; without effect but that 0 and 1 skip the "
+                         "autotuner")
     ap.add_argument("--no-autotune", action="store_true",
                     help="use the per-call heuristics instead of tuning the "
                          "plans (tuning runs before the timed region)")

@@ -9,9 +9,11 @@
 //   4. radix sort      stable, so the record order is deterministic
 //   5. tile bounds     record range of every tile
 //   6. work items      tiles cut into chunks; split chunks get partial slots
-//   7. k_grid_tiles    persistent tile-owning accumulation
-//   8. reduce          split tiles: grid += partials, in chunk order
-// The host synchronises once, after step 2, to size the sort buffers.
+//   7. k_prepare_records  the sorted records' descriptors
+//   8. k_grid_tiles    persistent tile-owning accumulation
+//   9. reduce          split tiles: grid += partials, in chunk order
+// The host synchronises once, after step 2, to size the sort buffers (and, with
+// several tile phases, after step 6, to size the partial tiles).
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -891,11 +893,13 @@ int read_scalars(gg_plan* plan, const gg_kernels* K, PlacedPoints points,
   return GG_OK;
 }
 
-// Slice bytes that 95 % of the call's taps come from (read_scalars), the most used bins of
-// planes first; the whole stack where that is more than four fifths of it (one
-// used evenly).  The planes of a telescope's visibilities crowd near zero: of a stack of 327 MB (601 planes,
-// support 4 to 72), 512-station tracks take 95 % of their taps from 67 MB,
-// 128-station ones from 114, uniform w from 290.
+// Slice bytes that 95 % of the call's taps come from (read_scalars), the most
+// used bins of planes first; the whole stack where that is more than four
+// fifths of it: one used evenly, whose other planes are used too (uniform w on
+// 327 MB: its 290 MB would make three groups, 5.31 ms, and four take 5.14).
+// The planes of a telescope's visibilities crowd near zero: of that stack (601
+// planes, support 4 to 72), 512-station tracks take 95 % of their taps from 67
+// MB, 128-station ones from 114.
 long long used_bytes(const gg_plan* plan, const gg_kernels* K) {
   const uint32_t* use =
       (const uint32_t*)((const char*)plan->h_scalars + kUseOffset);
@@ -1481,7 +1485,7 @@ int build_work_items(gg_plan* plan, const Bins& b, int num_ctas, int passes,
   GG_TRY(tile_queue_order(plan, b.geom, b.grid_size, false, s,
                           &ib->tile_order));
   GG_CUDA(launch_build_items(plan->tile_start.as<uint32_t>(), num_tiles,
-                             b.total, chunk, *ib, s));
+                             chunk, *ib, s));
   if (pphases > 1) {
     uint32_t slots = 0;
     GG_CUDA(cudaMemcpyAsync(&slots, ib->num_slots, sizeof(slots),

@@ -50,7 +50,7 @@ struct Vec2<double> { using type = double2; };
 // A placed visibility as the gridding kernel's records gather it: cell, meta
 // and the weighted visibility together, so that the gather of a record, in
 // tile order and so at random, is one sector of HBM and not three (3.1e7 track
-// points, 5.9e7 records: 3 GB less, 1 ms of 25).
+// points, 5.9e7 records: 2.55 ms with three, 1.10 with one).
 template <typename Real>
 struct alignas(4 * sizeof(Real)) Placed {
   uint32_t cell, meta;

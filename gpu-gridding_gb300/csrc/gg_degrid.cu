@@ -209,7 +209,7 @@ k_degrid_tiles(DegridArgs<Real> a) {
     for (int q = 0; q < kPerLane; ++q) {
       const int t = q * 32 + lane;
       if (t < nb) {
-        const uint32_t tile = a.low_bits >= 32 ? 0u : key[q] >> a.low_bits;
+        const uint32_t tile = key[q] >> a.low_bits;
         const int vg = (int)(tile / (uint32_t)a.geom.tiles_total);
         const int tl =
             a.tile_order[tile - (uint32_t)vg * (uint32_t)a.geom.tiles_total];

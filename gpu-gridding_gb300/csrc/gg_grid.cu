@@ -490,7 +490,7 @@ struct WarpSmem64 {
 };
 
 // The gridding kernel in FP64.  The FP64 pipe bounds it (a warp's FMA takes
-// 12 cycles of the SM however few of its lanes are active, four of them for
+// 16 cycles of the SM however few of its lanes are active, four of them for
 // 32 cells), so the lanes take a record's cells in the band packed row by row,
 // whatever the footprint's position, instead of a column each: of the cells
 // of a record on a band about half are inside its footprint (2048^2, 2e5
@@ -989,9 +989,39 @@ __global__ void k_tile_groups(const uint32_t* __restrict__ tile_start,
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(cells, mine);
 }
 
-// Failure-path probe: every thread waits, bounded by `limit` probes, on an
-// mbarrier that nothing arrives at -- the wait the gridding kernels use --
-// so the wait runs out, the kernel sets the error flag and returns.
+// The failure-report probe's wait: no other kernel waits on a barrier.
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "r"(count)
+               : "memory");
+}
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Acquire-wait for the completion of the phase with the given parity;
+// false when `limit` probes have failed.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
+                                          unsigned limit) {
+  for (unsigned i = 0; i < limit; ++i) {
+    if (mbar_test(bar, parity)) return true;
+    if (i >= 32) __nanosleep(64);
+  }
+  return false;
+}
+// Failure-report probe: every thread waits, bounded by `limit` probes, on an
+// mbarrier that nothing arrives at, so the wait runs out, the kernel sets the
+// error flag and returns.
 __global__ void k_wait_probe(unsigned limit, uint32_t* __restrict__ error) {
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) mbar_init(&bar, 1);
@@ -1083,10 +1113,9 @@ __global__ void k_item_emit(const uint32_t* __restrict__ tile_start,
   }
 }
 
-// The kernels take more than 48 KB of dynamic shared memory: opt in before
-// querying occupancy or launching.  The opt-in is made once per device, so
-// later launches (replays captured in a CUDA graph among them) make no
-// attribute call.
+// The kernels take 24 to 48 KB of dynamic shared memory: set before querying
+// occupancy or launching, once per device, so later launches (replays captured
+// in a CUDA graph among them) make no attribute call.
 template <typename Real, int TW, bool kWide, bool kPrepared>
 cudaError_t prepare_grid_kernel(void** fn, size_t* smem) {
   static std::atomic<unsigned long long> opted_in{0};
@@ -1133,8 +1162,7 @@ cudaError_t prepare_grid_kernel_for(int tile_u, bool wide, bool prepared,
 cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
                                int num_tiles, uint32_t* tile_start,
                                cudaStream_t s) {
-  // A tile per thread; with the whole key below the tile field no shift
-  // separates them, and every record is tile 0's.
+  // A tile per thread, and one more for the end.
   const int blocks = num_tiles / 256 + 1;
   k_tile_bounds<<<blocks, 256, 0, s>>>(keys, n, shift, num_tiles, tile_start);
   return cudaGetLastError();
@@ -1170,9 +1198,8 @@ cudaError_t launch_touched_spans(const uint32_t* tile_start, int num_tiles,
 }
 
 cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
-                               uint32_t num_records, uint32_t chunk,
-                               ItemBuffers b, cudaStream_t s) {
-  (void)num_records;
+                               uint32_t chunk, ItemBuffers b,
+                               cudaStream_t s) {
   uint32_t* A = b.chunks;
   uint32_t* B = b.split_chunks;
   const int blocks = (num_tiles + 256) / 256;   // one more thread: bounds

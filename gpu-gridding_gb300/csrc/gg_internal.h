@@ -18,6 +18,11 @@ namespace gg {
 size_t scan_temp_bytes(size_t n);
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n,
                                uint32_t* d_total, void* tmp, cudaStream_t s);
+// The same for two arrays of n entries, in place and in the same launches
+// (tmp: scan_temp_bytes(n)).
+cudaError_t exclusive_scan_pair_u32(uint32_t* a, uint32_t* b, size_t n,
+                                    uint32_t* total_a, uint32_t* total_b,
+                                    void* tmp, cudaStream_t s);
 // *total (device) = sum of in[0..n) in 64 bits.
 cudaError_t sum_u32(const uint32_t* in, size_t n, unsigned long long* total,
                     cudaStream_t s);
@@ -26,10 +31,6 @@ cudaError_t sum_u32(const uint32_t* in, size_t n, unsigned long long* total,
 // Sorts the first n pairs by key bits [0, end_bit).  Ping-pongs between
 // (keys, vals) and (keys_alt, vals_alt); on return *in_alt tells which pair
 // of buffers holds the result.  tmp must hold radix_temp_bytes(n).
-// The same for two arrays of n entries, in place and in the same launches.
-cudaError_t exclusive_scan_pair_u32(uint32_t* a, uint32_t* b, size_t n,
-                                    uint32_t* total_a, uint32_t* total_b,
-                                    void* tmp, cudaStream_t s);
 // Kernel launches of a scan of n entries (one array or a pair), and of a sort.
 int scan_launches(size_t n);
 int radix_passes(int end_bit);
@@ -84,7 +85,12 @@ __host__ __device__ inline int tile_v_of_shape(int shape) {
 // where offset tile grids save the most tile crossings, and the call has
 // enough of them for its `tiles` tiles, else one.  What four phases save
 // grows with the MACs (more per MAC in narrow tiles), what they cost (the
-// partial tiles of the later phases and their addition) with the tiles.
+// partial tiles of the later phases and their addition) with the tiles, and
+// there is a fixed cost of 30 to 40 us (a second wait for the host, which sizes
+// the partial tiles, and the reduction), 1.5e8 of them: 256^2, support 8 to 13,
+// 1.1e8 MACs 0.346 and 0.375, 2.3e8 0.511 and 0.498; 1024^2 0.298 and 0.327,
+// 0.454 and 0.426; 16-wide tiles, support 5 and 6, 512^2, 6.3e7 MACs 0.332 and
+// 0.347, 1.3e8 0.503 and 0.481.
 // Measured, ms with one and four phases (track points, 32-wide tiles where
 // support reaches 44, 16-wide for 18): 7.8e6 on 2048^2, support 44 6.85 and
 // 5.17, 18 3.09 and 2.50; on 8192^2 6.57 and 5.69, 3.07 and 3.03; 1e6 on
@@ -219,7 +225,7 @@ cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
 cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
                                int num_tiles, uint32_t* tile_start,
                                cudaStream_t s);
-// One CTA whose threads wait, bounded by `limit` probes, on an mbarrier
+// One block whose threads wait, bounded by `limit` probes, on an mbarrier
 // that nothing arrives at, then set *error (see gg_plan_probe_bounded_wait).
 cudaError_t launch_wait_probe(unsigned limit, uint32_t* error,
                               cudaStream_t s);
@@ -269,8 +275,8 @@ struct ItemBuffers {
   int2* tile_slot = nullptr;
 };
 cudaError_t launch_build_items(const uint32_t* tile_start, int num_tiles,
-                               uint32_t num_records, uint32_t chunk,
-                               ItemBuffers b, cudaStream_t s);
+                               uint32_t chunk, ItemBuffers b,
+                               cudaStream_t s);
 // Bytes of a prepared record (launch_grid_tiles' recs, one per record; spans
 // takes two more).
 template <typename Real>
@@ -348,7 +354,8 @@ inline long long cache_budget(int l2) {
 
 // ---- uniform weighting (gg_weights.cu) -------------------------------------
 // Keys each point by its density cell (grid_size^2 when off the grid), its
-// value the weight's bits (FP32) or its index, and counts the off-grid points into *d_num_skipped (which must start at 0).
+// value the weight's bits (FP32) or its index, and counts the off-grid points
+// into *d_num_skipped (which must start at 0).
 template <typename Real>
 cudaError_t launch_weight_keys(const Real* uu, const Real* vv,
                                const Real* weight, unsigned long long n,

@@ -25,11 +25,10 @@
 //   count is known only after placement, whose norm and skip totals go to
 //   the scratch array and reach the caller's outputs once the call is
 //   accepted);
-// * if a call's gridding kernel runs out of its bounded wait, that call has
-//   already returned GG_OK; the failure is reported by the next no-alloc
-//   call on the device (whoever makes it), which returns GG_ERR_CUDA
-//   without touching its outputs -- the incomplete grid is the previous
-//   call's;
+// * the array's error flag (set by gg_noalloc_probe_bounded_wait alone: the
+//   tile kernels wait for nothing) is reported by the next no-alloc call on the
+//   device (whoever makes it), which returns GG_ERR_CUDA without touching its
+//   outputs and clears it;
 // * the device address of the array is looked up (cudaGetSymbolAddress) by
 //   the first call on each device, which must therefore be made with that
 //   device current and before any stream capture begins.
@@ -207,8 +206,8 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
                         "no-alloc scratch layout exceeds the array");
 
   // The array keeps the previous call's contents: clear the counters this
-  // call accumulates into.  Word 6, the bounded-wait error flag of the
-  // tile kernel, is left for the check below.
+  // call accumulates into.  Word 6, the error flag, is left for the check
+  // below.
   NA_CUDA(cudaMemsetAsync(sc, 0, 6 * sizeof(uint32_t), s));
   NA_CUDA(cudaMemsetAsync(call_norm, 0, sizeof(double), s));
 
@@ -240,8 +239,8 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   if (host_sc[6]) {
     NA_CUDA(cudaMemsetAsync(sc + 6, 0, sizeof(uint32_t), s));
     return record_error(GG_ERR_CUDA,
-                        "an earlier no-alloc call's tile kernel ran out of "
-                        "its bounded wait; that call's grid is incomplete");
+                        "a kernel on the no-alloc array ran out of its "
+                        "bounded wait");
   }
   const uint32_t total = host_sc[0];
   const int shape = (int)(host_sc[5] & 0xFFu);
@@ -314,7 +313,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   ib.group_items = sc + 8;   // two entries: one plane group
   ib.num_groups = 1;
   ib.scan_tmp = scan_tmp;
-  NA_CUDA(launch_build_items(tile_start, num_tiles, total, chunk, ib, s));
+  NA_CUDA(launch_build_items(tile_start, num_tiles, chunk, ib, s));
   NA_CUDA(launch_grid_tiles<float>(items, sc + 8, sc + 4, nullptr, nullptr, vals,
                                    placed, view, geom, grid_size, d_grid, 0,
                                    (float*)partials, split_tiles, sc + 3,

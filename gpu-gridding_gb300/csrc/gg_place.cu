@@ -307,7 +307,7 @@ __global__ void k_emit(PlacedPoints points,
           group = group * (uint32_t)g.tile_phases + (uint32_t)phase;
         tile += group * (uint32_t)g.tiles_total;
       }
-      keys[pos] = low_bits >= 32 ? low : ((tile << low_bits) | low);
+      keys[pos] = (tile << low_bits) | low;
       vals[pos] = vid;
       ++pos;
     }

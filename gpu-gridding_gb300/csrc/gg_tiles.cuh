@@ -1,7 +1,7 @@
 // Pieces shared by the tile-owning kernels (gridding in gg_grid.cu,
 // degridding in gg_degrid.cu): the tile shape (2048 cells in eight bands,
-// lane = column, kRows rows per lane), bounded mbarrier waits, tap loads and
-// the slice descriptor of a record.
+// lane = column, kRows rows per lane), tap loads and the slice descriptor of a
+// record.
 #pragma once
 
 #include "gg_internal.h"
@@ -11,14 +11,10 @@ namespace gg {
 namespace {
 
 constexpr int kRows = 8;          // rows per lane (registers)
-constexpr int kWarps = 8;         // consumer warps per CTA
+constexpr int kWarps = 8;         // bands of a tile, one warp each
 constexpr int kConsumers = kWarps * 32;
 constexpr int kCells = kConsumers * kRows; // 2048 cells per tile
 static_assert(kRows - 1 <= kSlicePad, "slices need kRows-1 padding rows");
-// Bound on every mbarrier wait (each failed probe sleeps ~100 ns): a wait
-// that runs out (> ~1 s) sets the error flag and the CTA returns.
-constexpr unsigned kWaitLimit = 1u << 24;
-
 template <int TW>
 struct WarpShape {
   static constexpr int kLanesY = 32 / TW;          // lane rows per warp
@@ -27,36 +23,6 @@ struct WarpShape {
   static constexpr int kTileV = kWarps * kBand;
 };
 
-// ---- mbarrier helpers (shared::cta) --------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(count)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Acquire-wait for the completion of the phase with the given parity;
-// false when `limit` probes have failed.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          unsigned limit = kWaitLimit) {
-  for (unsigned i = 0; i < limit; ++i) {
-    if (mbar_test(bar, parity)) return true;
-    if (i >= 32) __nanosleep(64);
-  }
-  return false;
-}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return __ffma2_rn(a, b, c);
 }
@@ -109,13 +75,6 @@ __device__ __forceinline__ int slice_step(uint2 d) {
   const int pitch = 2 * (int)((d.y >> 16) & 0x3FFFu) + 2;
   return (int)d.y < 0 ? -pitch : pitch;
 }
-// Tap index of tile cell (0, col) of descriptor d with that step.
-__device__ __forceinline__ uint32_t slice_tap(uint2 d, int step, int col) {
-  const int z = (int)(short)(d.y & 0xFFFFu);
-  const int c = d.y & kMirrorU ? z - col : z + col;
-  return d.x + (uint32_t)min(max(c, -1), abs(step) - 1);
-}
-
 // kRows taps from `at` on, `step` taps apart.  kWide: the stack holds more
 // than 4 GiB; below that its byte offsets fit 32 bits, and each row costs one
 // 32-bit addition to a common base instead of a 64-bit one (5 % of the

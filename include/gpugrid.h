@@ -184,8 +184,8 @@ GG_API int gg_plan_set_slice_staging(gg_plan* plan, int mode);
  *                  64 items a team): more items balance the load better but
  *                  write more partial tiles
  *   sort_detail    order of a tile's records: 2 (default) by w-plane where
- *                  that pays (three plane groups or more), 1 by w-plane, 0
- *                  visibility order
+ *                  that pays (three plane groups or more, or a gridding pass
+ *                  whose kernels leave L2), 1 by w-plane, 0 visibility order
  *   ctas_per_sm    resident teams of eight warps (one for each band of a
  *                  tile) per SM, 0 (default) = as many as fit, else min(that,
  *                  what fits), 1..32
@@ -388,9 +388,7 @@ GG_API int gg_grid_wproj_d_batched_device(gg_plan* plan,
  * memset on the stream -- no allocation, no host synchronisation -- so it
  * may be captured in a CUDA graph.  Any other gridding call on the plan
  * discards the kept geometry (GG_ERR_INVALID_ARG on the next replay).  The
- * kernels argument must be the batched call's.  A failure inside the
- * gridding kernel (a bounded wait that ran out) is reported by the next
- * gg_plan_check or the next non-replay call. */
+ * kernels argument must be the batched call's. */
 GG_API int gg_grid_wproj_f_batched_replay(gg_plan* plan,
         const gg_kernels* kernels, const float* d_vis, const float* d_weight,
         unsigned long long* d_num_skipped, double* d_norm, float* d_grids,
@@ -413,15 +411,15 @@ GG_API int gg_grid_wproj_d_batched_replay(gg_plan* plan,
 GG_API int gg_plan_set_batch_limit(gg_plan* plan,
                                    unsigned long long max_points);
 
-/* Synchronises the stream and returns GG_ERR_CUDA if a gridding kernel of
- * this plan flagged a failure (a bounded wait that ran out). */
+/* Synchronises the stream and returns GG_ERR_CUDA if the plan's error flag is
+ * set.  The gridding and degridding kernels wait for nothing (each warp takes
+ * its own work), so only gg_plan_probe_bounded_wait sets it. */
 GG_API int gg_plan_check(gg_plan* plan, void* stream);
 
-/* Diagnostic of that failure path, safe to run: a kernel waits, bounded by
+/* Diagnostic of that report, safe to run: a kernel waits, bounded by
  * `iterations` probes (1..1048576, each failed probe sleeping ~64 ns), on
- * an mbarrier that nothing arrives at -- the kind of wait the gridding
- * kernels bound -- so the wait runs out, the kernel sets the plan's error
- * flag and returns.  Returns GG_ERR_CUDA (with its message) as the plan
+ * an mbarrier that nothing arrives at, so the wait runs out, the kernel sets
+ * the plan's error flag and returns.  Returns GG_ERR_CUDA (with its message) as the plan
  * then does from every call; the device and other plans stay usable. */
 GG_API int gg_plan_probe_bounded_wait(gg_plan* plan, unsigned iterations,
                                       void* stream);
@@ -440,11 +438,9 @@ GG_API int gg_plan_probe_bounded_wait(gg_plan* plan, unsigned iterations,
  * the array, so calls that overlap on the GPU race and must be serialised by
  * the caller.  The first call on each device looks up the array's device
  * address; make it with that device current and before any stream capture.
- * If a call's gridding kernel runs out of its bounded wait (see
- * gg_plan_check), that call has already returned GG_OK: the failure is
+ * The array's error flag, which gg_noalloc_probe_bounded_wait sets, is
  * reported by the next no-alloc call on the same device, which returns
- * GG_ERR_CUDA with its outputs untouched and clears the flag -- the
- * incomplete grid is the earlier call's.  Same semantics and results as
+ * GG_ERR_CUDA with its outputs untouched and clears it.  Same semantics and results as
  * gg_grid_wproj_f_device otherwise (grid and *d_norm accumulated,
  * *d_num_skipped set; one stream synchronisation per call). */
 GG_API int gg_grid_wproj_f_device_noalloc(const gg_kernels* kernels,
