@@ -27,7 +27,7 @@
 // Calls in ms, with a block of eight band warps and a producer sharing a
 // stream of records -> warps of their own: 2e5 points on 2048^2 0.513 ->
 // 0.467; 7.8e6 track points on 8192^2 (support 4 to 72) 7.9 -> 6.8; the
-// former in FP64 5.4 -> 2.9 (the multiply-adds alone 1.7); and with a tile's
+// former in FP64 5.4 -> 2.8 (the multiply-adds alone 1.7); and with a tile's
 // records in visibility order 0.449 and 6.4.
 //
 // The reference has no degridder; this one is pinned by the dot-product
@@ -271,12 +271,18 @@ k_degrid_tiles(DegridArgs<Real> a) {
         for (int j = 0; j < 4; ++j) {
           const int t = min(t0 + j, kUnit);
           word |= (uint32_t)(t < nb ? t : kUnit) << (8 * j);
-          Real re = 0, im = 0;
+          // As dot_record's sums, eight cells of a lane at a time: one chain
+          // of additions over all of a lane's cells left up to half as much
+          // error again (supports of 30 to 60), and took longer: 2e5 points
+          // of support 4 to 24 on 2048^2 2.82 ms, so 2.77; 6e4 of 10 to 60
+          // 4.73 and 4.24.
+          R2 X{}, Y{};
+          bool conj = false;
           if (t < nb) {
             const int4 e = sm.rec[t];
             const int gu = (int)(short)e.y, s = e.z - 1;
             const int su = e.y & kMirrorU ? -1 : 1;
-            const bool conj = e.y < 0;
+            conj = e.y < 0;
             const int c0 = max(gu - s, 0);
             const int w = min(gu + s, kDegridTileU - 1) - c0 + 1;
             const int top = sm.row0[t];
@@ -287,7 +293,7 @@ k_degrid_tiles(DegridArgs<Real> a) {
             const uint32_t x = (uint32_t)(e.x + r0 * e.w + su * (c0 - gu));
             const int2 o = sm.origin[t];
             const R2* const cells = grid + (size_t)(o.y + r0) * G + o.x + c0;
-            for (int k = lane; k < n; k += 32 * kAhead) {
+            auto add = [&](int k, R2& PX, R2& PY) {
               R2 tap[kAhead], cell[kAhead];
 #pragma unroll
               for (int h = 0; h < kAhead; ++h) {
@@ -304,14 +310,24 @@ k_degrid_tiles(DegridArgs<Real> a) {
 #pragma unroll
               for (int h = 0; h < kAhead; ++h) {
                 if (k + 32 * h >= n) break;
-                const Real ti = conj ? -tap[h].y : tap[h].y;
-                re = fma(ti, cell[h].y, fma(tap[h].x, cell[h].x, re));
-                im = fma(-ti, cell[h].x, fma(tap[h].x, cell[h].y, im));
+                PX.x = fma(tap[h].x, cell[h].x, PX.x);
+                PX.y = fma(tap[h].y, cell[h].y, PX.y);
+                PY.x = fma(tap[h].x, cell[h].y, PY.x);
+                PY.y = fma(tap[h].y, cell[h].x, PY.y);
               }
+            };
+            if (lane < n) add(lane, X, Y);
+            for (int k = lane + 32 * kAhead; k < n; k += 32 * kAhead) {
+              R2 PX{}, PY{};
+              add(k, PX, PY);
+              X.x += PX.x;
+              X.y += PX.y;
+              Y.x += PY.x;
+              Y.y += PY.y;
             }
           }
-          v[2 * j] = re;
-          v[2 * j + 1] = im;
+          v[2 * j] = X.x + (conj ? -X.y : X.y);
+          v[2 * j + 1] = Y.x - (conj ? -Y.y : Y.y);
         }
         __syncwarp();
         store(word, v);
