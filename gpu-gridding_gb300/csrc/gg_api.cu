@@ -1939,7 +1939,8 @@ template <typename Real>
 int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
                     const Real* uu, const Real* vv, const Real* ww,
                     Real cell_size_rad, Real w_scale, int grid_size,
-                    const Real* d_grid, Real* d_out, cudaStream_t s) {
+                    const Real* d_grid, Real* d_out, cudaStream_t s,
+                    const Real* host_grid = nullptr) {
   if (!plan || !K) return set_error(GG_ERR_INVALID_ARG, "plan or kernels is NULL");
   if (K->is_double != (sizeof(Real) == 8))
     return set_error(GG_ERR_INVALID_ARG,
@@ -2001,12 +2002,25 @@ int degrid_pipeline(gg_plan* plan, const gg_kernels* K, size_t num_points,
     plan->stats.num_ctas = grid_teams(num_ctas);
     GG_TRY(plan->rec_out.ensure((size_t)b.total * 2 * sizeof(Real)));
     uint32_t* sc = plan->scalars.as<uint32_t>();
+    if (host_grid) {
+      // The caller's grid, in host memory: d_grid is room for it.
+      GG_TRY(plan->tile_start.ensure((size_t)(b.num_tiles + 1) * 4));
+      GG_TRY(plan->tile_groups.ensure((size_t)num_strips(b.geom)));
+      GG_CUDA(launch_tile_bounds(b.keys, b.total, b.low_bits, b.num_tiles,
+                                 plan->tile_start.as<uint32_t>(), s));
+      GG_CUDA(launch_gather_tiles<Real>(
+          plan->tile_start.as<uint32_t>(), b.tile_order, b.geom, b.num_tiles,
+          b.total, plan->tile_groups.as<unsigned char>(), sc + kNumSplit,
+          grid_size, host_grid, const_cast<Real*>(d_grid), sms, s));
+      plan->stats.num_launches += 3;
+    }
     if (plan->grid_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->grid_wait, 0));
     if (plan->stack_wait) GG_CUDA(cudaStreamWaitEvent(s, plan->stack_wait, 0));
     GG_CUDA(launch_degrid_tiles<Real>(
         b.keys, b.vals, b.total, b.low_bits, b.tile_order, po.points,
         plan->rec_offset.as<uint32_t>(), sc + kCounter, view, b.geom,
-        grid_size, d_grid, plan->rec_out.p, num_ctas, s));
+        grid_size, d_grid, host_grid, sc + kNumSplit, plan->rec_out.p,
+        num_ctas, s));
     GG_CUDA(launch_degrid_finish<Real>(po.rec_count,
                                        plan->rec_offset.as<uint32_t>(),
                                        plan->rec_out.p, n, d_out, s));
@@ -2672,8 +2686,8 @@ int degrid_host(size_t num_w_planes, const int* support, int oversample,
   gg_kernels* K = nullptr;
   GG_TRY(host_kernels<Real>(st, num_w_planes, support, oversample,
                             conv_size_half, conv_func, s, uploads, &K));
-  // A grid the device addresses is read in place by the degridding kernel
-  // (each work item loads its tile once); others go up behind the cube.
+  // Of a grid the device addresses, the call's kernels bring over the tiles
+  // that hold records (launch_gather_tiles); others go up behind the cube.
   const void* direct =
       n ? direct_host_address(st, dev, grid, grid_bytes, 2 * sizeof(Real))
         : nullptr;
@@ -2689,8 +2703,8 @@ int degrid_host(size_t num_w_planes, const int* support, int oversample,
   const int rc = degrid_pipeline<Real>(
       plan, K, n, plan->in_uu.as<Real>(), plan->in_vv.as<Real>(),
       plan->in_ww.as<Real>(), cell_size_rad, w_scale, grid_size,
-      direct ? (const Real*)direct : plan->in_grid.as<Real>(),
-      plan->in_vis.as<Real>(), s);
+      plan->in_grid.as<Real>(), plan->in_vis.as<Real>(), s,
+      (const Real*)direct);
   plan->grid_wait = nullptr;
   plan->stack_wait = nullptr;
   GG_TRY(rc);

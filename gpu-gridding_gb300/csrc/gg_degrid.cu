@@ -95,8 +95,75 @@ struct DegridArgs {
   TileGeom geom;
   int grid_size;
   const Real* grid;
+  // A grid in the caller's host memory, or null: read in place where
+  // stays_at_host, else `grid` holds the cells that the tiles cover.
+  const Real* host;
+  const uint32_t* touched;    // virtual tiles with records
   typename Vec2<Real>::type* rec_out;  // partial result per emission slot
 };
+
+// Whether a grid in host memory is read there record by record.  Every unit
+// reads its tiles' values anew, over the link in that case, so only calls of
+// less than three records a tile do.  Host calls in ms, so and with the tiles
+// brought over first (support 2 to 8 on 8192^2): 5e3 points 0.35 and 0.53, 2e4
+// 0.65 and 0.81, 5e4 1.05 and 1.03, 4e5 2.97 and 1.76; 2e5 points of support 4
+// to 24 on 2048^2 1.51 and 0.75.
+__device__ __forceinline__ bool stays_at_host(uint32_t touched,
+                                              uint32_t total) {
+  return 3ull * touched > total;
+}
+
+// Marks the strips (TileGeom) of the tiles with records, and counts the virtual
+// tiles among them.  tile_start: by place in the queue order.
+__global__ void k_mark_strips(const uint32_t* __restrict__ tile_start,
+                              const int* __restrict__ tile_order, TileGeom g,
+                              int num_tiles, unsigned char* __restrict__ marks,
+                              uint32_t* __restrict__ touched) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool has = t < num_tiles && tile_start[t + 1] > tile_start[t];
+  if (has) {
+    const int vg = t / g.tiles_total, P = g.tile_phases;
+    const int tl = tile_order[t - vg * g.tiles_total];
+    const int tv = tl / g.tiles_u, tu = tl - tv * g.tiles_u;
+    const int first = tu * P - (vg & (P - 1));
+    for (int s = max(first, 0); s < min(first + P, g.strips_u); ++s)
+      marks[(size_t)tv * g.strips_u + s] = 1;
+  }
+  const uint32_t n = __popc(__ballot_sync(0xffffffffu, has));
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(touched, n);
+}
+
+// Brings the marked strips' cells from the caller's host memory, grid row by
+// grid row, each over the link once.  The link bounds it (16 blocks of 1024
+// threads are too few, 48 to 300 the same); beside the binning, on a stream of
+// its own, it got in the way of the cube's transfer (2e5 points on 2048^2 1.09
+// ms a call instead of 0.76).
+template <typename R2>
+__global__ void __launch_bounds__(256)
+k_gather_strips(const unsigned char* __restrict__ marks,
+                const uint32_t* __restrict__ touched, uint32_t total,
+                TileGeom g, int G, const R2* __restrict__ src,
+                R2* __restrict__ dst) {
+  constexpr int kAhead = 4;
+  if (stays_at_host(*touched, total)) return;
+  for (int row = blockIdx.x; row < G; row += gridDim.x) {
+    const unsigned char* mark = marks + (size_t)(row / g.tile_v) * g.strips_u;
+    const size_t at = (size_t)row * G;
+    for (int c0 = threadIdx.x; c0 < G; c0 += kAhead * blockDim.x) {
+      R2 v[kAhead];
+      bool on[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const int c = c0 + k * (int)blockDim.x;
+        on[k] = c < G && mark[c >> g.strip_shift];
+        if (on[k]) v[k] = src[at + c];
+      }
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+        if (on[k]) dst[at + c0 + k * blockDim.x] = v[k];
+    }
+  }
+}
 
 // Shared memory of one warp.  A record's int4: the tap index of the footprint
 // centre's column in the slice row of tile row 0; conjugated << 31 | columns
@@ -174,7 +241,9 @@ k_degrid_tiles(DegridArgs<Real> a) {
   SM& sm = reinterpret_cast<SM*>(g_smem_raw)[threadIdx.x >> 5];
   const int G = a.grid_size;
   const R2* __restrict__ taps = (const R2*)a.view.taps;
-  const R2* __restrict__ grid = (const R2*)a.grid;
+  const R2* __restrict__ grid =
+      (const R2*)(a.host && stays_at_host(*a.touched, a.cut.total) ? a.host
+                                                                   : a.grid);
   const uint32_t lt = (1u << lane) - 1u;
   if (lane == 0) {
     sm.rec[kUnit] = make_int4((int)kStackZero, 0, 0, 0);
@@ -523,8 +592,9 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
                                 PlacedPoints points,
                                 const uint32_t* rec_offset, uint32_t* counter,
                                 StackView view, TileGeom geom, int grid_size,
-                                const Real* grid, void* rec_out, int num_ctas,
-                                cudaStream_t s) {
+                                const Real* grid, const Real* host,
+                                const uint32_t* touched, void* rec_out,
+                                int num_ctas, cudaStream_t s) {
   if (geom.tile_u != kDegridTileU || geom.tile_v != DegridShape::kTileV)
     return cudaErrorInvalidValue;
   DegridArgs<Real> a;
@@ -546,6 +616,8 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
   a.geom = geom;
   a.grid_size = grid_size;
   a.grid = grid;
+  a.host = host;
+  a.touched = touched;
   a.rec_out = (typename Vec2<Real>::type*)rec_out;
   void* fn = nullptr;
   size_t smem = 0;
@@ -556,6 +628,24 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
   void* args[] = {&a};
   return cudaLaunchKernel(fn, dim3(num_ctas), dim3(kDegridThreads), args, smem,
                           s);
+}
+
+template <typename Real>
+cudaError_t launch_gather_tiles(const uint32_t* tile_start,
+                                const int* tile_order, TileGeom geom,
+                                int num_tiles, uint32_t total,
+                                unsigned char* marks, uint32_t* touched,
+                                int grid_size, const Real* host, Real* grid,
+                                int num_sms, cudaStream_t s) {
+  using R2 = typename Vec2<Real>::type;
+  cudaError_t e = cudaMemsetAsync(touched, 0, sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(marks, 0, num_strips(geom), s);
+  if (e != cudaSuccess) return e;
+  k_mark_strips<<<(num_tiles + 255) / 256, 256, 0, s>>>(
+      tile_start, tile_order, geom, num_tiles, marks, touched);
+  k_gather_strips<R2><<<std::min(grid_size, 8 * num_sms), 256, 0, s>>>(
+      marks, touched, total, geom, grid_size, (const R2*)host, (R2*)grid);
+  return cudaGetLastError();
 }
 
 template <typename Real>
@@ -573,10 +663,18 @@ template int degrid_tiles_ctas_per_sm<float>(bool);
 template int degrid_tiles_ctas_per_sm<double>(bool);
 template cudaError_t launch_degrid_tiles<float>(
     const uint32_t*, const uint32_t*, uint32_t, int, const int*, PlacedPoints,
-    const uint32_t*, uint32_t*, StackView, TileGeom, int, const float*, void*, int, cudaStream_t);
+    const uint32_t*, uint32_t*, StackView, TileGeom, int, const float*,
+    const float*, const uint32_t*, void*, int, cudaStream_t);
 template cudaError_t launch_degrid_tiles<double>(
     const uint32_t*, const uint32_t*, uint32_t, int, const int*, PlacedPoints,
-    const uint32_t*, uint32_t*, StackView, TileGeom, int, const double*, void*, int, cudaStream_t);
+    const uint32_t*, uint32_t*, StackView, TileGeom, int, const double*,
+    const double*, const uint32_t*, void*, int, cudaStream_t);
+template cudaError_t launch_gather_tiles<float>(
+    const uint32_t*, const int*, TileGeom, int, uint32_t, unsigned char*,
+    uint32_t*, int, const float*, float*, int, cudaStream_t);
+template cudaError_t launch_gather_tiles<double>(
+    const uint32_t*, const int*, TileGeom, int, uint32_t, unsigned char*,
+    uint32_t*, int, const double*, double*, int, cudaStream_t);
 template cudaError_t launch_degrid_finish<float>(const uint32_t*,
                                                  const uint32_t*, const void*,
                                                  unsigned long long, float*,
