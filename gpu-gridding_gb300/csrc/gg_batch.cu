@@ -53,6 +53,7 @@ k_place_batched(PlaceParams<Real> p, StackView v, PlaceOut out,
   o.meta = pack_meta(r.plane, r.ou, r.ov, r.conj_neg, r.skipped);
   o.v.x = rmul(w, p.vis[2 * i]);
   o.v.y = rmul(w, p.vis[2 * i + 1]);
+  o.meta |= odd_bit(o.v, r.skipped);
   ((Placed<Real>*)out.points.p)[i] = o;
   double t = 0.0;
   if (!r.skipped) {
@@ -80,8 +81,10 @@ k_revalue(const Real* __restrict__ vis, const Real* __restrict__ weight,
   R2 o;
   o.x = rmul(w, vis[2 * i]);
   o.y = rmul(w, vis[2 * i + 1]);
-  placed[i].v = o;
   const uint32_t m = placed[i].meta;
+  placed[i].v = o;
+  if constexpr (sizeof(Real) == 4)
+    placed[i].meta = (m & ~kMetaOdd) | odd_bit(o, meta_skipped(m));
   double t = 0.0;
   if (!meta_skipped(m)) {
     const int side = 2 * v.omax + 1;
@@ -103,20 +106,38 @@ k_chunk_totals(PlacedPoints points,
                unsigned long long* __restrict__ chunk_macs) {
   const int c = blockIdx.x;
   const unsigned long long b = chunk_begin[c], e = chunk_begin[c + 1];
+  // A thread's points in flight: a chunk is one block, so that the latency of
+  // its loads bounds it (16 grids of 62 500 points: 89 us one at a time).
+  constexpr int kAhead = 8;
   double n = 0.0;
   unsigned long long skip = 0, macs = 0;
-  for (unsigned long long i = b + threadIdx.x; i < e; i += kThreads) {
-    const uint32_t m = points.at(i).y;
-    if (meta_skipped(m)) {
-      ++skip;
-    } else {
-      const unsigned long long f = 2ull * v.support[meta_plane(m)] + 1;
-      macs += f * f;
-      n += nterm[i];
+  uint32_t odd = 0;
+  for (unsigned long long i0 = b + threadIdx.x; i0 < e;
+       i0 += kAhead * kThreads) {
+    uint32_t m[kAhead];
+    double t[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const unsigned long long i = i0 + j * kThreads;
+      m[j] = i < e ? points.at(i).y : 0u;
+      t[j] = i < e ? nterm[i] : 0.0;   // 0 for a skipped point
+    }
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      if (i0 + j * kThreads >= e) break;
+      odd |= m[j] & kMetaOdd;
+      n += t[j];
+      if (meta_skipped(m[j])) {
+        ++skip;
+      } else {
+        const unsigned long long f = 2ull * v.support[meta_plane(m[j])] + 1;
+        macs += f * f;
+      }
     }
   }
   n = block_sum(n);
-  skip = block_sum(skip);
+  // Threads with an odd point count as one (only none or some matters).
+  skip = block_sum(skip + (odd ? kOneOdd : 0ull));
   macs = block_sum(macs);
   if (threadIdx.x == 0) {
     chunk_norm[c] = n;
@@ -135,7 +156,8 @@ k_batch_finalize(int num_grids, const int* __restrict__ grid_chunk0,
                  const unsigned long long* __restrict__ chunk_macs,
                  int forced_shape, int phases, long long tiles, double* d_norm,
                  unsigned long long* d_num_skipped,
-                 unsigned long long* d_macs, uint32_t* d_shape) {
+                 unsigned long long* d_macs, uint32_t* d_shape,
+                 uint32_t* d_odd) {
   unsigned long long points = 0, skips = 0, macs = 0;
   for (int g = threadIdx.x; g < num_grids; g += kThreads) {
     double n = 0.0;
@@ -147,13 +169,15 @@ k_batch_finalize(int num_grids, const int* __restrict__ grid_chunk0,
       points += chunk_begin[c + 1] - chunk_begin[c];
     }
     if (d_norm) d_norm[g] += n;
-    if (d_num_skipped) d_num_skipped[g] = sk;
+    if (d_num_skipped) d_num_skipped[g] = sk % kOneOdd;
     skips += sk;
   }
   points = block_sum(points);
   skips = block_sum(skips);
   macs = block_sum(macs);
   if (threadIdx.x == 0) {
+    *d_odd = (uint32_t)(skips / kOneOdd);
+    skips %= kOneOdd;
     *d_macs = macs;
     *d_shape = choose_shape(macs, points - skips, forced_shape, phases, tiles);
   }
@@ -180,14 +204,15 @@ cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
                                 int forced_shape, double* d_norm,
                                 unsigned long long* d_num_skipped,
                                 unsigned long long* d_macs, uint32_t* d_shape,
-                                cudaStream_t s, int phases, long long tiles) {
+                                uint32_t* d_odd, cudaStream_t s, int phases,
+                                long long tiles) {
   if (num_chunks > 0)
     k_chunk_totals<<<num_chunks, kThreads, 0, s>>>(
         points, nterm, view, chunk_begin, chunk_norm, chunk_skip, chunk_macs);
   k_batch_finalize<<<1, kThreads, 0, s>>>(
       num_grids, grid_chunk0, chunk_begin, chunk_norm, chunk_skip,
       chunk_macs, forced_shape, phases, tiles, d_norm, d_num_skipped, d_macs,
-      d_shape);
+      d_shape, d_odd);
   return cudaGetLastError();
 }
 

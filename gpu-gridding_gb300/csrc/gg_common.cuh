@@ -21,7 +21,7 @@ constexpr int kMaxPlanes = 65535;
 // Packed placement of one visibility (written by the placement kernel).
 //   cell: u in bits 0-15, v in bits 16-31
 //   meta: plane in bits 0-15, (off_u + 8) in 16-19, (off_v + 8) in 20-23,
-//         conj_neg in bit 24, skipped in bit 25
+//         conj_neg in bit 24, skipped in bit 25, kMetaOdd in bit 26
 __host__ __device__ inline uint32_t pack_cell(int u, int v) {
   return (uint32_t)(u & 0xFFFF) | ((uint32_t)(v & 0xFFFF) << 16);
 }
@@ -33,6 +33,10 @@ __host__ __device__ inline uint32_t pack_meta(int plane, int ou, int ov,
          ((uint32_t)(ov + 8) << 20) | ((uint32_t)conj_neg << 24) |
          ((uint32_t)skipped << 25);
 }
+// A gridded FP32 point whose weighted visibility is infinite or not a number:
+// added cell by cell (launch_grid_odd), as the tile kernel's lanes outside its
+// footprint would make NaNs of their zero taps.
+constexpr uint32_t kMetaOdd = 1u << 26;
 __host__ __device__ inline int meta_plane(uint32_t m) { return (int)(m & 0xFFFF); }
 __host__ __device__ inline int meta_ou(uint32_t m) { return (int)((m >> 16) & 0xF) - 8; }
 __host__ __device__ inline int meta_ov(uint32_t m) { return (int)((m >> 20) & 0xF) - 8; }

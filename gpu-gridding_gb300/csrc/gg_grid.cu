@@ -180,6 +180,7 @@ __device__ __forceinline__ void prepare_record(const GridArgs<Real>& a,
   span = (uint32_t)(max(gv - s, 0) / kRows) |
          (uint32_t)(min(gv + s, WarpShape<TW>::kTileV - 1) / kRows) << 5 |
          (meta_conj(m) ? kSpanConj : 0u);
+  if (m & kMetaOdd) span = kSpanNone;   // k_grid_odd's
 }
 
 // Prepares the records of every work item of the call: one block per item at
@@ -646,6 +647,52 @@ k_grid_tiles_f64(GridArgs<double> a) {
       }
     }
     __syncwarp();   // acc is free for the next unit
+  }
+}
+
+// Adds the kMetaOdd points, a warp each at a time, its lanes on the footprint's
+// cells.
+__global__ void __launch_bounds__(256)
+k_grid_odd(const Placed<float>* __restrict__ placed, unsigned long long n,
+           const uint32_t* __restrict__ odd, StackView v, int G, float* grid,
+           long long grid_stride,
+           const unsigned long long* __restrict__ grid_offsets,
+           int num_grids) {
+  if (odd && *odd == 0) return;
+  const int lane = threadIdx.x & 31;
+  const unsigned long long warps = (unsigned long long)gridDim.x * 8;
+  for (unsigned long long i0 =
+           ((unsigned long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32;
+       i0 < n; i0 += warps * 32) {
+    const uint32_t mine = i0 + lane < n ? placed[i0 + lane].meta : 0u;
+    for (uint32_t b = __ballot_sync(0xffffffffu, (mine & kMetaOdd) != 0u); b;
+         b &= b - 1) {
+      const unsigned long long i = i0 + (__ffs(b) - 1);
+      int gi = 0;
+      for (int hi = num_grids - 1; gi < hi;) {   // i's grid
+        const int mid = (gi + hi + 1) >> 1;
+        if (grid_offsets[mid] <= i) gi = mid; else hi = mid - 1;
+      }
+      const Placed<float> pt = placed[i];
+      const SlicePlane plane = v.planes[meta_plane(pt.meta)];
+      const int s = plane.support, F = 2 * s + 1, pitch = slice_pitch(s);
+      const int ou = meta_ou(pt.meta), ov = meta_ov(pt.meta);
+      const float2* const taps =
+          (const float2*)v.taps + slice_origin(plane, v.omax, abs(ou), abs(ov));
+      const float sgn = meta_conj(pt.meta) ? -1.0f : 1.0f;
+      float* const corner =
+          grid + gi * grid_stride +
+          2 * ((size_t)(cell_v(pt.cell) - s) * G + (cell_u(pt.cell) - s));
+      for (int e = lane; e < F * F; e += 32) {
+        const int row = e / F, col = e - row * F;
+        const float2 t = taps[(ov < 0 ? F - 1 - row : row) * pitch +
+                              (ou < 0 ? F - 1 - col : col)];
+        const float ti = sgn * t.y;
+        float* const c = corner + 2 * ((size_t)row * G + col);
+        atomicAdd(c, pt.v.x * t.x - pt.v.y * ti);
+        atomicAdd(c + 1, pt.v.x * ti + pt.v.y * t.x);
+      }
+    }
   }
 }
 
@@ -1165,6 +1212,20 @@ cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
   // A tile per thread, and one more for the end.
   const int blocks = num_tiles / 256 + 1;
   k_tile_bounds<<<blocks, 256, 0, s>>>(keys, n, shift, num_tiles, tile_start);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
+                            const uint32_t* odd, StackView view, int grid_size,
+                            float* grid, long long grid_stride,
+                            const unsigned long long* grid_offsets,
+                            int num_grids, cudaStream_t s) {
+  const unsigned long long blocks = std::min<unsigned long long>(
+      (n + 255) / 256, 1216);
+  if (blocks == 0) return cudaSuccess;
+  k_grid_odd<<<(unsigned)blocks, 256, 0, s>>>(
+      (const Placed<float>*)placed, n, odd, view, grid_size, grid, grid_stride,
+      grid_offsets, num_grids);
   return cudaGetLastError();
 }
 

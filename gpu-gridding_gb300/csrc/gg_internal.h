@@ -127,9 +127,12 @@ struct PlaceOut {
   PlacedPoints points;        // [N] Placed<Real>, or pairs for degridding
   uint32_t* rec_count;        // [N] records (tiles touched) per visibility
   double* blk_norm;           // [num_blocks]
-  unsigned long long* blk_skip;   // [num_blocks]
+  unsigned long long* blk_skip;   // [num_blocks] skipped + kOneOdd * odd
   unsigned long long* blk_macs;   // [num_blocks]
 };
+// One kMetaOdd point in the skip counts' upper halves (a call has fewer than
+// 2^32 points).
+constexpr unsigned long long kOneOdd = 1ull << 32;
 // Points per block of the placement kernel (its per-block partials).
 constexpr int kPlaceBlock = 256;
 int place_num_blocks(unsigned long long n);
@@ -151,6 +154,7 @@ cudaError_t launch_norm_terms(PlacedPoints points, const Real* weight,
 // *d_macs = macs (all device pointers), and picks the tile shape and tile
 // phases for the call into *d_shape (choose_shape): forced_shape if >= 0,
 // phases if > 0, else from the mean footprint area (macs / gridded points).
+// *d_odd (may be null) = the kMetaOdd points.
 cudaError_t launch_place_finalize(const double* blk_norm,
                                   const unsigned long long* blk_skip,
                                   const unsigned long long* blk_macs,
@@ -158,8 +162,9 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   int forced_shape, double* d_norm,
                                   unsigned long long* d_num_skipped,
                                   unsigned long long* d_macs,
-                                  uint32_t* d_shape, cudaStream_t s,
-                                  int phases = 1, long long tiles = -1);
+                                  uint32_t* d_shape, uint32_t* d_odd,
+                                  cudaStream_t s, int phases = 1,
+                                  long long tiles = -1);
 // use[b] = how many of up to 8192 placed points, evenly spread, are gridded with
 // planes p of bin b = p * kPlaneBins / num_planes.
 constexpr int kPlaneBins = 256;
@@ -218,8 +223,8 @@ cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
                                 int forced_shape, double* d_norm,
                                 unsigned long long* d_num_skipped,
                                 unsigned long long* d_macs, uint32_t* d_shape,
-                                cudaStream_t s, int phases = 1,
-                                long long tiles = -1);
+                                uint32_t* d_odd, cudaStream_t s,
+                                int phases = 1, long long tiles = -1);
 
 // ---- work decomposition and gridding (gg_grid.cu) -------------------------
 cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
@@ -315,6 +320,15 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
                               int group_span = 1,
                               const int2* tile_slot = nullptr,
                               const uint32_t* tile_start = nullptr);
+// After launch_grid_tiles, whose kernel leaves kMetaOdd points out: adds these
+// to the grid (or to the caller's, in host memory) cell by cell, atomically; the
+// cells they reach come out infinite or as NaN whatever the order.  Returns at
+// once where *odd (if given) is 0.  grid_offsets as in launch_emit_records.
+cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
+                            const uint32_t* odd, StackView view, int grid_size,
+                            float* grid, long long grid_stride,
+                            const unsigned long long* grid_offsets,
+                            int num_grids, cudaStream_t s);
 // Direct mode of a single-grid call: per strip (num_strips), the first and
 // last virtual group (plane group and tile phase) with records there
 // (first | last << 16, 0xFFFF when none), and *cells += the grid cells of

@@ -42,6 +42,10 @@ k_place(PlaceParams<Real> p, StackView v, TileGeom g, PlaceOut out) {
       o.meta = meta;
       o.v.x = rmul(w, p.vis[2 * i]);
       o.v.y = rmul(w, p.vis[2 * i + 1]);
+      if (odd_bit(o.v, r.skipped)) {
+        o.meta |= kMetaOdd;
+        skip = kOneOdd;
+      }
       ((Placed<Real>*)out.points.p)[i] = o;
     } else {
       *(uint2*)(out.points.p + i * out.points.stride) = make_uint2(cell, meta);
@@ -125,7 +129,7 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
                                  double* d_norm,
                                  unsigned long long* d_num_skipped,
                                  unsigned long long* d_macs,
-                                 uint32_t* d_shape) {
+                                 uint32_t* d_shape, uint32_t* d_odd) {
   // One block; thread t sums blocks t, t+blockDim, ... in order, then a
   // fixed-shape shuffle and shared-memory tree: the same association on
   // every run, so the norm is deterministic.
@@ -164,6 +168,8 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
     m = lane < nw ? s_m[lane] : 0ull;
     n = warp_sum(n); s = warp_sum(s); m = warp_sum(m);
     if (lane == 0) {
+      if (d_odd) *d_odd = (uint32_t)(s / kOneOdd);
+      s %= kOneOdd;
       if (d_norm) *d_norm += n;
       if (d_num_skipped) *d_num_skipped = s;
       if (d_macs) *d_macs = m;
@@ -366,11 +372,12 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   int forced_shape, double* d_norm,
                                   unsigned long long* d_num_skipped,
                                   unsigned long long* d_macs,
-                                  uint32_t* d_shape, cudaStream_t s,
-                                  int phases, long long tiles) {
-  k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, blk_skip, blk_macs,
-                                      num_blocks, n, forced_shape, phases, tiles,
-                                      d_norm, d_num_skipped, d_macs, d_shape);
+                                  uint32_t* d_shape, uint32_t* d_odd,
+                                  cudaStream_t s, int phases,
+                                  long long tiles) {
+  k_place_finalize<<<1, 1024, 0, s>>>(
+      blk_norm, blk_skip, blk_macs, num_blocks, n, forced_shape, phases, tiles,
+      d_norm, d_num_skipped, d_macs, d_shape, d_odd);
   return cudaGetLastError();
 }
 
@@ -393,7 +400,8 @@ cudaError_t launch_norm_terms(PlacedPoints points, const Real* weight,
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, nullptr, nullptr, nb, n, 0,
-                                      1, -1, d_norm, nullptr, nullptr, nullptr);
+                                      1, -1, d_norm, nullptr, nullptr, nullptr,
+                                      nullptr);
   return cudaGetLastError();
 }
 

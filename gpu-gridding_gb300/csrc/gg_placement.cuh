@@ -25,6 +25,14 @@ __device__ __forceinline__ float rabs(float a) { return fabsf(a); }
 __device__ __forceinline__ double rabs(double a) { return fabs(a); }
 
 
+// kMetaOdd for a gridded point with weighted visibility v, or 0.
+template <typename R2>
+__device__ __forceinline__ uint32_t odd_bit(R2 v, int skipped) {
+  return sizeof(v.x) == 4 && !skipped && !(isfinite(v.x) && isfinite(v.y))
+             ? kMetaOdd
+             : 0u;
+}
+
 struct Placement {
   int gu, gv, ou, ov, plane, conj_neg, skipped, support;
 };
