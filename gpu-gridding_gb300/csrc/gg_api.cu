@@ -699,7 +699,6 @@ enum Scalar {
   kCounter,
   kShape,
   kDeviceError,   // set by a kernel whose bounded wait ran out; sticky
-  kOdd,           // the call's kMetaOdd points
   kScalarCount
 };
 // Tile shape of the degridding kernel (32 x 64 cells).
@@ -1186,8 +1185,7 @@ int place_and_count(gg_plan* plan, const gg_kernels* K,
                                 pp.defer_norm || plan->norm_added ? nullptr
                                                                   : d_norm,
                                 d_num_skipped, scalar64(plan, kMacs),
-                                sc + kShape, sc + kOdd, s, plan->call_phases,
-                                plan->call_tiles));
+                                sc + kShape, s, plan->call_phases, plan->call_tiles));
   if (!pp.defer_norm) plan->norm_added = true;
   GG_CUDA(launch_count_records(po.points, n, view, sc + kShape, po.rec_count,
                                s));
@@ -1315,7 +1313,7 @@ int bin_records(gg_plan* plan, const gg_kernels* K, size_t n,
   const int tile_v = tile_v_of_shape(shape);
   // (Points that launch_grid_odd adds come after all passes.)
   const bool split = plan->split_event && num_grids == 1 && spare >= 2 &&
-                     plan->h_scalars[kOdd] == 0 &&
+                     !(plan->h_scalars[kShape] & kShapeOdd) &&
                      plan->split_row > 0 && plan->split_row < grid_size &&
                      plan->split_row % tile_v == 0;
   int pgroups = 1;
@@ -1617,7 +1615,7 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
       (Real*)plan->host_grid, tile_groups, span, plan->tile_slot.as<int2>(),
       plan->tile_start.as<uint32_t>()));
   if constexpr (sizeof(Real) == 4) {
-    if (plan->h_scalars[kOdd]) {
+    if (plan->h_scalars[kShape] & kShapeOdd) {
       GG_CUDA(launch_grid_odd(po.points.p, n, nullptr, view, grid_size,
                               tile_groups ? (float*)plan->host_grid : d_grid,
                               grid_stride, d_grid_offsets, num_grids, s));
@@ -1749,7 +1747,7 @@ int batched_attempt(gg_plan* plan, const gg_kernels* K, int num_grids,
       plan->chunk_begin.as<unsigned long long>(), num_grids,
       plan->grid_chunk0.as<int>(), cp.norm, cp.skip, cp.macs,
       plan->forced_shape, plan->norm_added ? nullptr : d_norm, d_num_skipped,
-      scalar64(plan, kMacs), sc + kShape, sc + kOdd, s, plan->call_phases,
+      scalar64(plan, kMacs), sc + kShape, s, plan->call_phases,
       plan->call_tiles));
   plan->norm_added = true;
   GG_CUDA(launch_count_records(po.points, n, view, sc + kShape, po.rec_count,
@@ -1930,7 +1928,7 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
       kp.num_chunks, plan->chunk_begin.as<unsigned long long>(),
       kp.num_grids, plan->grid_chunk0.as<int>(), cp.norm, cp.skip, cp.macs,
       kp.shape, d_norm, d_num_skipped, scalar64(plan, kMacs), sc + kShape,
-      sc + kOdd, s));
+      s));
   if (kp.num_records == 0) return GG_OK;
   const long long grid_stride = 2LL * kp.grid_size * kp.grid_size;
   // A sub-plan's records go where its parent's last sub-batch had them, if that
@@ -1945,7 +1943,7 @@ int replay_pipeline(gg_plan* plan, const gg_kernels* K, const Real* vis,
       s, nullptr, nullptr, nullptr, nullptr, kp.group_span,
       plan->tile_slot.as<int2>(), plan->tile_start.as<uint32_t>()));
   if constexpr (sizeof(Real) == 4)
-    GG_CUDA(launch_grid_odd(plan->placed.p, kp.num_points, sc + kOdd, view,
+    GG_CUDA(launch_grid_odd(plan->placed.p, kp.num_points, sc + kShape, view,
                             kp.grid_size, d_grids, grid_stride,
                             plan->grid_offsets.as<unsigned long long>(),
                             kp.num_grids, s));

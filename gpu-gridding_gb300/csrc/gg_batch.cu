@@ -156,8 +156,7 @@ k_batch_finalize(int num_grids, const int* __restrict__ grid_chunk0,
                  const unsigned long long* __restrict__ chunk_macs,
                  int forced_shape, int phases, long long tiles, double* d_norm,
                  unsigned long long* d_num_skipped,
-                 unsigned long long* d_macs, uint32_t* d_shape,
-                 uint32_t* d_odd) {
+                 unsigned long long* d_macs, uint32_t* d_shape) {
   unsigned long long points = 0, skips = 0, macs = 0;
   for (int g = threadIdx.x; g < num_grids; g += kThreads) {
     double n = 0.0;
@@ -176,10 +175,11 @@ k_batch_finalize(int num_grids, const int* __restrict__ grid_chunk0,
   skips = block_sum(skips);
   macs = block_sum(macs);
   if (threadIdx.x == 0) {
-    *d_odd = (uint32_t)(skips / kOneOdd);
+    const uint32_t odd = skips >= kOneOdd ? kShapeOdd : 0u;
     skips %= kOneOdd;
     *d_macs = macs;
-    *d_shape = choose_shape(macs, points - skips, forced_shape, phases, tiles);
+    *d_shape = choose_shape(macs, points - skips, forced_shape, phases, tiles) |
+               odd;
   }
 }
 
@@ -204,15 +204,14 @@ cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
                                 int forced_shape, double* d_norm,
                                 unsigned long long* d_num_skipped,
                                 unsigned long long* d_macs, uint32_t* d_shape,
-                                uint32_t* d_odd, cudaStream_t s, int phases,
-                                long long tiles) {
+                                cudaStream_t s, int phases, long long tiles) {
   if (num_chunks > 0)
     k_chunk_totals<<<num_chunks, kThreads, 0, s>>>(
         points, nterm, view, chunk_begin, chunk_norm, chunk_skip, chunk_macs);
   k_batch_finalize<<<1, kThreads, 0, s>>>(
       num_grids, grid_chunk0, chunk_begin, chunk_norm, chunk_skip,
       chunk_macs, forced_shape, phases, tiles, d_norm, d_num_skipped, d_macs,
-      d_shape, d_odd);
+      d_shape);
   return cudaGetLastError();
 }
 

@@ -654,11 +654,11 @@ k_grid_tiles_f64(GridArgs<double> a) {
 // cells.
 __global__ void __launch_bounds__(256)
 k_grid_odd(const Placed<float>* __restrict__ placed, unsigned long long n,
-           const uint32_t* __restrict__ odd, StackView v, int G, float* grid,
+           const uint32_t* __restrict__ shape, StackView v, int G, float* grid,
            long long grid_stride,
            const unsigned long long* __restrict__ grid_offsets,
            int num_grids) {
-  if (odd && *odd == 0) return;
+  if (shape && !(*shape & kShapeOdd)) return;
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * 8;
   for (unsigned long long i0 =
@@ -1216,7 +1216,7 @@ cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
 }
 
 cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
-                            const uint32_t* odd, StackView view, int grid_size,
+                            const uint32_t* shape, StackView view, int grid_size,
                             float* grid, long long grid_stride,
                             const unsigned long long* grid_offsets,
                             int num_grids, cudaStream_t s) {
@@ -1224,7 +1224,7 @@ cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
       (n + 255) / 256, 1216);
   if (blocks == 0) return cudaSuccess;
   k_grid_odd<<<(unsigned)blocks, 256, 0, s>>>(
-      (const Placed<float>*)placed, n, odd, view, grid_size, grid, grid_stride,
+      (const Placed<float>*)placed, n, shape, view, grid_size, grid, grid_stride,
       grid_offsets, num_grids);
   return cudaGetLastError();
 }

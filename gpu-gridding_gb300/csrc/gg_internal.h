@@ -118,6 +118,8 @@ __host__ __device__ inline uint32_t choose_shape(unsigned long long macs,
       phases >= 8 ? 3u : (phases >= 4 ? 2u : (phases >= 2 ? 1u : 0u));
   return (uint32_t)shape | (pbits << 12);
 }
+// In a shape word: the call has kMetaOdd points.
+constexpr uint32_t kShapeOdd = 1u << 31;
 // Tile phases of a shape word made by choose_shape.
 __host__ __device__ inline int phases_of_shape(uint32_t word) {
   return 1 << ((word >> 12) & 3u);
@@ -154,7 +156,7 @@ cudaError_t launch_norm_terms(PlacedPoints points, const Real* weight,
 // *d_macs = macs (all device pointers), and picks the tile shape and tile
 // phases for the call into *d_shape (choose_shape): forced_shape if >= 0,
 // phases if > 0, else from the mean footprint area (macs / gridded points).
-// *d_odd (may be null) = the kMetaOdd points.
+// kShapeOdd is set in *d_shape where the call has kMetaOdd points.
 cudaError_t launch_place_finalize(const double* blk_norm,
                                   const unsigned long long* blk_skip,
                                   const unsigned long long* blk_macs,
@@ -162,9 +164,8 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   int forced_shape, double* d_norm,
                                   unsigned long long* d_num_skipped,
                                   unsigned long long* d_macs,
-                                  uint32_t* d_shape, uint32_t* d_odd,
-                                  cudaStream_t s, int phases = 1,
-                                  long long tiles = -1);
+                                  uint32_t* d_shape, cudaStream_t s,
+                                  int phases = 1, long long tiles = -1);
 // use[b] = how many of up to 8192 placed points, evenly spread, are gridded with
 // planes p of bin b = p * kPlaneBins / num_planes.
 constexpr int kPlaneBins = 256;
@@ -223,8 +224,8 @@ cudaError_t launch_batch_totals(PlacedPoints points, const double* nterm,
                                 int forced_shape, double* d_norm,
                                 unsigned long long* d_num_skipped,
                                 unsigned long long* d_macs, uint32_t* d_shape,
-                                uint32_t* d_odd, cudaStream_t s,
-                                int phases = 1, long long tiles = -1);
+                                cudaStream_t s, int phases = 1,
+                                long long tiles = -1);
 
 // ---- work decomposition and gridding (gg_grid.cu) -------------------------
 cudaError_t launch_tile_bounds(const uint32_t* keys, uint32_t n, int shift,
@@ -323,9 +324,10 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
 // After launch_grid_tiles, whose kernel leaves kMetaOdd points out: adds these
 // to the grid (or to the caller's, in host memory) cell by cell, atomically; the
 // cells they reach come out infinite or as NaN whatever the order.  Returns at
-// once where *odd (if given) is 0.  grid_offsets as in launch_emit_records.
+// once where the shape word at `shape` (if given) lacks kShapeOdd.
+// grid_offsets as in launch_emit_records.
 cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
-                            const uint32_t* odd, StackView view, int grid_size,
+                            const uint32_t* shape, StackView view, int grid_size,
                             float* grid, long long grid_stride,
                             const unsigned long long* grid_offsets,
                             int num_grids, cudaStream_t s);

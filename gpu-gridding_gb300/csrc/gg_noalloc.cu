@@ -172,7 +172,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   Carve c{scratch};
   uint32_t* sc = c.take<uint32_t>(16);  // 0 total, 1 items, 2 slots,
                                         // 3 split, 4 counter, 5 shape,
-                                        // 6 error, 7 odd points
+                                        // 6 error
   unsigned long long* macs = c.take<unsigned long long>(1);
   // This call's norm and skip totals, committed to the caller's outputs
   // only once the call is accepted.
@@ -229,7 +229,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
   NA_CUDA(launch_place<float>(pp, view, TileGeom{}, 0, 0, po, s));
   NA_CUDA(launch_place_finalize(blk_norm, blk_skip, blk_macs, nblk,
                                 num_points, -1, call_norm, call_skip, macs,
-                                sc + 5, sc + 7, s));
+                                sc + 5, s));
   NA_CUDA(launch_count_records(po.points, num_points, view, sc + 5, count, s));
   NA_CUDA(exclusive_scan_u32(count, offset, num_points, sc + 0, scan_tmp, s));
   uint32_t host_sc[8] = {0};
@@ -318,7 +318,7 @@ extern "C" GG_API int gg_grid_wproj_f_device_noalloc(
                                    placed, view, geom, grid_size, d_grid, 0,
                                    (float*)partials, split_tiles, sc + 3,
                                    num_tiles, num_ctas, s));
-  if (host_sc[7])
+  if (host_sc[5] & kShapeOdd)
     NA_CUDA(launch_grid_odd(placed, num_points, nullptr, view, grid_size,
                             d_grid, 0, nullptr, 1, s));
   return GG_OK;

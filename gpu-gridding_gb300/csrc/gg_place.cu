@@ -129,7 +129,7 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
                                  double* d_norm,
                                  unsigned long long* d_num_skipped,
                                  unsigned long long* d_macs,
-                                 uint32_t* d_shape, uint32_t* d_odd) {
+                                 uint32_t* d_shape) {
   // One block; thread t sums blocks t, t+blockDim, ... in order, then a
   // fixed-shape shuffle and shared-memory tree: the same association on
   // every run, so the norm is deterministic.
@@ -168,13 +168,14 @@ __global__ void k_place_finalize(const double* __restrict__ blk_norm,
     m = lane < nw ? s_m[lane] : 0ull;
     n = warp_sum(n); s = warp_sum(s); m = warp_sum(m);
     if (lane == 0) {
-      if (d_odd) *d_odd = (uint32_t)(s / kOneOdd);
+      const uint32_t odd = s >= kOneOdd ? kShapeOdd : 0u;
       s %= kOneOdd;
       if (d_norm) *d_norm += n;
       if (d_num_skipped) *d_num_skipped = s;
       if (d_macs) *d_macs = m;
       if (d_shape)
-        *d_shape = choose_shape(m, n_points - s, forced_shape, phases, tiles);
+        *d_shape =
+            choose_shape(m, n_points - s, forced_shape, phases, tiles) | odd;
     }
   }
 }
@@ -372,12 +373,11 @@ cudaError_t launch_place_finalize(const double* blk_norm,
                                   int forced_shape, double* d_norm,
                                   unsigned long long* d_num_skipped,
                                   unsigned long long* d_macs,
-                                  uint32_t* d_shape, uint32_t* d_odd,
-                                  cudaStream_t s, int phases,
-                                  long long tiles) {
-  k_place_finalize<<<1, 1024, 0, s>>>(
-      blk_norm, blk_skip, blk_macs, num_blocks, n, forced_shape, phases, tiles,
-      d_norm, d_num_skipped, d_macs, d_shape, d_odd);
+                                  uint32_t* d_shape, cudaStream_t s,
+                                  int phases, long long tiles) {
+  k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, blk_skip, blk_macs,
+                                      num_blocks, n, forced_shape, phases, tiles,
+                                      d_norm, d_num_skipped, d_macs, d_shape);
   return cudaGetLastError();
 }
 
@@ -400,8 +400,7 @@ cudaError_t launch_norm_terms(PlacedPoints points, const Real* weight,
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_place_finalize<<<1, 1024, 0, s>>>(blk_norm, nullptr, nullptr, nb, n, 0,
-                                      1, -1, d_norm, nullptr, nullptr, nullptr,
-                                      nullptr);
+                                      1, -1, d_norm, nullptr, nullptr, nullptr);
   return cudaGetLastError();
 }
 
