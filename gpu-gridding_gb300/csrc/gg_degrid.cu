@@ -99,38 +99,46 @@ struct DegridArgs {
   // A grid in the caller's host memory, or null: read in place where
   // stays_at_host, else `grid` holds the cells that the tiles cover.
   const Real* host;
-  const uint32_t* touched;    // virtual tiles with records
+  const uint32_t* marked;     // strips of the tiles with records
 };
 
-// Whether a grid in host memory is read there record by record.  Every unit
-// reads its tiles' values anew, over the link in that case, so only calls of
-// less than three records a tile do.  Host calls in ms, so and with the tiles
-// brought over first (support 2 to 8 on 8192^2): 5e3 points 0.35 and 0.53, 2e4
-// 0.65 and 0.81, 5e4 1.05 and 1.03, 4e5 2.97 and 1.76; 2e5 points of support 4
-// to 24 on 2048^2 1.51 and 0.75.
-__device__ __forceinline__ bool stays_at_host(uint32_t touched,
-                                              uint32_t total) {
-  return 3ull * touched > total;
+// Whether a grid in host memory is read there unit by unit.  Every unit reads its
+// tiles' values anew, over the link in that case, but those of its records'
+// bands alone and beside its work, so calls of less than nine records a tile of
+// cells to be brought over do (tile_phases strips; tiles of several phases share
+// theirs).  Host calls in ms, so and with the tiles brought over first; on
+// 8192^2, support 2 to 8: 2e4 points (4.4 records) 0.65 and 0.81, 5e4 (7.9) 1.04
+// and 1.03, 4e5 2.97 and 1.76; 8 to 20: 5e3 (3.4) 0.52 and 0.68, 2e4 (7.9) 0.91
+// and 1.03, 5e4 (15) 1.36 and 1.26; 20 to 36: 5e3 (4.9) 0.72 and 0.84, 2e4 (12)
+// 1.28 and 1.22; 40 to 72: 2e3 (4.8) 0.78 and 0.87, 5e3 (8.8) 1.12 and 1.11, 2e4
+// 1.87 and 1.57; on 2048^2, 2 to 8: 2e3 (5.7) 0.23 and 0.24, 2e4 (32) 0.38 and
+// 0.33; 4 to 24: 2e5 1.51 and 0.75.
+__device__ __forceinline__ bool stays_at_host(uint32_t marked, uint32_t total,
+                                              int phases) {
+  return 9ull * marked > (unsigned long long)total * (unsigned)phases;
 }
 
-// Marks the strips (TileGeom) of the tiles with records, and counts the virtual
-// tiles among them.  tile_start: by place in the queue order.
+// Marks the strips (TileGeom) of the tiles with records, a byte each, and counts
+// them.  tile_start: by place in the queue order.
 __global__ void k_mark_strips(const uint32_t* __restrict__ tile_start,
                               const int* __restrict__ tile_order, TileGeom g,
-                              int num_tiles, unsigned char* __restrict__ marks,
-                              uint32_t* __restrict__ touched) {
+                              int num_tiles, uint32_t* __restrict__ marks,
+                              uint32_t* __restrict__ marked) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool has = t < num_tiles && tile_start[t + 1] > tile_start[t];
-  if (has) {
+  uint32_t n = 0;
+  if (t < num_tiles && tile_start[t + 1] > tile_start[t]) {
     const int vg = t / g.tiles_total, P = g.tile_phases;
     const int tl = tile_order[t - vg * g.tiles_total];
     const int tv = tl / g.tiles_u, tu = tl - tv * g.tiles_u;
     const int first = tu * P - (vg & (P - 1));
-    for (int s = max(first, 0); s < min(first + P, g.strips_u); ++s)
-      marks[(size_t)tv * g.strips_u + s] = 1;
+    for (int s = max(first, 0); s < min(first + P, g.strips_u); ++s) {
+      const size_t at = (size_t)tv * g.strips_u + s;
+      const uint32_t bit = 1u << (8 * (at & 3));
+      n += (atomicOr(marks + at / 4, bit) & bit) == 0u;
+    }
   }
-  const uint32_t n = __popc(__ballot_sync(0xffffffffu, has));
-  if ((threadIdx.x & 31) == 0 && n) atomicAdd(touched, n);
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(marked, n);
 }
 
 // Brings the marked strips' cells from the caller's host memory, grid row by
@@ -141,11 +149,11 @@ __global__ void k_mark_strips(const uint32_t* __restrict__ tile_start,
 template <typename R2>
 __global__ void __launch_bounds__(256)
 k_gather_strips(const unsigned char* __restrict__ marks,
-                const uint32_t* __restrict__ touched, uint32_t total,
+                const uint32_t* __restrict__ marked, uint32_t total,
                 TileGeom g, int G, const R2* __restrict__ src,
                 R2* __restrict__ dst) {
   constexpr int kAhead = 4;
-  if (stays_at_host(*touched, total)) return;
+  if (stays_at_host(*marked, total, g.tile_phases)) return;
   for (int row = blockIdx.x; row < G; row += gridDim.x) {
     const unsigned char* mark = marks + (size_t)(row / g.tile_v) * g.strips_u;
     const size_t at = (size_t)row * G;
@@ -246,7 +254,8 @@ k_degrid_tiles(DegridArgs<Real> a) {
   const R2* __restrict__ taps = (const R2*)a.view.taps;
   const R2* __restrict__ grid = (const R2*)a.grid;
   if constexpr (kHost)
-    if (stays_at_host(*a.touched, a.cut.total)) grid = (const R2*)a.host;
+    if (stays_at_host(*a.marked, a.cut.total, a.geom.tile_phases))
+      grid = (const R2*)a.host;
   const uint32_t lt = (1u << lane) - 1u;
   if (lane == 0) {
     sm.rec[kUnit] = make_int4((int)kStackZero, 0, 0, 0);
@@ -600,7 +609,7 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
                                 const uint32_t* rec_offset, uint32_t* counter,
                                 StackView view, TileGeom geom, int grid_size,
                                 const Real* grid, const Real* host,
-                                const uint32_t* touched, void* rec_out,
+                                const uint32_t* marked, void* rec_out,
                                 int num_ctas, cudaStream_t s) {
   if (geom.tile_u != kDegridTileU || geom.tile_v != DegridShape::kTileV)
     return cudaErrorInvalidValue;
@@ -624,7 +633,7 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
   a.grid_size = grid_size;
   a.grid = grid;
   a.host = host;
-  a.touched = touched;
+  a.marked = marked;
   a.rec_out = (typename Vec2<Real>::type*)rec_out;
   void* fn = nullptr;
   size_t smem = 0;
@@ -642,17 +651,19 @@ template <typename Real>
 cudaError_t launch_gather_tiles(const uint32_t* tile_start,
                                 const int* tile_order, TileGeom geom,
                                 int num_tiles, uint32_t total,
-                                unsigned char* marks, uint32_t* touched,
+                                uint32_t* marks, uint32_t* marked,
                                 int grid_size, const Real* host, Real* grid,
                                 int num_sms, cudaStream_t s) {
   using R2 = typename Vec2<Real>::type;
-  cudaError_t e = cudaMemsetAsync(touched, 0, sizeof(uint32_t), s);
-  if (e == cudaSuccess) e = cudaMemsetAsync(marks, 0, num_strips(geom), s);
+  cudaError_t e = cudaMemsetAsync(marked, 0, sizeof(uint32_t), s);
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(marks, 0, strip_mark_bytes(geom), s);
   if (e != cudaSuccess) return e;
   k_mark_strips<<<(num_tiles + 255) / 256, 256, 0, s>>>(
-      tile_start, tile_order, geom, num_tiles, marks, touched);
+      tile_start, tile_order, geom, num_tiles, marks, marked);
   k_gather_strips<R2><<<std::min(grid_size, 8 * num_sms), 256, 0, s>>>(
-      marks, touched, total, geom, grid_size, (const R2*)host, (R2*)grid);
+      (const unsigned char*)marks, marked, total, geom, grid_size,
+      (const R2*)host, (R2*)grid);
   return cudaGetLastError();
 }
 
@@ -678,10 +689,10 @@ template cudaError_t launch_degrid_tiles<double>(
     const uint32_t*, uint32_t*, StackView, TileGeom, int, const double*,
     const double*, const uint32_t*, void*, int, cudaStream_t);
 template cudaError_t launch_gather_tiles<float>(
-    const uint32_t*, const int*, TileGeom, int, uint32_t, unsigned char*,
+    const uint32_t*, const int*, TileGeom, int, uint32_t, uint32_t*,
     uint32_t*, int, const float*, float*, int, cudaStream_t);
 template cudaError_t launch_gather_tiles<double>(
-    const uint32_t*, const int*, TileGeom, int, uint32_t, unsigned char*,
+    const uint32_t*, const int*, TileGeom, int, uint32_t, uint32_t*,
     uint32_t*, int, const double*, double*, int, cudaStream_t);
 template cudaError_t launch_degrid_finish<float>(const uint32_t*,
                                                  const uint32_t*, const void*,

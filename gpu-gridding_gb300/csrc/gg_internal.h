@@ -423,17 +423,20 @@ cudaError_t launch_degrid_tiles(const uint32_t* rec_key,
                                 const uint32_t* rec_offset, uint32_t* counter,
                                 StackView view, TileGeom geom, int grid_size,
                                 const Real* grid, const Real* host,
-                                const uint32_t* touched, void* rec_out,
+                                const uint32_t* marked, void* rec_out,
                                 int num_ctas, cudaStream_t s);
 // For a grid at `host`, in the caller's host memory: the cells of the tiles
 // with records (tile_start by place in the queue order) come to `grid`, unless
 // the records are so few a tile that launch_degrid_tiles (given host and
-// touched) reads them there.  marks: num_strips bytes; touched: one word.
+// marked) reads them there.  marks: strip_mark_bytes; marked: one word.
+inline size_t strip_mark_bytes(const TileGeom& g) {
+  return ((size_t)num_strips(g) + 3) / 4 * 4;
+}
 template <typename Real>
 cudaError_t launch_gather_tiles(const uint32_t* tile_start,
                                 const int* tile_order, TileGeom geom,
                                 int num_tiles, uint32_t total,
-                                unsigned char* marks, uint32_t* touched,
+                                uint32_t* marks, uint32_t* marked,
                                 int grid_size, const Real* host, Real* grid,
                                 int num_sms, cudaStream_t s);
 // out[v] = the sum of visibility v's count[v] partial results from

@@ -238,7 +238,7 @@ def test_sort_digit_widths(pkg, oracle_mod, n, G):
 @pytest.mark.parametrize("prec", ["f", "d"])
 @pytest.mark.parametrize("n,G,s_max,pinned", [
     (200_000, 2047, 24, False), (100_000, 1024, 30, True),
-    (3_000, 4096, 6, False), (40, 300, 4, True)])
+    (3_000, 4096, 6, False), (40, 300, 4, True), (12_000, 8192, 9, False)])
 def test_degrid_host_grid_comes_over_once(pkg, synthetic, torch, prec, n, G,
                                           s_max, pinned):
     """A grid in place at host: the tiles with records cross the link once (or,
