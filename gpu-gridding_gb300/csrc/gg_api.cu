@@ -1617,9 +1617,9 @@ int bin_and_grid(gg_plan* plan, const gg_kernels* K, size_t n,
   if constexpr (sizeof(Real) == 4) {
     if (plan->h_scalars[kShape] & kShapeOdd) {
       GG_CUDA(launch_grid_odd(po.points.p, n, nullptr, view, grid_size,
-                              tile_groups ? (float*)plan->host_grid : d_grid,
-                              grid_stride, d_grid_offsets, num_grids, s));
-      plan->stats.num_launches += 1;
+                              d_grid, grid_stride, d_grid_offsets, num_grids,
+                              s, tile_groups ? (float*)plan->host_grid : nullptr));
+      plan->stats.num_launches += tile_groups ? 2 : 1;
     }
   }
   plan->split_launched = upper_done >= 0;

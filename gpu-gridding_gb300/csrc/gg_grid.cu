@@ -651,7 +651,9 @@ k_grid_tiles_f64(GridArgs<double> a) {
 }
 
 // Adds the kMetaOdd points, a warp each at a time, its lanes on the footprint's
-// cells.
+// cells.  The atomics bound it; cells that are NaN already, as nearly all soon
+// are, need none (2.15e6 points on 8192^2, all of them odd: 24.3 ms a call, with
+// this test 14.9, none odd 4.8; a tenth 7.2 and 6.6).
 __global__ void __launch_bounds__(256)
 k_grid_odd(const Placed<float>* __restrict__ placed, unsigned long long n,
            const uint32_t* __restrict__ shape, StackView v, int G, float* grid,
@@ -689,10 +691,37 @@ k_grid_odd(const Placed<float>* __restrict__ placed, unsigned long long n,
                               (ou < 0 ? F - 1 - col : col)];
         const float ti = sgn * t.y;
         float* const c = corner + 2 * ((size_t)row * G + col);
-        atomicAdd(c, pt.v.x * t.x - pt.v.y * ti);
-        atomicAdd(c + 1, pt.v.x * ti + pt.v.y * t.x);
+        const float2 was = __ldcg((const float2*)c);   // a NaN stays one
+        if (!isnan(was.x)) atomicAdd(c, pt.v.x * t.x - pt.v.y * ti);
+        if (!isnan(was.y)) atomicAdd(c + 1, pt.v.x * ti + pt.v.y * t.x);
       }
     }
+  }
+}
+
+// host += sums where these are not zero: what the kMetaOdd points add, none of
+// which is finite.  Two cells a thread.
+__global__ void __launch_bounds__(256)
+k_add_odd(const float4* __restrict__ sums, unsigned long long pairs,
+          size_t cells, float2* __restrict__ host) {
+  const unsigned long long i =
+      (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pairs) return;
+  const bool two = 2 * i + 1 < cells;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (two) {
+    v = sums[i];
+  } else {
+    const float2 one = ((const float2*)sums)[2 * i];
+    v.x = one.x; v.y = one.y;
+  }
+  if (v.x != 0.0f || v.y != 0.0f) {
+    const float2 was = host[2 * i];
+    host[2 * i] = make_float2(was.x + v.x, was.y + v.y);
+  }
+  if (two && (v.z != 0.0f || v.w != 0.0f)) {
+    const float2 was = host[2 * i + 1];
+    host[2 * i + 1] = make_float2(was.x + v.z, was.y + v.w);
   }
 }
 
@@ -1219,13 +1248,24 @@ cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
                             const uint32_t* shape, StackView view, int grid_size,
                             float* grid, long long grid_stride,
                             const unsigned long long* grid_offsets,
-                            int num_grids, cudaStream_t s) {
+                            int num_grids, cudaStream_t s, float* host) {
+  const size_t cells = (size_t)grid_size * grid_size;
+  if (host) {
+    const cudaError_t e =
+        cudaMemsetAsync(grid, 0, cells * sizeof(float2), s);
+    if (e != cudaSuccess) return e;
+  }
   const unsigned long long blocks = std::min<unsigned long long>(
       (n + 255) / 256, 1216);
   if (blocks == 0) return cudaSuccess;
   k_grid_odd<<<(unsigned)blocks, 256, 0, s>>>(
       (const Placed<float>*)placed, n, shape, view, grid_size, grid, grid_stride,
       grid_offsets, num_grids);
+  if (host) {
+    const unsigned long long pairs = (cells + 1) / 2;
+    k_add_odd<<<(unsigned)((pairs + 255) / 256), 256, 0, s>>>(
+        (const float4*)grid, pairs, cells, (float2*)host);
+  }
   return cudaGetLastError();
 }
 

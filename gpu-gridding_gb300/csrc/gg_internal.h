@@ -322,15 +322,19 @@ cudaError_t launch_grid_tiles(const WorkItem* items,
                               const int2* tile_slot = nullptr,
                               const uint32_t* tile_start = nullptr);
 // After launch_grid_tiles, whose kernel leaves kMetaOdd points out: adds these
-// to the grid (or to the caller's, in host memory) cell by cell, atomically; the
-// cells they reach come out infinite or as NaN whatever the order.  Returns at
+// to the grid cell by cell, atomically; the cells they reach come out infinite or
+// as NaN whatever the order.  With host given, the caller's grid in host memory,
+// they are added in `grid`, whose cells are no longer needed, and these sums then
+// to host, whose atomics would each cross the link (a tenth of 2.15e6 points on
+// 8192^2: 107 ms a call, so 13).  Returns at
 // once where the shape word at `shape` (if given) lacks kShapeOdd.
 // grid_offsets as in launch_emit_records.
 cudaError_t launch_grid_odd(const void* placed, unsigned long long n,
                             const uint32_t* shape, StackView view, int grid_size,
                             float* grid, long long grid_stride,
                             const unsigned long long* grid_offsets,
-                            int num_grids, cudaStream_t s);
+                            int num_grids, cudaStream_t s,
+                            float* host = nullptr);
 // Direct mode of a single-grid call: per strip (num_strips), the first and
 // last virtual group (plane group and tile phase) with records there
 // (first | last << 16, 0xFFFF when none), and *cells += the grid cells of
